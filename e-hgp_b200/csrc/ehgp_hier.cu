@@ -17,7 +17,7 @@
 // B200 design:
 //  * events are assembled, given a rigorous FP64 level interval and sorted on the device
 //    (LSD radix over the level bits); only runs whose intervals overlap are settled exactly
-//    on the host (2304-bit level comparisons), so the facade order is exact;
+//    on the device (2304-bit level comparisons), so the facade order is exact;
 //  * a stable partition by closed rank gives every order's births and saddle families in
 //    facade order at once; births are hashed by facet on the device;
 //  * each strict arm descends on its own thread: exact facet miniball (FP64 Welzl, then
@@ -27,10 +27,10 @@
 //    the terminal facet does not depend on the locator state (a descent chain only
 //    reaches a minimum, and minima of lower level are bound before the arm's batch), so
 //    every arm of every batch descends in one launch;
-//  * the order-by-order hyper-Kruskal pass over the resolved arms is host code with
-//    incremental carrier counts.
+//  * the forest journal over the resolved arms is built on the device (ehgp_journal.cu).
 #include "ehgp_internal.cuh"
 #include "ehgp_exact.cuh"
+#include "ehgp_journal.cuh"
 #include "ehgp_sphere.cuh"
 
 #include <algorithm>
@@ -45,7 +45,6 @@
 #include <thread>
 #include <vector>
 
-#include <sys/mman.h>
 #if defined(__x86_64__)
 #include <immintrin.h>
 #endif
@@ -77,7 +76,7 @@ constexpr int kVisitStripes = 64;
 __device__ unsigned long long g_descent_visits[kVisitStripes];
 __device__ __forceinline__ void slow(int i) { atomicAdd(&g_descent_slow[i], 1ull); }
 
-// Descent status per arm.
+// Descent status of an arm.
 enum ArmStatus : uint8_t {
   kArmOk = 0,
   kArmUnresolved = 1,   // canonical top-k choice equals the facet
@@ -286,14 +285,13 @@ __global__ void k_ev_build(uint32_t np, uint32_t nh, const PairRecD* __restrict_
 __global__ void k_ev_gather(uint32_t m, const uint32_t* __restrict__ v0, const uint32_t* __restrict__ v1,
                             const uint32_t* __restrict__ state, int passes, const EvRec* __restrict__ ev,
                             const double* __restrict__ lmid, const double* __restrict__ lerr, EvRec* __restrict__ out,
-                            double* __restrict__ omid, double* __restrict__ oerr, uint32_t* __restrict__ perm) {
+                            double* __restrict__ omid, double* __restrict__ oerr) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const uint32_t s = radix_result(state, passes, v0, v1)[i];
   out[i] = ev[s];
   omid[i] = lmid[s];
   oerr[i] = lerr[s];
-  perm[i] = s;
 }
 
 // ---- scans (block-local then across blocks) -----------------------------------------
@@ -588,23 +586,6 @@ __global__ void k_rank_info(uint32_t m, const uint32_t* __restrict__ rank_order,
   const uint32_t fi = rank_order[i];
   cls_rp[i] = lclass[fi];
   size_rp[i] = ev[fi].size;
-}
-
-// One arm seed per support point of every saddle family (families = rank positions
-// fam_lo.. in journal order; arm_off = exclusive sum of their support sizes).
-__global__ void k_arm_expand(uint32_t nfam, uint32_t fam_lo, const uint32_t* __restrict__ rank_order,
-                             const EvRec* __restrict__ ev, const uint32_t* __restrict__ arm_off,
-                             uint32_t* __restrict__ arm_family, uint8_t* __restrict__ arm_local,
-                             uint32_t* __restrict__ arm_removed) {
-  const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nfam) return;
-  const EvRec& e = ev[rank_order[fam_lo + f]];
-  const uint32_t o = arm_off[f];
-  for (uint32_t j = 0; j < e.size; ++j) {
-    arm_family[o + j] = f;
-    arm_local[o + j] = (uint8_t)j;
-    arm_removed[o + j] = e.ids[j];
-  }
 }
 
 // ---- 3. strict-arm descent ----------------------------------------------------------
@@ -1048,26 +1029,39 @@ __device__ __forceinline__ int arm_facet(const EvRec& e, uint32_t removed, uint3
   return w;
 }
 
-// First probe of every arm: most arms are themselves a birth facet of their order.
-// Misses are queued with their facet for the descent steps.
-__global__ void k_arm_probe(DescentParams d, uint32_t a0, uint32_t narms,
-                            const uint32_t* __restrict__ fam_event /* rank_order + fam_lo */,
-                            const uint32_t* __restrict__ arm_family, const uint8_t* __restrict__ arm_local,
-                            const EvRec* __restrict__ ev, uint32_t* __restrict__ term, uint8_t* __restrict__ status,
-                            uint32_t* __restrict__ q_arm, uint32_t* __restrict__ q_fac, uint32_t* __restrict__ q_count) {
+// Arm seeds and their first probe, one thread per saddle family: one arm per support point
+// (F_u = (I u U) \ {u}); most arms are themselves a birth facet of their order.  Misses are queued
+// with their facet for the descent steps while they fit (q_count counts them all).
+__global__ void k_arm_probe(DescentParams d, uint32_t f0, uint32_t nfam, const uint32_t* __restrict__ fam_event,
+                            const uint32_t* __restrict__ armoff, const EvRec* __restrict__ ev,
+                            uint32_t* __restrict__ removed, uint32_t* __restrict__ term, uint32_t* __restrict__ q_arm,
+                            uint32_t* __restrict__ q_fac, uint32_t q_cap, uint32_t* __restrict__ q_count) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= narms) return;
-  const uint32_t a = a0 + i;
-  const EvRec e = ev[fam_event[arm_family[a]]];
-  uint32_t F[kMaxFacet + 1];
-  const int k = arm_facet(e, e.ids[arm_local[a]], F);
-  const uint32_t h = probe_facet(d, F, k);
-  term[a] = h;
-  status[a] = kArmOk;
-  if (h != kInvalid32) return;
-  const uint32_t slot = atomicAdd(q_count, 1u);
-  q_arm[slot] = a;
-  for (int j = 0; j < kMaxFacet; ++j) q_fac[(uint64_t)slot * kMaxFacet + j] = j < k ? F[j] : kInvalid32;
+  const bool on = i < nfam;
+  const uint32_t f = f0 + (on ? i : 0u), a0 = armoff[f];
+  const EvRec e = ev[fam_event[f]];
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t t = 0; t < 4; ++t) {  // the whole warp: its misses take their slots with one atomic
+    const bool arm = on && t < e.size;
+    uint32_t F[kMaxFacet + 1];
+    int k = 0;
+    bool miss = false;
+    if (arm) {
+      k = arm_facet(e, e.ids[t], F);
+      const uint32_t h = probe_facet(d, F, k);
+      removed[a0 + t] = e.ids[t];
+      term[a0 + t] = h;
+      miss = h == kInvalid32;
+    }
+    const uint32_t b = __ballot_sync(0xffffffffu, miss);
+    uint32_t base = 0;
+    if (lane == 0 && b) base = atomicAdd(q_count, (uint32_t)__popc(b));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const uint32_t slot = base + __popc(b & ((1u << lane) - 1u));
+    if (!miss || slot >= q_cap) continue;
+    q_arm[slot] = a0 + t;
+    for (int j = 0; j < kMaxFacet; ++j) q_fac[(uint64_t)slot * kMaxFacet + j] = j < k ? F[j] : kInvalid32;
+  }
 }
 
 // One strict descent step for every queued arm: exact miniball of F, exact canonical
@@ -1094,8 +1088,7 @@ __global__ void __launch_bounds__(128, EHGP_STEP_BLOCKS_PER_SM)
 k_arm_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, const uint32_t* __restrict__ in_fac,
            const uint32_t* __restrict__ rstate, int passes, const uint32_t* __restrict__ v0,
            const uint32_t* __restrict__ v1, uint32_t* __restrict__ out_arm, uint32_t* __restrict__ out_fac,
-           uint32_t* __restrict__ out_count, uint32_t* __restrict__ term, uint8_t* __restrict__ status,
-           unsigned long long* __restrict__ stats) {
+           uint32_t* __restrict__ out_count, uint32_t* __restrict__ term, unsigned long long* __restrict__ stats) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= m) return;
   // queue entry: in Morton order of the facets when the queue was sorted (passes >= 0)
@@ -1108,9 +1101,9 @@ k_arm_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, con
     k += F[j] != kInvalid32;
   }
   const Cloud c{d.px, d.py, d.pz, d.S};
-  auto fail = [&](int why) {  // stats[3] counts failed arms
-    status[a] = (uint8_t)why;
-    atomicAdd(stats + 3, 1ull);
+  auto fail = [&](int why) {  // failed arms, and the least of them with its status
+    atomicAdd(stats + 2, 1ull);
+    atomicMin(stats + 3, (unsigned long long)a << 8 | (unsigned long long)why);
   };
   Mini mb;
   if (!facet_miniball(c, F, k, mb)) { fail(kArmInternal); return; }
@@ -1131,7 +1124,7 @@ k_arm_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, con
     if (!flevel(mg.fs, glo, ghi)) exact_level_fp(c, mg.T, mg.ts, glo, ghi);
     if (!flevel(mb.fs, flo, fhi)) exact_level_fp(c, mb.T, mb.ts, flo, fhi);
     if (!(ghi < flo) && level_cmp_exact(c, mg.T, mg.ts, mb.T, mb.ts) >= 0) { fail(kArmPlateau); return; }
-    atomicAdd(stats + 2, 1ull);
+    atomicAdd(stats + 1, 1ull);
   }
   atomicAdd(stats, 1ull);
   const uint32_t h = probe_facet(d, G, k);
@@ -1147,121 +1140,11 @@ k_arm_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, con
 }  // namespace
 
 // ---- host state ---------------------------------------------------------------------
-// Streaming (non-temporal) store of one record of 4-byte words: the forest records are
-// written once and read at copy-out, so they bypass the caches that hold the union-find
-// arrays.  stream_fence() orders them before a release that publishes them.
-template <class T>
-inline void nt_store(T& dst, const T& v) {
-  static_assert(sizeof(T) % 4 == 0, "records of 4-byte words");
-#if defined(__x86_64__)
-  if (sizeof(T) % 16 == 0 && (reinterpret_cast<uintptr_t>(&dst) & 15) == 0) {  // whole 16-byte stores
-    __m128i* d = reinterpret_cast<__m128i*>(&dst);
-    for (size_t i = 0; i < sizeof(T) / 16; ++i) {
-      __m128i w;
-      std::memcpy(&w, reinterpret_cast<const char*>(&v) + 16 * i, 16);
-      _mm_stream_si128(d + i, w);
-    }
-    return;
-  }
-  const int* s = reinterpret_cast<const int*>(&v);
-  int* d = reinterpret_cast<int*>(&dst);
-  for (size_t i = 0; i < sizeof(T) / 4; ++i) _mm_stream_si32(d + i, s[i]);
-#else
-  dst = v;
-#endif
-}
-inline void stream_fence() {
-#if defined(__x86_64__)
-  _mm_sfence();
-#endif
-}
-
-constexpr uint32_t kUnborn = 0xFFFFFFFEu;  // HierDsu::rroot of a handle not yet born
-
-struct HierDsu {
-  uint32_t parent, rroot;  // rroot: the component's reduced root (at roots), kUnborn before the birth
-};
-
-// Anonymous mapping advised for transparent huge pages: the union-find array is read at
-// random, and 2 MB pages keep its translations in the TLB.  Capacity is kept across calls.
-struct HugeBuf {
-  void* p = nullptr;
-  size_t bytes = 0;
-  HugeBuf() = default;
-  HugeBuf(const HugeBuf&) = delete;
-  HugeBuf& operator=(const HugeBuf&) = delete;
-  ~HugeBuf() {
-    if (p) munmap(p, bytes);
-  }
-  bool ensure(size_t need) {
-    if (need <= bytes) return true;
-    if (p) munmap(p, bytes);
-    p = nullptr;
-    bytes = 0;
-    const size_t align = size_t{2} << 20, b = (need + align - 1) / align * align;
-    void* q = mmap(nullptr, b, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
-    if (q == MAP_FAILED) return false;
-    madvise(q, b, MADV_HUGEPAGE);
-    p = q;
-    bytes = b;
-    return true;
-  }
-};
-
-// Growable storage of plain C records that keeps its capacity across calls and leaves new
-// storage uninitialised; n counts the records in use.  Writers stay within the capacity
-// reserved up front (fits() reports an overrun, which is never written).
-template <class T>
-struct Arena {
-  std::unique_ptr<T[]> p;
-  uint64_t cap = 0, n = 0;
-  void reset(uint64_t need) {
-    if (need > cap) {
-      p.reset(new T[need]);
-      cap = need;
-    }
-    n = 0;
-  }
-  uint64_t size() const { return n; }
-  bool fits() const { return n <= cap; }
-  T& operator[](uint64_t i) { return p[i]; }
-  const T& operator[](uint64_t i) const { return p[i]; }
-  T* begin() { return p.get(); }
-  T* end() { return p.get() + n; }
-  void push_back(const T& x) {
-    if (n < cap) p[n] = x;
-    ++n;
-  }
-  template <class It>
-  void append(It first, It last) {
-    for (; first != last; ++first) push_back(*first);
-  }
-};
-
-struct HierOrderOut {  // one order's journal and forest arenas, local indices
-  Arena<ehgp_journal_batch> jb;
-  Arena<ehgp_role_record> roles;
-  Arena<ehgp_family_record> fam;
-  Arena<ehgp_forest_node> nodes;
-  Arena<uint32_t> children;
-  Arena<ehgp_forest_birth> births;
-  Arena<ehgp_forest_binding> bindings;
-  Arena<ehgp_forest_saddle> saddles;
-  Arena<ehgp_forest_group> groups;
-  Arena<ehgp_forest_batch> fb;
-  Arena<ehgp_forest_root> roots;
-  Arena<uint32_t> node_cls;  // level class of each node (kInvalid32: an order-one birth node)
-  Arena<uint32_t> fam_res;   // resulting root of each family's atomic group (local node id)
-  Arena<uint32_t> v_res;     // vertical maps from this order: each node's carrier-saddle root one order down
-  Arena<uint32_t> v_cls;     // and its own level class
-  int status = EHGP_OK;
-  const char* msg = "";
-  double ms = 0;
-};
-
-struct HierOff {
-  uint32_t jb, role, fam, node, child, birth, bind, sad, grp, root, vert;
-};
+constexpr int kStageSlots = 16;
+constexpr uint64_t kStageBytes = uint64_t{1} << 20;
+// Pageable bytes of one copy from which the pinned ring pays for its allocation (16 MB of page-locked
+// memory and the threads: a few ms, once per context).
+constexpr uint64_t kStageFrom = uint64_t{32} << 20;
 
 struct HierState {
   std::vector<void*> allocs;
@@ -1277,7 +1160,6 @@ struct HierState {
   uint64_t* key2 = nullptr;     // key-value sort scratch
   uint32_t* order0 = nullptr;
   uint32_t* order1 = nullptr;
-  uint32_t* perm = nullptr;
   double* pre_hi = nullptr;
   double* suf_lo = nullptr;
   double* bsum = nullptr;
@@ -1290,17 +1172,10 @@ struct HierState {
   uint32_t* radix_counts = nullptr;
   uint32_t* bfac = nullptr;
   uint32_t* slots = nullptr;
-  uint32_t* fam_event = nullptr;
-  uint32_t* arm_family = nullptr;
-  uint8_t* arm_local = nullptr;
   uint32_t* term = nullptr;
-  uint8_t* arm_status = nullptr;
-  unsigned long long* dstats = nullptr;
+  unsigned long long* dstats = nullptr;  // [0] descent steps, [1] strictness checks passed, [2] failed arms, [3] least (arm, status)
   uint32_t* qcount = nullptr;   // [0] first-probe misses, [1], [2] step outputs (ping-pong)
-  uint32_t* q_arm[2] = {nullptr, nullptr};
-  uint32_t* q_fac[2] = {nullptr, nullptr};
-  uint64_t q_cap = 0;
-  cudaEvent_t ev_block = nullptr;  // blocking-sync event: the descent loop waits without spinning a core
+  DeviceArena mem;              // the descent's queues, then the forest journal and its records
   uint32_t first_misses = 0, descent_rounds = 0;
   unsigned long long slow[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   unsigned long long visits[kVisitStripes] = {};  // ball-query node visits of the descent steps
@@ -1308,14 +1183,6 @@ struct HierState {
   uint32_t n = 0, K = 0, keff = 0;
   int S = 0;
   uint64_t events = 0, diagnostics = 0;
-  std::vector<HierOrderOut> outs;     // per-order arenas (capacity kept across calls)
-  HugeBuf dsu;
-  uint64_t pin_m = 0, pin_arms = 0;   // pinned host views of the last call
-  uint32_t* p_rank = nullptr;
-  uint32_t* p_cls = nullptr;
-  uint32_t* p_armoff = nullptr;
-  uint32_t* p_term = nullptr;
-  uint8_t* p_stat = nullptr;
   uint32_t* d_cls_rp = nullptr;       // device views (event capacity)
   uint32_t* d_size_rp = nullptr;
   uint32_t* d_armoff = nullptr;
@@ -1329,35 +1196,27 @@ struct HierState {
   uint32_t* run_off = nullptr;
   uint32_t* run_lo = nullptr;
   uint64_t tie_cap = 0, run_cap = 0;
-  // The result stays in the per-order arenas (local indices); off[k] holds the global
-  // offsets of order k's records, off[keff + 1] the totals.  Records take their global
-  // indices when they are copied out.  An empty `off` means no result.
-  std::vector<HierOff> off;
-  uint64_t arm_seeds = 0;  // d_removed holds the removed point of each arm seed
-  std::vector<std::vector<ehgp_vertical_assignment>> vert;  // per source order, global node ids
+  bool complete = false;   // `journal` and d_removed hold the result of the last call
+  uint64_t families = 0, births = 0, arm_seeds = 0;
+  JournalOut journal;
   uint32_t decision = EHGP_ERR_NOT_BUILT;
-  double ms_device = 0, ms_forest = 0, ms_descent = 0, ms_orders = 0;
-  double ms_host[4] = {0, 0, 0, 0};  // exact facade ties, order passes, (unused), vertical maps
+  double ms_device = 0, ms_forest = 0, ms_descent = 0, ms_ties = 0;
   uint64_t descent_steps = 0, arms = 0, exact_boundaries = 0;
   cudaEvent_t ev_step[2] = {nullptr, nullptr};  // around each descent-step launch
   double ms_steps = 0;                          // summed k_arm_step launch times
   uint64_t step_launches = 0;
-  // Schedule of the host forest pass and of the descent parts (results never depend on it):
-  // single-role batches per published chunk, arms per descent part, host pool threads
-  // (0: every hardware thread).
-  uint32_t chunk_batches = 1u << 14, part_arms = 1u << 22, pool_threads = 0;
+  uint32_t part_arms = 0;  // arms per part of the descent (0: one part); results never depend on it
+  // pinned ring through which results reach pageable memory
+  char* stage = nullptr;
+  cudaEvent_t stage_ev[kStageSlots] = {};
 };
 
 void hier_free(Ctx& ctx) {
   if (!ctx.hier) return;
   for (void* p : ctx.hier->allocs) cudaFree(p);
-  for (void* p : {(void*)ctx.hier->q_arm[0], (void*)ctx.hier->q_arm[1], (void*)ctx.hier->q_fac[0],
-                  (void*)ctx.hier->q_fac[1]})
-    if (p) cudaFree(p);
-  for (void* p : {(void*)ctx.hier->p_rank, (void*)ctx.hier->p_cls, (void*)ctx.hier->p_armoff,
-                  (void*)ctx.hier->p_term, (void*)ctx.hier->p_stat})
-    if (p) cudaFreeHost(p);
-  if (ctx.hier->ev_block) cudaEventDestroy(ctx.hier->ev_block);
+  if (ctx.hier->stage) cudaFreeHost(ctx.hier->stage);
+  for (cudaEvent_t ev : ctx.hier->stage_ev)
+    if (ev) cudaEventDestroy(ev);
   for (void* q : {(void*)ctx.hier->tie_num, (void*)ctx.hier->tie_a2, (void*)ctx.hier->tie_idx,
                   (void*)ctx.hier->tie_tmp, (void*)ctx.hier->tie_pos, (void*)ctx.hier->run_off,
                   (void*)ctx.hier->run_lo})
@@ -1403,7 +1262,6 @@ cudaError_t ensure_events(HierState& h, uint64_t m) {
   HA(h.key2, cap);
   HA(h.order0, cap);
   HA(h.order1, cap);
-  HA(h.perm, cap);
   HA(h.pre_hi, cap);
   HA(h.suf_lo, cap);
   HA(h.bsum, cap / 1024 + 2);
@@ -1415,16 +1273,12 @@ cudaError_t ensure_events(HierState& h, uint64_t m) {
   HA(h.counters, 32);
   HA(h.radix_counts, 256ull * ((cap + kRadixTile - 1) / kRadixTile) + 256);
   HA(h.bfac, cap * kMaxFacet);
-  HA(h.fam_event, cap);
   HA(h.d_cls_rp, cap);
   HA(h.d_size_rp, cap);
   HA(h.d_armoff, cap + 1);
   HA(h.dstats, 4);
   const uint64_t arms = 4 * cap;
-  HA(h.arm_family, arms);
-  HA(h.arm_local, arms);
   HA(h.term, arms);
-  HA(h.arm_status, arms);
   HA(h.d_removed, arms);
   uint64_t slots = 1;
   while (slots < 2 * cap + 1024) slots <<= 1;
@@ -1463,7 +1317,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
   GeomBuffers& g = ctx.gb;
   uint64_t launches = 0;
   h.decision = EHGP_ERR_NOT_BUILT;
-  h.off.clear();
+  h.complete = false;
   h.arm_seeds = 0;
   h.n = n;
   h.K = K;
@@ -1481,7 +1335,6 @@ int hier_run(Ctx& ctx, uint32_t K) {
     if (s != EHGP_OK) return s;
   }
   nh = ctx.hb.count;
-  const auto t0 = std::chrono::steady_clock::now();
   cudaEventRecord(ctx.ev0, st);
   const uint64_t total = (uint64_t)np + nh;
   cudaError_t e = ensure_events(h, total + 1);
@@ -1513,7 +1366,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
     // facade order: the event keys (FP64 level midpoints, diagnostics last) move with the indices
     const int passes = radix_sort_kv(st, (uint32_t)total, h.order0, h.order1, h.key, h.key2, 64, rs, &launches);
     k_ev_gather<<<nblk(total, kT), kT, 0, st>>>((uint32_t)total, h.order0, h.order1, ctx.radix.state, passes, h.ev_raw,
-                                                 h.lmid_raw, h.lerr_raw, h.ev, h.lmid, h.lerr, h.perm);
+                                                 h.lmid_raw, h.lerr_raw, h.ev, h.lmid, h.lerr);
     ++launches;
   }
   int scale_h[4];
@@ -1628,6 +1481,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
   const uint64_t fam_lo = rb[2], fam_hi = rb[std::min<uint32_t>(keff + 2, 16)];
   const uint64_t nfam = fam_hi - fam_lo;
   uint64_t narms = 0;
+  uint32_t herr = 0;
   if (m) {
     k_rank_info<<<nblk(m, kT), kT, 0, st>>>(m, h.rank_order, h.ev, h.lclass, h.d_cls_rp, h.d_size_rp);
     ++launches;
@@ -1645,981 +1499,261 @@ int hier_run(Ctx& ctx, uint32_t K) {
     narms = na;
   }
   if (narms > h.cap_arms) return abi_fail(&ctx, EHGP_ERR_CAPACITY, "strict arms exceed the hierarchy buffers");
-  // pinned host views
-  if (h.pin_m < m + 1 || h.pin_arms < narms + 1) {
-    for (void* p : {(void*)h.p_rank, (void*)h.p_cls, (void*)h.p_armoff, (void*)h.p_term, (void*)h.p_stat})
-      if (p) cudaFreeHost(p);
-    h.p_rank = h.p_cls = h.p_armoff = h.p_term = nullptr;
-    h.p_stat = nullptr;
-    const uint64_t pm = (m + 1) + (m + 1) / 8, pa = (narms + 1) + (narms + 1) / 8;
-    if (cudaMallocHost(&h.p_rank, pm * 4) != cudaSuccess || cudaMallocHost(&h.p_cls, pm * 4) != cudaSuccess ||
-        cudaMallocHost(&h.p_armoff, pm * 4) != cudaSuccess || cudaMallocHost(&h.p_term, pa * 4) != cudaSuccess ||
-        cudaMallocHost(&h.p_stat, pa) != cudaSuccess) {
-      h.pin_m = h.pin_arms = 0;
-      return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "pinned host buffers for the hierarchy");
-    }
-    h.pin_m = pm;
-    h.pin_arms = pa;
-  }
-  const uint32_t* rank_order = h.p_rank;
-  const uint32_t* cls_rp = h.p_cls;
-  const uint32_t* arm_off = h.p_armoff;
-  const uint32_t* term = h.p_term;
-  const uint8_t* astat = h.p_stat;
-  if (m) {
-    cudaMemcpyAsync(h.p_rank, h.rank_order, (uint64_t)m * 4, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(h.p_cls, h.d_cls_rp, (uint64_t)m * 4, cudaMemcpyDeviceToHost, st);
-  }
-  if (nfam) cudaMemcpyAsync(h.p_armoff, h.d_armoff, (nfam + 1) * 4, cudaMemcpyDeviceToHost, st);
-  if (narms) {
-    k_arm_expand<<<nblk(nfam, kT), kT, 0, st>>>((uint32_t)nfam, (uint32_t)fam_lo, h.rank_order, h.ev, h.d_armoff,
-                                               h.arm_family, h.arm_local, h.d_removed);
-    ++launches;
-  }
-  // the facade, rank partition, births and arm seeds are complete: the descent runs order
-  // by order below, overlapped with the host forest pass
-  uint32_t herr = 0;
-  cudaMemcpyAsync(&herr, h.counters + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "strict-arm seeds");
-  if (herr) return abi_fail(&ctx, EHGP_ERR_CAPACITY, "the birth facet table is full");
-  if (narms) {
-    if (!h.qcount && (e = halloc(h, &h.qcount, 4)) != cudaSuccess)
-      return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "descent queue");
-    if (h.q_cap < narms) {  // worst case: every arm misses
-      for (void* p : {(void*)h.q_arm[0], (void*)h.q_arm[1], (void*)h.q_fac[0], (void*)h.q_fac[1]})
-        if (p) cudaFree(p);
-      h.q_arm[0] = h.q_arm[1] = h.q_fac[0] = h.q_fac[1] = nullptr;
-      const uint64_t qc = narms + narms / 8 + 1024;
-      if (cudaMalloc(&h.q_arm[0], qc * 4) != cudaSuccess || cudaMalloc(&h.q_arm[1], qc * 4) != cudaSuccess ||
-          cudaMalloc(&h.q_fac[0], qc * 4 * kMaxFacet) != cudaSuccess ||
-          cudaMalloc(&h.q_fac[1], qc * 4 * kMaxFacet) != cudaSuccess)
-        return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "descent queue buffers do not fit the device");
-      h.q_cap = qc;
-    }
-  }
   h.arms = narms;
   h.exact_boundaries = unc;
-  // ---- host: journal, seeds and the forest journal ------------------------------------
-  // Orders are independent (their handles, components and nodes never meet), so each
-  // order runs on its own host thread with local indices; records take the global offsets
-  // the reference's single pass would give when they are copied out.
-  const auto t1 = std::chrono::steady_clock::now();
-  const uint64_t birth_count = n + nb_higher;
-  // union-find state packed per birth handle: one cache line touch per arm
-  if (!h.dsu.ensure(birth_count * sizeof(HierDsu)))  // each order initialises its own handle range
-    return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "the union-find array does not fit host memory");
-  HierDsu* dsu = static_cast<HierDsu*>(h.dsu.p);
-  // per-order arenas and union-find state persist across calls (no page faults when warm)
-  if (h.outs.size() < keff + 1) h.outs.resize(keff + 1);
-  auto& outs = h.outs;
-  for (uint32_t k = 1; k <= keff; ++k) {
-    HierOrderOut& o = outs[k];
-    o.status = EHGP_OK;
-    o.msg = "";
+  JournalIn in;
+  in.n = n;
+  in.keff = keff;
+  in.handles = (uint32_t)(n + nb_higher);
+  in.families = (uint32_t)nfam;
+  in.arms = (uint32_t)narms;
+  for (uint32_t k = 1; k <= keff + 1; ++k) {
+    in.fam0[k] = (uint32_t)(rb[std::min<uint32_t>(k + 1, 16)] - fam_lo);
+    in.han0[k] = k == 1 ? 0 : (uint32_t)(n + rb[k] - rb[2]);
   }
-  const auto t_init = std::chrono::steady_clock::now();
-  // Each order runs a lean sequential core (union-find over its batches; it writes the arm
-  // bindings in place and handles multi-role batches whole) and publishes chunks of
-  // single-role batches with the running counters at their start; a shared pool of host
-  // threads rebuilds those batches' journal and forest records from the bindings while the
-  // cores go on.  Record positions and contents equal those of one sequential pass.
-  struct Cnt {
-    uint64_t bi, si;
-    uint32_t jb, role, birth, sad, grp, node, child, count;
-    uint64_t carriers, reduced;
-  };
-  const uint32_t kChunkBatches = h.chunk_batches;
-  constexpr uint32_t kSnapBlock = 4096;
-  struct Progress {
-    std::vector<std::unique_ptr<Cnt[]>> blocks;  // published chunk starts, kSnapBlock per block
-    std::atomic<uint32_t> published{0}, claimed{0}, replayed{0};
-    std::atomic<int> done{0}, bad{0};
-    // vertical maps from this order (k >= 2): parallel gathers, then one sweep
-    std::atomic<uint32_t> va_claimed{0}, va_done{0};
-    std::atomic<int> vb_claimed{0}, vb_done{0}, vstat{EHGP_OK};
-  };
-  std::vector<Progress> prog(keff + 1);
-  auto order_range = [&](uint32_t k, uint64_t& b_lo, uint64_t& b_hi, uint64_t& s_lo, uint64_t& s_hi,
-                         uint64_t& arm_lo, uint64_t& arm_hi) {
-    b_lo = k == 1 ? 0 : rb[k];
-    b_hi = k == 1 ? 0 : rb[k + 1];
-    s_lo = rb[k + 1];
-    s_hi = rb[k + 2 > 16 ? 16 : k + 2];
-    arm_lo = s_hi > s_lo ? arm_off[s_lo - fam_lo] : 0;
-    arm_hi = s_hi > s_lo ? arm_off[s_hi - fam_lo] : 0;
-  };
-  // fam_lim[k]: saddle positions below it have their terminal handles on the host (the
-  // descent of an order arrives in parts cut at batch boundaries); stop_all ends waits
-  std::unique_ptr<std::atomic<uint64_t>[]> fam_lim(new std::atomic<uint64_t>[keff + 1]);
-  for (uint32_t k = 0; k <= keff; ++k) fam_lim[k].store(0);
-  std::atomic<int> stop_all{0};
-  // This order's union-find handles: every one a root, not yet born (done by the order's
-  // thread while the device descends its first part).
-  auto init_dsu = [&](uint32_t k) {
-    const uint64_t h_lo = k == 1 ? 0 : n + (rb[k] - rb[2]), h_hi = k == 1 ? n : n + (rb[k + 1] - rb[2]);
-    for (uint64_t i = h_lo; i < h_hi; ++i) dsu[i] = {(uint32_t)i, kUnborn};
-  };
-  auto run_core = [&](uint32_t k, HierOrderOut& o) {
-    const auto to0 = std::chrono::steady_clock::now();
-    Progress& pg = prog[k];
-    auto fail_o = [&](const char* m) {
-      o.status = EHGP_ERR_DEGENERATE;
-      o.msg = m;
-    };
-    auto find = [&](uint32_t x) {  // path halving; roots follow the least-handle union rule alone
-      while (dsu[x].parent != x) {
-        dsu[x].parent = dsu[dsu[x].parent].parent;
-        x = dsu[x].parent;
-      }
-      return x;
-    };
-    uint64_t b_lo, b_hi, s_lo, s_hi, arm_lo, arm_hi;
-    order_range(k, b_lo, b_hi, s_lo, s_hi, arm_lo, arm_hi);
-    const uint64_t births_k = k == 1 ? n : b_hi - b_lo, fams_k = s_hi - s_lo, arms_k = arm_hi - arm_lo;
-    const uint64_t h_lo = k == 1 ? 0 : n + (rb[k] - rb[2]), h_hi = h_lo + births_k;  // this order's handles
-    // capacities are upper bounds (one batch holds at least one role; a group at least one
-    // saddle; a multifusion's children are distinct prior roots of its arms' carriers)
-    o.jb.reset(births_k + fams_k);
-    o.fb.reset(births_k + fams_k);
-    o.roles.reset(births_k + fams_k);
-    o.fam.reset(fams_k);
-    o.saddles.reset(fams_k);
-    o.groups.reset(fams_k);
-    o.births.reset(births_k);
-    o.bindings.reset(arms_k);
-    o.nodes.reset((k == 1 ? n : 0) + fams_k);
-    o.children.reset(arms_k);
-    o.roots.reset(births_k);
-    o.node_cls.reset((k == 1 ? n : 0) + fams_k);
-    o.fam_res.reset(fams_k);
-    // this order's union-find handles
-    pg.blocks.clear();
-    // chunks <= batches / kChunkBatches + multi-role batches + 1 <= batches + 1
-    pg.blocks.resize((births_k + fams_k + 1) / kSnapBlock + 2);
-    Cnt c{b_lo, s_lo, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    uint32_t nchunk = 0;
-    Cnt open = c;  // start of the chunk being filled
-    auto close_chunk = [&] {
-      if (open.count == 0) return;
-      const uint32_t blk = nchunk / kSnapBlock;
-      if (!pg.blocks[blk]) pg.blocks[blk].reset(new Cnt[kSnapBlock]);
-      pg.blocks[blk][nchunk % kSnapBlock] = open;
-      ++nchunk;
-      stream_fence();  // the chunk's bindings
-      pg.published.store(nchunk, std::memory_order_release);
-    };
-    auto reopen = [&] {
-      open = c;
-      open.count = 0;
-    };
-    struct Role {
-      uint32_t proj, role, fi, pos;
-    };
-    struct Arm {
-      uint32_t seed, carrier, prior;
-    };
-    struct Plan {
-      uint32_t c_off, c_cnt, p_off, p_cnt, s_off, s_cnt, kind, created, result;
-    };
-    std::vector<Role> batch_roles;
-    std::vector<uint32_t> fam_pos, fam_local, arm_b_off, cars, qp, plan_of, plan_car, plan_prior, plan_sad, tmp,
-        new_births;
-    std::vector<Arm> arms_b;
-    std::vector<Plan> plans;
-    std::vector<ehgp_forest_node> gnodes;
-    uint64_t& bi = c.bi;
-    uint64_t& si = c.si;
-    uint64_t& carriers = c.carriers;
-    uint64_t& reduced = c.reduced;
-    bool singles = k == 1;
-    uint64_t lim = 0;  // saddle positions below lim have their terminal handles
-    auto core = [&]() {
-      while (singles || bi < b_hi || si < s_hi) {
-        uint32_t cls = kInvalid32, lev = kInvalid32;
-        if (!singles) {
-          const uint32_t cls_b = bi < b_hi ? cls_rp[bi] : kInvalid32;
-          const uint32_t cls_s = si < s_hi ? cls_rp[si] : kInvalid32;
-          if (cls_s <= cls_b && si >= lim) {  // the batch holds saddles: wait for their part of the descent
-            while ((lim = fam_lim[k].load(std::memory_order_acquire)) <= si) {
-              if (stop_all.load(std::memory_order_acquire)) {
-                fail_o("the strict-arm descent stopped");
-                return;
-              }
-              std::this_thread::sleep_for(std::chrono::microseconds(20));
-            }
-          }
-          cls = std::min(cls_b, cls_s);
-          lev = cls_b <= cls_s ? rank_order[bi] : rank_order[si];
-          // single-role batches (almost every batch off ties): union-find only here
-          const bool one_b = cls_b == cls && !(bi + 1 < b_hi && cls_rp[bi + 1] == cls) && cls_s != cls;
-          const bool one_s = cls_s == cls && !(si + 1 < s_hi && cls_rp[si + 1] == cls) && cls_b != cls;
-          if (one_b) {
-            const uint32_t handle = n + (uint32_t)(bi - rb[2]);
-            dsu[handle].rroot = kInvalid32;
-            ++carriers;
-            ++c.jb; ++c.role; ++c.birth;
-            ++bi;
-            if (++open.count == kChunkBatches) { close_chunk(); reopen(); }
-            continue;
-          }
-          if (one_s) {
-            const uint32_t pos = (uint32_t)(si - fam_lo), fidx = (uint32_t)(si - s_lo);
-            const uint32_t a0 = arm_off[pos], a1 = arm_off[pos + 1];
-            uint32_t dc[4], pr[4];
-            int ndc = 0, np = 0;
-            for (uint32_t a = a0; a < a1; ++a) {
-              // two-stage prefetch: the arm's record 64 arms ahead, its parent's 32 ahead
-              if (a + 64 < arm_hi) __builtin_prefetch(&dsu[term[a + 64] < birth_count ? term[a + 64] : 0]);
-              if (a + 32 < arm_hi && term[a + 32] >= h_lo && term[a + 32] < h_hi) __builtin_prefetch(&dsu[dsu[term[a + 32]].parent]);
-              if (term[a] < h_lo || term[a] >= h_hi || dsu[term[a]].rroot == kUnborn) {
-                fail_o("a strict arm descended to a minimum that is not yet born");
-                return;
-              }
-              const uint32_t c0 = find(term[a]);
-              const uint32_t p0 = dsu[c0].rroot;
-              nt_store(o.bindings[a - arm_lo], ehgp_forest_binding{a, fidx, c0, p0});
-              bool dup = false;
-              for (int t = 0; t < ndc; ++t) dup |= dc[t] == c0;
-              if (dup) continue;
-              int j = ndc++;
-              while (j > 0 && dc[j - 1] > c0) { dc[j] = dc[j - 1]; --j; }
-              dc[j] = c0;
-              if (p0 != kInvalid32) {
-                int q = np++;
-                while (q > 0 && pr[q - 1] > p0) { pr[q] = pr[q - 1]; --q; }
-                pr[q] = p0;
-                if ((q > 0 && pr[q - 1] == p0) || (q + 1 < np && pr[q + 1] == p0)) {
-                  fail_o("a frozen carrier class repeats a reduced root");
-                  return;
-                }
-              }
-            }
-            uint32_t result;
-            if (np == 1) {
-              result = pr[0];
-            } else {
-              if (np == 0 && k == 1) {
-                fail_o("an order-one group has no root");
-                return;
-              }
-              result = c.node++;
-              if (np >= 2) c.child += (uint32_t)np;
-            }
-            // commit: the distinct carriers are pre-batch roots; the least survives
-            for (int t = 1; t < ndc; ++t) dsu[dc[t]].parent = dc[0];
-            carriers -= (uint64_t)(ndc - 1);
-            dsu[dc[0]].rroot = result;
-            reduced = reduced - (uint64_t)np + 1;
-            ++c.jb; ++c.role; ++c.sad; ++c.grp;
-            ++si;
-            if (++open.count == kChunkBatches) { close_chunk(); reopen(); }
-            continue;
-          }
-        }
-        // a multi-role batch, whole: the arenas' counts follow the core's counters
-        close_chunk();
-        o.jb.n = c.jb; o.fb.n = c.jb; o.roles.n = c.role; o.fam.n = (uint32_t)(si - s_lo); o.births.n = c.birth;
-        o.bindings.n = si < s_hi ? arm_off[si - fam_lo] - arm_lo : arms_k;
-        o.saddles.n = c.sad; o.groups.n = c.grp; o.nodes.n = c.node; o.children.n = c.child;
-        const uint32_t bidx = (uint32_t)o.jb.size();
-        ehgp_journal_batch jb{k, lev, (uint32_t)o.roles.size(), 0, 0, 0};
-        ehgp_forest_batch fb{};
-        fb.order = k;
-        fb.level_event = lev;
-        fb.pre_carriers = (uint32_t)carriers;
-        fb.pre_roots = (uint32_t)reduced;
-        batch_roles.clear();
-        if (singles) {
-          for (uint32_t p = 0; p < n; ++p) batch_roles.push_back({p, 0, kInvalid32, p});
-        } else {
-          while (bi < b_hi && cls_rp[bi] == cls) {
-            batch_roles.push_back({n + rank_order[bi], 0, rank_order[bi], (uint32_t)(bi - rb[2])});
-            ++bi;
-          }
-          const size_t nbr = batch_roles.size();
-          while (si < s_hi && cls_rp[si] == cls) {
-            batch_roles.push_back({n + rank_order[si], 1, rank_order[si], (uint32_t)(si - fam_lo)});
-            ++si;
-          }
-          if (nbr && nbr < batch_roles.size())
-            std::inplace_merge(batch_roles.begin(), batch_roles.begin() + nbr, batch_roles.end(),
-                               [](const Role& x, const Role& y) { return x.proj < y.proj; });
-        }
-        singles = false;
-        // journal roles and saddle families
-        fam_pos.clear();
-        fam_local.clear();
-        for (size_t q = 0; q < batch_roles.size(); ++q) {
-          const Role& r = batch_roles[q];
-          const uint32_t ridx = (uint32_t)o.roles.size();
-          o.roles.push_back({bidx, r.proj, r.role});
-          if (r.role == 0) {
-            ++jb.birth_roles;
-            continue;
-          }
-          ++jb.saddle_roles;
-          // arm seeds follow the rank partition: the family at position p owns seeds arm_off[p]..
-          fam_local.push_back((uint32_t)o.fam.size());
-          o.fam.push_back({r.fi, r.proj, ridx, bidx, k, arm_off[r.pos], arm_off[r.pos + 1] - arm_off[r.pos]});
-          fam_pos.push_back(r.pos);
-        }
-        jb.role_count = (uint32_t)batch_roles.size();
-        o.jb.push_back(jb);
-        // arms resolved against the pre-batch components
-        arms_b.clear();
-        arm_b_off.clear();
-        for (uint32_t q = 0; q < fam_pos.size(); ++q) {
-          const uint32_t fpos = fam_pos[q];
-          arm_b_off.push_back((uint32_t)arms_b.size());
-          for (uint64_t a = arm_off[fpos]; a < arm_off[fpos + 1]; ++a) {
-            // two-stage prefetch: the arm's record 64 arms ahead, its parent's 32 ahead
-            if (a + 64 < arm_hi) __builtin_prefetch(&dsu[term[a + 64] < birth_count ? term[a + 64] : 0]);
-            if (a + 32 < arm_hi && term[a + 32] >= h_lo && term[a + 32] < h_hi) __builtin_prefetch(&dsu[dsu[term[a + 32]].parent]);
-            if (term[a] < h_lo || term[a] >= h_hi || dsu[term[a]].rroot == kUnborn) {
-              fail_o("a strict arm descended to a minimum that is not yet born");
-              return;
-            }
-            const uint32_t c0 = find(term[a]);
-            arms_b.push_back({(uint32_t)a, c0, dsu[c0].rroot});
-          }
-        }
-        arm_b_off.push_back((uint32_t)arms_b.size());
-        // frozen-root quotient: transitive carrier classes, ordered by least carrier
-        plans.clear();
-        plan_car.clear();
-        plan_prior.clear();
-        plan_sad.clear();
-        if (!fam_pos.empty()) {
-          cars.clear();
-          for (const Arm& a : arms_b) cars.push_back(a.carrier);
-          std::sort(cars.begin(), cars.end());
-          cars.erase(std::unique(cars.begin(), cars.end()), cars.end());
-          const uint32_t nc = (uint32_t)cars.size();
-          auto qi = [&](uint32_t x) { return (uint32_t)(std::lower_bound(cars.begin(), cars.end(), x) - cars.begin()); };
-          qp.resize(nc);
-          std::iota(qp.begin(), qp.end(), 0u);
-          auto qf = [&](uint32_t x) {
-            while (qp[x] != x) x = qp[x] = qp[qp[x]];
-            return x;
-          };
-          for (uint32_t q = 0; q + 1 < arm_b_off.size(); ++q) {
-            const uint32_t a0 = qf(qi(arms_b[arm_b_off[q]].carrier));
-            for (uint32_t a = arm_b_off[q] + 1; a < arm_b_off[q + 1]; ++a) {
-              const uint32_t x = qf(a0), y = qf(qi(arms_b[a].carrier));
-              if (x != y) qp[std::max(x, y)] = std::min(x, y);
-            }
-          }
-          plan_of.assign(nc, kInvalid32);
-          for (uint32_t i = 0; i < nc; ++i) {
-            const uint32_t r0 = qf(i);
-            if (plan_of[r0] == kInvalid32) {
-              plan_of[r0] = (uint32_t)plans.size();
-              plans.push_back({0, 0, 0, 0, 0, 0, 0, kInvalid32, 0});
-            }
-          }
-          for (uint32_t i = 0; i < nc; ++i) {
-            Plan& p = plans[plan_of[qf(i)]];
-            ++p.c_cnt;
-            if (dsu[cars[i]].rroot != kInvalid32) ++p.p_cnt;
-          }
-          for (uint32_t q = 0; q + 1 < arm_b_off.size(); ++q) ++plans[plan_of[qf(qi(arms_b[arm_b_off[q]].carrier))]].s_cnt;
-          uint32_t co = 0, po = 0, so = 0;
-          for (Plan& p : plans) {
-            p.c_off = co; p.p_off = po; p.s_off = so;
-            co += p.c_cnt; po += p.p_cnt; so += p.s_cnt;
-            p.c_cnt = p.p_cnt = p.s_cnt = 0;
-          }
-          plan_car.resize(co);
-          plan_prior.resize(po);
-          plan_sad.resize(so);
-          for (uint32_t i = 0; i < nc; ++i) {
-            Plan& p = plans[plan_of[qf(i)]];
-            plan_car[p.c_off + p.c_cnt++] = cars[i];
-            if (dsu[cars[i]].rroot != kInvalid32) plan_prior[p.p_off + p.p_cnt++] = dsu[cars[i]].rroot;
-          }
-          for (uint32_t q = 0; q + 1 < arm_b_off.size(); ++q) {
-            Plan& p = plans[plan_of[qf(qi(arms_b[arm_b_off[q]].carrier))]];
-            plan_sad[p.s_off + p.s_cnt++] = q;
-          }
-          uint32_t pending = 0;
-          for (Plan& p : plans) {
-            uint32_t* pr = plan_prior.data() + p.p_off;
-            std::sort(pr, pr + p.p_cnt);
-            if (std::adjacent_find(pr, pr + p.p_cnt) != pr + p.p_cnt) {
-              fail_o("a frozen carrier class repeats a reduced root");
-              return;
-            }
-            if (p.p_cnt == 1) {
-              p.kind = 1;
-              p.created = kInvalid32;
-              p.result = pr[0];
-            } else {
-              if (p.p_cnt == 0 && k == 1) {
-                fail_o("an order-one group has no root");
-                return;
-              }
-              p.kind = p.p_cnt == 0 ? 0 : 2;
-              p.created = (uint32_t)o.nodes.size() + pending++;
-              p.result = p.created;
-            }
-          }
-        }
-        fb.saddle_offset = (uint32_t)o.saddles.size();
-        fb.group_offset = (uint32_t)o.groups.size();
-        gnodes.clear();
-        for (const Plan& p : plans) {
-          const uint32_t g_soff = (uint32_t)o.saddles.size();
-          const uint32_t gidx = (uint32_t)o.groups.size();
-          for (uint32_t t = 0; t < p.s_cnt; ++t) {
-            const uint32_t q = plan_sad[p.s_off + t];
-            const uint32_t fidx = fam_local[q];
-            const uint32_t arm_o = (uint32_t)o.bindings.size();
-            tmp.clear();
-            uint32_t nprior = 0;
-            for (uint32_t a = arm_b_off[q]; a < arm_b_off[q + 1]; ++a) {
-              const Arm& am = arms_b[a];
-              o.bindings.push_back({am.seed, fidx, am.carrier, am.prior});
-              tmp.push_back(am.carrier);
-            }
-            std::sort(tmp.begin(), tmp.end());
-            tmp.erase(std::unique(tmp.begin(), tmp.end()), tmp.end());
-            for (uint32_t c0 : tmp) nprior += dsu[c0].rroot != kInvalid32;  // carriers are pre-batch roots
-            o.saddles.push_back({fidx, o.fam[fidx].event, bidx, arm_o, arm_b_off[q + 1] - arm_b_off[q],
-                                 (uint32_t)tmp.size(), (uint32_t)tmp.size() - nprior, nprior, gidx});
-          }
-          const uint32_t ccnt = p.kind == 2 ? p.p_cnt : 0u;
-          o.groups.push_back({bidx, g_soff, (uint32_t)o.saddles.size() - g_soff, p.c_cnt, p.c_cnt - p.p_cnt, p.p_cnt,
-                              (uint32_t)o.children.size(), ccnt, p.created, p.result, p.kind});
-          if (p.kind != 1)
-            gnodes.push_back({k, lev, p.kind == 0 ? 1u : 2u, (uint32_t)o.children.size(), ccnt, kInvalid32, gidx});
-          if (p.kind == 2)
-            o.children.append(plan_prior.begin() + p.p_off, plan_prior.begin() + p.p_off + p.p_cnt);
-        }
-        o.nodes.append(gnodes.begin(), gnodes.end());
-        // births of this batch (hidden from this batch's arms); handles are global
-        fb.birth_offset = (uint32_t)o.births.size();
-        new_births.clear();
-        for (const Role& r : batch_roles) {
-          if (r.role != 0) continue;
-          const uint32_t handle = k == 1 ? r.proj : n + r.pos;
-          uint32_t node = kInvalid32;
-          if (k == 1) {
-            node = (uint32_t)o.nodes.size();
-            o.nodes.push_back({1, kInvalid32, 0, (uint32_t)o.children.size(), 0, handle, kInvalid32});
-          }
-          o.births.push_back({r.proj, bidx, k, handle, node});
-          new_births.push_back(handle);
-        }
-        // commit: unions (least handle survives), reduced roots, then births
-        for (const Plan& p : plans) {
-          uint32_t r0 = find(plan_car[p.c_off]);
-          uint32_t had_reduced = dsu[r0].rroot != kInvalid32;
-          for (uint32_t i = 1; i < p.c_cnt; ++i) {
-            const uint32_t r1 = find(plan_car[p.c_off + i]);
-            if (r1 == r0) continue;
-            had_reduced += dsu[r1].rroot != kInvalid32;
-            const uint32_t lo = std::min(r0, r1), hi = std::max(r0, r1);
-            dsu[hi].parent = lo;
-            r0 = lo;
-            --carriers;
-          }
-          dsu[r0].rroot = p.result;
-          reduced = reduced - had_reduced + 1;
-        }
-        for (size_t t = 0; t < new_births.size(); ++t) {
-          const uint32_t hnd = new_births[t];
-          dsu[hnd].rroot = k == 1 ? o.births[fb.birth_offset + t].order_one_node : kInvalid32;
-          ++carriers;
-          if (k == 1) ++reduced;
-        }
-        fb.birth_count = (uint32_t)new_births.size();
-        fb.saddle_count = (uint32_t)o.saddles.size() - fb.saddle_offset;
-        fb.group_count = (uint32_t)o.groups.size() - fb.group_offset;
-        fb.post_carriers = (uint32_t)carriers;
-        fb.post_roots = (uint32_t)reduced;
-        o.fb.push_back(fb);
-        for (uint64_t i = c.node; i < o.nodes.n && i < o.nodes.cap; ++i)
-          o.node_cls[i] = o.nodes[i].level_event == kInvalid32 ? kInvalid32 : cls;
-        for (uint64_t sd = c.sad; sd < o.saddles.n && sd < o.saddles.cap; ++sd)
-          o.fam_res[o.saddles[sd].family] = o.groups[o.saddles[sd].group].result_node;
-        c.jb = (uint32_t)o.jb.n; c.role = (uint32_t)o.roles.n; c.birth = (uint32_t)o.births.n;
-        c.sad = (uint32_t)o.saddles.n; c.grp = (uint32_t)o.groups.n; c.node = (uint32_t)o.nodes.n;
-        c.child = (uint32_t)o.children.n;
-        reopen();
-      }
-    };
-    core();
-    if (o.status == EHGP_OK) {
-      close_chunk();
-      o.jb.n = c.jb; o.fb.n = c.jb; o.roles.n = c.role; o.fam.n = fams_k; o.births.n = c.birth; o.bindings.n = arms_k;
-      o.saddles.n = c.sad; o.groups.n = c.grp; o.nodes.n = c.node; o.children.n = c.child;
-      if (!o.jb.fits() || !o.roles.fits() || !o.nodes.fits() || !o.children.fits() || !o.groups.fits() ||
-          !o.saddles.fits() || !o.births.fits() || !o.fb.fits() || !o.fam.fits() || !o.bindings.fits())
-        fail_o("internal: a forest arena bound was exceeded");
+  in.ev = h.rank_order + fam_lo;
+  in.cls = h.d_cls_rp + fam_lo;
+  in.armoff = h.d_armoff;
+  in.term = h.term;
+  // ---- strict-arm descent ----
+  // One part unless a schedule says otherwise: the fewer parts, the fewer rounds, and a round
+  // is a few launches and a look at its queue's length.
+  const uint32_t part_fams = h.part_arms ? std::max(1u, h.part_arms / 4u) : (uint32_t)nfam;
+  const uint64_t journal = journal_bytes(in);
+  // queue entries: about a third of the arms miss their first probe; a longer queue grows
+  uint64_t q_cap = std::min<uint64_t>(narms, std::max<uint64_t>(narms * 3 / 8, 1u << 16)) + 32;
+  uint32_t *q_arm[2], *q_fac[2];
+  auto queues = [&]() -> cudaError_t {
+    cudaError_t r = h.mem.reset(std::max(journal, q_cap * 2 * (4 + 4 * kMaxFacet) + 4096));
+    for (int i = 0; i < 2; ++i) {
+      if (r == cudaSuccess) r = h.mem.take(&q_arm[i], q_cap);
+      if (r == cudaSuccess) r = h.mem.take(&q_fac[i], q_cap * kMaxFacet);
     }
-    if (o.status == EHGP_OK) {
-      // final roots of this order (local node ids)
-      for (uint64_t hnd = h_lo; hnd < h_hi; ++hnd)
-        if (dsu[hnd].parent == hnd && dsu[hnd].rroot != kInvalid32 && dsu[hnd].rroot != kUnborn)
-          o.roots.push_back({k, (uint32_t)hnd, dsu[hnd].rroot});
-      std::sort(o.roots.begin(), o.roots.end(),
-                [](const ehgp_forest_root& x, const ehgp_forest_root& y) { return x.node < y.node; });
+    return r;
+  };
+  auto no_queue = [&] {
+    cudaGetLastError();
+    return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "descent queue buffers do not fit the device");
+  };
+  if (queues() != cudaSuccess) return no_queue();
+  if (!h.qcount && (e = halloc(h, &h.qcount, 4)) != cudaSuccess)
+    return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "descent queue");
+  const DescentParams dp{n, 2 * n - 2, g.tnodes, b.px, b.py, b.pz, h.S, h.slots, (uint32_t)(h.cap_slots - 1), h.bfac,
+                         (uint32_t)nb_higher};
+  uint32_t misses = 0, max_rounds = 0;
+  h.descent_steps = 0;
+  h.ms_steps = 0;
+  h.step_launches = 0;
+  for (cudaEvent_t& ev : h.ev_step)
+    if (!ev && cudaEventCreate(&ev) != cudaSuccess) ev = nullptr;
+  cudaEventRecord(ctx.evk0, st);
+  cudaMemsetAsync(h.dstats + 3, 0xff, sizeof(unsigned long long), st);
+  for (uint32_t f0 = 0; f0 < nfam; f0 += part_fams) {
+    const uint32_t nf = std::min<uint32_t>(part_fams, (uint32_t)nfam - f0);
+    uint32_t pending = 0;
+    for (;;) {  // count -> grow -> queue
+      cudaMemsetAsync(h.qcount, 0, 4 * sizeof(uint32_t), st);
+      k_arm_probe<<<nblk(nf, kT), kT, 0, st>>>(dp, f0, nf, in.ev, h.d_armoff, h.ev, h.d_removed, h.term, q_arm[0],
+                                               q_fac[0], (uint32_t)q_cap, h.qcount);
+      ++launches;
+      cudaMemcpyAsync(&pending, h.qcount, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+      cudaMemcpyAsync(&herr, h.counters + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+      if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "strict-arm seeds");
+      if (herr) return abi_fail(&ctx, EHGP_ERR_CAPACITY, "the birth facet table is full");
+      if (pending <= q_cap) break;
+      q_cap = pending;
+      if (queues() != cudaSuccess) return no_queue();
     }
-    o.v_res.reset(o.nodes.n);
-    o.v_cls.reset(o.nodes.n);
-    o.ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - to0).count();
-    stream_fence();
-    pg.done.store(1, std::memory_order_release);
-  };
-  // Rebuilds the records of one published chunk of single-role batches.
-  auto replay = [&](uint32_t k, uint32_t j) {
-    HierOrderOut& o = outs[k];
-    Progress& pg = prog[k];
-    Cnt c = pg.blocks[j / kSnapBlock][j % kSnapBlock];
-    uint64_t b_lo, b_hi, s_lo, s_hi, arm_lo, arm_hi;
-    order_range(k, b_lo, b_hi, s_lo, s_hi, arm_lo, arm_hi);
-    (void)b_lo;
-    (void)arm_hi;
-    for (uint32_t t = 0; t < c.count; ++t) {
-      const uint32_t cls_b = c.bi < b_hi ? cls_rp[c.bi] : kInvalid32;
-      const uint32_t cls_s = c.si < s_hi ? cls_rp[c.si] : kInvalid32;
-      const uint32_t cls = std::min(cls_b, cls_s);
-      const uint32_t lev = cls_b <= cls_s ? rank_order[c.bi] : rank_order[c.si];
-      const bool one_b = cls_b == cls && !(c.bi + 1 < b_hi && cls_rp[c.bi + 1] == cls) && cls_s != cls;
-      const bool one_s = cls_s == cls && !(c.si + 1 < s_hi && cls_rp[c.si + 1] == cls) && cls_b != cls;
-      const uint32_t bidx = c.jb;
-      if (one_b) {
-        const uint32_t pos = (uint32_t)(c.bi - rb[2]), fi = rank_order[c.bi];
-        nt_store(o.jb[bidx], ehgp_journal_batch{k, lev, c.role, 1, 1, 0});
-        nt_store(o.roles[c.role], ehgp_role_record{bidx, n + fi, 0});
-        nt_store(o.births[c.birth], ehgp_forest_birth{n + fi, bidx, k, n + pos, kInvalid32});
-        nt_store(o.fb[bidx], ehgp_forest_batch{k, lev, c.birth, 1, c.sad, 0, c.grp, 0, (uint32_t)c.carriers,
-                                               (uint32_t)c.reduced, (uint32_t)(c.carriers + 1), (uint32_t)c.reduced});
-        ++c.carriers;
-        ++c.jb; ++c.role; ++c.birth;
-        ++c.bi;
-        continue;
+    misses += pending;
+    int cur = 0;
+    uint32_t rounds = 0;
+    while (pending) {
+      if (++rounds > (uint32_t)kDescentSteps) {
+        h.decision = EHGP_ERR_DEGENERATE;
+        return abi_fail(&ctx, EHGP_ERR_DEGENERATE, "a strict arm descent exceeded its step budget");
       }
-      if (!one_s) {
-        pg.bad.store(1);
-        return;
-      }
-      const uint32_t pos = (uint32_t)(c.si - fam_lo), fi = rank_order[c.si], fidx = (uint32_t)(c.si - s_lo);
-      const uint32_t a0 = arm_off[pos], a1 = arm_off[pos + 1];
-      const uint32_t ridx = c.role;
-      nt_store(o.jb[bidx], ehgp_journal_batch{k, lev, ridx, 1, 0, 1});
-      nt_store(o.roles[ridx], ehgp_role_record{bidx, n + fi, 1});
-      nt_store(o.fam[fidx], ehgp_family_record{fi, n + fi, ridx, bidx, k, a0, a1 - a0});
-      uint32_t dc[4], pr[4];
-      int ndc = 0, np = 0;
-      for (uint32_t a = a0; a < a1; ++a) {
-        const ehgp_forest_binding& bd = o.bindings[a - arm_lo];
-        bool dup = false;
-        for (int q = 0; q < ndc; ++q) dup |= dc[q] == bd.carrier;
-        if (dup) continue;
-        dc[ndc++] = bd.carrier;
-        if (bd.prior_root != kInvalid32) {
-          int q = np++;
-          while (q > 0 && pr[q - 1] > bd.prior_root) { pr[q] = pr[q - 1]; --q; }
-          pr[q] = bd.prior_root;
-        }
-      }
-      const uint32_t kind = np == 1 ? 1u : np == 0 ? 0u : 2u;
-      const uint32_t created = kind == 1 ? kInvalid32 : c.node;
-      const uint32_t result = kind == 1 ? pr[0] : created;
-      const uint32_t ccnt = kind == 2 ? (uint32_t)np : 0u;
-      nt_store(o.saddles[c.sad], ehgp_forest_saddle{fidx, fi, bidx, a0 - (uint32_t)arm_lo, a1 - a0, (uint32_t)ndc,
-                                                    (uint32_t)(ndc - np), (uint32_t)np, c.grp});
-      nt_store(o.groups[c.grp], ehgp_forest_group{bidx, c.sad, 1, (uint32_t)ndc, (uint32_t)(ndc - np), (uint32_t)np,
-                                                  c.child, ccnt, created, result, kind});
-      o.fam_res[fidx] = result;
-      if (kind != 1) {
-        o.node_cls[c.node] = cls;
-        o.nodes[c.node++] = {k, lev, kind == 0 ? 1u : 2u, c.child, ccnt, kInvalid32, c.grp};
-      }
-      for (uint32_t q = 0; q < ccnt; ++q) o.children[c.child + q] = pr[q];
-      c.child += ccnt;
-      nt_store(o.fb[bidx], ehgp_forest_batch{k, lev, c.birth, 0, c.sad, 1, c.grp, 1, (uint32_t)c.carriers,
-                                             (uint32_t)c.reduced, (uint32_t)(c.carriers - (uint64_t)(ndc - 1)),
-                                             (uint32_t)(c.reduced - (uint64_t)np + 1)});
-      c.carriers -= (uint64_t)(ndc - 1);
-      c.reduced = c.reduced - (uint64_t)np + 1;
-      ++c.jb; ++c.role; ++c.sad; ++c.grp;
-      ++c.si;
-    }
-  };
-  // ---- vertical maps: each reduced node of order k >= 2 at level a maps, on the closed
-  // cut at a, to the root of order k - 1 whose component contains it.  A carrier birth of
-  // the node's group is an event of rank k; that event is a saddle of order k - 1, whose
-  // group's resulting root (level <= a) is climbed through multifusion parents of level <= a
-  // (the contract serializer's assignment, reference/morsehgp3d_oracle/serialization.py:1040-1099).
-  // They run in the same pool as soon as orders k and k - 1 are complete: chunks of source
-  // nodes gather their targets in parallel, then one offline sweep per order climbs them
-  // (node ids grow with level in both forests, so the target forest's parent links are
-  // united in id order as the source levels rise; the image is one find with path compression).
-  constexpr uint32_t kVChunk = 1u << 15;
-  if (h.vert.size() < keff + 1) h.vert.resize(keff + 1);
-  auto vcls = [](const HierOrderOut& o, uint32_t node) -> int64_t {
-    const uint32_t c = o.node_cls[node];
-    return c == kInvalid32 ? -1 : (int64_t)c;
-  };
-  auto complete = [&](uint32_t k) {
-    Progress& pg = prog[k];
-    return pg.done.load(std::memory_order_acquire) &&
-           pg.replayed.load(std::memory_order_acquire) == pg.published.load(std::memory_order_acquire);
-  };
-  auto v_gather = [&](uint32_t k, uint32_t chunk) {
-    HierOrderOut& src = outs[k];
-    const HierOrderOut& tgt = outs[k - 1];
-    const uint64_t h_lo = n + (rb[k] - rb[2]);  // first birth handle of order k
-    const uint64_t i_hi = std::min<uint64_t>(src.nodes.size(), (uint64_t)(chunk + 1) * kVChunk);
-    for (uint64_t i = (uint64_t)chunk * kVChunk; i < i_hi; ++i) {
-      const ehgp_forest_node& nd = src.nodes[i];
-      const ehgp_forest_group& g = src.groups[nd.atomic_group];
-      const uint64_t carrier = src.bindings[src.saddles[g.saddle_offset].arm_offset].carrier;
-      // the carrier's birth (rank k) and its saddle family of order k - 1 share the rank
-      // segment position, so the family's local index is carrier - h_lo
-      const uint64_t f = carrier - h_lo;
-      if (carrier < h_lo || f >= tgt.fam.size()) {
-        prog[k].vstat.store(EHGP_ERR_DEGENERATE);
-        src.v_res[i] = kInvalid32;
-        continue;
-      }
-      src.v_res[i] = tgt.fam_res[f];
-      src.v_cls[i] = src.node_cls[i];
-    }
-  };
-  auto v_sweep = [&](uint32_t k) {
-    const HierOrderOut& src = outs[k];
-    const HierOrderOut& tgt = outs[k - 1];
-    std::vector<ehgp_vertical_assignment>& vo = h.vert[k];
-    vo.clear();
-    if (prog[k].vstat.load() != EHGP_OK) return;
-    const uint32_t t_n = (uint32_t)tgt.nodes.size();
-    std::vector<uint32_t> up(t_n);
-    std::iota(up.begin(), up.end(), 0u);
-    auto find_up = [&](uint32_t x) {
-      while (up[x] != x) {
-        up[x] = up[up[x]];
-        x = up[x];
-      }
-      return x;
-    };
-    uint32_t sweep = 0;  // next target node whose child links are not yet united
-    for (uint64_t i = 0; i < src.nodes.size(); ++i) {
-      const uint32_t R = src.v_res[i];
-      const int64_t lev = vcls(src, (uint32_t)i);
-      if (R >= t_n || vcls(tgt, R) > lev) {
-        prog[k].vstat.store(EHGP_ERR_DEGENERATE);
-        return;
-      }
-      while (sweep < t_n && vcls(tgt, sweep) <= lev) {
-        const ehgp_forest_node& p = tgt.nodes[sweep];
-        if (p.kind == 2)
-          for (uint32_t c = 0; c < p.child_count; ++c) up[find_up(tgt.children[p.child_offset + c])] = sweep;
-        ++sweep;
-      }
-      vo.push_back({(uint32_t)i, find_up(R), k, src.nodes[i].level_event});  // local ids; offsets at copy-out
-    }
-  };
-  // One step of vertical work (a gather chunk or a sweep) if one is ready; `pending` is
-  // cleared while some vertical map is unfinished.
-  auto vertical_step = [&](bool& pending) {
-    for (uint32_t k = keff; k >= 2; --k) {
-      Progress& pg = prog[k];
-      if (pg.vb_done.load(std::memory_order_acquire)) continue;
-      pending = false;
-      if (!complete(k) || !complete(k - 1)) continue;
-      if (outs[k].status != EHGP_OK || outs[k - 1].status != EHGP_OK || prog[k].bad.load() || prog[k - 1].bad.load()) {
-        int z = 0;
-        if (pg.vb_claimed.compare_exchange_strong(z, 1)) pg.vb_done.store(1, std::memory_order_release);
-        continue;
-      }
-      const uint32_t na = (uint32_t)((outs[k].nodes.size() + kVChunk - 1) / kVChunk);
-      uint32_t c = pg.va_claimed.load(std::memory_order_relaxed);
-      while (c < na) {
-        if (pg.va_claimed.compare_exchange_weak(c, c + 1)) {
-          v_gather(k, c);
-          pg.va_done.fetch_add(1, std::memory_order_acq_rel);
-          return true;
-        }
-      }
-      if (pg.va_done.load(std::memory_order_acquire) == na) {
-        int z = 0;
-        if (pg.vb_claimed.compare_exchange_strong(z, 1)) {
-          v_sweep(k);
-          pg.vb_done.store(1, std::memory_order_release);
-          return true;
-        }
-      }
-    }
-    return false;
-  };
-  // claims and replays published chunks, highest order first, then the vertical maps, until
-  // every core is done and every chunk and map is finished
-  auto work = [&] {
-    uint32_t idle = 0;  // idle rounds: a short spin, then 50 us sleeps (the cores need the CPUs)
-    for (;;) {
-      bool did = false, all = true;
-      for (uint32_t k = keff; k >= 1; --k) {
-        Progress& pg = prog[k];
-        const int done = pg.done.load(std::memory_order_acquire);
-        const uint32_t pub = pg.published.load(std::memory_order_acquire);
-        uint32_t cl = pg.claimed.load(std::memory_order_relaxed);
-        while (cl < pub) {
-          if (pg.claimed.compare_exchange_weak(cl, cl + 1)) {
-            replay(k, cl);  // published chunks are complete even when the core stops later
-            stream_fence();
-            pg.replayed.fetch_add(1, std::memory_order_acq_rel);
-            did = true;
-            break;
-          }
-        }
-        if (!done || pg.claimed.load(std::memory_order_relaxed) < pg.published.load(std::memory_order_acquire))
-          all = false;
-        if (did) break;
-      }
-      if (!did && vertical_step(all)) did = true;
-      if (did) {
-        idle = 0;
-        continue;
-      }
-      if (all) return;
-      if (++idle < 64) std::this_thread::yield();
-      else std::this_thread::sleep_for(std::chrono::microseconds(50));
-    }
-  };
-  // The strict-arm descent runs order by order, highest first, on this thread; an order's
-  // union-find core starts as soon as its terminal handles are on the host, while the
-  // device descends the lower orders.  ready[k]: 0 waiting, 1 go, 2 stopped.
-  std::unique_ptr<std::atomic<int>[]> ready(new std::atomic<int>[keff + 1]);
-  for (uint32_t k = 0; k <= keff; ++k) ready[k].store(0);
-  int dstatus = EHGP_OK;
-  const char* dmsg = "";
-  cudaError_t dcuda = cudaSuccess;
-  {
-    const uint32_t hw = h.pool_threads ? h.pool_threads : std::max(1u, std::thread::hardware_concurrency());
-    const uint32_t extra = hw > keff + 1 ? std::min(hw - keff - 1, 32u) : 0u;  // one CPU for this thread
-    std::vector<std::thread> pool;
-    for (uint32_t k = 1; k <= keff; ++k)
-      pool.emplace_back([&, k] {
-        init_dsu(k);
-        int r;
-        while ((r = ready[k].load(std::memory_order_acquire)) == 0) std::this_thread::sleep_for(std::chrono::microseconds(20));
-        if (r == 1) {
-          run_core(k, outs[k]);
-        } else {
-          outs[k].status = EHGP_ERR_DEGENERATE;
-          outs[k].msg = "the strict-arm descent stopped";
-          prog[k].done.store(1, std::memory_order_release);
-        }
-        work();
-      });
-    for (uint32_t i = 0; i < extra; ++i) pool.emplace_back(work);
-    // descent, order by order; the host thread sleeps in its waits (the cores need the CPUs)
-    if (!h.ev_block && cudaEventCreateWithFlags(&h.ev_block, cudaEventBlockingSync | cudaEventDisableTiming) != cudaSuccess)
-      h.ev_block = nullptr;
-    auto wait_stream = [&]() -> cudaError_t {
-      if (!h.ev_block) return cudaStreamSynchronize(st);
-      cudaError_t r = cudaEventRecord(h.ev_block, st);
-      return r == cudaSuccess ? cudaEventSynchronize(h.ev_block) : r;
-    };
-    const DescentParams dp{n, 2 * n - 2, g.tnodes, b.px, b.py, b.pz, h.S, h.slots, (uint32_t)(h.cap_slots - 1), h.bfac,
-                           (uint32_t)nb_higher};
-    uint32_t misses = 0, max_rounds = 0;
-    unsigned long long failed_before = 0;
-    h.descent_steps = 0;
-    h.ms_steps = 0;
-    h.step_launches = 0;
-    for (cudaEvent_t& ev : h.ev_step)
-      if (!ev && cudaEventCreate(&ev) != cudaSuccess) ev = nullptr;
-    cudaEventRecord(ctx.evk0, st);
-    uint32_t k = keff;
-    auto stop = [&](int status, const char* msg) {
-      dstatus = status;
-      dmsg = msg;
-    };
-    const uint32_t kPartArms = h.part_arms;  // arms per part of an order's descent (about)
-    std::vector<uint64_t> plo(keff + 1);
-    for (uint32_t j = 1; j <= keff; ++j) plo[j] = rb[j + 1];
-    // Descends the next part of order k (cut at a batch boundary after about kPartArms arms)
-    // and publishes it to the order's core; false on a failure.
-    auto part = [&](uint32_t k) -> bool {
-      const uint64_t s_hi = rb[k + 2 > 16 ? 16 : k + 2];
-      uint64_t& p_lo = plo[k];
-      // the part ends at a batch boundary after about kPartArms arms
-      uint64_t p_hi = p_lo;
-      {
-        uint64_t lo = p_lo, hi = s_hi;  // first position whose arms reach the budget
-        const uint64_t goal = (uint64_t)arm_off[p_lo - fam_lo] + kPartArms;
-        while (lo < hi) {
-          const uint64_t mid = (lo + hi) / 2;
-          if ((uint64_t)arm_off[mid + 1 - fam_lo] >= goal) hi = mid; else lo = mid + 1;
-        }
-        p_hi = std::min<uint64_t>(lo + 1, s_hi);
-        while (p_hi < s_hi && cls_rp[p_hi] == cls_rp[p_hi - 1]) ++p_hi;
-      }
-      const uint32_t a_lo = arm_off[p_lo - fam_lo], a_hi = arm_off[p_hi - fam_lo];
-      if (a_hi > a_lo) {
-        const uint32_t na = a_hi - a_lo;
-        cudaMemsetAsync(h.qcount, 0, 4 * sizeof(uint32_t), st);
-        k_arm_probe<<<nblk(na, kT), kT, 0, st>>>(dp, a_lo, na, h.rank_order + fam_lo, h.arm_family, h.arm_local,
-                                                 h.ev, h.term, h.arm_status, h.q_arm[0], h.q_fac[0], h.qcount);
+      uint32_t* oc = h.qcount + 1 + (1 - cur);
+      cudaMemsetAsync(oc, 0, sizeof(uint32_t), st);
+      if (h.ev_step[0]) cudaEventRecord(h.ev_step[0], st);
+      int spasses = -1;  // large queues run in Morton order of their facets
+      if (pending >= kSortQueueMin && pending <= h.cap_events) {
+        k_queue_keys<<<nblk(pending, kT), kT, 0, st>>>(pending, q_fac[cur], b.code, h.key, h.order0);
         ++launches;
-        uint32_t pending = 0;
-        cudaMemcpyAsync(&pending, h.qcount, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-        if ((dcuda = wait_stream()) != cudaSuccess) return false;
-        misses += pending;
-        int cur = 0;
-        uint32_t rounds = 0;
-        while (pending) {
-          if (++rounds > (uint32_t)kDescentSteps) {
-            stop(EHGP_ERR_DEGENERATE, "a strict arm descent exceeded its step budget");
-            break;
-          }
-          uint32_t* oc = h.qcount + 1 + (1 - cur);
-          cudaMemsetAsync(oc, 0, sizeof(uint32_t), st);
-          if (h.ev_step[0]) cudaEventRecord(h.ev_step[0], st);
-          int spasses = -1;  // large queues run in Morton order of their facets
-          if (pending >= kSortQueueMin && pending <= h.cap_events) {
-            k_queue_keys<<<nblk(pending, kT), kT, 0, st>>>(pending, h.q_fac[cur], b.code, h.key, h.order0);
-            ++launches;
-            spasses = radix_sort_kv(st, pending, h.order0, h.order1, h.key, h.key2, 24, rs, &launches);
-          }
-          k_arm_step<<<nblk(pending, 128), 128, 0, st>>>(dp, pending, h.q_arm[cur], h.q_fac[cur], ctx.radix.state,
-                                                         spasses, h.order0, h.order1, h.q_arm[1 - cur],
-                                                         h.q_fac[1 - cur], oc, h.term, h.arm_status, h.dstats);
-          if (h.ev_step[1]) cudaEventRecord(h.ev_step[1], st);
-          ++launches;
-          ++h.step_launches;
-          cudaMemcpyAsync(&pending, oc, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-          if ((dcuda = wait_stream()) != cudaSuccess) break;
-          if (h.ev_step[0] && h.ev_step[1]) {
-            float sm = 0.f;
-            if (cudaEventElapsedTime(&sm, h.ev_step[0], h.ev_step[1]) == cudaSuccess) h.ms_steps += sm;
-          }
-          cur = 1 - cur;
-        }
-        if (dcuda != cudaSuccess || dstatus != EHGP_OK) return false;
-        max_rounds = std::max(max_rounds, rounds);
-        unsigned long long dst[4] = {0, 0, 0, 0};
-        cudaMemcpyAsync(h.p_term + a_lo, h.term + a_lo, (uint64_t)na * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(dst, h.dstats, sizeof(dst), cudaMemcpyDeviceToHost, st);
-        if ((dcuda = wait_stream()) != cudaSuccess) return false;
-        h.descent_steps = dst[0];
-        if (dst[3] > failed_before) {  // an arm of this part failed: report the first one
-          failed_before = dst[3];
-          if ((dcuda = cudaMemcpy(h.p_stat + a_lo, h.arm_status + a_lo, na, cudaMemcpyDeviceToHost)) != cudaSuccess)
-            return false;
-          static const char* msg[] = {"", "a strict arm descent is unresolved", "a strict arm descent met a plateau",
-                                      "a strict arm descent exceeded its ball-query capacity",
-                                      "a strict arm descent exceeded its step budget",
-                                      "a strict arm descent found no consistent exact miniball or top-k"};
-          for (uint32_t a = a_lo; a < a_hi; ++a)
-            if (astat[a] != kArmOk) {
-              stop(astat[a] == kArmCapacity ? EHGP_ERR_CAPACITY : EHGP_ERR_DEGENERATE,
-                   msg[astat[a] < 6 ? astat[a] : 5]);
-              break;
-            }
-          if (dstatus != EHGP_OK) return false;
-        }
+        spasses = radix_sort_kv(st, pending, h.order0, h.order1, h.key, h.key2, 24, rs, &launches);
       }
-      fam_lim[k].store(p_hi, std::memory_order_release);
-      ready[k].store(1, std::memory_order_release);
-      p_lo = p_hi;
-      return true;
-    };
-    // The first parts of the four largest orders first, so that their cores start early; then
-    // each order's remaining parts, highest order first.
-    bool dok = true;
-    for (k = keff; dok && k >= 1 && k + 4 > keff; --k)
-      if (plo[k] < rb[k + 2 > 16 ? 16 : k + 2]) dok = part(k);
-    for (k = keff; dok && k >= 1; --k) {
-      const uint64_t s_hi = rb[k + 2 > 16 ? 16 : k + 2];
-      while (dok && plo[k] < s_hi) dok = part(k);
-      if (!dok) break;
-      fam_lim[k].store(s_hi, std::memory_order_release);
-      ready[k].store(1, std::memory_order_release);
-    }
-    if (dcuda != cudaSuccess || dstatus != EHGP_OK) stop_all.store(1, std::memory_order_release);
-    // orders left waiting after a failure stop without running
-    for (uint32_t j = 1; j <= keff; ++j) {
-      int expect = 0;
-      ready[j].compare_exchange_strong(expect, 2);
-    }
-    cudaEventRecord(ctx.evk1, st);
-    cudaMemcpyFromSymbolAsync(h.slow, g_descent_slow, sizeof(h.slow), 0, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyFromSymbolAsync(h.visits, g_descent_visits, sizeof(h.visits), 0, cudaMemcpyDeviceToHost, st);
-    cudaEventRecord(ctx.ev1, st);
-    if (dcuda == cudaSuccess) dcuda = cudaStreamSynchronize(st);
-    h.first_misses = misses;
-    h.descent_rounds = max_rounds;
-    for (auto& t : pool) t.join();
-    for (uint32_t j = 1; j <= keff; ++j)
-      if (outs[j].status == EHGP_OK && prog[j].bad.load()) {
-        outs[j].status = EHGP_ERR_DEGENERATE;
-        outs[j].msg = "internal: a forest chunk replay disagrees with its core";
+      k_arm_step<<<nblk(pending, 128), 128, 0, st>>>(dp, pending, q_arm[cur], q_fac[cur], ctx.radix.state, spasses,
+                                                     h.order0, h.order1, q_arm[1 - cur], q_fac[1 - cur], oc, h.term,
+                                                     h.dstats);
+      if (h.ev_step[1]) cudaEventRecord(h.ev_step[1], st);
+      ++launches;
+      ++h.step_launches;
+      cudaMemcpyAsync(&pending, oc, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+      if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "strict-arm descent");
+      if (h.ev_step[0] && h.ev_step[1]) {
+        float sm = 0.f;
+        if (cudaEventElapsedTime(&sm, h.ev_step[0], h.ev_step[1]) == cudaSuccess) h.ms_steps += sm;
       }
+      cur = 1 - cur;
+    }
+    max_rounds = std::max(max_rounds, rounds);
   }
-  if (dcuda != cudaSuccess) return abi_cuda_fail(&ctx, dcuda, "strict-arm descent");
+  cudaEventRecord(ctx.evk1, st);
+  unsigned long long dst[4] = {0, 0, 0, 0};
+  cudaMemcpyAsync(dst, h.dstats, sizeof(dst), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyFromSymbolAsync(h.slow, g_descent_slow, sizeof(h.slow), 0, cudaMemcpyDeviceToHost, st);
+  cudaMemcpyFromSymbolAsync(h.visits, g_descent_visits, sizeof(h.visits), 0, cudaMemcpyDeviceToHost, st);
+  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "strict-arm descent");
+  h.first_misses = misses;
+  h.descent_rounds = max_rounds;
+  h.descent_steps = dst[0];
+  if (dst[2]) {  // report the first failed arm
+    static const char* msg[] = {"", "a strict arm descent is unresolved", "a strict arm descent met a plateau",
+                                "a strict arm descent exceeded its ball-query capacity",
+                                "a strict arm descent exceeded its step budget",
+                                "a strict arm descent found no consistent exact miniball or top-k"};
+    const uint32_t why = (uint32_t)(dst[3] & 0xff);
+    const int status = why == kArmCapacity ? EHGP_ERR_CAPACITY : EHGP_ERR_DEGENERATE;
+    h.decision = (uint32_t)status;
+    return abi_fail(&ctx, status, msg[why < 6 ? why : 5]);
+  }
+  // ---- forest journal, in the queues' memory ----
+  if ((e = h.mem.reset(journal)) != cudaSuccess) return no_queue();
+  const int js = journal_run(ctx, in, h.mem, h.journal, &launches);
+  if (js != EHGP_OK) return js;
+  cudaEventRecord(ctx.ev1, st);
+  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "forest journal");
   {
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx.ev0, ctx.ev1);
     h.ms_device = ms;
+    cudaEventElapsedTime(&ms, ctx.evk1, ctx.ev1);
+    h.ms_forest = ms;
     if (narms) {
       cudaEventElapsedTime(&ms, ctx.evk0, ctx.evk1);
       ctx.kernel_ms = ms;
       h.ms_descent = ms;
     }
   }
-  if (dstatus != EHGP_OK) {
-    h.decision = (uint32_t)dstatus;
-    return abi_fail(&ctx, dstatus, dmsg);
-  }
-  const auto t_orders = std::chrono::steady_clock::now();
-  for (uint32_t k = 1; k <= keff; ++k)
-    if (outs[k].status != EHGP_OK) return abi_fail(&ctx, outs[k].status, outs[k].msg);
-  h.ms_orders = 0;
-  for (uint32_t k = 1; k <= keff; ++k) h.ms_orders = std::max(h.ms_orders, outs[k].ms);
-  // global offsets of each order's records (the reference's single pass emits orders in turn)
-  std::vector<HierOff> off(keff + 2);
-  off[1] = HierOff{0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (uint32_t k = 1; k <= keff; ++k) {
-    const HierOrderOut& o = outs[k];
-    const HierOff& a = off[k];
-    off[k + 1] = {a.jb + (uint32_t)o.jb.size(),         a.role + (uint32_t)o.roles.size(),
-                  a.fam + (uint32_t)o.fam.size(),       a.node + (uint32_t)o.nodes.size(),
-                  a.child + (uint32_t)o.children.size(), a.birth + (uint32_t)o.births.size(),
-                  a.bind + (uint32_t)o.bindings.size(), a.sad + (uint32_t)o.saddles.size(),
-                  a.grp + (uint32_t)o.groups.size(),    a.root + (uint32_t)o.roots.size(), 0u};
-  }
-  const auto t_merge = std::chrono::steady_clock::now();
-  {
-    uint32_t vtot = 0;
-    for (uint32_t k = 1; k <= keff; ++k) {
-      if (k >= 2 && prog[k].vstat.load() != EHGP_OK)
-        return abi_fail(&ctx, prog[k].vstat.load(), "a reduced node has no lower-order image through its carrier saddle");
-      off[k].vert = vtot;
-      if (k >= 2) vtot += (uint32_t)h.vert[k].size();
-    }
-    off[keff + 1].vert = vtot;
-  }
-  const auto t2 = std::chrono::steady_clock::now();
-  h.ms_forest = std::chrono::duration<double, std::milli>(t2 - t1).count();
-  {
-    using msd = std::chrono::duration<double, std::milli>;
-    h.ms_host[0] = ms_ties;
-    h.ms_host[1] = msd(t_orders - t_init).count();
-    h.ms_host[2] = msd(t_merge - t_orders).count();
-    h.ms_host[3] = msd(t2 - t_merge).count();
-  }
-  (void)t0;
+  h.ms_ties = ms_ties;
   ctx.last_launches = launches;
-  ctx.last_ms = h.ms_device + h.ms_forest;
-  h.off = std::move(off);
+  ctx.last_ms = h.ms_device;
   h.arm_seeds = narms;
+  h.families = nfam;
+  h.births = in.handles;
+  h.complete = true;
   h.decision = EHGP_OK;
   return EHGP_OK;
+}
+
+// One device range and the host memory it goes to.
+struct CopyOut {
+  char* dst;
+  const char* src;
+  uint64_t bytes;
+};
+
+namespace {
+
+// Streaming copy into memory that is not read back here (the caches keep the staging ring).
+void stream_copy(char* dst, const char* src, uint64_t bytes) {
+#if defined(__x86_64__)
+  const uint64_t lead = std::min<uint64_t>(bytes, (16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15);
+  std::memcpy(dst, src, lead);
+  dst += lead;
+  src += lead;
+  bytes -= lead;
+  uint64_t i = 0;
+  for (; i + 64 <= bytes; i += 64)
+    for (int q = 0; q < 4; ++q)
+      _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i) + q, _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i) + q));
+  std::memcpy(dst + i, src + i, bytes - i);
+  _mm_sfence();
+#else
+  std::memcpy(dst, src, bytes);
+#endif
+}
+
+}  // namespace
+
+// Copies device ranges to host memory.  Pinned destinations and small ranges go straight there;
+// large pageable ones go through a ring of pinned slots that host threads empty while the next
+// chunks cross the bus (a pageable cudaMemcpy stages through one thread instead).
+cudaError_t copy_out(Ctx& ctx, HierState& h, const std::vector<CopyOut>& list) {
+  cudaStream_t st = ctx.stream;
+  cudaError_t e = cudaSuccess;
+  std::vector<CopyOut> chunks;
+  uint64_t all = 0;
+  for (const CopyOut& c : list) all += c.bytes;
+  for (const CopyOut& c : list) {
+    cudaPointerAttributes at{};
+    const bool pinned = cudaPointerGetAttributes(&at, c.dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    if (pinned || c.bytes <= kStageBytes || all < kStageFrom) {
+      if ((e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+      continue;
+    }
+    for (uint64_t o = 0; o < c.bytes; o += kStageBytes)
+      chunks.push_back({c.dst + o, c.src + o, std::min(kStageBytes, c.bytes - o)});
+  }
+  if (chunks.empty()) return cudaStreamSynchronize(st);
+  if (!h.stage) {
+    if ((e = cudaMallocHost(reinterpret_cast<void**>(&h.stage), kStageSlots * kStageBytes)) != cudaSuccess) {
+      h.stage = nullptr;
+      return e;
+    }
+    for (cudaEvent_t& ev : h.stage_ev)
+      if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
+  }
+  const size_t total = chunks.size();
+  std::atomic<size_t> issued{0}, next{0};
+  std::atomic<int> failed{0};
+  std::vector<std::atomic<uint8_t>> done(total);
+  for (auto& d : done) d.store(0, std::memory_order_relaxed);
+  auto drain = [&] {
+    for (size_t t; (t = next.fetch_add(1)) < total;) {
+      while (issued.load(std::memory_order_acquire) <= t && !failed.load(std::memory_order_acquire)) std::this_thread::yield();
+      if (failed.load(std::memory_order_acquire)) return;
+      const int slot = (int)(t % kStageSlots);
+      if (cudaEventSynchronize(h.stage_ev[slot]) != cudaSuccess) {
+        failed.store(1, std::memory_order_release);
+        return;
+      }
+      stream_copy(chunks[t].dst, h.stage + slot * kStageBytes, chunks[t].bytes);
+      done[t].store(1, std::memory_order_release);
+    }
+  };
+  const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
+  const size_t workers = std::min<size_t>({total, (size_t)8, (size_t)(hw - 1)});
+  std::vector<std::thread> pool;
+  try {
+    for (size_t i = 0; i < workers; ++i) pool.emplace_back([&] {
+      cudaSetDevice(ctx.device);
+      drain();
+    });
+  } catch (...) {  // no more threads: the ones that started do the work
+  }
+  if (pool.empty()) {
+    for (const CopyOut& c : chunks)
+      if ((e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+    return cudaStreamSynchronize(st);
+  }
+  for (size_t t = 0; t < total && !failed.load(std::memory_order_acquire); ++t) {
+    if (t >= (size_t)kStageSlots)
+      while (!done[t - kStageSlots].load(std::memory_order_acquire) && !failed.load(std::memory_order_acquire))
+        std::this_thread::yield();
+    const int slot = (int)(t % kStageSlots);
+    e = cudaMemcpyAsync(h.stage + slot * kStageBytes, chunks[t].src, chunks[t].bytes, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaEventRecord(h.stage_ev[slot], st);
+    if (e != cudaSuccess) {
+      failed.store(1, std::memory_order_release);
+      break;
+    }
+    issued.store(t + 1, std::memory_order_release);
+  }
+  for (auto& th : pool) th.join();
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return e;
+  return es != cudaSuccess ? es : failed.load() ? cudaErrorUnknown : cudaSuccess;
 }
 
 }  // namespace ehgp
@@ -2648,20 +1782,20 @@ int ehgp_hierarchy(ehgp_ctx* ctx, uint32_t K, ehgp_hier_counts* counts) {
       const ehgp::HierState& h = *ctx->hier;
       counts->events = h.events;
       counts->diagnostics = h.diagnostics;
-      if (!h.off.empty()) {
-        const ehgp::HierOff& t = h.off.back();
-        counts->journal_batches = t.jb;
-        counts->role_records = t.role;
-        counts->families = t.fam;
+      if (h.complete) {
+        const ehgp::JournalOut& j = h.journal;
+        counts->journal_batches = j.n_batches;
+        counts->role_records = j.n_roles;
+        counts->families = h.families;
         counts->arm_seeds = h.arm_seeds;
-        counts->birth_records = t.birth;
-        counts->nodes = t.node;
-        counts->children = t.child;
-        counts->arm_bindings = t.bind;
-        counts->saddle_records = t.sad;
-        counts->atomic_groups = t.grp;
-        counts->final_roots = t.root;
-        counts->vertical_assignments = t.vert;
+        counts->birth_records = h.births;
+        counts->nodes = j.n_nodes;
+        counts->children = j.n_children;
+        counts->arm_bindings = h.arm_seeds;
+        counts->saddle_records = h.families;
+        counts->atomic_groups = j.n_groups;
+        counts->final_roots = j.roots.size();
+        counts->vertical_assignments = j.n_vert;
       }
       counts->k_eff = h.keff;
     }
@@ -2674,10 +1808,9 @@ int ehgp_hier_schedule(ehgp_ctx* ctx, uint32_t chunk_batches, uint32_t part_arms
   if (!ctx) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   if (!ctx->hier) ctx->hier = new ehgp::HierState();
-  ehgp::HierState& h = *ctx->hier;
-  h.chunk_batches = chunk_batches ? chunk_batches : 1u << 14;
-  h.part_arms = part_arms ? part_arms : 1u << 22;
-  h.pool_threads = host_threads;
+  (void)chunk_batches;  // the forest journal runs on the device
+  (void)host_threads;
+  ctx->hier->part_arms = part_arms;
   return EHGP_OK;
 }
 
@@ -2685,123 +1818,30 @@ int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out) {
   if (!ctx || !out) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   if (!ctx->hier) return ehgp::abi_fail(ctx, EHGP_ERR_NOT_BUILT, "no hierarchy result is resident");
-  const ehgp::HierState& h = *ctx->hier;
-  if (out->events && h.events) {
-    const cudaError_t e = cudaMemcpy(out->events, h.ev, h.events * sizeof(ehgp::EvRec), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "facade copy");
-  }
-  if (h.off.empty()) return EHGP_OK;
-  if (out->arm_removed && h.arm_seeds) {
-    const cudaError_t e = cudaMemcpy(out->arm_removed, h.d_removed, h.arm_seeds * 4, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "arm seed copy");
-  }
-  // Each order's arenas go to their global offsets with local indices shifted, in chunks
-  // spread over the host cores.
-  using ehgp::HierOff;
-  const uint32_t keff = (uint32_t)h.off.size() - 2;
-  std::vector<std::function<void()>> tasks;
-  constexpr uint64_t kChunk = 1u << 18;
-  auto shift = [](uint32_t v, uint32_t d) { return v == ehgp::kInvalid32 ? v : v + d; };
-  auto add = [&](void* dst_base, uint64_t count, auto&& one) {
-    if (!dst_base) return;
-    for (uint64_t lo = 0; lo < count; lo += kChunk) {
-      const uint64_t hi = std::min(count, lo + kChunk);
-      tasks.emplace_back([=] {
-        for (uint64_t i = lo; i < hi; ++i) one(i);
-      });
-    }
+  ehgp::HierState& h = *ctx->hier;
+  const ehgp::JournalOut& j = h.journal;
+  std::vector<ehgp::CopyOut> list;
+  auto add = [&](void* dst, const void* src, uint64_t count, uint64_t size) {
+    if (dst && count) list.push_back({static_cast<char*>(dst), static_cast<const char*>(src), count * size});
   };
-  for (uint32_t k = 1; k <= keff; ++k) {
-    const ehgp::HierOrderOut& o = h.outs[k];
-    const HierOff f = h.off[k];
-    add(out->journal_batches, o.jb.size(), [&o, f, out](uint64_t i) {
-      ehgp_journal_batch x = o.jb[i];
-      x.role_offset += f.role;
-      ehgp::nt_store(out->journal_batches[f.jb + i], x);
-    });
-    add(out->batches, o.fb.size(), [&o, f, out](uint64_t i) {
-      ehgp_forest_batch y = o.fb[i];
-      y.birth_offset += f.birth;
-      y.saddle_offset += f.sad;
-      y.group_offset += f.grp;
-      ehgp::nt_store(out->batches[f.jb + i], y);
-    });
-    add(out->roles, o.roles.size(), [&o, f, out](uint64_t i) {
-      ehgp_role_record x = o.roles[i];
-      x.batch += f.jb;
-      ehgp::nt_store(out->roles[f.role + i], x);
-    });
-    add(out->families, o.fam.size(), [&o, f, out](uint64_t i) {
-      ehgp_family_record x = o.fam[i];
-      x.role_record += f.role;
-      x.batch += f.jb;
-      ehgp::nt_store(out->families[f.fam + i], x);
-    });
-    add(out->nodes, o.nodes.size(), [&o, f, out, shift](uint64_t i) {
-      ehgp_forest_node x = o.nodes[i];
-      x.child_offset += f.child;
-      x.atomic_group = shift(x.atomic_group, f.grp);
-      ehgp::nt_store(out->nodes[f.node + i], x);
-    });
-    add(out->children, o.children.size(), [&o, f, out](uint64_t i) { out->children[f.child + i] = o.children[i] + f.node; });
-    add(out->births, o.births.size(), [&o, f, out, shift](uint64_t i) {
-      ehgp_forest_birth x = o.births[i];
-      x.batch += f.jb;
-      x.order_one_node = shift(x.order_one_node, f.node);
-      ehgp::nt_store(out->births[f.birth + i], x);
-    });
-    add(out->bindings, o.bindings.size(), [&o, f, out, shift](uint64_t i) {
-      ehgp_forest_binding x = o.bindings[i];
-      x.family += f.fam;
-      x.prior_root = shift(x.prior_root, f.node);
-      ehgp::nt_store(out->bindings[f.bind + i], x);
-    });
-    add(out->saddles, o.saddles.size(), [&o, f, out](uint64_t i) {
-      ehgp_forest_saddle x = o.saddles[i];
-      x.family += f.fam;
-      x.batch += f.jb;
-      x.arm_offset += f.bind;
-      x.group += f.grp;
-      ehgp::nt_store(out->saddles[f.sad + i], x);
-    });
-    add(out->groups, o.groups.size(), [&o, f, out, shift](uint64_t i) {
-      ehgp_forest_group x = o.groups[i];
-      x.batch += f.jb;
-      x.saddle_offset += f.sad;
-      x.child_offset += f.child;
-      x.created_node = shift(x.created_node, f.node);
-      x.result_node = shift(x.result_node, f.node);
-      ehgp::nt_store(out->groups[f.grp + i], x);
-    });
-    add(out->roots, o.roots.size(), [&o, f, out](uint64_t i) {
-      ehgp_forest_root x = o.roots[i];
-      x.node += f.node;
-      ehgp::nt_store(out->roots[f.root + i], x);
-    });
-    if (k >= 2 && k < h.vert.size()) {
-      const std::vector<ehgp_vertical_assignment>& v = h.vert[k];
-      const uint32_t tnode = h.off[k - 1].node;
-      add(out->vertical, v.size(), [&v, f, tnode, out](uint64_t i) {
-        ehgp_vertical_assignment x = v[i];
-        x.source_node += f.node;
-        x.target_node += tnode;
-        ehgp::nt_store(out->vertical[f.vert + i], x);
-      });
-    }
+  add(out->events, h.ev, h.events, sizeof(ehgp::EvRec));
+  if (h.complete) {
+    add(out->journal_batches, j.jb, j.n_batches, sizeof *j.jb);
+    add(out->roles, j.roles, j.n_roles, sizeof *j.roles);
+    add(out->families, j.fam, h.families, sizeof *j.fam);
+    add(out->arm_removed, h.d_removed, h.arm_seeds, 4);
+    add(out->nodes, j.nodes, j.n_nodes, sizeof *j.nodes);
+    add(out->children, j.children, j.n_children, 4);
+    add(out->births, j.births, h.births, sizeof *j.births);
+    add(out->bindings, j.bindings, h.arm_seeds, sizeof *j.bindings);
+    add(out->saddles, j.saddles, h.families, sizeof *j.saddles);
+    add(out->groups, j.groups, j.n_groups, sizeof *j.groups);
+    add(out->batches, j.fb, j.n_batches, sizeof *j.fb);
+    add(out->vertical, j.vert, j.n_vert, sizeof *j.vert);
+    if (out->roots && !j.roots.empty()) std::memcpy(out->roots, j.roots.data(), j.roots.size() * sizeof j.roots[0]);
   }
-  if (!tasks.empty()) {
-    const uint32_t hw = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-    const uint32_t nt = (uint32_t)std::min<uint64_t>(hw, tasks.size());
-    std::atomic<uint64_t> next{0};
-    auto work = [&] {
-      for (uint64_t t; (t = next.fetch_add(1)) < tasks.size();) tasks[t]();
-      ehgp::stream_fence();  // the streaming stores are complete before the join
-    };
-    std::vector<std::thread> pool;
-    for (uint32_t i = 1; i < nt; ++i) pool.emplace_back(work);
-    work();
-    for (auto& t : pool) t.join();
-  }
+  const cudaError_t e = ehgp::copy_out(*ctx, h, list);
+  if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "hierarchy copy");
   return EHGP_OK;
 }
 
@@ -2812,9 +1852,8 @@ int ehgp_hier_stats(const ehgp_ctx* ctx, double* ms, uint64_t* stats) {
     ms[0] = h.ms_device;
     ms[1] = h.ms_descent;
     ms[2] = h.ms_forest;
-    ms[3] = h.ms_orders;
-    for (int i = 0; i < 4; ++i) ms[4 + i] = h.ms_host[i];
-    for (uint32_t k = 1; k <= 16; ++k) ms[7 + k] = k < h.outs.size() ? h.outs[k].ms : 0.0;
+    for (int i = 3; i < 25; ++i) ms[i] = 0.0;
+    ms[4] = h.ms_ties;
   }
   if (stats) {
     stats[0] = h.arms;

@@ -1,0 +1,73 @@
+// Forest journal of the direct Morse hierarchy on the device (ehgp_journal.cu): inputs, the
+// records it leaves in HBM, and the memory it works in.
+#pragma once
+
+#include "ehgp_internal.cuh"
+
+namespace ehgp {
+
+// Device memory handed out in order from one kept block; what does not fit goes to further
+// blocks, which the next reset folds into one of the total size.
+class DeviceArena {
+ public:
+  DeviceArena() = default;
+  DeviceArena(const DeviceArena&) = delete;
+  DeviceArena& operator=(const DeviceArena&) = delete;
+  ~DeviceArena() { release(); }
+  // Forgets every piece handed out; nothing on the device may still use them.
+  cudaError_t reset(uint64_t want);
+  cudaError_t take(void** p, uint64_t bytes);
+  template <class T>
+  cudaError_t take(T** p, uint64_t count) {
+    return take(reinterpret_cast<void**>(p), count * sizeof(T));
+  }
+  void release();
+  uint64_t bytes() const;
+
+ private:
+  struct Block {
+    char* p;
+    uint64_t size, used;
+  };
+  std::vector<Block> blocks_;
+};
+
+constexpr int kJournalOrders = 18;  // orders 1..10 and the ends of their ranges
+
+// The resolved arms of every order.  Families (saddles) and birth handles of orders >= 2 are
+// both numbered by rank-partition position: family f is the event at rb2 + f, and handle n + i
+// the event at rb2 + i, so family f of order k and handle n + f of order k + 1 are one event.
+struct JournalIn {
+  uint32_t n = 0, keff = 0;
+  uint32_t handles = 0, families = 0, arms = 0;
+  uint32_t fam0[kJournalOrders] = {};   // first family of order k (k = 1..keff + 1)
+  uint32_t han0[kJournalOrders] = {};   // first handle of order k
+  const uint32_t* ev = nullptr;         // [families] facade index (ascending within an order)
+  const uint32_t* cls = nullptr;        // [families] level class (ascending within an order)
+  const uint32_t* armoff = nullptr;     // [families + 1]
+  const uint32_t* term = nullptr;       // [arms] birth handle that ends the arm's descent
+};
+
+// Records in the reference's arena order with global indices (device pointers into the arena).
+struct JournalOut {
+  ehgp_journal_batch* jb = nullptr;
+  ehgp_role_record* roles = nullptr;
+  ehgp_family_record* fam = nullptr;
+  ehgp_forest_node* nodes = nullptr;
+  uint32_t* children = nullptr;
+  ehgp_forest_birth* births = nullptr;
+  ehgp_forest_binding* bindings = nullptr;
+  ehgp_forest_saddle* saddles = nullptr;
+  ehgp_forest_group* groups = nullptr;
+  ehgp_forest_batch* fb = nullptr;
+  ehgp_vertical_assignment* vert = nullptr;
+  std::vector<ehgp_forest_root> roots;  // on the host (one per surviving component)
+  uint64_t n_batches = 0, n_roles = 0, n_nodes = 0, n_children = 0, n_groups = 0, n_vert = 0;
+};
+
+// Device bytes the journal takes from its arena for these counts (nodes and children, which
+// it counts itself, not included).
+uint64_t journal_bytes(const JournalIn& in);
+int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out, uint64_t* launches);
+
+}  // namespace ehgp

@@ -206,7 +206,6 @@ int ehgp_server_create(int device, const ehgp_server_limits* limits, ehgp_server
   // before any measurement: about 120 KB per point covers the 50,653-point lattice's
   // supports and hierarchy with room
   s->bytes_per_point = 120.0 * 1024.0;
-  const uint32_t hw = std::max(1u, std::thread::hardware_concurrency());
   for (uint32_t w = 0; w < limits->workers; ++w) {
     ehgp_limits cl{limits->max_points, limits->hbm_fraction};
     Worker wk;
@@ -215,8 +214,6 @@ int ehgp_server_create(int device, const ehgp_server_limits* limits, ehgp_server
       for (auto& x : s->workers) ehgp_ctx_destroy(x.ctx);
       return st;
     }
-    // the host passes of the workers share the CPUs
-    ehgp_hier_schedule(wk.ctx, 0, 0, std::max(12u, hw / limits->workers));
     s->workers.push_back(std::move(wk));
   }
   for (uint32_t w = 0; w < limits->workers; ++w) s->workers[w].thread = std::thread(worker_loop, s.get(), w);

@@ -461,19 +461,16 @@ int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out);
 
 /* Schedule of later ehgp_hierarchy calls on ctx; results never depend on it.  No
  * counterpart in the reference, whose forest journal is one sequential pass
- * (src/cpu/hierarchy/direct_morse_forest_journal.cpp:1042-2150): single-role batches
- * per chunk that the host pool rebuilds in parallel (0: 16384), strict arms per part
- * of the descent that an order's union-find core consumes while the device descends
- * the next (0: 4,194,304), and host threads (0: every hardware thread). */
+ * (src/cpu/hierarchy/direct_morse_forest_journal.cpp:1042-2150): about how many strict
+ * arms a part of the descent takes (0: all in one part; smaller parts need less
+ * queue memory and more launches).  chunk_batches and host_threads scheduled a
+ * host forest pass; the journal is built on the device and they have no effect. */
 int ehgp_hier_schedule(ehgp_ctx* ctx, uint32_t chunk_batches, uint32_t part_arms, uint32_t host_threads);
 
-/* Timing of the last ehgp_hierarchy call: ms[0] device stages (CUDA events),
- * ms[1] the strict-arm descent kernels, ms[2] the host forest pass, ms[3] its
- * slowest order (orders run on parallel host threads), ms[4] the exact
- * ordering of the facade runs that FP64 level intervals leave open (on the device), ms[5..7] the host forest pass split
- * into the order passes, the record offsets and the vertical maps,
- * ms[8 + k - 1] the union-find core of order k (k <= 16,
- * zero above the last order);
+/* Timing of the last ehgp_hierarchy call: ms[0] the whole call on the device timeline (CUDA
+ * events), ms[1] the strict-arm descent, ms[2] the forest journal, ms[4] the exact
+ * ordering of the facade runs that FP64 level intervals leave open; ms[3] and ms[5..23]
+ * are zero (they held the host forest pass);
  * stats[0] strict arms, [1] descent steps, [2] facade boundaries settled
  * exactly (2304-bit level comparisons on the device), [3] facade events, [4] arms that are not themselves a
  * birth facet, [5] descent rounds (longest chain), [6..12] slow-path counts of
