@@ -174,7 +174,9 @@ struct GeomBuffers {
 
 // Buffers of the pair-support stage.
 struct PairBuffers {
-  uint32_t* W = nullptr;            // [n * 32] witness lists (32 nearest, FP64 order)
+  uint32_t* W = nullptr;            // [n * 64] witness lists (64 nearest, FP64 order)
+  void* tasks = nullptr;            // [2 * task_cap] walks handed over between rounds
+  uint32_t task_cap = 0;
   double* R2 = nullptr;             // [n] squared witness radius
   void* raw = nullptr;              // [capacity] 64-byte records, unordered
   void* sorted = nullptr;           // [capacity] records in (u, v) order

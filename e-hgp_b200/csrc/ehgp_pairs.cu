@@ -16,18 +16,23 @@
 //
 // B200 design (replacing the reference's CPU frontier of node pairs with BigInt
 // bounds, pair_support_stream.cpp:1518-2249):
-//  * every point u owns a witness list W_u = its 32 nearest other points
-//    (FP64 order); R_u^2 is the 32nd squared distance;
-//  * one thread per u, in Morton order, walks the LBVH over partners v that
-//    follow u in Morton order (each unordered pair is visited once);
+//  * every point u owns a witness list W_u = its 64 nearest other points
+//    (FP64 order); R_u^2 is the 64th squared distance;
+//  * one warp per u, in Morton order, walks the LBVH over partners v that
+//    follow u in Morton order (each unordered pair is visited once), 32 nodes a
+//    step, one per lane; a walk that grows long hands the rest of its stack to
+//    further warps (points at the rim of a cluster have walks hundreds of times
+//    the usual length);
 //  * a subtree B of partners is pruned when at least s_max - 1 witnesses w of
 //    u satisfy max_{v in B} (w - u).(w - v) < 0 with certainty (binary32
 //    bound with a conservative margin): every pair (u, v in B) then has more
 //    than s_max - 2 strict interior points;
-//  * a leaf pair whose sphere lies in the strict 32-NN ball of u or of v
+//  * a leaf pair whose sphere lies in the strict 64-NN ball of u or of v
 //    (|u - v| < R_u: every point of the closed diametral ball is within |u - v|
-//    of u) is classified from that witness list alone; any other leaf pair
-//    runs an exact closed-ball query over the LBVH with early rejection;
+//    of u) is classified from that witness list alone; any other leaf pair is
+//    dropped when enough witnesses of u or of v lie inside its sphere for
+//    certain, and else runs an exact closed-ball query over the LBVH with early
+//    rejection;
 //  * every side decision is FP64 with a rigorous error bound, then exact
 //    integers at the cloud scale inside the bound.
 #include "ehgp_internal.cuh"
@@ -39,7 +44,10 @@ namespace ehgp {
 namespace {
 
 constexpr int kThreads = 128;
-constexpr int kStack = 128;
+constexpr uint32_t kStack = 512; // warp traversal stack
+// While the stack holds more than this, one node is taken per step: depth first, a walk adds at
+// most the tree's depth (63 + log2 n + 1) to it.
+constexpr uint32_t kStackWide = kStack - 64 - 128;
 constexpr int kW = 64;           // witnesses per point (two per lane)
 constexpr int kMaxInterior = 9;  // s_max - 2 for K >= 10
 
@@ -78,56 +86,155 @@ __device__ __forceinline__ double box_ub(const TNode& t, double qx, double qy, d
   return (dx * dx + dy * dy + dz * dz) * (1.0 + 4.0 * kDistRelErr);
 }
 
-// ---- 32 nearest neighbours (FP64 order; witnesses, no exactness needed) --------
+__device__ __forceinline__ uint32_t lanemask_lt() {
+  uint32_t m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
+
+constexpr int kWarpsPerBlock = kThreads / 32;
+
+// ---- 64 nearest neighbours (FP64 order; witnesses, no exactness needed) --------
+// One warp per point.  The 64 nearest points so far are kept sorted across the warp (lane l holds
+// the l-th and the (32 + l)-th); candidates are collected 32 at a time and merged in.  The walk takes
+// 32 nodes of a shared stack per step, and is pruned from the start at the largest distance to
+// 64 points next to u in Morton order.
+// Bound: latency of the walk's dependent node loads.  A thread per point with its list in local
+// memory took 5.69 ms on 29,791 lattice points and 2.40 on 8,009 clustered ones; this 0.51 and 0.17.
+struct DistId {
+  double d;
+  uint32_t id;
+};
+__device__ __forceinline__ DistId shfl_xor(const DistId& x, int o) {
+  return DistId{__shfl_xor_sync(0xffffffffu, x.d, o), __shfl_xor_sync(0xffffffffu, x.id, o)};
+}
+__device__ __forceinline__ DistId lesser(const DistId& a, const DistId& b) { return b.d < a.d ? b : a; }
+__device__ __forceinline__ DistId greater_of(const DistId& a, const DistId& b) { return b.d < a.d ? a : b; }
+
+// Ascending order of a bitonic sequence (one element per lane).
+__device__ __forceinline__ DistId bitonic_merge(DistId x, uint32_t lane) {
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    const DistId o = shfl_xor(x, j);
+    const bool take = ((lane & j) == 0) ? o.d < x.d : x.d < o.d;
+    if (take) x = o;
+  }
+  return x;
+}
+__device__ __forceinline__ DistId bitonic_sort(DistId x, uint32_t lane) {
+#pragma unroll
+  for (uint32_t k = 2; k <= 32; k <<= 1)
+#pragma unroll
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      const DistId o = shfl_xor(x, j);
+      const bool up = ((lane & j) == 0) == ((lane & k) == 0 || k == 32);
+      if (up ? o.d < x.d : x.d < o.d) x = o;
+    }
+  return x;
+}
+
+struct KnnShared {
+  uint32_t stack[kStack];
+  double cd[64];
+  uint32_t cid[64];
+};
+
 __global__ void __launch_bounds__(kThreads)
 k_witness_knn(uint32_t n, uint32_t kw, uint32_t root, const TNode* __restrict__ tn,
               const uint32_t* __restrict__ leaf_pid, const double* __restrict__ px, const double* __restrict__ py,
               const double* __restrict__ pz, uint32_t* __restrict__ W, double* __restrict__ R2,
               uint32_t* __restrict__ err) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t p = leaf_pid[i];
+  __shared__ KnnShared shared[kWarpsPerBlock];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint32_t pos = blockIdx.x * kWarpsPerBlock + warp;
+  if (pos >= n) return;
+  KnnShared& sh = shared[warp];
+  const uint32_t p = leaf_pid[pos];
   const double qx = px[p], qy = py[p], qz = pz[p];
-  double cd[kW];
-  uint32_t cid[kW];
-  int cnt = 0;
-  uint32_t stack[kStack];
-  int top = 0;
-  stack[top++] = root;
+  if (n - 1 <= (uint32_t)kW) {  // every other point is a witness (kw = n - 1)
+    for (uint32_t j = lane; j < (uint32_t)kW; j += 32)
+      W[(uint64_t)p * kW + j] = j < n - 1 ? leaf_pid[j < pos ? j : j + 1] : kInvalid32;
+    if (lane == 0) R2[p] = INFINITY;
+    return;
+  }
+  double seed = 0.0;  // at least 64 points lie within it
+  const uint32_t w0 = min(pos > 32u ? pos - 32u : 0u, n - 65u);
+  for (uint32_t j = lane; j <= 64; j += 32) {
+    const uint32_t q = leaf_pid[w0 + j];
+    seed = fmax(seed, d2fp(qx, qy, qz, px[q], py[q], pz[q]));
+  }
+  for (int o = 16; o > 0; o >>= 1) seed = fmax(seed, __shfl_xor_sync(0xffffffffu, seed, o));
+  DistId lo{INFINITY, kInvalid32}, hi{INFINITY, kInvalid32};
+  double thr = seed;
+  uint32_t top = 1, cnt = 0;
+  if (lane == 0) sh.stack[0] = root;
+  __syncwarp();
+  auto merge = [&](uint32_t m) {  // the first m <= 32 collected candidates
+    DistId x{INFINITY, kInvalid32};
+    if (lane < m) x = DistId{sh.cd[lane], sh.cid[lane]};
+    x = bitonic_sort(x, lane);
+    x = shfl_xor(x, 31);                            // descending
+    hi = bitonic_merge(lesser(hi, x), lane);        // the 32 least of the upper half and the new ones
+    const DistId r = shfl_xor(hi, 31);
+    const DistId l2 = lesser(lo, r);
+    hi = bitonic_merge(greater_of(lo, r), lane);
+    lo = bitonic_merge(l2, lane);
+    thr = fmin(seed, __shfl_sync(0xffffffffu, hi.d, 31));
+  };
   while (top > 0) {
-    const uint32_t node = stack[--top];
-    const TNode t = load_node(tn, node);
-    const double thr = (cnt >= (int)kw) ? cd[kw - 1] : INFINITY;
-    if (t.left == kInvalid32) {
-      const uint32_t q = t.right;
-      if (q == p) continue;
-      const double d = d2fp(qx, qy, qz, px[q], py[q], pz[q]);
-      if (d >= thr) continue;
-      int j = (cnt < (int)kw) ? cnt++ : (int)kw - 1;
-      while (j > 0 && cd[j - 1] > d) {
-        cd[j] = cd[j - 1];
-        cid[j] = cid[j - 1];
-        --j;
+    const uint32_t batch = top > kStackWide ? 1u : min(top, 32u);
+    uint32_t node = kInvalid32;
+    if (lane < batch) node = sh.stack[top - 1 - lane];
+    __syncwarp();
+    top -= batch;
+    bool take = false, expand = false;
+    double d = 0.0;
+    TNode t;
+    if (node != kInvalid32) {
+      t = load_node(tn, node);
+      if (t.left == kInvalid32) {
+        if (t.right != p) {
+          d = d2fp(qx, qy, qz, px[t.right], py[t.right], pz[t.right]);
+          take = d <= thr;
+        }
+      } else {
+        expand = box_lb(t, qx, qy, qz) <= thr;
       }
-      cd[j] = d;
-      cid[j] = q;
-      continue;
     }
-    if (box_lb(t, qx, qy, qz) > thr) continue;
-    const TNode L = load_node(tn, t.left), R = load_node(tn, t.right);
-    const double ll = box_lb(L, qx, qy, qz), lr = box_lb(R, qx, qy, qz);
-    if (top + 2 > kStack) { atomicOr(err, kErrCapacity); return; }
-    if (ll <= lr) {
-      if (lr <= thr) stack[top++] = t.right;
-      if (ll <= thr) stack[top++] = t.left;
-    } else {
-      if (ll <= thr) stack[top++] = t.left;
-      if (lr <= thr) stack[top++] = t.right;
+    const uint32_t tb = __ballot_sync(0xffffffffu, take), eb = __ballot_sync(0xffffffffu, expand);
+    if (take) {
+      const uint32_t at = cnt + __popc(tb & lanemask_lt());
+      sh.cd[at] = d;
+      sh.cid[at] = t.right;
+    }
+    if (expand) {
+      const uint32_t at = top + 2 * __popc(eb & lanemask_lt());
+      sh.stack[at] = t.right;
+      sh.stack[at + 1] = t.left;
+    }
+    top += 2 * __popc(eb);
+    cnt += __popc(tb);
+    if (top + 64 > kStack) {  // deeper than an LBVH can be
+      if (lane == 0) atomicOr(err, kErrCapacity);
+      return;
+    }
+    __syncwarp();
+    if (cnt >= 32) {
+      merge(32);
+      cnt -= 32;
+      __syncwarp();
+      if (lane < cnt) {
+        sh.cd[lane] = sh.cd[32 + lane];
+        sh.cid[lane] = sh.cid[32 + lane];
+      }
+      __syncwarp();
     }
   }
-  for (int j = 0; j < kW; ++j) W[(uint64_t)p * kW + j] = j < cnt ? cid[j] : kInvalid32;
-  // witness radius: every point strictly closer than R2 is in W (R2 = +inf when W is all other points)
-  R2[p] = (cnt >= (int)kw && n - 1 > kw) ? cd[kw - 1] : INFINITY;
+  if (cnt) merge(cnt);
+  W[(uint64_t)p * kW + lane] = lo.id;
+  W[(uint64_t)p * kW + 32 + lane] = hi.id;
+  // witness radius: every point strictly closer than R2 is in W
+  if (lane == 31) R2[p] = hi.d;
 }
 
 // ---- exact side of w relative to the diametral sphere of (u, v) ---------------------
@@ -165,20 +272,28 @@ static_assert(sizeof(PairRec) == 64, "pair record is one 64-byte line");
 
 // ---- warp-per-point enumeration ---------------------------------------------------
 // One warp owns one point u; lane l holds witnesses l and l + 32 of W_u.
-constexpr int kWarpsPerBlock = kThreads / 32;
-constexpr int kQueue = 256;  // warp-cooperative ball-query frontier (power of two)
+constexpr int kQueue = 256;       // warp-cooperative ball-query frontier (power of two)
+constexpr uint32_t kLeaves = 64;  // partners waiting for their classification
+constexpr uint32_t kRecs = 16;    // records waiting to leave with one atomic
+// Work a warp does before it hands its stack over: a step looks at 32 nodes or at one partner.
+// 8,009 clustered points, K = 10: 29.9 ms with every walk in one warp, one node a step (the longest
+// walks ran alone at the end, with a global query for most partners), 7.1 ms like this; lattices,
+// whose walks are short, 4.7 ms both ways (29,791 points).
+constexpr uint32_t kPairSteps = 128;
+// A handed-over walk: Morton position of u, node count, nodes.
+constexpr uint32_t kTaskNodes = 6;
+struct PairTask {
+  uint32_t pos, count, node[kTaskNodes];
+};
 
 struct WarpShared {
+  float4 wit[kW];                 // w - u (binary32), |w - u|^2
   uint32_t stack[kStack];
   uint32_t queue[kQueue];
   uint32_t ids[kMaxInterior + 64];
+  uint32_t leaf[kLeaves + 32];
+  PairRec rec[kRecs];
 };
-
-__device__ __forceinline__ uint32_t lanemask_lt() {
-  uint32_t m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
 
 // Appends the ids of flagged lanes (two flags per lane) to sh.ids[base...];
 // returns the number appended.  Writes only while the total stays <= cap.
@@ -293,134 +408,215 @@ __device__ void warp_ball_query(WarpBall& b, WarpShared& sh, uint32_t iu, uint32
   __syncwarp();
 }
 
+// Writes the warp's finished records: one atomic for all of them (every record of the cloud takes
+// its place on one address), whole lines.
+__device__ __forceinline__ void flush_records(const WarpShared& sh, uint32_t& kept, PairRec* __restrict__ out,
+                                              uint32_t out_cap, uint32_t* __restrict__ counters, uint32_t lane) {
+  __syncwarp();
+  uint32_t slot = 0;
+  if (lane == 0 && kept) slot = atomicAdd(counters, kept);
+  slot = __shfl_sync(0xffffffffu, slot, 0);
+  const uint32_t room = slot < out_cap ? min(kept, out_cap - slot) : 0u;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(sh.rec);
+  uint32_t* dst = reinterpret_cast<uint32_t*>(out + slot);
+  for (uint32_t w = lane; w < room * 16; w += 32) dst[w] = src[w];
+  kept = 0;
+  __syncwarp();
+}
+
+// tasks == nullptr: warp i starts the walk of Morton position i at the root; else it goes on with
+// tasks[i].  Walks longer than kPairSteps leave the rest of their stack in next[0 .. *next_count)
+// (those that do not fit are counted only).
 __global__ void __launch_bounds__(kThreads)
 k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, const uint32_t* __restrict__ leaf_pid,
         const uint32_t* __restrict__ n_begin, const uint32_t* __restrict__ n_end, const double* __restrict__ px,
         const double* __restrict__ py, const double* __restrict__ pz, const int* __restrict__ scale,
         const uint32_t* __restrict__ W, const double* __restrict__ R2, PairRec* __restrict__ out,
         uint32_t out_cap, uint32_t* __restrict__ counters, unsigned long long* __restrict__ stats,
-        uint32_t* __restrict__ err) {
+        uint32_t* __restrict__ err, const PairTask* __restrict__ tasks, uint32_t ntask, PairTask* __restrict__ next,
+        uint32_t next_cap, uint32_t* __restrict__ next_count) {
   __shared__ WarpShared shared[kWarpsPerBlock];
+  __shared__ unsigned long long s_stats[5];
+  if (threadIdx.x < 5) s_stats[threadIdx.x] = 0;
+  __syncthreads();
   // work counters (identical in every lane; lane 0 publishes them)
   unsigned long long visits = 0, local_pairs = 0, ball_queries = 0, ball_nodes = 0, emitted = 0;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t pos = blockIdx.x * kWarpsPerBlock + warp;
-  if (pos >= n) return;  // uniform per warp
-  WarpShared& sh = shared[warp];
-  const uint32_t iu = leaf_pid[pos];
-  const Pt u = point(px, py, pz, iu);
-  const int S = scale[0];
-  const double r2u = R2[iu];
-  // this lane's two witnesses of u
-  const uint32_t w0 = W[(uint64_t)iu * kW + lane], w1 = W[(uint64_t)iu * kW + 32 + lane];
-  float ax0 = 0.f, ay0 = 0.f, az0 = 0.f, ax1 = 0.f, ay1 = 0.f, az1 = 0.f;
-  if (w0 != kInvalid32) { ax0 = (float)(px[w0] - u.x); ay0 = (float)(py[w0] - u.y); az0 = (float)(pz[w0] - u.z); }
-  if (w1 != kInvalid32) { ax1 = (float)(px[w1] - u.x); ay1 = (float)(py[w1] - u.y); az1 = (float)(pz[w1] - u.z); }
-  const uint32_t nw = __popc(__ballot_sync(0xffffffffu, w0 != kInvalid32)) +
-                      __popc(__ballot_sync(0xffffffffu, w1 != kInvalid32));
-  const uint32_t need = cap + 1;
-  uint32_t top = 0;
-  if (lane == 0) sh.stack[0] = root;
-  top = 1;
-  __syncwarp();
-  const double lo = 1.0 - 4.0 * kDistRelErr, hi = 1.0 + 4.0 * kDistRelErr;
-  while (top > 0) {
-    const uint32_t node = sh.stack[top - 1];
-    --top;
+  const uint32_t wi = blockIdx.x * kWarpsPerBlock + warp;
+  if (wi < (tasks ? ntask : n)) {  // uniform per warp
+    WarpShared& sh = shared[warp];
+    const uint32_t pos = tasks ? tasks[wi].pos : wi;
+    const uint32_t iu = leaf_pid[pos];
+    const Pt u = point(px, py, pz, iu);
+    const int S = scale[0];
+    const double r2u = R2[iu];
+    // this lane's two witnesses of u
+    const uint32_t w0 = W[(uint64_t)iu * kW + lane], w1 = W[(uint64_t)iu * kW + 32 + lane];
+    float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+    if (w0 != kInvalid32) { a0.x = (float)(px[w0] - u.x); a0.y = (float)(py[w0] - u.y); a0.z = (float)(pz[w0] - u.z); }
+    if (w1 != kInvalid32) { a1.x = (float)(px[w1] - u.x); a1.y = (float)(py[w1] - u.y); a1.z = (float)(pz[w1] - u.z); }
+    a0.w = a0.x * a0.x + a0.y * a0.y + a0.z * a0.z;
+    a1.w = a1.x * a1.x + a1.y * a1.y + a1.z * a1.z;
+    sh.wit[lane] = a0;
+    sh.wit[32 + lane] = a1;
+    const uint32_t nw = __popc(__ballot_sync(0xffffffffu, w0 != kInvalid32)) +
+                        __popc(__ballot_sync(0xffffffffu, w1 != kInvalid32));  // the first nw slots
+    const uint32_t need = cap + 1;
+    uint32_t top = 1, nleaf = 0, kept = 0, steps = 0;
+    if (tasks) {
+      top = tasks[wi].count;
+      if (lane < top) sh.stack[lane] = tasks[wi].node[lane];
+    } else if (lane == 0) {
+      sh.stack[0] = root;
+    }
     __syncwarp();
-    if (n_end[node] <= pos + 1) continue;  // every partner precedes u in Morton order
-    const TNode t = load_node(tn, node);
-    ++visits;
-    if (t.left != kInvalid32) {
-      if (nw >= need) {
-        const float lx = (float)((double)t.lo[0] - u.x), ly = (float)((double)t.lo[1] - u.y),
-                    lz = (float)((double)t.lo[2] - u.z);
-        const float hx = (float)((double)t.hi[0] - u.x), hy = (float)((double)t.hi[1] - u.y),
-                    hz = (float)((double)t.hi[2] - u.z);
-        // max over v in box of (w-u).(w-v) = sum_i a_i (a_i - (a_i >= 0 ? lo_i : hi_i)), a = w - u
-        auto inside = [&](float ax, float ay, float az, bool valid) {
-          const float tx = ax * (ax - (ax >= 0.f ? lx : hx));
-          const float ty = ay * (ay - (ay >= 0.f ? ly : hy));
-          const float tz = az * (az - (az >= 0.f ? lz : hz));
-          const float mag = fabsf(tx) + fabsf(ty) + fabsf(tz) + ax * ax + ay * ay + az * az;
-          return valid && (tx + ty + tz < -1e-5f * mag);
-        };
-        const uint32_t cnt = __popc(__ballot_sync(0xffffffffu, inside(ax0, ay0, az0, w0 != kInvalid32))) +
-                             __popc(__ballot_sync(0xffffffffu, inside(ax1, ay1, az1, w1 != kInvalid32)));
-        if (cnt >= need) continue;
+    const double lo = 1.0 - 4.0 * kDistRelErr, hi = 1.0 + 4.0 * kDistRelErr;
+    // Classifies the pair (u, v) with the whole warp and keeps its record when it is relevant.
+    auto pair = [&](uint32_t iv) {
+      const Pt v = point(px, py, pz, iv);
+      const double d2 = d2fp(u.x, u.y, u.z, v.x, v.y, v.z);
+      WarpBall b{0u, 0u, kInvalid32, false};
+      if (d2 * hi < r2u * lo) {
+        ++local_pairs;
+        warp_classify(b, sh, w0, w1, iu, iv, u, v, px, py, pz, S, cap);
+      } else {
+        const uint32_t v0 = W[(uint64_t)iv * kW + lane], v1 = W[(uint64_t)iv * kW + 32 + lane];
+        if (d2 * hi < R2[iv] * lo) {
+          ++local_pairs;
+          warp_classify(b, sh, v0, v1, iu, iv, u, v, px, py, pz, S, cap);
+        } else {
+          // witnesses of u, or of v, strictly inside this one sphere for certain: enough of them
+          // reject the pair without a global query.  (w - u).(w - v) = |e|^2 - e.(q - p) with
+          // e = w - p for the end p the witness belongs to and q the other end; the margin
+          // covers binary32 differences.
+          const double vx = v.x - u.x, vy = v.y - u.y, vz = v.z - u.z;
+          auto inside = [&](double ex, double ey, double ez, double sx, double sy, double sz) {
+            const double ee = ex * ex + ey * ey + ez * ez, tx = ex * sx, ty = ey * sy, tz = ez * sz;
+            return ee - (tx + ty + tz) < -1e-5 * (ee + fabs(tx) + fabs(ty) + fabs(tz));
+          };
+          auto of_u = [&](uint32_t w, const float4& a) {
+            return w != kInvalid32 && w != iv && inside(a.x, a.y, a.z, vx, vy, vz);
+          };
+          auto of_v = [&](uint32_t w) {
+            return w != kInvalid32 && w != iu && inside(px[w] - v.x, py[w] - v.y, pz[w] - v.z, -vx, -vy, -vz);
+          };
+          const uint32_t cu = __popc(__ballot_sync(0xffffffffu, of_u(w0, a0))) +
+                              __popc(__ballot_sync(0xffffffffu, of_u(w1, a1)));
+          if (cu >= need) return;
+          const uint32_t cv = __popc(__ballot_sync(0xffffffffu, of_v(v0))) + __popc(__ballot_sync(0xffffffffu, of_v(v1)));
+          if (cv >= need) return;
+          ++ball_queries;
+          steps += 8;
+          warp_ball_query(b, sh, iu, iv, u, v, root, tn, leaf_pid, n_begin, n_end, px, py, pz, S, cap, err, ball_nodes);
+        }
       }
-      if (top + 2 > kStack) {
-        if (lane == 0) atomicOr(err, kErrCapacity);
-        return;
-      }
-      if (lane == 0) {
-        sh.stack[top] = t.right;
-        sh.stack[top + 1] = t.left;
-      }
-      top += 2;
       __syncwarp();
-      continue;
-    }
-    const uint32_t iv = t.right;
-    const Pt v = point(px, py, pz, iv);
-    const double d2 = d2fp(u.x, u.y, u.z, v.x, v.y, v.z);
-    WarpBall b{0u, 0u, kInvalid32, false};
-    if (d2 * hi < r2u * lo) {
-      ++local_pairs;
-      warp_classify(b, sh, w0, w1, iu, iv, u, v, px, py, pz, S, cap);
-    } else if (d2 * hi < R2[iv] * lo) {
-      ++local_pairs;
-      const uint32_t v0 = W[(uint64_t)iv * kW + lane], v1 = W[(uint64_t)iv * kW + 32 + lane];
-      warp_classify(b, sh, v0, v1, iu, iv, u, v, px, py, pz, S, cap);
-    } else {
-      // witnesses of u strictly inside this one sphere: enough of them rejects
-      // the pair without a global query
-      auto strictly_inside = [&](uint32_t w, float ax, float ay, float az) {
-        if (w == kInvalid32 || w == iv) return false;
-        const double dx = (double)ax, dy = (double)ay, dz = (double)az;  // w - u (binary32-rounded)
-        const double vx = v.x - u.x, vy = v.y - u.y, vz = v.z - u.z;
-        // (w-u).(w-v) = |a|^2 - a.(v-u); margin covers the binary32 rounding of a
-        const double aa = dx * dx + dy * dy + dz * dz, av = dx * vx + dy * vy + dz * vz;
-        return aa - av < -1e-5 * (aa + fabs(dx * vx) + fabs(dy * vy) + fabs(dz * vz));
-      };
-      const uint32_t inside = __popc(__ballot_sync(0xffffffffu, strictly_inside(w0, ax0, ay0, az0))) +
-                              __popc(__ballot_sync(0xffffffffu, strictly_inside(w1, ax1, ay1, az1)));
-      if (inside >= need) continue;
-      ++ball_queries;
-      warp_ball_query(b, sh, iu, iv, u, v, root, tn, leaf_pid, n_begin, n_end, px, py, pz, S, cap, err, ball_nodes);
-    }
-    __syncwarp();
-    if (b.rejected || b.interior > cap) continue;
-    ++emitted;
-    if (lane == 0) {
-      const uint32_t slot = atomicAdd(counters, 1u);
-      if (slot < out_cap) {
-        PairRec r;
+      if (b.rejected || b.interior > cap) return;
+      ++emitted;
+      // interior ids ascending: lane i holds the i-th, its rank is the number of lesser ids
+      const uint32_t mine = lane < b.interior ? sh.ids[lane] : kInvalid32;
+      uint32_t rank = 0;
+      for (uint32_t i = 0; i < b.interior; ++i) rank += __shfl_sync(0xffffffffu, mine, i) < mine ? 1u : 0u;
+      PairRec& r = sh.rec[kept];
+      if (lane == 0) {
         r.u = min(iu, iv);
         r.v = max(iu, iv);
         r.interior = b.interior;
         r.shell = b.shell + 2;
         r.witness = b.witness;
-        for (uint32_t j = 0; j < kMaxInterior; ++j) r.ids[j] = j < b.interior ? sh.ids[j] : kInvalid32;
-        for (uint32_t a = 1; a < b.interior; ++a) {  // ascending interior ids
-          const uint32_t x = r.ids[a];
-          uint32_t j = a;
-          while (j > 0 && r.ids[j - 1] > x) { r.ids[j] = r.ids[j - 1]; --j; }
-          r.ids[j] = x;
-        }
         r.pad[0] = r.pad[1] = 0;
-        out[slot] = r;
       }
+      if (lane < b.interior) r.ids[rank] = mine;
+      else if (lane < (uint32_t)kMaxInterior) r.ids[lane] = kInvalid32;
+      if (++kept == kRecs) flush_records(sh, kept, out, out_cap, counters, lane);
+      __syncwarp();
+    };
+    while (top > 0 || nleaf > 0) {
+      if (nleaf >= kLeaves || top == 0) {
+        for (uint32_t i = 0; i < nleaf; ++i) pair(sh.leaf[i]);
+        steps += nleaf;
+        nleaf = 0;
+        __syncwarp();
+        continue;
+      }
+      if (steps >= kPairSteps && top > 1) {  // hand the rest over (the top first: its nodes are the smallest)
+        const uint32_t made = (top + kTaskNodes - 1) / kTaskNodes;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(next_count, made);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (at + made <= next_cap) {
+          for (uint32_t i = lane; i < made; i += 32) {
+            PairTask t;
+            t.pos = pos;
+            t.count = min(kTaskNodes, top - i * kTaskNodes);
+            for (uint32_t j = 0; j < kTaskNodes; ++j) t.node[j] = j < t.count ? sh.stack[i * kTaskNodes + j] : 0u;
+            next[at + i] = t;
+          }
+          top = 0;
+          __syncwarp();
+          continue;
+        }
+        if (lane == 0) atomicSub(next_count, made);  // no room: the walk goes on here
+        steps = 0;
+      }
+      const uint32_t batch = top > kStackWide ? 1u : min(top, 32u);
+      uint32_t node = kInvalid32;
+      if (lane < batch) node = sh.stack[top - 1 - lane];
+      __syncwarp();
+      top -= batch;
+      visits += batch;
+      ++steps;
+      bool open = false;
+      TNode t;
+      t.left = t.right = kInvalid32;
+      float lx = 0.f, ly = 0.f, lz = 0.f, hx = 0.f, hy = 0.f, hz = 0.f;
+      if (node != kInvalid32 && n_end[node] > pos + 1) {  // every partner follows u in Morton order
+        t = load_node(tn, node);
+        open = true;
+        lx = (float)((double)t.lo[0] - u.x), ly = (float)((double)t.lo[1] - u.y), lz = (float)((double)t.lo[2] - u.z);
+        hx = (float)((double)t.hi[0] - u.x), hy = (float)((double)t.hi[1] - u.y), hz = (float)((double)t.hi[2] - u.z);
+      }
+      if (nw >= need) {
+        // max over v in box of (w-u).(w-v) = sum_i a_i (a_i - (a_i >= 0 ? lo_i : hi_i)), a = w - u: below 0
+        // with certainty for `need` witnesses, no pair of u with the box is relevant
+        uint32_t in = 0;
+        for (uint32_t w = 0; w < nw; ++w) {
+          const float4 a = sh.wit[w];
+          const float tx = a.x * (a.x - (a.x >= 0.f ? lx : hx));
+          const float ty = a.y * (a.y - (a.y >= 0.f ? ly : hy));
+          const float tz = a.z * (a.z - (a.z >= 0.f ? lz : hz));
+          in += tx + ty + tz < -1e-5f * (fabsf(tx) + fabsf(ty) + fabsf(tz) + a.w) ? 1u : 0u;
+          if ((w & 7u) == 7u && __all_sync(0xffffffffu, !open || in >= need)) break;
+        }
+        open = open && in < need;
+      }
+      const bool is_leaf = open && t.left == kInvalid32, expand = open && !is_leaf;
+      const uint32_t lb = __ballot_sync(0xffffffffu, is_leaf), eb = __ballot_sync(0xffffffffu, expand);
+      if (is_leaf) sh.leaf[nleaf + __popc(lb & lanemask_lt())] = t.right;
+      nleaf += __popc(lb);
+      if (expand) {
+        const uint32_t at = top + 2 * __popc(eb & lanemask_lt());
+        sh.stack[at] = t.right;
+        sh.stack[at + 1] = t.left;
+      }
+      top += 2 * __popc(eb);
+      if (top + 64 > kStack) {  // deeper than an LBVH can be
+        if (lane == 0) atomicOr(err, kErrCapacity);
+        top = nleaf = 0;
+      }
+      __syncwarp();
     }
-    __syncwarp();
+    flush_records(sh, kept, out, out_cap, counters, lane);
   }
   if (lane == 0) {
-    atomicAdd(stats + 0, visits);
-    atomicAdd(stats + 1, local_pairs);
-    atomicAdd(stats + 2, ball_queries);
-    atomicAdd(stats + 3, ball_nodes);
-    atomicAdd(stats + 4, emitted);
+    atomicAdd(s_stats + 0, visits);
+    atomicAdd(s_stats + 1, local_pairs);
+    atomicAdd(s_stats + 2, ball_queries);
+    atomicAdd(s_stats + 3, ball_nodes);
+    atomicAdd(s_stats + 4, emitted);
   }
+  __syncthreads();
+  if (threadIdx.x < 5 && s_stats[threadIdx.x]) atomicAdd(stats + threadIdx.x, s_stats[threadIdx.x]);
 }
 
 __global__ void __launch_bounds__(256)
@@ -500,6 +696,8 @@ cudaError_t pairs_alloc(Ctx& ctx) {
   EHGP_ALLOC(p.R2, n * sizeof(double));
   EHGP_ALLOC(p.counters, 8 * sizeof(uint32_t));
   EHGP_ALLOC(p.stats, 8 * sizeof(unsigned long long));
+  p.task_cap = (uint32_t)(2 * n + 4096);  // handed-over walks per round (what does not fit goes on in place)
+  EHGP_ALLOC(p.tasks, 2ull * p.task_cap * sizeof(PairTask));
 #undef EHGP_ALLOC
   // records: about 38 per point in lattices and uniform clouds; grown on demand
   return pairs_records_alloc(ctx, 48 * n + 1024);
@@ -530,7 +728,7 @@ int pairs_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
   const uint32_t kw = (n - 1 < (uint32_t)kW) ? n - 1 : (uint32_t)kW;
   uint64_t launches = 0;
   cudaEventRecord(ctx.ev0, st);
-  k_witness_knn<<<nblocks(n), kThreads, 0, st>>>(n, kw, root, g.tnodes, b.leaf_pid, b.px, b.py, b.pz, p.W, p.R2,
+  k_witness_knn<<<nblocks(n, kWarpsPerBlock), kThreads, 0, st>>>(n, kw, root, g.tnodes, b.leaf_pid, b.px, b.py, b.pz, p.W, p.R2,
                                                   ctx.d_err);
   ++launches;
   uint32_t hc[2] = {0, 0};
@@ -541,17 +739,28 @@ int pairs_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
     cudaMemsetAsync(p.counters, 0, 8 * sizeof(uint32_t), st);
     cudaMemsetAsync(p.stats, 0, 8 * sizeof(unsigned long long), st);
     cudaEventRecord(ctx.evk0, st);
-    k_pairs<<<nblocks(n, kWarpsPerBlock), kThreads, 0, st>>>(n, cap, root, g.tnodes, b.leaf_pid, b.n_begin, b.n_end,
-                                                             b.px, b.py, b.pz, g.scale, p.W, p.R2, (PairRec*)p.raw,
-                                                             p.capacity, p.counters, p.stats, ctx.d_err);
-    cudaEventRecord(ctx.evk1, st);
-    ++launches;
     unsigned long long hs[8];
-    cudaMemcpyAsync(hc, p.counters, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(hc + 1, ctx.d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(hs, p.stats, sizeof(hs), cudaMemcpyDeviceToHost, st);
-    e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return abi_cuda_fail(&ctx, e, "pair enumeration");
+    PairTask* task[2] = {(PairTask*)p.tasks, (PairTask*)p.tasks + p.task_cap};
+    uint32_t ntask = 0;  // 0: the walks from the root; then those that were handed over, while there are any
+    for (int round = 0;; ++round) {
+      const uint32_t warps = round ? ntask : n;
+      k_pairs<<<nblocks(warps, kWarpsPerBlock), kThreads, 0, st>>>(
+          n, cap, root, g.tnodes, b.leaf_pid, b.n_begin, b.n_end, b.px, b.py, b.pz, g.scale, p.W, p.R2, (PairRec*)p.raw,
+          p.capacity, p.counters, p.stats, ctx.d_err, round ? task[round & 1] : nullptr, ntask, task[(round + 1) & 1],
+          p.task_cap, p.counters + 1);
+      ++launches;
+      uint32_t hn[2];
+      cudaEventRecord(ctx.evk1, st);
+      cudaMemcpyAsync(hn, p.counters, sizeof(hn), cudaMemcpyDeviceToHost, st);
+      cudaMemcpyAsync(hc + 1, ctx.d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+      cudaMemcpyAsync(hs, p.stats, sizeof(hs), cudaMemcpyDeviceToHost, st);
+      e = cudaStreamSynchronize(st);
+      if (e != cudaSuccess) return abi_cuda_fail(&ctx, e, "pair enumeration");
+      hc[0] = hn[0];
+      ntask = hn[1];
+      if (ntask == 0 || hc[1]) break;
+      cudaMemsetAsync(p.counters + 1, 0, sizeof(uint32_t), st);
+    }
     {
       float kms = 0.f;
       cudaEventElapsedTime(&kms, ctx.evk0, ctx.evk1);
