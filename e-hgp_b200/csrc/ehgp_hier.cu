@@ -1089,52 +1089,85 @@ k_arm_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, con
            const uint32_t* __restrict__ rstate, int passes, const uint32_t* __restrict__ v0,
            const uint32_t* __restrict__ v1, uint32_t* __restrict__ out_arm, uint32_t* __restrict__ out_fac,
            uint32_t* __restrict__ out_count, uint32_t* __restrict__ term, unsigned long long* __restrict__ stats) {
+  // Work counters leave through shared memory with the block's last warp (no warp waits for another);
+  // a global atomic per arm and counter queues every arm on one address.
+  __shared__ unsigned int s_count[4], s_warps;  // node visits, steps, equal cutoffs, strictness checks
+  const uint32_t lane = threadIdx.x & 31u;
+  if (threadIdx.x < 4) s_count[threadIdx.x] = 0;
+  if (threadIdx.x == 4) s_warps = 0;
+  __syncthreads();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= m) return;
-  // queue entry: in Morton order of the facets when the queue was sorted (passes >= 0)
-  const uint32_t i = passes >= 0 ? radix_result(rstate, passes, v0, v1)[t] : t;
-  const uint32_t a = in_arm[i];
-  uint32_t F[kMaxFacet];
+  uint32_t F[kMaxFacet], G[kMaxFacet];
+  uint32_t a = 0, visits = 0, stepped = 0, equal = 0, strict = 0;
   int k = 0;
-  for (int j = 0; j < kMaxFacet; ++j) {
-    F[j] = in_fac[(uint64_t)i * kMaxFacet + j];
-    k += F[j] != kInvalid32;
+  bool go_on = false;  // G is no birth facet: queued for the next step
+  if (t < m) {
+    // queue entry: in Morton order of the facets when the queue was sorted (passes >= 0)
+    const uint32_t i = passes >= 0 ? radix_result(rstate, passes, v0, v1)[t] : t;
+    a = in_arm[i];
+    for (int j = 0; j < kMaxFacet; ++j) {
+      F[j] = in_fac[(uint64_t)i * kMaxFacet + j];
+      k += F[j] != kInvalid32;
+    }
+    const Cloud c{d.px, d.py, d.pz, d.S};
+    auto step = [&]() -> int {
+      Mini mb;
+      if (!facet_miniball(c, F, k, mb)) return kArmInternal;
+      int cut_below = 0;
+      const int s = topk_choice(d, c, mb, k, G, &cut_below, &visits);
+      if (s != kArmOk) return s;
+      bool same = true;
+      for (int j = 0; j < k; ++j) same &= G[j] == F[j];
+      if (same) return kArmUnresolved;
+      if (!cut_below) {  // beta(G) <= cutoff = beta(F): the decrease must be strict
+        equal = 1;
+        Mini mg;
+        if (!facet_miniball(c, G, k, mg)) return kArmInternal;
+        double glo, ghi, flo, fhi;
+        if (!flevel(mg.fs, glo, ghi)) exact_level_fp(c, mg.T, mg.ts, glo, ghi);
+        if (!flevel(mb.fs, flo, fhi)) exact_level_fp(c, mb.T, mb.ts, flo, fhi);
+        if (!(ghi < flo) && level_cmp_exact(c, mg.T, mg.ts, mb.T, mb.ts) >= 0) return kArmPlateau;
+        strict = 1;
+      }
+      stepped = 1;
+      return kArmOk;
+    };
+    const int why = step();
+    if (why != kArmOk) {  // failed arms, and the least of them with its status
+      atomicAdd(stats + 2, 1ull);
+      atomicMin(stats + 3, (unsigned long long)a << 8 | (unsigned long long)why);
+    } else {
+      const uint32_t h = probe_facet(d, G, k);
+      go_on = h == kInvalid32;
+      if (!go_on) term[a] = h;
+    }
   }
-  const Cloud c{d.px, d.py, d.pz, d.S};
-  auto fail = [&](int why) {  // failed arms, and the least of them with its status
-    atomicAdd(stats + 2, 1ull);
-    atomicMin(stats + 3, (unsigned long long)a << 8 | (unsigned long long)why);
-  };
-  Mini mb;
-  if (!facet_miniball(c, F, k, mb)) { fail(kArmInternal); return; }
-  uint32_t G[kMaxFacet];
-  int cut_below = 0;
-  uint32_t visits = 0;
-  const int s = topk_choice(d, c, mb, k, G, &cut_below, &visits);
-  atomicAdd(&g_descent_visits[blockIdx.x % kVisitStripes], (unsigned long long)visits);
-  if (s != kArmOk) { fail(s); return; }
-  bool same = true;
-  for (int j = 0; j < k; ++j) same &= G[j] == F[j];
-  if (same) { fail(kArmUnresolved); return; }
-  if (!cut_below) {  // beta(G) <= cutoff = beta(F): the decrease must be strict
-    slow(6);
-    Mini mg;
-    if (!facet_miniball(c, G, k, mg)) { fail(kArmInternal); return; }
-    double glo, ghi, flo, fhi;
-    if (!flevel(mg.fs, glo, ghi)) exact_level_fp(c, mg.T, mg.ts, glo, ghi);
-    if (!flevel(mb.fs, flo, fhi)) exact_level_fp(c, mb.T, mb.ts, flo, fhi);
-    if (!(ghi < flo) && level_cmp_exact(c, mg.T, mg.ts, mb.T, mb.ts) >= 0) { fail(kArmPlateau); return; }
-    atomicAdd(stats + 1, 1ull);
+  __syncwarp();
+  const uint32_t b = __ballot_sync(0xffffffffu, go_on);
+  uint32_t base = 0;
+  if (lane == 0 && b) base = atomicAdd(out_count, (uint32_t)__popc(b));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (go_on) {
+    const uint32_t slot = base + __popc(b & ((1u << lane) - 1u));
+    out_arm[slot] = a;
+    for (int j = 0; j < kMaxFacet; ++j) out_fac[(uint64_t)slot * kMaxFacet + j] = j < k ? G[j] : kInvalid32;
   }
-  atomicAdd(stats, 1ull);
-  const uint32_t h = probe_facet(d, G, k);
-  if (h != kInvalid32) {
-    term[a] = h;
-    return;
-  }
-  const uint32_t slot = atomicAdd(out_count, 1u);
-  out_arm[slot] = a;
-  for (int j = 0; j < kMaxFacet; ++j) out_fac[(uint64_t)slot * kMaxFacet + j] = j < k ? G[j] : kInvalid32;
+  visits = __reduce_add_sync(0xffffffffu, visits);
+  stepped = __reduce_add_sync(0xffffffffu, stepped);
+  equal = __reduce_add_sync(0xffffffffu, equal);
+  strict = __reduce_add_sync(0xffffffffu, strict);
+  if (lane != 0) return;
+  atomicAdd(s_count + 0, visits);
+  atomicAdd(s_count + 1, stepped);
+  atomicAdd(s_count + 2, equal);
+  atomicAdd(s_count + 3, strict);
+  __threadfence_block();
+  if (atomicAdd(&s_warps, 1u) + 1 < blockDim.x / 32) return;
+  __threadfence_block();
+  atomicAdd(&g_descent_visits[blockIdx.x % kVisitStripes], (unsigned long long)atomicAdd(s_count + 0, 0u));
+  atomicAdd(stats, (unsigned long long)atomicAdd(s_count + 1, 0u));
+  atomicAdd(&g_descent_slow[6], (unsigned long long)atomicAdd(s_count + 2, 0u));
+  atomicAdd(stats + 1, (unsigned long long)atomicAdd(s_count + 3, 0u));
 }
 
 }  // namespace
