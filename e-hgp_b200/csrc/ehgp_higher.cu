@@ -39,6 +39,7 @@
 #include <array>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 namespace ehgp {
@@ -332,7 +333,7 @@ k_gather(uint32_t n, uint32_t root, const TNode* __restrict__ tn, const uint32_t
 // u; those lie in C(a) too, so classifying against C(a) rejects it.
 // The neighbour list (points within the gather radius L, sorted by distance)
 // certifies rho_s when rho_s <= L / 2: every unlisted point has rho >= L / 2.
-constexpr int kDirThreads = 128;  // one block per point: four warps share its sorted list
+constexpr int kDirThreads = 224;  // one block per point: seven warps share its sorted list, 3 x 224 directions
 constexpr int kMaxCand = 256;     // candidate-set capacity per point
 constexpr int kLargeCand = 1024;  // large sets: staged whole in shared memory with their face mask
 constexpr int kHugeCand = 4096;   // huge sets: staged in shared memory, face mask in global scratch
@@ -364,39 +365,92 @@ __device__ __forceinline__ double cone_exit(const CertParams& cp, double sk, dou
   return g * (1.0 + 1e-12);
 }
 
-// Bitonic sort of one value per lane, descending across the warp (lane 0 the largest).
-__device__ __forceinline__ float warp_sort_desc(float v, uint32_t lane) {
+// The `need` largest lower bounds of 1 / rho_shr seen by one direction, descending, in registers: the
+// first kMaxNeed - need slots hold infinity, so the threshold is always the last slot.
+struct TopInv {
+  float v[kMaxNeed];
+  __device__ __forceinline__ void init(uint32_t need) {
 #pragma unroll
-  for (uint32_t k = 2; k <= 32; k <<= 1) {
+    for (int j = 0; j < kMaxNeed; ++j) v[j] = j < kMaxNeed - (int)need ? INFINITY : 0.0f;
+  }
+  __device__ __forceinline__ float thr() const { return v[kMaxNeed - 1]; }
+  __device__ __forceinline__ void add(float x) {  // x > thr()
 #pragma unroll
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      const float o = __shfl_xor_sync(0xffffffffu, v, j);
-      v = (((lane & j) == 0) == ((lane & k) == 0)) ? fmaxf(v, o) : fminf(v, o);
+    for (int j = 0; j < kMaxNeed; ++j) {
+      const float hi = fmaxf(v[j], x);
+      x = fminf(v[j], x);
+      v[j] = hi;
     }
   }
-  return v;
-}
+};
 
-// top holds the 32 largest values seen so far, descending across the warp; merges in one
-// value per lane: the larger of top[j] and the j-th smallest new value forms a bitonic
-// sequence that holds the 32 largest of both, and a bitonic merge orders it.
-__device__ __forceinline__ float warp_top_merge(float top, float v, uint32_t lane) {
-  const float s = warp_sort_desc(v, lane);
-  float x = fmaxf(top, __shfl_sync(0xffffffffu, s, 31u - lane));
-#pragma unroll
-  for (uint32_t j = 16; j > 0; j >>= 1) {
-    const float o = __shfl_xor_sync(0xffffffffu, x, j);
-    x = ((lane & j) == 0) ? fmaxf(x, o) : fminf(x, o);
+// The cone that holds the directions of a warp's lanes (unit axis, cosine and sine of its half-angle).
+// Points are first tested against it 32 at a time, one per lane, and only those that some lane may
+// need are looked at by every lane.
+struct ConeGroup {
+  float a0, a1, a2, cr, sr;
+  __device__ __forceinline__ void init(float u0, float u1, float u2, bool on) {
+    float x = on ? u0 : 0.f, y = on ? u1 : 0.f, z = on ? u2 : 0.f;
+    for (int o = 16; o > 0; o >>= 1) {
+      x += __shfl_xor_sync(0xffffffffu, x, o);
+      y += __shfl_xor_sync(0xffffffffu, y, o);
+      z += __shfl_xor_sync(0xffffffffu, z, o);
+    }
+    const float l = sqrtf(x * x + y * y + z * z);
+    const float inv = l > 1e-3f ? 1.0f / l : 0.0f;  // (no axis: half-angle 180 degrees)
+    a0 = x * inv;
+    a1 = y * inv;
+    a2 = z * inv;
+    float c = on ? u0 * a0 + u1 * a1 + u2 * a2 : 1.0f;
+    for (int o = 16; o > 0; o >>= 1) c = fminf(c, __shfl_xor_sync(0xffffffffu, c, o));
+    cr = l > 1e-3f ? fminf(c, 1.0f) : -1.0f;
+    sr = sqrtf(fmaxf(0.0f, 1.0f - cr * cr));
   }
+  // Upper bound of the cosine between the unit direction r and any of the lanes' directions
+  // (binary32 roundings are below the slack).
+  __device__ __forceinline__ float cos_max(const float4& r) const {
+    const float c = a0 * r.x + a1 * r.y + a2 * r.z;
+    if (c >= cr) return 1.0f;
+    return fminf(1.0f, c * cr + sqrtf(fmaxf(0.0f, 1.0f - c * c)) * sr + 1e-5f);
+  }
+};
+__device__ __forceinline__ float warp_min(float x) {
+  for (int o = 16; o > 0; o >>= 1) x = fminf(x, __shfl_xor_sync(0xffffffffu, x, o));
   return x;
 }
+__device__ __forceinline__ float warp_max(float x) {
+  for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+  return x;
+}
+// Upper bound of cos(max(angle - delta, 0)) from an upper bound of the angle's cosine.
+__device__ __forceinline__ float cos_low(float c, float cdf, float sdlf) {
+  const float cs = fminf(1.0f, c + 1e-5f);  // cosine of a lower bound of the angle
+  if (cs >= cdf) return 1.0f;
+  const float sn = sqrtf(fmaxf(0.0f, (1.0f - cs) * (1.0f + cs)));
+  return cs * cdf + sn * sdlf + 1e-6f;
+}
 
-// register budget of the direction table: 10 blocks of 128 threads per SM (51 registers; its
-// shared list is 20.6 KB per block); measured higher-stage wall at 50k 113.6 ms at 7, 111.7 at 10
-#ifndef EHGP_DIRTABLE_BLOCKS_PER_SM
-#define EHGP_DIRTABLE_BLOCKS_PER_SM 10
-#endif
-__global__ void __launch_bounds__(kDirThreads, EHGP_DIRTABLE_BLOCKS_PER_SM)
+// Lower bound of 1 / rho_p(u) over the cone of s, binary32 without divides:
+// 2 cos(angle + delta) / |p - a|; 0 when the bound is not positive.  Every binary32 rounding
+// (about 1e-7 relative) is covered by the 1e-5 margins and the 1e-6 absolute slack on the
+// cosines, always in the safe direction.  `best` is an upper bound of the value that needs no
+// square root (the sine is not negative): values at most `best` cannot pass a threshold above it.
+__device__ __forceinline__ float inv_rho_best(float c, float w, float cdf) {
+  const float cs = fmaxf(-1.0f, c - 1e-5f);
+  return 2.0f * (cs * cdf) * w;
+}
+__device__ __forceinline__ float inv_rho(float c, float w, float cdf, float sdlf) {
+  const float cs = fmaxf(-1.0f, c - 1e-5f);  // cosine of an upper bound of the angle
+  const float sn = sqrtf(fmaxf(0.0f, (1.0f - cs) * (1.0f + cs)));
+  const float cshr = cs * cdf - sn * sdlf - 1e-6f;  // lower bound of cos(angle + delta)
+  return cshr > 1e-6f ? 2.0f * cshr * w * (1.0f - 1e-5f) : 0.0f;
+}
+
+// Register budget: 6 blocks of 7 warps per SM (48 registers).
+// Bound: FP32 and integer issue.  50,653 lattice points, K = 10, gathers and tables of both rounds: 34.7 ms
+// with 32 points per step of one direction (the `need` largest merged across the warp by a bitonic
+// network), 20.3 with a direction per lane, 15.7 with points tested against the warp's cone first.
+__global__ void __launch_bounds__(kDirThreads, 6)
 k_dirtable(uint32_t n, uint32_t list_cap, CertParams cp, const uint32_t* __restrict__ leaf_pid, uint32_t* __restrict__ nb,
            const uint32_t* __restrict__ nbc, const double* __restrict__ px, const double* __restrict__ py,
            const double* __restrict__ pz, const double* __restrict__ gather_r2, uint8_t* __restrict__ todo,
@@ -468,85 +522,85 @@ k_dirtable(uint32_t n, uint32_t list_cap, CertParams cp, const uint32_t* __restr
   const uint32_t need = cp.need;
   double worst_needed = 0.0;  // largest certified rho_s (the list must cover 2 rho_s)
   bool ok = true;
-  // Each warp takes batches of 32 directions; lane j prepares direction j of the batch, then
-  // the warp scans the sorted list for one direction at a time, 32 points per step.
+  // One direction per lane (neighbouring lanes hold neighbouring directions), one point of the sorted
+  // list per step for the whole warp: a point behind all 32 cones costs its dot product.
   for (uint32_t dbase = warp * 32u; dbase < (uint32_t)kDirs; dbase += kDirThreads) {
     const uint32_t dl = dbase + lane;
-    float s0f = 0.f, s1f = 0.f, s2f = 0.f;
-    double ext_c = 0.0;
-    if (dl < (uint32_t)kDirs) {
+    const bool on = dl < (uint32_t)kDirs;
+    float u0 = 0.f, u1 = 0.f, u2 = 0.f;
+    double ext_d = 0.0;
+    if (on) {
       const double s0 = cp.dirs[3 * dl], s1 = cp.dirs[3 * dl + 1], s2 = cp.dirs[3 * dl + 2];
-      s0f = (float)s0;
-      s1f = (float)s1;
-      s2f = (float)s2;
+      u0 = (float)s0;
+      u1 = (float)s1;
+      u2 = (float)s2;
       // AABB support bound over the cone
       const double ext = cone_ext(cp, s0, ax, 0) + cone_ext(cp, s1, ay, 1) + cone_ext(cp, s2, az, 2);
       // the centre of a well-centred sphere lies in conv(S), inside the AABB: r is at most
       // the distance at which the ray a + r u leaves the AABB, maximised over the cone
       // axis by axis (min over axes of the per-axis maxima bounds the max of the min)
       const double exit_r = fmin(fmin(cone_exit(cp, s0, ax, 0), cone_exit(cp, s1, ay, 1)), cone_exit(cp, s2, az, 2));
-      ext_c = fmin(ext * (1.0 + 1e-12), exit_r);
+      ext_d = fmin(ext * (1.0 + 1e-12), exit_r);
     }
-    const uint32_t nd = min(32u, (uint32_t)kDirs - dbase);
-    float my_rho = 0.f;
-    for (uint32_t jd = 0; jd < nd; ++jd) {
-      const float u0 = __shfl_sync(0xffffffffu, s0f, jd), u1 = __shfl_sync(0xffffffffu, s1f, jd),
-                  u2 = __shfl_sync(0xffffffffu, s2f, jd);
-      const double ext_d = __shfl_sync(0xffffffffu, ext_c, jd);
-      // The `need` smallest shrunk thresholds, kept as the `need` largest lower bounds of
-      // 1 / rho_shr (binary32, no divides):  1/rho_p(u) >= 2 cos(angle + delta) / |p - a|.
-      // Every binary32 rounding (about 1e-7 relative) is covered by the 1e-5 margins and the
-      // 1e-6 absolute slack on the cosines, always in the safe direction.  The scan stops at
-      // the first step whose nearest point has rho >= |p - a| / 2 > min(kth, ext); points
-      // past that bound can neither enter the `need` largest nor lower min(kth, ext).
-      const float inv_ext = 1.0f / __double2float_ru(ext_d);
-      float top = 0.0f;  // lane j: the j-th largest lower bound so far
-      float thr = 0.0f;  // top[need - 1]
-      for (uint32_t base = 0; base < m; base += 32) {
-        const uint32_t i = base + lane;
-        const float lim = 0.5f * (1.0f - 1e-5f) * fmaxf(thr, inv_ext);
-        const float4 r = i < m ? rel[i] : make_float4(0.f, 0.f, 0.f, 0.f);  // r.w = 1 / |p - a|
-        if (lim > __shfl_sync(0xffffffffu, r.w, 0)) break;
-        float inv = 0.0f;
-        if (i < m && !(lim > r.w)) {
-          const float c = u0 * r.x + u1 * r.y + u2 * r.z;
-          const float cs = fmaxf(-1.0f, c - 1e-5f);  // cosine of an upper bound of the angle
-          const float sn = sqrtf(fmaxf(0.0f, (1.0f - cs) * (1.0f + cs)));
-          const float cshr = cs * cdf - sn * sdlf - 1e-6f;  // lower bound of cos(angle + delta)
-          if (cshr > 1e-6f) inv = 2.0f * cshr * r.w * (1.0f - 1e-5f);  // lower bound of 1 / rho_p(u)
-        }
-        if (__any_sync(0xffffffffu, inv > thr)) {
-          top = warp_top_merge(top, inv, lane);
-          thr = __shfl_sync(0xffffffffu, top, need - 1);
+    // The scan of a direction stops at the first point with rho >= |p - a| / 2 > min(kth, ext): points
+    // past that bound can neither enter the `need` largest nor lower min(kth, ext).
+    const float inv_ext = on ? 1.0f / __double2float_ru(ext_d) : INFINITY;
+    ConeGroup grp;
+    grp.init(u0, u1, u2, on);
+    TopInv top;
+    top.init(on ? need : 0u);
+    float lim = 0.5f * (1.0f - 1e-5f) * inv_ext;
+    for (uint32_t base = 0; base < m; base += 32) {
+      const uint32_t i = base + lane;
+      const float4 mine = i < m ? rel[i] : make_float4(0.f, 0.f, 0.f, 0.f);  // .w = 1 / |p - a|
+      const float lim_min = warp_min(lim), thr_min = warp_min(top.thr());
+      if (lim_min > __shfl_sync(0xffffffffu, mine.w, 0)) break;
+      const bool some = i < m && !(lim_min > mine.w) && inv_rho_best(grp.cos_max(mine) + 2e-5f, mine.w, cdf) > thr_min;
+      for (uint32_t todo_pts = __ballot_sync(0xffffffffu, some); todo_pts; todo_pts &= todo_pts - 1) {
+        const float4 r = rel[base + __ffs((int)todo_pts) - 1];
+        const float c = u0 * r.x + u1 * r.y + u2 * r.z;
+        if (!(lim > r.w) && inv_rho_best(c, r.w, cdf) > top.thr()) {
+          const float inv = inv_rho(c, r.w, cdf, sdlf);
+          if (inv > top.thr()) {
+            top.add(inv);
+            lim = 0.5f * (1.0f - 1e-5f) * fmaxf(top.thr(), inv_ext);
+          }
         }
       }
-      const double kth = thr > 0.0f ? (1.0 / (double)thr) * (1.0 + 1e-12) : INFINITY;
-      const double rho_s = fmin(kth, ext_d);
-      const float rho_sf = __double2float_ru(rho_s);  // per-cone bound, rounded up
-      if (lane == jd) my_rho = rho_sf;
+    }
+    const double kth = top.thr() > 0.0f ? (1.0 / (double)top.thr()) * (1.0 + 1e-12) : INFINITY;
+    const double rho_s = fmin(kth, ext_d);
+    const float rho_sf = on ? __double2float_ru(rho_s) : 0.0f;  // per-cone bound, rounded up
+    if (on) {
+      rho_tab[(uint64_t)a * kDirs + dl] = rho_sf;
       // certified when every unlisted point (rho >= L/2) cannot lower it
       if (!(rho_s <= half_L)) ok = false;
       worst_needed = fmax(worst_needed, rho_s);
-      // mark the candidates of this cone: rho_lo_p(s) <= rho_s, i.e. 2 cos(max(angle - delta, 0)) rho_s >= |p - a|;
-      // rho_lo >= |p - a| / 2 > rho_s stops the scan (monotone along the sorted list)
-      for (uint32_t base = 0; base < m; base += 32) {
-        const uint32_t i = base + lane;
-        const float4 r = i < m ? rel[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const bool stop = !(i < m) || (0.5f * (1.0f - 1e-5f) > rho_sf * r.w);
-        if (__shfl_sync(0xffffffffu, stop, 0)) break;
+    }
+    // mark the candidates of these cones: rho_lo_p(s) <= rho_s, i.e. 2 cos(max(angle - delta, 0)) rho_s >= |p - a|;
+    // rho_lo >= |p - a| / 2 > rho_s stops a scan (monotone along the sorted list); a point that is marked
+    // already (by these or other cones) needs no test
+    const float rho_max = warp_max(rho_sf);
+    for (uint32_t base = 0; base < m; base += 32) {
+      const uint32_t i = base + lane;
+      const float4 mine = i < m ? rel[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (0.5f * (1.0f - 1e-5f) > rho_max * __shfl_sync(0xffffffffu, mine.w, 0)) break;
+      const uint32_t seen = *(volatile uint32_t*)&mark[base >> 5];
+      const bool some = i < m && !(seen >> lane & 1u) && !(0.5f * (1.0f - 1e-5f) > rho_max * mine.w) &&
+                        2.0f * cos_low(grp.cos_max(mine), cdf, sdlf) * rho_max * mine.w * (1.0f + 3e-5f) >= 1.0f;
+      uint32_t found = 0;
+      for (uint32_t todo_pts = __ballot_sync(0xffffffffu, some); todo_pts; todo_pts &= todo_pts - 1) {
+        const int q = __ffs((int)todo_pts) - 1;
+        const float4 r = rel[base + q];
         bool f = false;
-        if (!stop) {
-          const float c = u0 * r.x + u1 * r.y + u2 * r.z;
-          const float cs = fminf(1.0f, c + 1e-5f);  // cosine of a lower bound of the angle
-          const float sn = sqrtf(fmaxf(0.0f, (1.0f - cs) * (1.0f + cs)));
-          const float clo = (cs >= cdf) ? 1.0f : cs * cdf + sn * sdlf + 1e-6f;  // upper bound of cos(max(angle - delta, 0))
+        if (!(0.5f * (1.0f - 1e-5f) > rho_sf * r.w)) {
+          const float clo = cos_low(u0 * r.x + u1 * r.y + u2 * r.z, cdf, sdlf);
           f = clo > 0.0f && 2.0f * clo * rho_sf * r.w * (1.0f + 2e-5f) >= 1.0f;
         }
-        const uint32_t bits = __ballot_sync(0xffffffffu, f);
-        if (lane == 0 && bits) atomicOr(&mark[base >> 5], bits);
+        if (__any_sync(0xffffffffu, f)) found |= 1u << q;
       }
+      if (lane == 0 && found) atomicOr(&mark[base >> 5], found);
     }
-    if (lane < nd) rho_tab[(uint64_t)a * kDirs + dl] = my_rho;
   }
   for (int off = 16; off > 0; off >>= 1) worst_needed = fmax(worst_needed, __shfl_xor_sync(0xffffffffu, worst_needed, off));
   if (lane == 0) worst_w[warp] = worst_needed;
@@ -585,56 +639,79 @@ k_dirtable(uint32_t n, uint32_t list_cap, CertParams cp, const uint32_t* __restr
 // Owners whose gather radius holds more than kMaxNb points (edges of dense clusters whose
 // bounds reach into a sparse background, points near the hull) take this path, with the
 // same certificate: their neighbour lists are counted, allocated in one arena and written
-// (one thread per owner, depth first, whole subtrees inside the radius taken as ranges); a
+// (one warp per owner, whole subtrees inside the radius taken as ranges); a
 // block per owner then stages its list in chunks and keeps, per direction, the `need` largest
 // lower bounds of 1 / rho_shr with every neighbour seen (the list is not sorted, so there is
 // no early exit), marks the candidates and writes C(a) sorted by binary32 distance.
-constexpr int kBigStack = 128;    // traversal stack: the LBVH is at most 63 + log2(n) + 1 deep
-constexpr int kBigThreads = 256;  // one block of eight warps per large owner
+constexpr int kBigStack = 512;    // warp traversal stack
+constexpr uint32_t kBigWide = kBigStack - 64 - 128;  // the LBVH is at most 63 + log2(n) + 1 deep
+constexpr int kBigThreads = 672;  // one block of 21 warps per large owner, one direction per thread
 constexpr int kBigChunk = 2048;   // neighbours staged per step
 
+// One warp per owner, 32 nodes of a shared stack per step, one per lane; whole subtrees inside the
+// radius are copied by the warp.  Above kBigWide entries one node is taken per step (depth first), so
+// the stack stays within kBigStack.  off == nullptr: the pass only counts.
+// 8,009 clustered points, K = 10 (three rounds of a count and a write): 5.3 ms with one node per step.
 __global__ void __launch_bounds__(128)
 k_gather_big(uint32_t nbig, const uint32_t* __restrict__ big, uint32_t root, const TNode* __restrict__ tn,
              const uint32_t* __restrict__ leaf_pid, const uint32_t* __restrict__ n_begin,
              const uint32_t* __restrict__ n_end, const double* __restrict__ px, const double* __restrict__ py,
              const double* __restrict__ pz, const double* __restrict__ gather_r2, const uint64_t* __restrict__ off,
              uint32_t* __restrict__ arena, uint32_t* __restrict__ cnt, uint32_t* __restrict__ err) {
-  // one warp per owner: every lane takes the same walk (warp-uniform branches, broadcast loads);
-  // lane 0 appends single leaves, and a whole subtree inside the radius is copied by the 32
-  // lanes; the list keeps the order of one thread's walk
+  __shared__ uint32_t stacks[4][kBigStack];
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
   if (i >= nbig) return;
+  uint32_t* stack = stacks[threadIdx.x >> 5];
   const uint32_t a = big[i];
   const double ax = px[a], ay = py[a], az = pz[a];
   const double R2 = gather_r2[a] * (1.0 + 32.0 * kU);
   const uint64_t cap = arena ? off[i + 1] - off[i] : 0;
   uint32_t* out = arena ? arena + off[i] : nullptr;
   uint64_t c = 0;
-  uint32_t stack[kBigStack];
-  int top = 0;
-  stack[top++] = root;
+  uint32_t top = 1;
+  if (lane == 0) stack[0] = root;
+  __syncwarp();
   while (top > 0) {
-    const uint32_t node = stack[--top];
-    const TNode t = load_node(tn, node);
-    if (t.left == kInvalid32) {
-      const uint32_t pid = t.right;
-      const double dx = px[pid] - ax, dy = py[pid] - ay, dz = pz[pid] - az;
-      if (pid != a && dx * dx + dy * dy + dz * dz <= R2) {
-        if (lane == 0 && c < cap) out[c] = pid;
-        ++c;
+    const uint32_t batch = top > kBigWide ? 1u : min(top, 32u);
+    uint32_t node = kInvalid32;
+    if (lane < batch) node = stack[top - 1 - lane];
+    __syncwarp();
+    top -= batch;
+    bool take = false, expand = false;
+    uint32_t bb = 0, be = 0;
+    TNode t;
+    if (node != kInvalid32) {
+      t = load_node(tn, node);
+      if (t.left == kInvalid32) {
+        const double dx = px[t.right] - ax, dy = py[t.right] - ay, dz = pz[t.right] - az;
+        take = t.right != a && dx * dx + dy * dy + dz * dz <= R2;
+      } else {
+        const double lx = fmax(fmax((double)t.lo[0] - ax, ax - (double)t.hi[0]), 0.0);
+        const double ly = fmax(fmax((double)t.lo[1] - ay, ay - (double)t.hi[1]), 0.0);
+        const double lz = fmax(fmax((double)t.lo[2] - az, az - (double)t.hi[2]), 0.0);
+        if (!((lx * lx + ly * ly + lz * lz) * (1.0 - 16.0 * kU) > R2)) {
+          const double ux = fmax(fabs((double)t.lo[0] - ax), fabs((double)t.hi[0] - ax));
+          const double uy = fmax(fabs((double)t.lo[1] - ay), fabs((double)t.hi[1] - ay));
+          const double uz = fmax(fabs((double)t.lo[2] - az), fabs((double)t.hi[2] - az));
+          if ((ux * ux + uy * uy + uz * uz) * (1.0 + 16.0 * kU) < R2) {  // the whole subtree is inside
+            bb = n_begin[node];
+            be = n_end[node];
+          } else {
+            expand = true;
+          }
+        }
       }
-      continue;
     }
-    const double lx = fmax(fmax((double)t.lo[0] - ax, ax - (double)t.hi[0]), 0.0);
-    const double ly = fmax(fmax((double)t.lo[1] - ay, ay - (double)t.hi[1]), 0.0);
-    const double lz = fmax(fmax((double)t.lo[2] - az, az - (double)t.hi[2]), 0.0);
-    if ((lx * lx + ly * ly + lz * lz) * (1.0 - 16.0 * kU) > R2) continue;
-    const double ux = fmax(fabs((double)t.lo[0] - ax), fabs((double)t.hi[0] - ax));
-    const double uy = fmax(fabs((double)t.lo[1] - ay), fabs((double)t.hi[1] - ay));
-    const double uz = fmax(fabs((double)t.lo[2] - az), fabs((double)t.hi[2] - az));
-    if ((ux * ux + uy * uy + uz * uz) * (1.0 + 16.0 * kU) < R2) {  // the whole subtree is inside
-      const uint32_t q_hi = n_end[node];
-      for (uint32_t q0 = n_begin[node]; q0 < q_hi; q0 += 32) {
+    const uint32_t tb = __ballot_sync(0xffffffffu, take), eb = __ballot_sync(0xffffffffu, expand);
+    if (take) {
+      const uint64_t pos = c + __popc(tb & lanemask_lt());
+      if (pos < cap) out[pos] = t.right;
+    }
+    c += __popc(tb);
+    for (uint32_t rb = __ballot_sync(0xffffffffu, be > bb); rb; rb &= rb - 1) {  // ranges, one after another
+      const int src = __ffs((int)rb) - 1;
+      const uint32_t q_lo = __shfl_sync(0xffffffffu, bb, src), q_hi = __shfl_sync(0xffffffffu, be, src);
+      for (uint32_t q0 = q_lo; q0 < q_hi; q0 += 32) {
         const uint32_t q = q0 + lane;
         const uint32_t pid = q < q_hi ? leaf_pid[q] : kInvalid32;
         const bool keep = q < q_hi && pid != a;
@@ -643,14 +720,18 @@ k_gather_big(uint32_t nbig, const uint32_t* __restrict__ big, uint32_t root, con
         if (keep && pos < cap) out[pos] = pid;
         c += __popc(bal);
       }
-      continue;
     }
-    if (top + 2 > kBigStack) {
+    if (expand) {
+      const uint32_t at = top + 2 * __popc(eb & lanemask_lt());
+      stack[at] = t.right;
+      stack[at + 1] = t.left;
+    }
+    top += 2 * __popc(eb);
+    if (top + 64 > (uint32_t)kBigStack) {  // deeper than an LBVH can be
       if (lane == 0) atomicOr(err, kErrCapacity);
       return;
     }
-    stack[top++] = t.right;
-    stack[top++] = t.left;
+    __syncwarp();
   }
   if (lane != 0) return;
   if (!arena) cnt[i] = (uint32_t)c;
@@ -658,8 +739,8 @@ k_gather_big(uint32_t nbig, const uint32_t* __restrict__ big, uint32_t root, con
 }
 
 // Dynamic shared memory of k_dirtable_big.
-constexpr size_t kBigSmem = (size_t)kBigChunk * 16 + (size_t)kDirs * kMaxNeed * 4 + (size_t)kDirs * 4 + 16 +
-                            (size_t)kDirs * 8 + (size_t)kMaxCand * 8;
+constexpr size_t kBigSmem = (size_t)kBigChunk * 16 + (size_t)kMaxCand * 8;
+static_assert(kBigThreads >= kDirs && kBigThreads <= 32 * 32, "one direction per thread");
 
 __global__ void __launch_bounds__(kBigThreads)
 k_dirtable_big(uint32_t nbig, CertParams cp, const uint32_t* __restrict__ big, const uint64_t* __restrict__ off,
@@ -669,14 +750,10 @@ k_dirtable_big(uint32_t nbig, CertParams cp, const uint32_t* __restrict__ big, c
                float* __restrict__ rho_tab) {
   extern __shared__ __align__(16) unsigned char smem[];
   float4* rel = reinterpret_cast<float4*>(smem);               // [kBigChunk] unit direction, 1 / |p - a|
-  float* topt = reinterpret_cast<float*>(rel + kBigChunk);     // [kDirs][kMaxNeed] descending
-  float* rho = topt + kDirs * kMaxNeed;                        // [kDirs] certified per-cone bounds
-  double* ext = reinterpret_cast<double*>(reinterpret_cast<uintptr_t>(rho + kDirs + 3) & ~uintptr_t(7));  // [kDirs]
-  uint32_t* cid = reinterpret_cast<uint32_t*>(ext + kDirs);    // [kMaxCand]
+  uint32_t* cid = reinterpret_cast<uint32_t*>(rel + kBigChunk);  // [kMaxCand]
   float* cds = reinterpret_cast<float*>(cid + kMaxCand);       // [kMaxCand] binary32 |p - a|
   __shared__ double s_worst[kBigThreads / 32];
-  __shared__ float s_rmax[kBigThreads / 32];
-  __shared__ uint32_t s_c;
+  __shared__ uint32_t s_c, mark[kBigChunk / 32];
   const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31u;
   if (blockIdx.x >= nbig) return;
   const uint32_t a = big[blockIdx.x];
@@ -688,18 +765,30 @@ k_dirtable_big(uint32_t nbig, CertParams cp, const uint32_t* __restrict__ big, c
   const double cd = cos(cp.delta), sdl = sin(cp.delta);
   const float cdf = (float)cd, sdlf = (float)sdl;
   const uint32_t need = cp.need;
-  for (uint32_t d = t; d < (uint32_t)kDirs; d += kBigThreads) {
-    const double s0 = cp.dirs[3 * d], s1 = cp.dirs[3 * d + 1], s2 = cp.dirs[3 * d + 2];
+  // one direction per thread, its `need` largest bounds in registers over the whole list (which is not
+  // sorted, so every point is looked at; one behind the 32 cones of a warp costs its dot product)
+  const bool on = t < (uint32_t)kDirs;
+  float u0 = 0.f, u1 = 0.f, u2 = 0.f;
+  double ext = 0.0;
+  if (on) {
+    const double s0 = cp.dirs[3 * t], s1 = cp.dirs[3 * t + 1], s2 = cp.dirs[3 * t + 2];
+    u0 = (float)s0;
+    u1 = (float)s1;
+    u2 = (float)s2;
     const double e = cone_ext(cp, s0, ax, 0) + cone_ext(cp, s1, ay, 1) + cone_ext(cp, s2, az, 2);
     const double exit_r = fmin(fmin(cone_exit(cp, s0, ax, 0), cone_exit(cp, s1, ay, 1)), cone_exit(cp, s2, az, 2));
-    ext[d] = fmin(e * (1.0 + 1e-12), exit_r);
-    for (uint32_t j = 0; j < (uint32_t)kMaxNeed; ++j) topt[d * kMaxNeed + j] = 0.0f;
+    ext = fmin(e * (1.0 + 1e-12), exit_r);
   }
+  const float inv_ext = on ? 1.0f / __double2float_ru(ext) : INFINITY;
+  ConeGroup grp;
+  grp.init(u0, u1, u2, on);
+  TopInv top;
+  top.init(on ? need : 0u);
+  float lim = 0.5f * (1.0f - 1e-5f) * inv_ext;
   if (t == 0) s_c = 0;
-  __syncthreads();
-  // 1. per cone, the `need` largest lower bounds of 1 / rho_shr over the whole list
-  for (uint64_t base = 0; base < m; base += kBigChunk) {
-    const uint32_t cnt = (uint32_t)min((uint64_t)kBigChunk, m - base);
+  // stages the points base .. base + cnt - 1 of the list: unit direction, 1 / |p - a|
+  auto stage = [&](uint64_t base, uint32_t cnt) {
+    __syncthreads();
     for (uint32_t j = t; j < cnt; j += kBigThreads) {
       const uint32_t p = list[base + j];
       const double x = px[p] - ax, y = py[p] - ay, z = pz[p] - az;
@@ -709,90 +798,84 @@ k_dirtable_big(uint32_t nbig, CertParams cp, const uint32_t* __restrict__ big, c
       rel[j] = make_float4((float)(x * inv), (float)(y * inv), (float)(z * inv), 1.0f / df);
     }
     __syncthreads();
-    for (uint32_t d = warp; d < (uint32_t)kDirs; d += kBigThreads / 32) {
-      const float u0 = cp.dirs[3 * d], u1 = cp.dirs[3 * d + 1], u2 = cp.dirs[3 * d + 2];
-      const float inv_ext = 1.0f / __double2float_ru(ext[d]);
-      float top = lane < need ? topt[d * kMaxNeed + lane] : 0.0f;
-      float thr = __shfl_sync(0xffffffffu, top, need - 1);
-      for (uint32_t sb = 0; sb < cnt; sb += 32) {
-        const uint32_t j = sb + lane;
-        const float lim = 0.5f * (1.0f - 1e-5f) * fmaxf(thr, inv_ext);
-        const float4 r = j < cnt ? rel[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        float inv = 0.0f;
-        if (j < cnt && !(lim > r.w)) {
-          const float c = u0 * r.x + u1 * r.y + u2 * r.z;
-          const float cs = fmaxf(-1.0f, c - 1e-5f);
-          const float sn = sqrtf(fmaxf(0.0f, (1.0f - cs) * (1.0f + cs)));
-          const float cshr = cs * cdf - sn * sdlf - 1e-6f;
-          if (cshr > 1e-6f) inv = 2.0f * cshr * r.w * (1.0f - 1e-5f);
-        }
-        if (__any_sync(0xffffffffu, inv > thr)) {
-          top = warp_top_merge(top, inv, lane);
-          thr = __shfl_sync(0xffffffffu, top, need - 1);
+  };
+  // 1. per cone, the `need` largest lower bounds of 1 / rho_shr over the whole list
+  for (uint64_t base = 0; base < m; base += kBigChunk) {
+    const uint32_t cnt = (uint32_t)min((uint64_t)kBigChunk, m - base);
+    stage(base, cnt);
+    for (uint32_t sb = 0; sb < cnt; sb += 32) {
+      const uint32_t j = sb + lane;
+      const float4 mine = j < cnt ? rel[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float lim_min = warp_min(lim), thr_min = warp_min(top.thr());
+      const bool some = j < cnt && !(lim_min > mine.w) && inv_rho_best(grp.cos_max(mine) + 2e-5f, mine.w, cdf) > thr_min;
+      for (uint32_t todo_pts = __ballot_sync(0xffffffffu, some); todo_pts; todo_pts &= todo_pts - 1) {
+        const float4 r = rel[sb + __ffs((int)todo_pts) - 1];
+        const float c = u0 * r.x + u1 * r.y + u2 * r.z;
+        if (!(lim > r.w) && inv_rho_best(c, r.w, cdf) > top.thr()) {
+          const float inv = inv_rho(c, r.w, cdf, sdlf);
+          if (inv > top.thr()) {
+            top.add(inv);
+            lim = 0.5f * (1.0f - 1e-5f) * fmaxf(top.thr(), inv_ext);
+          }
         }
       }
-      if (lane < need) topt[d * kMaxNeed + lane] = top;
     }
-    __syncthreads();
   }
   // certified per-cone bounds (same rule as the list path)
   double worst = 0.0;
-  float rmax = 0.0f;
+  float rho_sf = 0.0f;
   bool ok = true;
-  for (uint32_t d = t; d < (uint32_t)kDirs; d += kBigThreads) {
-    const float thr = topt[d * kMaxNeed + need - 1];
-    const double kth = thr > 0.0f ? (1.0 / (double)thr) * (1.0 + 1e-12) : INFINITY;
-    const double rho_s = fmin(kth, ext[d]);
-    const float rho_sf = __double2float_ru(rho_s);
-    rho[d] = rho_sf;
-    rho_tab[(uint64_t)a * kDirs + d] = rho_sf;
+  if (on) {
+    const double kth = top.thr() > 0.0f ? (1.0 / (double)top.thr()) * (1.0 + 1e-12) : INFINITY;
+    const double rho_s = fmin(kth, ext);
+    rho_sf = __double2float_ru(rho_s);
+    rho_tab[(uint64_t)a * kDirs + t] = rho_sf;
     if (!(rho_s <= half_L)) ok = false;
-    worst = fmax(worst, rho_s);
-    rmax = fmaxf(rmax, rho_sf);
+    worst = rho_s;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    worst = fmax(worst, __shfl_xor_sync(0xffffffffu, worst, o));
-    rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-  }
-  if (lane == 0) {
-    s_worst[warp] = worst;
-    s_rmax[warp] = rmax;
-  }
+  for (int o = 16; o > 0; o >>= 1) worst = fmax(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+  if (lane == 0) s_worst[warp] = worst;
   ok = __syncthreads_and(ok);
-  for (int w = 0; w < kBigThreads / 32; ++w) {
-    worst = fmax(worst, s_worst[w]);
-    rmax = fmaxf(rmax, s_rmax[w]);
-  }
+  for (int w = 0; w < kBigThreads / 32; ++w) worst = fmax(worst, s_worst[w]);
   if (!ok) {  // the list must grow to 2 rho_s (with room); the owner stays on this path
     if (t == 0) need_r[a] = worst;
     return;
   }
-  // 2. candidates: rho_lo_p(s) <= rho_s for some cone s
-  for (uint64_t j = t; j < m; j += kBigThreads) {
-    const uint32_t p = list[j];
-    const double x = px[p] - ax, y = py[p] - ay, z = pz[p] - az;
-    const double dd = sqrt(x * x + y * y + z * z);
-    const double inv = dd > 0.0 ? 1.0 / dd : 0.0;
-    const float df = (float)dd;
-    const float rw = 1.0f / df;
-    if (0.5f * (1.0f - 1e-5f) > rmax * rw) continue;  // beyond 2 rho_s of every cone
-    const float r0 = (float)(x * inv), r1 = (float)(y * inv), r2 = (float)(z * inv);
-    bool f = false;
-    for (uint32_t d = 0; d < (uint32_t)kDirs && !f; ++d) {
-      const float rho_sf = rho[d];
-      if (0.5f * (1.0f - 1e-5f) > rho_sf * rw) continue;
-      const float c = cp.dirs[3 * d] * r0 + cp.dirs[3 * d + 1] * r1 + cp.dirs[3 * d + 2] * r2;
-      const float cs = fminf(1.0f, c + 1e-5f);
-      const float sn = sqrtf(fmaxf(0.0f, (1.0f - cs) * (1.0f + cs)));
-      const float clo = (cs >= cdf) ? 1.0f : cs * cdf + sn * sdlf + 1e-6f;
-      f = clo > 0.0f && 2.0f * clo * rho_sf * rw * (1.0f + 2e-5f) >= 1.0f;
-    }
-    if (f) {
-      const uint32_t at = atomicAdd(&s_c, 1u);
-      if (at < (uint32_t)kMaxCand) {
-        cid[at] = p;
-        cds[at] = df;
+  // 2. candidates: rho_lo_p(s) <= rho_s for some cone s (each warp its 32 cones)
+  const float rho_max = warp_max(rho_sf);
+  for (uint64_t base = 0; base < m; base += kBigChunk) {
+    const uint32_t cnt = (uint32_t)min((uint64_t)kBigChunk, m - base);
+    __syncthreads();  // the marks of the chunk before have been read
+    for (uint32_t w = t; w < (uint32_t)kBigChunk / 32; w += kBigThreads) mark[w] = 0;
+    stage(base, cnt);
+    for (uint32_t sb = 0; sb < cnt; sb += 32) {
+      const uint32_t j = sb + lane;
+      const float4 mine = j < cnt ? rel[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const uint32_t seen = *(volatile uint32_t*)&mark[sb >> 5];
+      const bool some = j < cnt && !(seen >> lane & 1u) && !(0.5f * (1.0f - 1e-5f) > rho_max * mine.w) &&
+                        2.0f * cos_low(grp.cos_max(mine), cdf, sdlf) * rho_max * mine.w * (1.0f + 3e-5f) >= 1.0f;
+      uint32_t found = 0;
+      for (uint32_t todo_pts = __ballot_sync(0xffffffffu, some); todo_pts; todo_pts &= todo_pts - 1) {
+        const int q = __ffs((int)todo_pts) - 1;
+        const float4 r = rel[sb + q];
+        bool f = false;
+        if (!(0.5f * (1.0f - 1e-5f) > rho_sf * r.w)) {
+          const float clo = cos_low(u0 * r.x + u1 * r.y + u2 * r.z, cdf, sdlf);
+          f = clo > 0.0f && 2.0f * clo * rho_sf * r.w * (1.0f + 2e-5f) >= 1.0f;
+        }
+        if (__any_sync(0xffffffffu, f)) found |= 1u << q;
       }
+      if (lane == 0 && found) atomicOr(&mark[sb >> 5], found);
+    }
+    __syncthreads();
+    for (uint32_t j = t; j < cnt; j += kBigThreads) {
+      if (!(mark[j >> 5] >> (j & 31) & 1u)) continue;
+      const uint32_t at = atomicAdd(&s_c, 1u);
+      if (at >= (uint32_t)kMaxCand) continue;
+      const uint32_t p = list[base + j];
+      const double x = px[p] - ax, y = py[p] - ay, z = pz[p] - az;
+      cid[at] = p;
+      cds[at] = (float)sqrt(x * x + y * y + z * z);
     }
   }
   __syncthreads();
@@ -1640,6 +1723,29 @@ void icosphere(std::vector<float>& dirs, double& delta) {
     }
   }
   delta *= 1.05;  // margin for the binary32 rounding of the stored directions
+  // Groups of 32 neighbouring directions (one per warp step of the direction tables): halves along
+  // the widest axis, cut at multiples of 32.
+  std::function<void(size_t, size_t)> split = [&](size_t lo, size_t hi) {
+    if (hi - lo <= 32) return;
+    int axis = 0;
+    double widest = -1;
+    for (int k = 0; k < 3; ++k) {
+      double mn = 2, mx = -2;
+      for (size_t i = lo; i < hi; ++i) {
+        mn = std::min(mn, v[i][k]);
+        mx = std::max(mx, v[i][k]);
+      }
+      if (mx - mn > widest) {
+        widest = mx - mn;
+        axis = k;
+      }
+    }
+    const size_t mid = lo + ((hi - lo + 31) / 32 + 1) / 2 * 32;
+    std::sort(v.begin() + lo, v.begin() + hi, [axis](const auto& x, const auto& y) { return x[axis] < y[axis]; });
+    split(lo, mid);
+    split(mid, hi);
+  };
+  split(0, v.size());
   dirs.clear();
   for (auto& p : v)
     for (int k = 0; k < 3; ++k) dirs.push_back((float)p[k]);
