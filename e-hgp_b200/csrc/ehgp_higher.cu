@@ -97,15 +97,12 @@ struct SetPt {
 
 __device__ __forceinline__ double ptmax(const SetPt& p) { return fmax(fabs(p.x), fmax(fabs(p.y), fabs(p.z))); }
 
-// A minimal support waiting for classification: side(w) = sgn * sign(A q - p.N)
-// with p = fl(w - a), q = fl(|p|^2); the FP value is decided outside +-bnd.
-struct QEntry {
+// Circumsphere of a minimal support: side(w) = sgn * sign(A q - p.N) with p = fl(w - a),
+// q = fl(|p|^2); the FP value is decided outside +-bnd.
+struct Sphere {
   double A, Nx, Ny, Nz, bnd;
-  uint32_t ids[4];  // ids[0] = owner a; ids[3] = kInvalid32 for a triangle
-  int16_t size, sgn;
-  float cut;  // candidates (sorted by distance from a) with |p - a|^2 above cut lie outside
+  int size, sgn;
 };
-static_assert(sizeof(QEntry) == 64, "queue entries are 64 bytes");
 
 // The exact fallbacks take their ids by value and return the signs packed two bits each
 // (sign + 1), so that no array of the hot path needs an address (and local memory).
@@ -125,15 +122,22 @@ __device__ __noinline__ uint32_t quad_signs_packed(Cloud c, uint32_t i0, uint32_
   for (int k = 0; k < 5; ++k) r |= (uint32_t)(sg[k] + 1) << (2 * k);
   return r;
 }
+__device__ __noinline__ int side_exact_ids(Cloud c, uint32_t i0, uint32_t i1, uint32_t i2, uint32_t i3, int size, uint32_t w) {
+  const uint32_t id[4] = {i0, i1, i2, i3};
+  return side_exact(c, id, size, w);
+}
 __device__ __forceinline__ int packed_sign(uint32_t p, int k) { return (int)((p >> (2 * k)) & 3u) - 1; }
 
 // Triangle (a, a + e1, a + e2): minimal iff its three angles are acute.
-// Returns 0 minimal (E filled), 1 boundary reduced, 2 obtuse, 3 collinear; *adm is
+// Returns 0 minimal (E filled), 1 boundary reduced, 2 obtuse, 3 collinear, and without kExact 4 when
+// binary64 does not decide (the loops that every support runs through make no call: what
+// lives across a call goes to local memory and back); *adm is
 // false when the circumradius certainly exceeds rmax (no relevant tetrahedron
 // has this face: its circumsphere contains the face's circumcircle).
-__device__ int tri_eval(const Cloud& c, const SetPt& e1, const SetPt& e2, uint32_t i0, uint32_t i1, uint32_t i2,
+template <bool kExact>
+__device__ __forceinline__ int tri_eval(const Cloud& c, const SetPt& e1, const SetPt& e2, uint32_t i0, uint32_t i1, uint32_t i2,
                         double Mp, double rmax2,
-                        QEntry& E, double& eA, double& eN, bool& adm) {
+                        Sphere& E, double& eA, double& eN, bool& adm) {
   const double M = fmax(ptmax(e1), ptmax(e2)) * (1.0 + 1e-15), M2 = M * M;
   const double G11 = e1.q, G22 = e2.q, G12 = (e1.x * e2.x + e1.y * e2.y) + e1.z * e2.z;
   const double db = G11 - G12, dc = G22 - G12;
@@ -141,6 +145,7 @@ __device__ int tri_eval(const Cloud& c, const SetPt& e1, const SetPt& e2, uint32
   const double bG = kFilt * 3.0 * M2 + kTiny, bD = kFilt * 6.0 * M2 + kTiny, b4 = kFilt * 18.0 * M2 * M2 + kTiny;
   int sg0 = fsign(G12, bG), sg1 = fsign(db, bD), sg2 = fsign(dc, bD), sg3 = fsign(detG, b4);
   if (sg0 == 2 || sg1 == 2 || sg2 == 2 || sg3 == 2) {
+    if (!kExact) return 4;
     const uint32_t pk = tri_signs_packed(c, i0, i1, i2);
     sg0 = packed_sign(pk, 0);
     sg1 = packed_sign(pk, 1);
@@ -174,10 +179,11 @@ __device__ int tri_eval(const Cloud& c, const SetPt& e1, const SetPt& e2, uint32
 }
 
 // Tetrahedron (a, a + e1, a + e2, a + e3): minimal iff the four barycentric
-// coordinates l_i / (2 detE^2) of its circumcentre are positive.
-__device__ int quad_eval(const Cloud& c, const SetPt& e1, const SetPt& e2, const SetPt& e3, uint32_t i0, uint32_t i1,
+// coordinates l_i / (2 detE^2) of its circumcentre are positive.  Returns as tri_eval.
+template <bool kExact>
+__device__ __forceinline__ int quad_eval(const Cloud& c, const SetPt& e1, const SetPt& e2, const SetPt& e3, uint32_t i0, uint32_t i1,
                          uint32_t i2, uint32_t i3,
-                         double Mp, QEntry& E, double& eA, double& eN) {
+                         double Mp, Sphere& E, double& eA, double& eN) {
   const double M = fmax(fmax(ptmax(e1), ptmax(e2)), ptmax(e3)) * (1.0 + 1e-15), M2 = M * M, M3 = M2 * M;
   const double c23x = e2.y * e3.z - e2.z * e3.y, c23y = e2.z * e3.x - e2.x * e3.z, c23z = e2.x * e3.y - e2.y * e3.x;
   const double c31x = e3.y * e1.z - e3.z * e1.y, c31y = e3.z * e1.x - e3.x * e1.z, c31z = e3.x * e1.y - e3.y * e1.x;
@@ -194,6 +200,7 @@ __device__ int quad_eval(const Cloud& c, const SetPt& e1, const SetPt& e2, const
   const double bE = kFilt * 6.0 * M3 + kTiny, bl = kFilt * 108.0 * M6 + kTiny, b0 = kFilt * 396.0 * M6 + kTiny;
   int sg0 = fsign(detE, bE), sg1 = fsign(l0, b0), sg2 = fsign(l1, bl), sg3 = fsign(l2, bl), sg4 = fsign(l3, bl);
   if (sg0 == 2 || sg1 == 2 || sg2 == 2 || sg3 == 2 || sg4 == 2) {
+    if (!kExact) return 4;
     const uint32_t pk = quad_signs_packed(c, i0, i1, i2, i3);
     sg0 = packed_sign(pk, 0);
     sg1 = packed_sign(pk, 1);
@@ -1045,14 +1052,20 @@ k_cand_large(uint32_t nown, const uint32_t* __restrict__ owners, const uint32_t*
 }
 
 // ---- 3. owner-local enumeration ---------------------------------------------------------
-// One warp per owner a.  C(a) is staged in shared memory as rounded differences
-// p - a; the support candidates are C(a) with ids > a.  Lanes test triangles
-// (pairs j < k) and tetrahedra (triples j < k < l, load-balanced over the pairs
-// whose three a-faces pass the circumradius bound) for minimality; a minimal
-// support whose circumradius certainly exceeds the radius bound of the cone
-// holding its centre direction is dropped, the others are classified against
-// C(a) by the whole warp, 32 points per step, with ballot counts and an early
-// exit once the interior exceeds s_max - size.
+// One block per owner a (or per chunk of a large owner's pairs).  C(a) is staged in shared memory as
+// rounded differences p - a; the support candidates are C(a) with ids > a.  Lanes test triangles
+// (pairs j < k, binary64) and tetrahedra (triples j < k < l whose three a-faces pass the
+// circumradius bound, binary32) and queue what they cannot reject; full warps then decide the queued
+// supports in binary64, drop those whose circumradius certainly exceeds the radius bound of the
+// cone holding their centre direction, and classify the rest against C(a), one support per lane.
+// What binary64 does not decide goes to a queue of its own, and from there to the exact integers.
+// No loop that every support runs through makes a call: with the exact fallbacks called inside the
+// loops, what lived across the calls was written to local memory and read back on every turn (1.2 G
+// local loads and 0.5 G stores of 8.1 G instructions at 12,289 uniform points; 33 M and 10 M of 3.4 G
+// now).  Bound: instruction issue (69 % of the slots, FP64 pipe 20 %).
+// k_higher, 50,653 lattice points, K = 10: 60.1 ms with a warp per support in binary64, 51.3 with a
+// support per lane, 37.7 with the binary32 test, 15.0 without calls in the loops; 12,289 uniform
+// points 16.0 -> 4.3 ms.
 struct HigherRec {
   uint32_t size;
   uint32_t ids[4];
@@ -1074,8 +1087,7 @@ struct Ctl {
 #endif
 // warps per owner block in k_higher (they share its staged candidate set), and the blocks per
 // SM its register budget is sized for: 65536 / (256 threads x 4 blocks) = 64 per thread, 32 warps
-// per SM (measured at 50k: 8 x 4 blocks 60.1 ms, 8 x 3 63.5, 8 x 2 81.4; earlier builds 4 x 4
-// 83, 4 x 5 82, 12 x 2 83, 8 x 3 77)
+// per SM (50,653 lattice points, K = 10: 15.0 ms at 4 blocks, 15.3 at 3, 18.3 at 2)
 constexpr int kHOwnerWarps = EHGP_HIGHER_OWNER_WARPS;
 constexpr int kHBlocksPerSM = EHGP_HIGHER_BLOCKS_PER_SM;
 constexpr int kCube = 32;       // cube-map cells per face edge for centre directions
@@ -1085,161 +1097,339 @@ struct HigherTables {
   const float* dirs;       // [kDirs * 3]
   const uint16_t* cells;   // [6 * kCube * kCube * kCellDirs]
   const float* rho;        // [n * kDirs] per-cone radius bounds, by PointId
-  double cos_lim;          // cos(delta) raised by a margin: inside the cone for sure
+  float cos_lim;           // cos(delta) raised by a margin: inside the cone for sure
 };
 
 template <int KC>
 struct OwnerSmemT {  // one owner's staged candidate set (at most KC), shared by the block's warps
-  uint32_t sid[KC];
   SetPt spt[KC];
+  float4 fpt[KC];    // support candidates: p - a and |p - a|^2 in binary32, scaled (see quad_outside)
   uint16_t supi[KC];
   float rho[kDirs];
 };
 // The face mask sits beside it: adm[j * (KC / 32) + w] bit k (j < k): face (a, j, k) within the bound.
 using OwnerSmem = OwnerSmemT<kMaxCand>;
 
-struct WarpQueue {  // one warp's queued supports
-  uint32_t iids[kMaxInteriorH];
-  QEntry q[32];
+// One warp's queues of supports: positions j < k < l among the support candidates (l = kNoPoint for a
+// triangle).  `found` holds those that the enumeration could not reject, `hard` those that binary64
+// does not decide, `kept` the minimal ones whose cone bound does not exclude them.  Each is worked
+// off 32 at a time, so that the steps that few supports reach run with full warps.
+constexpr uint16_t kNoPoint = 0xffffu;
+struct WarpQueue {
+  ushort4 found[64], hard[64], kept[64];
 };
 
-__device__ __forceinline__ int cube_cell(double ux, double uy, double uz) {
-  const double ax = fabs(ux), ay = fabs(uy), az = fabs(uz);
+__device__ __forceinline__ int cube_cell(float ux, float uy, float uz) {
+  const float ax = fabsf(ux), ay = fabsf(uy), az = fabsf(uz);
   int face;
-  double s, t;
+  float s, t;
   if (ax >= ay && ax >= az) {
-    face = ux > 0 ? 0 : 1; s = uy / ax; t = uz / ax;
+    const float inv = __fdividef(1.0f, ax);
+    face = ux > 0 ? 0 : 1; s = uy * inv; t = uz * inv;
   } else if (ay >= az) {
-    face = uy > 0 ? 2 : 3; s = ux / ay; t = uz / ay;
+    const float inv = __fdividef(1.0f, ay);
+    face = uy > 0 ? 2 : 3; s = ux * inv; t = uz * inv;
   } else {
-    face = uz > 0 ? 4 : 5; s = ux / az; t = uy / az;
+    const float inv = __fdividef(1.0f, az);
+    face = uz > 0 ? 4 : 5; s = ux * inv; t = uy * inv;
   }
-  const int i = min(kCube - 1, max(0, (int)floor((s + 1.0) * 0.5 * kCube)));
-  const int j = min(kCube - 1, max(0, (int)floor((t + 1.0) * 0.5 * kCube)));
+  const int i = min(kCube - 1, max(0, (int)floorf((s + 1.0f) * 0.5f * kCube)));
+  const int j = min(kCube - 1, max(0, (int)floorf((t + 1.0f) * 0.5f * kCube)));
   return (face * kCube + i) * kCube + j;
 }
 
 // True when the sphere's circumradius certainly exceeds the bound of a cone
-// that certainly holds its centre direction: no relevant support.
-__device__ bool cone_rejects(const QEntry& E, double eA, double eN, const float* rho, const HigherTables& tb) {
+// that certainly holds its centre direction: no relevant support.  The direction and its cosines
+// are binary32 (errors below 1e-6, which cos_lim's margin of 4e-6 covers; a cell off by one lists
+// other cones, each of which is checked); the radius is binary64.
+__device__ bool cone_rejects(const Sphere& E, double eA, double eN, const float* rho, const HigherTables& tb) {
   const double nn = sqrt(E.Nx * E.Nx + E.Ny * E.Ny + E.Nz * E.Nz);
   const double en = eN * 1.7320508075688772;
   if (!(en <= 1e-7 * nn)) return false;  // direction not well determined
   const double r_lo = (nn - en) / (2.0 * (fabs(E.A) + eA)) * (1.0 - 1e-12);
   // centre offset N / (2A); the sign of A is the certified orientation sgn
   const double inv = (E.sgn > 0 ? 1.0 : -1.0) / nn;
-  const double ux = E.Nx * inv, uy = E.Ny * inv, uz = E.Nz * inv;
-  const uint16_t* cl = tb.cells + (uint64_t)cube_cell(ux, uy, uz) * kCellDirs;
-  double bound = INFINITY;
+  const float ux = (float)(E.Nx * inv), uy = (float)(E.Ny * inv), uz = (float)(E.Nz * inv);
+  const uint4 cl = *reinterpret_cast<const uint4*>(tb.cells + (uint64_t)cube_cell(ux, uy, uz) * kCellDirs);
+  const uint32_t w[4] = {cl.x, cl.y, cl.z, cl.w};
+  float bound = INFINITY;
+#pragma unroll
   for (int i = 0; i < kCellDirs; ++i) {
-    const uint32_t s = cl[i];
+    const uint32_t s = (w[i >> 1] >> (16 * (i & 1))) & 0xffffu;
     if (s == 0xffffu) break;
-    const double cs = (double)tb.dirs[3 * s] * ux + (double)tb.dirs[3 * s + 1] * uy + (double)tb.dirs[3 * s + 2] * uz;
-    if (cs >= tb.cos_lim) bound = fmin(bound, (double)rho[s]);
+    const float cs = tb.dirs[3 * s] * ux + tb.dirs[3 * s + 1] * uy + tb.dirs[3 * s + 2] * uz;
+    if (cs >= tb.cos_lim) bound = fminf(bound, rho[s]);
   }
-  return r_lo > bound * (1.0 + 1e-9);
+  return r_lo > (double)bound * (1.0 + 1e-9);
 }
 
 // Every point of the closed ball lies within its diameter of a: |p - a|^2 <= 4 r^2 = |N|^2 / A^2.
 // The cut adds 2e-5 for the FP64 values of A and N (relative errors below 1e-7 when the cut
 // is used at all) and for the binary32 distances that order C(a); otherwise no cut.
-__device__ float sphere_cut(const QEntry& E, double eA, double eN) {
+__device__ float sphere_cut(const Sphere& E, double eA, double eN) {
   const double nn2 = E.Nx * E.Nx + E.Ny * E.Ny + E.Nz * E.Nz;
   if (!(eA <= 1e-7 * fabs(E.A)) || !(3.0 * eN * eN <= 1e-14 * nn2)) return INFINITY;
   return __double2float_ru(nn2 / (E.A * E.A) * (1.0 + 2e-5));
 }
 
-// Classifies the queued supports against C(a) with the whole warp and emits the relevant ones.
-template <int KC, typename Count>
-__device__ __forceinline__ void classify_queue(const OwnerSmemT<KC>& S, WarpQueue& Q, uint32_t qn, uint32_t m, const Cloud& c,
-                               uint32_t smax, HigherRec* out, uint32_t cap, uint32_t* counter, uint32_t lane,
-                               Count& emitted) {
-  for (uint32_t e = 0; e < qn; ++e) {
-    const QEntry E = Q.q[e];
-    const uint32_t icap = smax - (uint32_t)E.size;
-    uint32_t interior = 0, shell = (uint32_t)E.size, wit = kInvalid32;
-    bool reject = false;
-    for (uint32_t base = 0; base < m; base += 32) {
-      // C(a) is sorted by distance from a: the rest of it lies beyond the sphere's diameter
-      if (S.spt[base].q > (double)E.cut) break;
-      const uint32_t i = base + lane;
-      int sd = 1;
-      uint32_t w = kInvalid32;
-      if (i < m) {
-        w = S.sid[i];
-        if (w != E.ids[1] && w != E.ids[2] && w != E.ids[3]) {
-          const SetPt p = S.spt[i];
-          const double v = E.A * p.q - ((p.x * E.Nx + p.y * E.Ny) + p.z * E.Nz);
-          sd = fsign(v, E.bnd);
-          if (sd == 2) sd = side_exact(c, Q.q[e].ids, E.size, w);  // the queue entry's ids (shared memory)
-          sd *= E.sgn;
-        }
-      }
-      const uint32_t bi = __ballot_sync(0xffffffffu, sd < 0), bs = __ballot_sync(0xffffffffu, sd == 0);
-      if (sd < 0) {
-        const uint32_t at = interior + __popc(bi & lanemask_lt());
-        if (at < icap) Q.iids[at] = w;
-      }
-      interior += __popc(bi);
-      if (interior > icap) {
-        reject = true;
-        break;
-      }
-      if (bs) {
-        shell += __popc(bs);
-        wit = min(wit, __reduce_min_sync(0xffffffffu, sd == 0 ? w : kInvalid32));
-      }
-    }
-    __syncwarp();
-    if (!reject) {  // warp-uniform: the record is written by 16 lanes, one word each
-      uint32_t slot = 0;
-      if (lane == 0) {
-        for (uint32_t i = 1; i < interior; ++i) {  // interior ids ascending, in place
-          const uint32_t x = Q.iids[i];
-          uint32_t j = i;
-          while (j > 0 && Q.iids[j - 1] > x) {
-            Q.iids[j] = Q.iids[j - 1];
-            --j;
-          }
-          Q.iids[j] = x;
-        }
-        slot = atomicAdd(counter, 1u);
-        ++emitted;
-      }
-      slot = __shfl_sync(0xffffffffu, slot, 0);
-      __syncwarp();
-      // support ids ascending (a triangle's fourth slot sorts last and is written as 0)
-      uint32_t s0 = E.ids[0], s1 = E.ids[1], s2 = E.ids[2], s3 = E.size == 4 ? E.ids[3] : kInvalid32;
-      auto cswap = [](uint32_t& x, uint32_t& y) {
-        const uint32_t lo = min(x, y), hi = max(x, y);
-        x = lo;
-        y = hi;
-      };
-      cswap(s0, s1);
-      cswap(s2, s3);
-      cswap(s0, s2);
-      cswap(s1, s3);
-      cswap(s1, s2);
-      if (E.size != 4) s3 = 0u;
-      if (slot < cap && lane < 16) {
-        uint32_t v;
-        if (lane == 0) v = (uint32_t)E.size;
-        else if (lane == 1) v = s0;
-        else if (lane == 2) v = s1;
-        else if (lane == 3) v = s2;
-        else if (lane == 4) v = s3;
-        else if (lane == 5) v = interior;
-        else if (lane == 6) v = shell;
-        else if (lane == 7) v = wit;
-        else v = lane - 8 < interior ? Q.iids[lane - 8] : kInvalid32;
-        reinterpret_cast<uint32_t*>(out + slot)[lane] = v;
-      }
-    }
-    __syncwarp();
+// What the steps of one owner's enumeration share.
+struct OwnerArgs {
+  const uint32_t* clist;  // C(a)
+  uint32_t a, m, smax, cap;
+  double Mp, rmax2;
+  Cloud c;
+  HigherTables tb;
+  HigherRec* out;
+  uint32_t* counter;
+};
+
+// Sphere of a queued support; status as tri_eval.  *adm: a triangle's face bound.
+template <bool kExact, int KC>
+__device__ __forceinline__ int queued_sphere(const OwnerArgs& o, const OwnerSmemT<KC>& S, const ushort4& t, uint32_t& i1,
+                                             uint32_t& i2, uint32_t& i3, Sphere& E, double& eA, double& eN, bool& adm) {
+  const uint32_t ij = S.supi[t.x], ik = S.supi[t.y];
+  i1 = o.clist[ij];
+  i2 = o.clist[ik];
+  adm = false;
+  if (t.z == kNoPoint) {
+    i3 = kInvalid32;
+    return tri_eval<kExact>(o.c, S.spt[ij], S.spt[ik], o.a, i1, i2, o.Mp, o.rmax2, E, eA, eN, adm);
   }
+  const uint32_t il = S.supi[t.z];
+  i3 = o.clist[il];
+  return quad_eval<kExact>(o.c, S.spt[ij], S.spt[ik], S.spt[il], o.a, i1, i2, i3, o.Mp, E, eA, eN);
 }
 
-__device__ __forceinline__ void decode_pair(uint64_t t, uint32_t& lo, uint32_t& hi) {
+// Appends the lanes' entries to a queue of n entries.
+__device__ __forceinline__ void enqueue(ushort4* q, uint32_t& n, bool push, const ushort4& t) {
+  const uint32_t b = __ballot_sync(0xffffffffu, push);
+  if (push) q[n + __popc(b & lanemask_lt())] = t;
+  n += __popc(b);
+}
+
+// Drops the first 32 of n (at most 64) queue entries.
+__device__ __forceinline__ void drop32(ushort4* q, uint32_t& n, uint32_t lane) {
+  __syncwarp();
+  const ushort4 rest = q[32 + lane];
+  __syncwarp();
+  if (lane + 32 < n) q[lane] = rest;
+  n = n > 32 ? n - 32 : 0;
+  __syncwarp();
+}
+
+// Supports of `hard`, one per lane (count of them), decided exactly: their status, the triangles' face
+// bits in adm, the minimal ones that no cone bound excludes to `kept`.  Returns, packed, the
+// minimal (low), kept and admitted supports of the warp (10 bits each).
+template <int KC>
+__device__ __noinline__ uint32_t sift_hard(const OwnerArgs& o, const OwnerSmemT<KC>& S, WarpQueue& Q, uint32_t count,
+                                           uint32_t kept, uint32_t* adm) {
+  constexpr uint32_t kWords = KC / 32;
+  const uint32_t lane = threadIdx.x & 31u;
+  __syncwarp();
+  bool minimal = false, keep = false, face = false;
+  ushort4 t = make_ushort4(0, 0, 0, 0);
+  if (lane < count) {
+    t = Q.hard[lane];
+    uint32_t i1, i2, i3;
+    Sphere E;
+    double eA, eN;
+    minimal = queued_sphere<true, KC>(o, S, t, i1, i2, i3, E, eA, eN, face) == 0;
+    if (face) atomicOr(&adm[t.x * kWords + (t.y >> 5)], 1u << (t.y & 31));
+    if (t.z == kNoPoint && o.smax < 3) minimal = false;
+    keep = minimal && !cone_rejects(E, eA, eN, S.rho, o.tb);
+  }
+  uint32_t n = kept;
+  enqueue(Q.kept, n, keep, t);
+  const uint32_t mb = __popc(__ballot_sync(0xffffffffu, minimal)), fb = __popc(__ballot_sync(0xffffffffu, face));
+  __syncwarp();
+  return mb | (n - kept) << 10 | fb << 20;
+}
+
+// Places of the warp's records (one atomic) and the record of a lane that has one: the support, and
+// the points at the given positions (16 bits each) as interior ids, ascending.
+template <int KC>
+__device__ __forceinline__ uint32_t emit_records(const OwnerArgs& o, const OwnerSmemT<KC>& S, bool live, int size,
+                                                 uint32_t i1, uint32_t i2, uint32_t i3, uint32_t interior, uint32_t shell,
+                                                 uint32_t wit, unsigned long long in_lo, unsigned long long in_hi) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t b = __ballot_sync(0xffffffffu, live);
+  uint32_t slot = 0;
+  if (lane == 0 && b) slot = atomicAdd(o.counter, (uint32_t)__popc(b));
+  slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(b & lanemask_lt());
+  if (live && slot < o.cap) {
+    uint32_t id[kMaxInteriorH];
+#pragma unroll
+    for (int q = 0; q < kMaxInteriorH; ++q) {
+      const uint32_t at = (uint32_t)((q < 4 ? in_lo >> (16 * q) : in_hi >> (16 * (q - 4))) & 0xffffu);
+      id[q] = (uint32_t)q < interior ? o.clist[at] : kInvalid32;
+    }
+#pragma unroll
+    for (int r = 0; r < kMaxInteriorH; ++r)  // odd-even transposition
+#pragma unroll
+      for (int q = r & 1; q + 1 < kMaxInteriorH; q += 2) {
+        const uint32_t lo = min(id[q], id[q + 1]), hi = max(id[q], id[q + 1]);
+        id[q] = lo;
+        id[q + 1] = hi;
+      }
+    // support ids ascending (a triangle's fourth slot sorts last and is written as 0)
+    uint32_t s0 = o.a, s1 = i1, s2 = i2, s3 = i3;
+    auto cswap = [](uint32_t& x, uint32_t& y) {
+      const uint32_t lo = min(x, y), hi = max(x, y);
+      x = lo;
+      y = hi;
+    };
+    cswap(s0, s1);
+    cswap(s2, s3);
+    cswap(s0, s2);
+    cswap(s1, s3);
+    cswap(s1, s2);
+    if (size != 4) s3 = 0u;
+    uint4* rec = reinterpret_cast<uint4*>(o.out + slot);
+    rec[0] = make_uint4((uint32_t)size, s0, s1, s2);
+    rec[1] = make_uint4(s3, interior, shell, wit);
+    rec[2] = make_uint4(id[0], id[1], id[2], id[3]);
+    rec[3] = make_uint4(id[4], id[5], id[6], id[7]);
+  }
+  return (uint32_t)__popc(b);
+}
+
+// Classifies the kept supports of the lanes in `which` exactly where binary64 does not decide (a point
+// on or next to the sphere, or a support whose own signs are not decided).
+template <int KC>
+__device__ __noinline__ uint32_t classify_exact(const OwnerArgs& o, const OwnerSmemT<KC>& S, const WarpQueue& Q,
+                                                uint32_t which) {
+  const uint32_t lane = threadIdx.x & 31u;
+  bool live = which >> lane & 1u, adm;
+  Sphere E;
+  E.A = E.Nx = E.Ny = E.Nz = E.bnd = 0.0;
+  E.size = 3;
+  E.sgn = 1;
+  uint32_t i1 = 0, i2 = 0, i3 = kInvalid32, pj = 0, pk = 0, pl = kInvalid32;
+  if (live) {
+    const ushort4 t = Q.kept[lane];
+    double eA, eN;
+    queued_sphere<true, KC>(o, S, t, i1, i2, i3, E, eA, eN, adm);
+    pj = S.supi[t.x];
+    pk = S.supi[t.y];
+    if (t.z != kNoPoint) pl = S.supi[t.z];
+  }
+  const uint32_t icap = o.smax - (uint32_t)E.size;
+  uint32_t interior = 0, shell = (uint32_t)E.size, wit = kInvalid32;
+  unsigned long long in_lo = 0, in_hi = 0;
+  for (uint32_t i = 0; i < o.m && live; ++i) {
+    if (i == pj || i == pk || i == pl) continue;
+    const SetPt p = S.spt[i];
+    int sd = fsign(E.A * p.q - ((p.x * E.Nx + p.y * E.Ny) + p.z * E.Nz), E.bnd);
+    if (sd == 2) sd = side_exact_ids(o.c, o.a, i1, i2, i3, E.size, o.clist[i]);
+    sd *= E.sgn;
+    if (sd == 0) {
+      ++shell;
+      wit = min(wit, o.clist[i]);
+    } else if (sd < 0) {
+      if (interior == icap) {
+        live = false;
+      } else {
+        ++interior;
+        in_hi = in_hi << 16 | in_lo >> 48;
+        in_lo = in_lo << 16 | i;
+      }
+    }
+  }
+  __syncwarp();
+  return emit_records<KC>(o, S, live, E.size, i1, i2, i3, interior, shell, wit, in_lo, in_hi);
+}
+
+// Classifies the first `count` (at most 32) kept supports against C(a), one per lane, and emits the
+// relevant ones: every lane walks C(a) (a point is one broadcast from shared memory for 32 spheres)
+// until its sphere's diameter or too many interior points.  Lanes that binary64 leaves open are
+// returned in *open; returns the number of records.
+template <int KC>
+__device__ __forceinline__ uint32_t classify_kept(const OwnerArgs& o, const OwnerSmemT<KC>& S, const WarpQueue& Q,
+                                                  uint32_t count, uint32_t* open) {
+  const uint32_t lane = threadIdx.x & 31u;
+  bool live = lane < count, undecided = false;
+  double A = 0.0, Nx = 0.0, Ny = 0.0, Nz = 0.0, bnd = 0.0;
+  int size = 3;
+  float cut = 0.f;
+  uint32_t i1 = 0, i2 = 0, i3 = kInvalid32;
+  uint32_t pj = 0, pk = 0, pl = kInvalid32;  // positions of the support's points
+  if (live) {
+    const ushort4 t = Q.kept[lane];
+    Sphere E;
+    double eA, eN;
+    bool adm;
+    undecided = queued_sphere<false, KC>(o, S, t, i1, i2, i3, E, eA, eN, adm) != 0;
+    size = t.z == kNoPoint ? 3 : 4;
+    if (!undecided) {
+      cut = sphere_cut(E, eA, eN);
+      // oriented so that a point outside has a positive value
+      A = E.sgn < 0 ? -E.A : E.A;
+      Nx = E.sgn < 0 ? -E.Nx : E.Nx;
+      Ny = E.sgn < 0 ? -E.Ny : E.Ny;
+      Nz = E.sgn < 0 ? -E.Nz : E.Nz;
+      bnd = E.bnd;
+    }
+    pj = S.supi[t.x];
+    pk = S.supi[t.y];
+    if (t.z != kNoPoint) pl = S.supi[t.z];
+  }
+  const uint32_t icap = o.smax - (uint32_t)size;
+  uint32_t interior = 0;
+  unsigned long long in_lo = 0, in_hi = 0;  // positions of the interior points, 16 bits each, last one first
+  bool walk = live && !undecided;
+  for (uint32_t i0 = 0; i0 < o.m; i0 += 4) {
+    // C(a) is sorted by distance from a: the rest of it lies beyond the sphere's diameter (points looked
+    // at beyond it are outside)
+    walk = walk && !(S.spt[i0].q > (double)cut);
+    if (!__any_sync(0xffffffffu, walk)) break;
+    const uint32_t i_end = min(i0 + 4, o.m);
+    for (uint32_t i = i0; i < i_end; ++i) {
+      const SetPt p = S.spt[i];
+      const double v = A * p.q - ((p.x * Nx + p.y * Ny) + p.z * Nz);
+      if (!walk || v > bnd) continue;
+      if (v < -bnd) {
+        if (interior == icap) {
+          walk = live = false;
+        } else {
+          ++interior;
+          in_hi = in_hi << 16 | in_lo >> 48;
+          in_lo = in_lo << 16 | i;
+        }
+      } else if (i != pj && i != pk && i != pl) {  // (the support's own points always are undecided)
+        undecided = true;
+        walk = false;
+      }
+    }
+  }
+  *open = __ballot_sync(0xffffffffu, live && undecided);
+  return emit_records<KC>(o, S, live && !undecided, size, i1, i2, i3, interior, (uint32_t)size, kInvalid32, in_lo, in_hi);
+}
+
+// True when the tetrahedron (a, a + e1, a + e2, a + e3) certainly is not minimal: some barycentric
+// numerator l_i of its circumcentre is negative.  Binary32 on coordinates scaled by a power of two
+// to at most 2: the polynomials of quad_eval, with at most 19 roundings on a path (each coordinate
+// and |e|^2 rounded once), so |computed - exact| <= 24 2^-24 m with the same m: l_1..3 108 M^6, l_0
+// 396 M^6; 1e-36 covers underflow.  What is left (some 15 % of the tests) goes on to binary64.
+__device__ __forceinline__ bool quad_outside(const float4& e1, const float4& e2, const float4& e3) {
+  const float M = fmaxf(fmaxf(fmaxf(fabsf(e1.x), fabsf(e1.y)), fmaxf(fabsf(e1.z), fabsf(e2.x))),
+                        fmaxf(fmaxf(fmaxf(fabsf(e2.y), fabsf(e2.z)), fmaxf(fabsf(e3.x), fabsf(e3.y))), fabsf(e3.z)));
+  const float c23x = e2.y * e3.z - e2.z * e3.y, c23y = e2.z * e3.x - e2.x * e3.z, c23z = e2.x * e3.y - e2.y * e3.x;
+  const float c31x = e3.y * e1.z - e3.z * e1.y, c31y = e3.z * e1.x - e3.x * e1.z, c31z = e3.x * e1.y - e3.y * e1.x;
+  const float c12x = e1.y * e2.z - e1.z * e2.y, c12y = e1.z * e2.x - e1.x * e2.z, c12z = e1.x * e2.y - e1.y * e2.x;
+  const float Nx = (e1.w * c23x + e2.w * c31x) + e3.w * c12x;
+  const float Ny = (e1.w * c23y + e2.w * c31y) + e3.w * c12y;
+  const float Nz = (e1.w * c23z + e2.w * c31z) + e3.w * c12z;
+  const float l1 = (Nx * c23x + Ny * c23y) + Nz * c23z;
+  const float l2 = (Nx * c31x + Ny * c31y) + Nz * c31z;
+  const float l3 = (Nx * c12x + Ny * c12y) + Nz * c12z;
+  const float det = (e1.x * c23x + e1.y * c23y) + e1.z * c23z;
+  const float l0 = 2.0f * det * det - ((l1 + l2) + l3);
+  const float M2 = M * M, m = (24.0f * 0x1p-24f * 1.00001f) * (M2 * M2 * M2);
+  const float bl = 108.0f * m + 1e-36f, b0 = 396.0f * m + 1e-36f;
+  return fminf(fminf(l1, l2), l3) < -bl || l0 < -b0;
+}
+
+__device__ __forceinline__ void decode_pair(uint32_t t, uint32_t& lo, uint32_t& hi) {
   uint32_t i = (uint32_t)((sqrt(8.0 * (double)t + 1.0) - 1.0) / 2.0);
   while ((uint64_t)(i + 1) * i / 2 > t) --i;
   while ((uint64_t)(i + 2) * (i + 1) / 2 <= t) ++i;
@@ -1281,6 +1471,7 @@ __device__ __forceinline__ void higher_owner(uint32_t a, const uint32_t* __restr
   constexpr uint32_t kWords = KC / 32;
   __shared__ double s_Mp;
   __shared__ uint32_t s_mc;
+  __shared__ uint32_t s_next[2];  // next pairs of the triangle and tetrahedron loops
   __shared__ float s_rmax[kHOwnerWarps];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   WarpQueue& Q = wq[warp];
@@ -1299,7 +1490,6 @@ __device__ __forceinline__ void higher_owner(uint32_t a, const uint32_t* __restr
       s.y = py[p] - ay;
       s.z = pz[p] - az;
       s.q = (s.x * s.x + s.y * s.y) + s.z * s.z;
-      S.sid[i] = p;
       S.spt[i] = s;
       Mp = fmax(Mp, ptmax(s));
     }
@@ -1324,144 +1514,234 @@ __device__ __forceinline__ void higher_owner(uint32_t a, const uint32_t* __restr
   if (threadIdx.x == 0) {
     s_Mp = Mp * (1.0 + 1e-15);
     s_mc = mc;
+    s_next[0] = s_next[1] = 0;
   }
   __syncthreads();
   Mp = s_Mp;
   mc = s_mc;
+  if (phases & kPhTet) {  // binary32 copies of the support candidates, scaled to at most 2
+    const double scale = Mp > 0.0 ? exp2((double)-ilogb(Mp)) : 1.0;
+    for (uint32_t j = threadIdx.x; j < mc; j += 32 * kHOwnerWarps) {
+      const SetPt p = S.spt[S.supi[j]];
+      S.fpt[j] = make_float4((float)(p.x * scale), (float)(p.y * scale), (float)(p.z * scale),
+                             (float)((p.q * scale) * scale));
+    }
+    __syncthreads();
+  }
   rmax = s_rmax[0];
   for (int w = 1; w < kHOwnerWarps; ++w) rmax = fmaxf(rmax, s_rmax[w]);
   const double rmax2 = (double)rmax * (double)rmax * (1.0 + 1e-12);
   // per-lane work counters: 32-bit where a block's share of an owner cannot reach 2^32 (sets of
   // up to 1,024 candidates, or a chunk of pairs), else 64-bit (registers are the scarce unit)
   using Count = typename std::conditional<(KC <= 1024), uint32_t, unsigned long long>::type;
-  Count tested = 0, minimal = 0, pruned = 0, classified = 0, emitted = 0, admitted = 0;
-  const uint64_t P2 = min((uint64_t)mc * (mc - 1) / 2, t_hi);
-  // --- triangles (a, j, k); also the face bound adm(j, k) for the tetrahedra
-  for (uint64_t t0 = t_lo + 32 * warp; (phases & kPhTri) && t0 < P2; t0 += 32 * kHOwnerWarps) {
-    const uint64_t t = t0 + lane;
-    bool push = false;
-    QEntry E;
-    if (t < P2) {
-      uint32_t j, k;
-      decode_pair(t, j, k);
-      const uint32_t ij = S.supi[j], ik = S.supi[k];
-      E.ids[0] = a;
-      E.ids[1] = S.sid[ij];
-      E.ids[2] = S.sid[ik];
-      E.ids[3] = kInvalid32;
-      double eA, eN;
-      bool face_ok;
-      ++tested;
-      const int st = tri_eval(c, S.spt[ij], S.spt[ik], E.ids[0], E.ids[1], E.ids[2], Mp, rmax2, E, eA, eN, face_ok);
-      if (face_ok) {
-        atomicOr(&adm[j * kWords + (k >> 5)], 1u << (k & 31));
-        ++admitted;
-      }
-      if (st == 0 && ctl.smax >= 3) {
-        ++minimal;
-        if (cone_rejects(E, eA, eN, S.rho, tb)) ++pruned;
-        else {
-          push = true;
-          E.cut = sphere_cut(E, eA, eN);
+  Count tested = 0, admitted = 0;
+  uint32_t n_minimal = 0, n_classified = 0, n_emitted = 0;  // of the warp
+  const OwnerArgs o{clist, a, m, ctl.smax, ctl.cap, Mp, rmax2, c, tb, out, counter};
+  const uint32_t words = (mc + 31) / 32;  // mask words in use per candidate
+  const uint32_t lo = (uint32_t)t_lo, P2 = (uint32_t)min((uint64_t)mc * (mc - 1) / 2, t_hi);  // below 2^28
+  // the warps take 32 pairs at a time as they become free (pairs differ widely in tetrahedra)
+  auto next_pairs = [&](int which) {
+    uint32_t t0 = 0;
+    if (lane == 0) t0 = atomicAdd(s_next + which, 32u);
+    return lo + __shfl_sync(0xffffffffu, t0, 0);
+  };
+  // common faces of the pair (j, k) in mask word w, beyond k
+  auto common = [&](uint32_t j_, uint32_t k_, uint32_t w) {
+    const uint32_t w0 = (k_ + 1) >> 5;
+    if (w < w0) return 0u;
+    const uint32_t bits = adm[j_ * kWords + w] & adm[k_ * kWords + w];
+    return w == w0 ? bits & (0xffffffffu << ((k_ + 1) & 31)) : bits;
+  };
+  uint32_t nf = 0, nh = 0, nk = 0;  // entries of the warp's queues
+  // state of the tetrahedron loop: pairs of the lanes (small sets) or of the warp (large sets), and the
+  // tetrahedra of theirs that are left
+  uint32_t j = 0, k = 0, excl = 0, total = 0, q0 = 0, faces = 0, wb = words, bits = 0;
+  bool tri = (phases & kPhTri) != 0, tet = ctl.smax >= 4 && (phases & kPhTet) != 0;
+  while (tri || tet) {
+    bool flush = false;  // nothing more comes from this loop
+    if (tri) {
+      // --- triangles (a, j, k); also the face bound adm(j, k) for the tetrahedra
+      while (nf < 32 && nh <= 32) {
+        const uint32_t t0 = next_pairs(0), t = t0 + lane;
+        if (t0 >= P2) {
+          flush = true;
+          break;
         }
-      }
-    }
-    const uint32_t b = __ballot_sync(0xffffffffu, push);
-    if (push) Q.q[__popc(b & lanemask_lt())] = E;
-    __syncwarp();
-    classified += __popc(b);
-    classify_queue(S, Q, __popc(b), m, c, ctl.smax, out, ctl.cap, counter, lane, emitted);
-  }
-  if ((phases & kPhTri) && (phases & kPhTet)) __syncthreads();  // the face mask is complete
-  // --- tetrahedra (a, j, k, l), j < k < l with adm(j,k), adm(j,l), adm(k,l)
-  if (ctl.smax >= 4 && (phases & kPhTet)) {
-    for (uint64_t t0 = t_lo + 32 * warp; t0 < P2; t0 += 32 * kHOwnerWarps) {
-      const uint64_t t = t0 + lane;
-      uint32_t j = 0, k = 0, cnt = 0;
-      if (t < P2) {
-        decode_pair(t, j, k);
-        if ((adm[j * kWords + (k >> 5)] >> (k & 31)) & 1u) {
-          const uint32_t w0 = (k + 1) >> 5;
-          for (uint32_t w = w0; w < kWords; ++w) {
-            uint32_t bits = adm[j * kWords + w] & adm[k * kWords + w];
-            if (w == w0) bits &= ((k + 1) & 31) ? (0xffffffffu << ((k + 1) & 31)) : 0xffffffffu;
-            cnt += __popc(bits);
+        int st = 3;
+        uint32_t tj = 0, tk = 0;
+        if (t < P2) {
+          decode_pair(t, tj, tk);
+          const uint32_t ij = S.supi[tj], ik = S.supi[tk];
+          Sphere E;
+          double eA, eN;
+          bool face_ok = false;
+          ++tested;
+          st = tri_eval<false>(c, S.spt[ij], S.spt[ik], a, o.clist[ij], o.clist[ik], Mp, rmax2, E, eA, eN, face_ok);
+          if (st != 4 && face_ok) {
+            atomicOr(&adm[tj * kWords + (tk >> 5)], 1u << (tk & 31));
+            ++admitted;
           }
         }
+        const ushort4 e = make_ushort4((uint16_t)tj, (uint16_t)tk, kNoPoint, 0);
+        enqueue(Q.found, nf, st == 0 && ctl.smax >= 3, e);
+        enqueue(Q.hard, nh, st == 4, e);
       }
-      uint32_t incl = cnt;
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, off);
-        if ((int)lane >= off) incl += x;
-      }
-      const uint32_t excl = incl - cnt, total = __shfl_sync(0xffffffffu, incl, 31);
-      for (uint32_t q0 = 0; q0 < total; q0 += 32) {
-        const uint32_t q = q0 + lane;
-        // owner lane: the largest o with excl_o <= q
-        uint32_t o = 0;
-        for (uint32_t step = 16; step > 0; step >>= 1) {
-          const uint32_t v = __shfl_sync(0xffffffffu, excl, o + step);
-          if (v <= q) o += step;
-        }
-        const uint32_t oj = __shfl_sync(0xffffffffu, j, o), ok = __shfl_sync(0xffffffffu, k, o);
-        const uint32_t oe = __shfl_sync(0xffffffffu, excl, o);
-        bool push = false;
-        QEntry E;
-        if (q < total) {
-          uint32_t r = q - oe, l = 0;
-          const uint32_t w0 = (ok + 1) >> 5;
-          for (uint32_t w = w0; w < kWords; ++w) {
-            uint32_t bits = adm[oj * kWords + w] & adm[ok * kWords + w];
-            if (w == w0) bits &= ((ok + 1) & 31) ? (0xffffffffu << ((ok + 1) & 31)) : 0xffffffffu;
-            const uint32_t pc = __popc(bits);
-            if (r < pc) {
-              l = w * 32 + select_bit(bits, r);
+    } else {
+      // --- tetrahedra (a, j, k, l), j < k < l with adm(j,k), adm(j,l), adm(k,l)
+      while (nf < 32) {
+        if (q0 >= total) {  // the next pairs
+          q0 = total = 0;
+          if (KC <= kMaxCand) {
+            // small sets: few tetrahedra per pair, so the lanes share those of 32 pairs
+            const uint32_t t0 = next_pairs(1), t = t0 + lane;
+            if (t0 >= P2) {
+              flush = true;
               break;
             }
-            r -= pc;
-          }
-          const uint32_t ij = S.supi[oj], ik = S.supi[ok], il = S.supi[l];
-          E.ids[0] = a;
-          E.ids[1] = S.sid[ij];
-          E.ids[2] = S.sid[ik];
-          E.ids[3] = S.sid[il];
-          double eA, eN;
-          ++tested;
-          if (quad_eval(c, S.spt[ij], S.spt[ik], S.spt[il], E.ids[0], E.ids[1], E.ids[2], E.ids[3], Mp, E, eA, eN) == 0) {
-            ++minimal;
-            if (cone_rejects(E, eA, eN, S.rho, tb)) ++pruned;
-            else {
-              push = true;
-              E.cut = sphere_cut(E, eA, eN);
+            uint32_t cnt = 0;
+            if (t < P2) {
+              decode_pair(t, j, k);
+              if ((adm[j * kWords + (k >> 5)] >> (k & 31)) & 1u)
+                for (uint32_t w = (k + 1) >> 5; w < words; ++w) cnt += __popc(common(j, k, w));
             }
+            bits = cnt;
+          } else {
+            // large sets: many tetrahedra per pair, so the warp takes one pair after another and a lane
+            // one mask word of every 32
+            wb += 32;
+            if (wb >= words) {
+              while (faces == 0) {
+                const uint32_t t0 = next_pairs(1), t = t0 + lane;
+                if (t0 >= P2) break;
+                bool face = false;
+                if (t < P2) {
+                  decode_pair(t, j, k);
+                  face = (adm[j * kWords + (k >> 5)] >> (k & 31)) & 1u;
+                }
+                faces = __ballot_sync(0xffffffffu, face);
+              }
+              if (faces == 0) {
+                flush = true;
+                break;
+              }
+              wb = ((__shfl_sync(0xffffffffu, k, __ffs((int)faces) - 1) + 1) >> 5) & ~31u;
+            }
+            const int src = __ffs((int)faces) - 1;
+            const uint32_t oj = __shfl_sync(0xffffffffu, j, src), ok = __shfl_sync(0xffffffffu, k, src);
+            bits = wb + lane < words ? common(oj, ok, wb + lane) : 0u;
           }
+          uint32_t incl = KC <= kMaxCand ? bits : __popc(bits);
+          const uint32_t own = incl;
+          for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, incl, off);
+            if ((int)lane >= off) incl += x;
+          }
+          excl = incl - own;
+          total = __shfl_sync(0xffffffffu, incl, 31);
+        } else {
+          const uint32_t q = q0 + lane;
+          uint32_t src = 0;  // the largest lane with excl <= q
+          for (uint32_t step = 16; step > 0; step >>= 1) {
+            const uint32_t v = __shfl_sync(0xffffffffu, excl, src + step);
+            if (v <= q) src += step;
+          }
+          const uint32_t oe = __shfl_sync(0xffffffffu, excl, src);
+          const uint32_t ob = __shfl_sync(0xffffffffu, bits, src);
+          const int from = KC <= kMaxCand ? (int)src : __ffs((int)faces) - 1;
+          const uint32_t oj = __shfl_sync(0xffffffffu, j, from), ok = __shfl_sync(0xffffffffu, k, from);
+          bool push = false;
+          uint32_t l = 0;
+          if (q < total) {
+            uint32_t r = q - oe;
+            if (KC <= kMaxCand) {
+              for (uint32_t w = (ok + 1) >> 5; w < words; ++w) {
+                const uint32_t x = common(oj, ok, w), pc = __popc(x);
+                if (r < pc) {
+                  l = w * 32 + select_bit(x, r);
+                  break;
+                }
+                r -= pc;
+              }
+            } else {
+              l = (wb + src) * 32 + select_bit(ob, r);
+            }
+            ++tested;
+            push = !quad_outside(S.fpt[oj], S.fpt[ok], S.fpt[l]);
+          }
+          enqueue(Q.found, nf, push, make_ushort4((uint16_t)oj, (uint16_t)ok, (uint16_t)l, 0));
+          q0 += 32;
         }
-        const uint32_t b = __ballot_sync(0xffffffffu, push);
-        if (push) Q.q[__popc(b & lanemask_lt())] = E;
-        __syncwarp();
-        classified += __popc(b);
-        classify_queue(S, Q, __popc(b), m, c, ctl.smax, out, ctl.cap, counter, lane, emitted);
+        // a pair of a large set is done with its last mask words
+        if (KC > kMaxCand && q0 >= total && wb + 32 >= words) faces &= faces - 1;
       }
     }
+    // --- the queues, 32 supports at a time (all of them when this loop has ended)
+    const bool last = flush && !(tri && tet);
+    for (;;) {
+      if (nk >= 32 || (last && nf == 0 && nh == 0 && nk)) {
+        __syncwarp();
+        uint32_t open;
+        n_emitted += classify_kept<KC>(o, S, Q, min(nk, 32u), &open);
+        if (open) n_emitted += classify_exact<KC>(o, S, Q, open);
+        drop32(Q.kept, nk, lane);
+      } else if (nh >= 32 || (flush && nh && nf == 0)) {
+        const uint32_t r = sift_hard<KC>(o, S, Q, min(nh, 32u), nk, adm);
+        n_minimal += r & 1023u;
+        nk += r >> 10 & 1023u;
+        n_classified += r >> 10 & 1023u;
+        if (lane == 0) admitted += r >> 20;
+        drop32(Q.hard, nh, lane);
+      } else if (nf >= 32 || (flush && nf)) {
+        __syncwarp();
+        int st = 3;
+        bool keep = false;
+        ushort4 e = make_ushort4(0, 0, 0, 0);
+        if (lane < nf) {
+          e = Q.found[lane];
+          uint32_t i1, i2, i3;
+          Sphere E;
+          double eA, eN;
+          bool face;
+          st = queued_sphere<false, KC>(o, S, e, i1, i2, i3, E, eA, eN, face);
+          keep = st == 0 && !cone_rejects(E, eA, eN, S.rho, tb);
+        }
+        n_minimal += __popc(__ballot_sync(0xffffffffu, st == 0));
+        const uint32_t before = nk;
+        enqueue(Q.kept, nk, keep, e);
+        n_classified += nk - before;
+        enqueue(Q.hard, nh, st == 4, e);
+        drop32(Q.found, nf, lane);
+      } else {
+        break;
+      }
+    }
+    if (!flush) continue;
+    if (!tri) break;
+    tri = false;
+    if (phases & kPhTet) __syncthreads();  // the face mask is complete
   }
   for (int off = 16; off > 0; off >>= 1) {
     tested += __shfl_xor_sync(0xffffffffu, tested, off);
-    minimal += __shfl_xor_sync(0xffffffffu, minimal, off);
-    pruned += __shfl_xor_sync(0xffffffffu, pruned, off);
     admitted += __shfl_xor_sync(0xffffffffu, admitted, off);
   }
+  // the block's counters leave with one atomic per counter
+  __shared__ unsigned long long s_stats[8];
+  if (threadIdx.x < 8) s_stats[threadIdx.x] = 0;
+  __syncthreads();
   if (lane == 0) {
-    atomicAdd(stats + 0, (unsigned long long)tested);
-    atomicAdd(stats + 1, (unsigned long long)classified);
-    atomicAdd(stats + 2, (unsigned long long)emitted);
+    atomicAdd(s_stats + 0, (unsigned long long)tested);
+    atomicAdd(s_stats + 1, (unsigned long long)n_classified);
+    atomicAdd(s_stats + 2, (unsigned long long)n_emitted);
     if (warp == 0 && (phases & kPhStats)) {
-      atomicAdd(stats + 3, (unsigned long long)m);
-      atomicAdd(stats + 4, (unsigned long long)mc);
+      s_stats[3] = m;
+      s_stats[4] = mc;
     }
-    atomicAdd(stats + 5, (unsigned long long)minimal);
-    atomicAdd(stats + 6, (unsigned long long)pruned);
-    atomicAdd(stats + 7, (unsigned long long)admitted);
+    atomicAdd(s_stats + 5, (unsigned long long)n_minimal);
+    atomicAdd(s_stats + 6, (unsigned long long)(n_minimal - n_classified));
+    atomicAdd(s_stats + 7, (unsigned long long)admitted);
   }
+  __syncthreads();
+  if (threadIdx.x < 8 && s_stats[threadIdx.x]) atomicAdd(stats + threadIdx.x, s_stats[threadIdx.x]);
 }
 
 __global__ void __launch_bounds__(32 * kHOwnerWarps, kHBlocksPerSM)
@@ -1589,27 +1869,23 @@ __global__ void k_predicate(uint32_t pred, uint32_t count, const double* __restr
     s.q = (s.x * s.x + s.y * s.y) + s.z * s.z;
     return s;
   };
-  auto status = [&](const uint32_t* sup, int size, QEntry& E, double& eA, double& eN) -> int {
+  auto status = [&](const uint32_t* sup, int size, Sphere& E, double& eA, double& eN) -> int {
     if (size == 1) return 0;
     if (size == 2) return sup[0] == sup[1] ? 3 : 0;
     const SetPt e1 = setpt(sup[1], sup[0]), e2 = setpt(sup[2], sup[0]);
     double Mp = fmax(ptmax(e1), ptmax(e2));
-    E.ids[0] = sup[0];
-    E.ids[1] = sup[1];
-    E.ids[2] = sup[2];
-    E.ids[3] = size == 4 ? sup[3] : kInvalid32;
     if (size == 3) {
       bool adm;
-      return tri_eval(c, e1, e2, sup[0], sup[1], sup[2], Mp * (1.0 + 1e-15), INFINITY, E, eA, eN, adm);
+      return tri_eval<true>(c, e1, e2, sup[0], sup[1], sup[2], Mp * (1.0 + 1e-15), INFINITY, E, eA, eN, adm);
     }
     const SetPt e3 = setpt(sup[3], sup[0]);
     Mp = fmax(Mp, ptmax(e3));
-    return quad_eval(c, e1, e2, e3, sup[0], sup[1], sup[2], sup[3], Mp * (1.0 + 1e-15), E, eA, eN);
+    return quad_eval<true>(c, e1, e2, e3, sup[0], sup[1], sup[2], sup[3], Mp * (1.0 + 1e-15), E, eA, eN);
   };
   if (pred == 1) {  // side of the last id against the support sphere of the others
     const int size = (int)count - 1;
     const uint32_t w = ids[size];
-    QEntry E;
+    Sphere E;
     double eA = 0, eN = 0;
     const int st = size >= 3 ? status(ids, size, E, eA, eN) : -1;
     if (st == 0) {  // a minimal support: the enumeration's classification
@@ -1626,7 +1902,7 @@ __global__ void k_predicate(uint32_t pred, uint32_t count, const double* __restr
       res = A.sign() == 0 ? 2 : side_exact(c, ids, size, w) * (A.sign() < 0 ? -1 : 1);  // 2: no sphere
     }
   } else if (pred == 2) {  // status of a 1- to 4-point support: 0 minimal, 1 boundary, 2 exterior, 3 dependent
-    QEntry E;
+    Sphere E;
     double eA = 0, eN = 0;
     res = status(ids, (int)count, E, eA, eN);
   } else if (pred == 3) {  // sign of level(left) - level(right); ids: left size, left ids, right ids
@@ -1864,7 +2140,7 @@ cudaError_t higher_alloc(Ctx& ctx) {
   EHGP_ALLOC(h.rho, n * kDirs * sizeof(float));
 #undef EHGP_ALLOC
   h.delta = delta;
-  h.cos_lim = std::cos(delta) + 1e-6;
+  h.cos_lim = std::cos(delta) + 4e-6;
   if ((e = cudaMemcpy(h.cells, cells.data(), cells.size() * sizeof(uint16_t), cudaMemcpyHostToDevice)) != cudaSuccess)
     return e;
   return cudaMemcpy(h.dirs, dirs.data(), dirs.size() * sizeof(float), cudaMemcpyHostToDevice);
@@ -2205,7 +2481,7 @@ int higher_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
   }
   uint32_t hc[2];
   cudaError_t e = cudaSuccess;
-  const HigherTables tb{h.dirs, h.cells, h.rho, h.cos_lim};
+  const HigherTables tb{h.dirs, h.cells, h.rho, (float)h.cos_lim};
   // count -> allocate -> emit: the enumeration counts every record and writes those that fit;
   // when the count exceeds the buffer, the buffer grows to it and the enumeration runs again
   for (int attempt = 0; attempt < 2; ++attempt) {
