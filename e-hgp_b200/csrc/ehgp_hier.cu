@@ -145,7 +145,9 @@ __device__ void fsphere(const double* __restrict__ px, const double* __restrict_
   s.az = pz[ids[0]];
   double e[3][3];
   double M = 0.0;
-  for (int j = 1; j < size; ++j) {
+#pragma unroll
+  for (int j = 1; j < 4; ++j) {
+    if (j >= size) continue;
     e[j - 1][0] = px[ids[j]] - s.ax;
     e[j - 1][1] = py[ids[j]] - s.ay;
     e[j - 1][2] = pz[ids[j]] - s.az;
@@ -412,12 +414,13 @@ __device__ bool tie_less(const WL* knum, const WL* ka2, const EvRec* rec, uint32
   return a.size < b.size;
 }
 
-// rec[i]: copy of the member's record (members of run r are run_off[r] .. run_off[r + 1] - 1,
+// rec[i], mid[i], err[i]: copies of the member's record and level interval (members of run r are run_off[r] .. run_off[r + 1] - 1,
 // at facade positions run_lo[r] ...); idx / tmp: scratch of the member count.
 __global__ void k_tie_sort(uint32_t nruns, const uint32_t* __restrict__ run_off, const uint32_t* __restrict__ run_lo,
                            const WL* __restrict__ knum, const WL* __restrict__ ka2, const EvRec* __restrict__ rec,
-                           uint32_t* __restrict__ idx, uint32_t* __restrict__ tmp, EvRec* __restrict__ ev,
-                           uint8_t* __restrict__ eqprev) {
+                           const double* __restrict__ mid, const double* __restrict__ err, uint32_t* __restrict__ idx,
+                           uint32_t* __restrict__ tmp, EvRec* __restrict__ ev, double* __restrict__ lmid,
+                           double* __restrict__ lerr, uint8_t* __restrict__ eqprev) {
   const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nruns) return;
   const uint32_t b = run_off[r], L = run_off[r + 1] - b;
@@ -440,15 +443,21 @@ __global__ void k_tie_sort(uint32_t nruns, const uint32_t* __restrict__ run_off,
   const uint32_t p0 = run_lo[r];
   for (uint32_t t = 0; t < L; ++t) {
     ev[p0 + t] = rec[src[t]];
+    lmid[p0 + t] = mid[src[t]];  // the level intervals follow their events
+    lerr[p0 + t] = err[src[t]];
     if (t > 0) eqprev[p0 + t] = tie_level_cmp(knum, ka2, src[t - 1], src[t]) == 0 ? 1 : 0;
   }
 }
 
 // Gathers the facade records of the uncertain runs (the member copies of the tie sort).
 __global__ void k_run_gather(uint32_t cnt, const uint32_t* __restrict__ idx, const EvRec* __restrict__ ev,
-                             EvRec* __restrict__ out) {
+                             const double* __restrict__ lmid, const double* __restrict__ lerr, EvRec* __restrict__ out,
+                             double* __restrict__ omid, double* __restrict__ oerr) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < cnt) out[i] = ev[idx[i]];
+  if (i >= cnt) return;
+  out[i] = ev[idx[i]];
+  omid[i] = lmid[idx[i]];
+  oerr[i] = lerr[idx[i]];
 }
 
 // Support records of facade events: out[5i] = size, out[5i + 1..4] = ids (unused 0); an
@@ -600,7 +609,20 @@ struct DescentParams {
   uint32_t mask;
   const uint32_t* bfac;
   uint32_t nbirths;
+  const uint32_t* birth_event;  // facade index of the birth of handle n + i
+  const double* lmid;           // level intervals of the facade, mid -+ err
+  const double* lerr;
 };
+
+// A queued facet (64 bytes): its ids, ascending (unused kInvalid32), and what its level must lie
+// strictly below: the support of the facet it came from (unused kInvalid32; the first one kInvalid32:
+// nothing to check) and the lower end of that one's level interval.
+struct __align__(16) QFacet {
+  uint32_t F[kMaxFacet];
+  uint32_t prev[4];
+  double prev_lo;
+};
+static_assert(sizeof(QFacet) == 64, "four 16-byte words");
 
 __device__ uint32_t probe_facet(const DescentParams& d, const uint32_t* F, int k) {
   if (k == 1) return F[0];  // order-one births are the singletons, handle = PointId
@@ -1035,7 +1057,7 @@ __device__ __forceinline__ int arm_facet(const EvRec& e, uint32_t removed, uint3
 __global__ void k_arm_probe(DescentParams d, uint32_t f0, uint32_t nfam, const uint32_t* __restrict__ fam_event,
                             const uint32_t* __restrict__ armoff, const EvRec* __restrict__ ev,
                             uint32_t* __restrict__ removed, uint32_t* __restrict__ term, uint32_t* __restrict__ q_arm,
-                            uint32_t* __restrict__ q_fac, uint32_t q_cap, uint32_t* __restrict__ q_count) {
+                            QFacet* __restrict__ q_fac, uint32_t q_cap, uint32_t* __restrict__ q_count) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool on = i < nfam;
   const uint32_t f = f0 + (on ? i : 0u), a0 = armoff[f];
@@ -1060,114 +1082,504 @@ __global__ void k_arm_probe(DescentParams d, uint32_t f0, uint32_t nfam, const u
     const uint32_t slot = base + __popc(b & ((1u << lane) - 1u));
     if (!miss || slot >= q_cap) continue;
     q_arm[slot] = a0 + t;
-    for (int j = 0; j < kMaxFacet; ++j) q_fac[(uint64_t)slot * kMaxFacet + j] = j < k ? F[j] : kInvalid32;
+    QFacet q;
+    for (int j = 0; j < kMaxFacet; ++j) q.F[j] = j < k ? F[j] : kInvalid32;
+    for (int j = 0; j < 4; ++j) q.prev[j] = kInvalid32;
+    q.prev_lo = 0.0;
+    q_fac[slot] = q;
   }
 }
 
-// One strict descent step for every queued arm: exact miniball of F, exact canonical
-// top-k choice G at its centre, certified beta(G) < beta(F); G is probed and either
-// binds the arm or is queued for the next step.
-// Blocks per SM the descent step's register budget is sized for: 8 x 128 threads gives 64
-// registers and 32 warps per SM; the spills cost less than the latency they hide (measured at
-// 50k: 3 blocks 246 ms, 4 222, 6 188, 8 172, 10 168, 12 176).
-#ifndef EHGP_STEP_BLOCKS_PER_SM
-#define EHGP_STEP_BLOCKS_PER_SM 8
-#endif
 // Sort keys of a descent queue: the top 24 bits of the Morton code of each facet's least
 // point, so that a warp's threads descend from nearby facets (shared traversal paths,
 // less divergence).  The order of processing never changes a result.
-__global__ void k_queue_keys(uint32_t m, const uint32_t* __restrict__ in_fac, const uint64_t* __restrict__ code,
+__global__ void k_queue_keys(uint32_t m, const QFacet* __restrict__ in_fac, const uint64_t* __restrict__ code,
                              uint64_t* __restrict__ key, uint32_t* __restrict__ val) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
-  key[i] = code[in_fac[(uint64_t)i * kMaxFacet]] >> 39;
+  key[i] = code[in_fac[i].F[0]] >> 39;
   val[i] = i;
 }
 
-__global__ void __launch_bounds__(128, EHGP_STEP_BLOCKS_PER_SM)
-k_arm_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, const uint32_t* __restrict__ in_fac,
-           const uint32_t* __restrict__ rstate, int passes, const uint32_t* __restrict__ v0,
-           const uint32_t* __restrict__ v1, uint32_t* __restrict__ out_arm, uint32_t* __restrict__ out_fac,
-           uint32_t* __restrict__ out_count, uint32_t* __restrict__ term, unsigned long long* __restrict__ stats) {
+// ---- one strict descent step for every queued arm -------------------------------------------------
+// Exact miniball of F, exact canonical top-k choice G at its centre, certified beta(G) < beta(F); G is
+// probed and either binds the arm or is queued for the next step.  A round is three launches:
+//  k_facet_ball  proposes the support of F's miniball in binary32 and certifies it in binary64;
+//  k_facet_step  takes the points inside the ball from the LBVH, forms G, checks the level, probes;
+//  k_facet_exact runs the arms that either of them left open: the exact fallbacks for every decision.
+// The first two make no call (what lives across one goes to local memory) and keep no array in local
+// memory; when G is not a birth, the next round's k_facet_ball checks that its level decreased; a birth's
+// level interval is known.  Bound: latency of the walk's node loads and its divergence.
+// One kernel with the exact fallbacks in its loops, a binary64 miniball of F and one of G per step and a
+// sorted candidate list per thread took 104.4 ms over all rounds at 50,653 lattice points (32.2 M
+// steps) and 27.6 at 12,289 uniform ones; the three launches take 32.5 and 11.8 ms.
+
+// Counts places of the lanes that have `on` set; `at` of the others is not defined.
+__device__ __forceinline__ uint32_t warp_slot(bool on, uint32_t* count) {
+  const uint32_t lane = threadIdx.x & 31u, b = __ballot_sync(0xffffffffu, on);
+  uint32_t base = 0;
+  if (lane == 0 && b) base = atomicAdd(count, (uint32_t)__popc(b));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  return base + __popc(b & ((1u << lane) - 1u));
+}
+
+// Side of the point at offset (x, y, z) from T[0] of the sphere of T: -1 inside, 1 outside, 0 when binary64
+// does not decide (the bounds of inside_closed).
+__device__ __forceinline__ int side_fp(const FSphere& fs, int ts, double x, double y, double z) {
+  const double Mp = fmax(fs.M, fmax(fabs(x), fmax(fabs(y), fabs(z)))) * (1.0 + 1e-15);
+  const double q = (x * x + y * y) + z * z;
+  const double v = fs.A * q - ((x * fs.Nx + y * fs.Ny) + z * fs.Nz);
+  const double M2 = fs.M * fs.M, M4 = M2 * M2;
+  const double Am = ts <= 2 ? 1.0 : (ts == 3 ? 18.0 * M4 : 6.0 * M2 * fs.M);
+  const double Nm = ts == 1 ? 0.0 : (ts == 2 ? fs.M : (ts == 3 ? 36.0 * M4 * fs.M : 18.0 * M4));
+  const double bnd = kFilt * (Am * 3.0 * Mp * Mp + 3.0 * Mp * Nm) + kTiny;
+  const double w = fs.A < 0.0 ? -v : v;
+  if (!(fabs(fs.A) > fs.eA)) return 0;
+  return w < -bnd ? -1 : (w > bnd ? 1 : 0);
+}
+
+// The circumcentre of T lies strictly inside its hull for certain (the bounds of hull_centre).
+__device__ __forceinline__ bool hull_fp(const Cloud& c, const uint32_t (&T)[4], int ts) {
+  if (ts <= 2) return ts == 2;
+  double e[3][3], M = 0.0;
+#pragma unroll
+  for (int j = 1; j < 4; ++j) {
+    if (j >= ts) {
+      e[j - 1][0] = e[j - 1][1] = e[j - 1][2] = 0.0;
+      continue;
+    }
+    e[j - 1][0] = c.px[T[j]] - c.px[T[0]];
+    e[j - 1][1] = c.py[T[j]] - c.py[T[0]];
+    e[j - 1][2] = c.pz[T[j]] - c.pz[T[0]];
+    M = fmax(M, fmax(fabs(e[j - 1][0]), fmax(fabs(e[j - 1][1]), fabs(e[j - 1][2]))));
+  }
+  M *= (1.0 + 1e-15);
+  const double M2 = M * M;
+  if (ts == 3) {
+    const double G11 = (e[0][0] * e[0][0] + e[0][1] * e[0][1]) + e[0][2] * e[0][2];
+    const double G22 = (e[1][0] * e[1][0] + e[1][1] * e[1][1]) + e[1][2] * e[1][2];
+    const double G12 = (e[0][0] * e[1][0] + e[0][1] * e[1][1]) + e[0][2] * e[1][2];
+    const double b2 = kFilt * 6.0 * M2 + kTiny;
+    return G12 > kFilt * 3.0 * M2 + kTiny && G11 - G12 > b2 && G22 - G12 > b2 &&
+           G11 * G22 - G12 * G12 > kFilt * 18.0 * M2 * M2 + kTiny;
+  }
+  const double* e1 = e[0];
+  const double* e2 = e[1];
+  const double* e3 = e[2];
+  const double c23x = e2[1] * e3[2] - e2[2] * e3[1], c23y = e2[2] * e3[0] - e2[0] * e3[2], c23z = e2[0] * e3[1] - e2[1] * e3[0];
+  const double c31x = e3[1] * e1[2] - e3[2] * e1[1], c31y = e3[2] * e1[0] - e3[0] * e1[2], c31z = e3[0] * e1[1] - e3[1] * e1[0];
+  const double c12x = e1[1] * e2[2] - e1[2] * e2[1], c12y = e1[2] * e2[0] - e1[0] * e2[2], c12z = e1[0] * e2[1] - e1[1] * e2[0];
+  const double q1 = (e1[0] * e1[0] + e1[1] * e1[1]) + e1[2] * e1[2];
+  const double q2 = (e2[0] * e2[0] + e2[1] * e2[1]) + e2[2] * e2[2];
+  const double q3 = (e3[0] * e3[0] + e3[1] * e3[1]) + e3[2] * e3[2];
+  const double detE = (e1[0] * c23x + e1[1] * c23y) + e1[2] * c23z;
+  const double Nx = (q1 * c23x + q2 * c31x) + q3 * c12x;
+  const double Ny = (q1 * c23y + q2 * c31y) + q3 * c12y;
+  const double Nz = (q1 * c23z + q2 * c31z) + q3 * c12z;
+  const double l1 = (Nx * c23x + Ny * c23y) + Nz * c23z;
+  const double l2 = (Nx * c31x + Ny * c31y) + Nz * c31z;
+  const double l3 = (Nx * c12x + Ny * c12y) + Nz * c12z;
+  const double l0 = (2.0 * detE) * detE - ((l1 + l2) + l3);
+  const double M6 = M2 * M2 * M2, bl = kFilt * 108.0 * M6 + kTiny;
+  return fabs(detE) > kFilt * 6.0 * M2 * M + kTiny && l0 > kFilt * 396.0 * M6 + kTiny && l1 > bl && l2 > bl && l3 > bl;
+}
+
+constexpr int kFT = 128;           // threads per block of the two fast kernels
+constexpr int kBallRounds = 24;    // pivots of the proposal before an arm is left open
+
+// Miniball of every queued facet: T (ascending ids, unused kInvalid32) when it is certified and its level lies
+// below the one it must, else the entry goes to `hard` and T.x is kInvalid32.
+// The proposal pivots on the farthest point: the ball of the support so far and that point (at most five
+// points, Welzl's recursion with the new point on the sphere) until nothing lies outside.  Binary32 on
+// differences scaled by a power of two, in shared memory (dynamic indices).
+__global__ void __launch_bounds__(kFT, 8)
+k_facet_ball(DescentParams d, uint32_t m, const QFacet* __restrict__ in_fac, const uint32_t* __restrict__ rstate, int passes,
+             const uint32_t* __restrict__ v0, const uint32_t* __restrict__ v1, uint4* __restrict__ support,
+             uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count) {
+  __shared__ float sx[kMaxFacet][kFT], sy[kMaxFacet][kFT], sz[kMaxFacet][kFT];
+  const uint32_t t = blockIdx.x * kFT + threadIdx.x, w = threadIdx.x;
+  bool open = false;
+  uint32_t i = 0;
+  if (t < m) {
+    i = passes >= 0 ? radix_result(rstate, passes, v0, v1)[t] : t;
+    const QFacet& e = in_fac[i];
+    const uint32_t f0 = e.F[0];
+    const double ax = d.px[f0], ay = d.py[f0], az = d.pz[f0];
+    int k = 0;
+    float M = 0.f;
+    for (int q = 0; q < kMaxFacet; ++q) {
+      const uint32_t id = e.F[q];
+      if (id == kInvalid32) break;
+      const float x = (float)(d.px[id] - ax), y = (float)(d.py[id] - ay), z = (float)(d.pz[id] - az);
+      sx[q][w] = x;
+      sy[q][w] = y;
+      sz[q][w] = z;
+      M = fmaxf(M, fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))));
+      ++k;
+    }
+    open = !(M > 1e-30f && M < 1e30f);
+    const float scale = open ? 1.f : exp2f((float)-ilogbf(M));
+    for (int q = 0; q < k; ++q) {
+      sx[q][w] *= scale;
+      sy[q][w] *= scale;
+      sz[q][w] *= scale;
+    }
+    float cx = 0.f, cy = 0.f, cz = 0.f, r2 = 0.f;
+    uint32_t T = 0;  // positions of the support's points, 8 bits each
+    int ts = 1, round = 0;
+    auto outside = [&](uint32_t q) {
+      const float x = sx[q][w] - cx, y = sy[q][w] - cy, z = sz[q][w] - cz;
+      return x * x + y * y + z * z > r2 * (1.f + 1e-5f) + 1e-12f;
+    };
+    // ball through the points of `idx` (8 bits each), s of them
+    auto ball = [&](uint32_t idx, int s) {
+      T = idx;
+      ts = s;
+      const uint32_t a = idx & 255u, p1 = idx >> 8 & 255u;
+      const float ox = sx[a][w], oy = sy[a][w], oz = sz[a][w];
+      const float x1 = sx[p1][w] - ox, y1 = sy[p1][w] - oy, z1 = sz[p1][w] - oz;
+      const float q1 = x1 * x1 + y1 * y1 + z1 * z1;
+      float A = 1.f, n0 = x1, n1 = y1, n2 = z1;  // two points
+      if (s > 2) {
+        const uint32_t p2 = idx >> 16 & 255u;
+        const float x2 = sx[p2][w] - ox, y2 = sy[p2][w] - oy, z2 = sz[p2][w] - oz;
+        const float q2 = x2 * x2 + y2 * y2 + z2 * z2;
+        if (s == 3) {
+          const float g = x1 * x2 + y1 * y2 + z1 * z2;
+          const float f1 = q2 * (q1 - g), f2 = q1 * (q2 - g);
+          A = q1 * q2 - g * g;
+          n0 = f1 * x1 + f2 * x2;
+          n1 = f1 * y1 + f2 * y2;
+          n2 = f1 * z1 + f2 * z2;
+        } else {
+          const uint32_t p3 = idx >> 24;
+          const float x3 = sx[p3][w] - ox, y3 = sy[p3][w] - oy, z3 = sz[p3][w] - oz;
+          const float q3 = x3 * x3 + y3 * y3 + z3 * z3;
+          const float ax3 = y2 * z3 - z2 * y3, ay3 = z2 * x3 - x2 * z3, az3 = x2 * y3 - y2 * x3;
+          const float bx3 = y3 * z1 - z3 * y1, by3 = z3 * x1 - x3 * z1, bz3 = x3 * y1 - y3 * x1;
+          const float cx3 = y1 * z2 - z1 * y2, cy3 = z1 * x2 - x1 * z2, cz3 = x1 * y2 - y1 * x2;
+          A = x1 * ax3 + y1 * ay3 + z1 * az3;
+          n0 = q1 * ax3 + q2 * bx3 + q3 * cx3;
+          n1 = q1 * ay3 + q2 * by3 + q3 * cy3;
+          n2 = q1 * az3 + q2 * bz3 + q3 * cz3;
+        }
+      }
+      const float inv = __fdividef(0.5f, A);
+      n0 *= inv;
+      n1 *= inv;
+      n2 *= inv;
+      cx = ox + n0;
+      cy = oy + n1;
+      cz = oz + n2;
+      r2 = n0 * n0 + n1 * n1 + n2 * n2;
+    };
+    for (; !open && round < kBallRounds; ++round) {
+      float far = r2 * (1.f + 1e-5f) + 1e-12f;
+      uint32_t f = 255u;
+      for (int q = 0; q < k; ++q) {
+        const float x = sx[q][w] - cx, y = sy[q][w] - cy, z = sz[q][w] - cz;
+        const float dd = x * x + y * y + z * z;
+        if (dd > far) {
+          far = dd;
+          f = (uint32_t)q;
+        }
+      }
+      if (f == 255u) break;
+      const uint32_t old = T;
+      const int n_old = ts;
+      cx = sx[f][w];
+      cy = sy[f][w];
+      cz = sz[f][w];
+      r2 = 0.f;
+      T = f;
+      ts = 1;
+      for (int j = 0; j < n_old; ++j) {
+        const uint32_t pj = old >> (8 * j) & 255u;
+        if (!outside(pj)) continue;
+        ball(f | pj << 8, 2);
+        for (int l = 0; l < j; ++l) {
+          const uint32_t pl = old >> (8 * l) & 255u;
+          if (!outside(pl)) continue;
+          ball(f | pj << 8 | pl << 16, 3);
+          for (int n = 0; n < l; ++n) {
+            const uint32_t pn = old >> (8 * n) & 255u;
+            if (outside(pn)) ball(f | pj << 8 | pl << 16 | pn << 24, 4);
+          }
+        }
+      }
+    }
+    open = open || round == kBallRounds || ts < 2;
+    // certificate in binary64
+    uint4 out = make_uint4(kInvalid32, kInvalid32, kInvalid32, kInvalid32);
+    if (!open) {
+      uint32_t id[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) id[j] = j < ts ? e.F[T >> (8 * j) & 255u] : kInvalid32;
+      auto cswap = [](uint32_t& x, uint32_t& y) {
+        const uint32_t lo = min(x, y), hi = max(x, y);
+        x = lo;
+        y = hi;
+      };
+      cswap(id[0], id[1]);
+      cswap(id[2], id[3]);
+      cswap(id[0], id[2]);
+      cswap(id[1], id[3]);
+      cswap(id[1], id[2]);
+      const Cloud c{d.px, d.py, d.pz, d.S};
+      open = !hull_fp(c, id, ts);
+      FSphere fs;
+      if (!open) {
+        fsphere(d.px, d.py, d.pz, id, ts, fs);
+        double lo, hi;
+        open = !flevel(fs, lo, hi) || (e.prev[0] != kInvalid32 && !(hi < e.prev_lo));
+      }
+      for (int q = 0; q < k && !open; ++q) {
+        const uint32_t p = e.F[q];
+        if (p == id[0] || p == id[1] || p == id[2] || p == id[3]) continue;
+        open = side_fp(fs, ts, d.px[p] - fs.ax, d.py[p] - fs.ay, d.pz[p] - fs.az) >= 0;
+      }
+      if (!open) out = make_uint4(id[0], id[1], id[2], id[3]);
+    }
+    support[i] = out;
+  }
+  const uint32_t slot = warp_slot(open, hard_count);
+  if (open) hard[slot] = i;
+}
+
+constexpr int kStepStack = 32;  // traversal entries per thread (an arm that needs more is left open)
+constexpr int kStepIn = 20;     // points inside the ball per thread (likewise)
+
+// The step of every facet with a certified support: points strictly inside its miniball come from the LBVH;
+// with fewer than k of them the choice is those and the least support points (which lie on the sphere),
+// with exactly k those.  Any point that binary64 does not place, more than k inside points, or an arm that
+// would fail goes to `hard`.
+__global__ void __launch_bounds__(kFT, 6)
+k_facet_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, const QFacet* __restrict__ in_fac,
+             const uint4* __restrict__ support, const uint32_t* __restrict__ rstate, int passes,
+             const uint32_t* __restrict__ v0, const uint32_t* __restrict__ v1, uint32_t* __restrict__ out_arm,
+             QFacet* __restrict__ out_fac, uint32_t* __restrict__ out_count, uint32_t* __restrict__ term,
+             unsigned long long* __restrict__ stats, uint32_t* __restrict__ hard, uint32_t* __restrict__ hard_count) {
+  __shared__ uint32_t stack[kStepStack][kFT], inside[kStepIn][kFT];
   // Work counters leave through shared memory with the block's last warp (no warp waits for another);
   // a global atomic per arm and counter queues every arm on one address.
-  __shared__ unsigned int s_count[4], s_warps;  // node visits, steps, equal cutoffs, strictness checks
-  const uint32_t lane = threadIdx.x & 31u;
-  if (threadIdx.x < 4) s_count[threadIdx.x] = 0;
-  if (threadIdx.x == 4) s_warps = 0;
+  __shared__ unsigned int s_count[3], s_warps;  // node visits, steps, equal cutoffs
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x;
+  if (w < 3) s_count[w] = 0;
+  if (w == 3) s_warps = 0;
   __syncthreads();
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t F[kMaxFacet], G[kMaxFacet];
-  uint32_t a = 0, visits = 0, stepped = 0, equal = 0, strict = 0;
-  int k = 0;
-  bool go_on = false;  // G is no birth facet: queued for the next step
+  const uint32_t t = blockIdx.x * kFT + w;
+  uint32_t i = 0, visits = 0, stepped = 0, equal = 0, G[kMaxFacet];
+  bool open = false, go_on = false;
+  double llo = 0.0, lhi = 0.0;
+  uint32_t T[4] = {kInvalid32, kInvalid32, kInvalid32, kInvalid32};
   if (t < m) {
-    // queue entry: in Morton order of the facets when the queue was sorted (passes >= 0)
-    const uint32_t i = passes >= 0 ? radix_result(rstate, passes, v0, v1)[t] : t;
-    a = in_arm[i];
-    for (int j = 0; j < kMaxFacet; ++j) {
-      F[j] = in_fac[(uint64_t)i * kMaxFacet + j];
-      k += F[j] != kInvalid32;
+    i = passes >= 0 ? radix_result(rstate, passes, v0, v1)[t] : t;
+    const uint4 sup = support[i];
+    T[0] = sup.x;
+    T[1] = sup.y;
+    T[2] = sup.z;
+    T[3] = sup.w;
+  }
+  if (T[0] != kInvalid32) {
+    const int ts = T[2] == kInvalid32 ? 2 : (T[3] == kInvalid32 ? 3 : 4);
+    double cx, cy, cz, R2, ed;
+    {
+      FSphere fs;
+      fsphere(d.px, d.py, d.pz, T, ts, fs);
+      flevel(fs, llo, lhi);  // certified by k_facet_ball
+      // FP64 centre and its error: c~ = a + N / (2A)
+      const double inv = 0.5 / fs.A;
+      const double ox = fs.Nx * inv, oy = fs.Ny * inv, oz = fs.Nz * inv;
+      cx = fs.ax + ox;
+      cy = fs.ay + oy;
+      cz = fs.az + oz;
+      const double on = sqrt(ox * ox + oy * oy + oz * oz);
+      const double nn = sqrt(fs.Nx * fs.Nx + fs.Ny * fs.Ny + fs.Nz * fs.Nz);
+      const double relA = fs.eA / fmax(fabs(fs.A) - fs.eA, 1e-300);
+      const double relN = fs.eN * 1.7320508075688772 / fmax(nn, 1e-300);
+      const double dc = on * (relA + relN) * 1.01 + 4.0 * kU * (fabs(cx) + fabs(cy) + fabs(cz)) + kTiny;
+      const double R = sqrt(lhi) * (1.0 + 1e-12) + dc;
+      R2 = R * R * (1.0 + 1e-12);
+      ed = 2.0 * R * dc + dc * dc + 8.0 * kU * R2 + kTiny;
+      open = !(relA < 0.5) || !isfinite(dc) || !(fabs(cx) < 0x1p60 && fabs(cy) < 0x1p60 && fabs(cz) < 0x1p60 && R2 < 0x1p100);
     }
-    const Cloud c{d.px, d.py, d.pz, d.S};
-    auto step = [&]() -> int {
-      Mini mb;
-      if (!facet_miniball(c, F, k, mb)) return kArmInternal;
-      int cut_below = 0;
-      const int s = topk_choice(d, c, mb, k, G, &cut_below, &visits);
-      if (s != kArmOk) return s;
-      bool same = true;
-      for (int j = 0; j < k; ++j) same &= G[j] == F[j];
-      if (same) return kArmUnresolved;
-      if (!cut_below) {  // beta(G) <= cutoff = beta(F): the decrease must be strict
-        equal = 1;
-        Mini mg;
-        if (!facet_miniball(c, G, k, mg)) return kArmInternal;
-        double glo, ghi, flo, fhi;
-        if (!flevel(mg.fs, glo, ghi)) exact_level_fp(c, mg.T, mg.ts, glo, ghi);
-        if (!flevel(mb.fs, flo, fhi)) exact_level_fp(c, mb.T, mb.ts, flo, fhi);
-        if (!(ghi < flo) && level_cmp_exact(c, mg.T, mg.ts, mb.T, mb.ts) >= 0) return kArmPlateau;
-        strict = 1;
+    // binary32 prune as in topk_choice: a lower bound of the distance to a node box, from the rounded centre
+    const float qx = (float)cx, qy = (float)cy, qz = (float)cz;
+    const float dq = fmaxf(__double2float_ru(fabs(cx - (double)qx)),
+                           fmaxf(__double2float_ru(fabs(cy - (double)qy)), __double2float_ru(fabs(cz - (double)qz))));
+    const float R2f = __double2float_ru(R2);
+    const double in2 = llo - ed, out2 = lhi + ed;  // FP distances below / above them are inside / outside for certain
+    uint32_t n_in = 0;
+    int top = 0;
+    if (!open) stack[top++][w] = d.root;
+    while (top > 0) {
+      const TNode nd = load_node(d.tn, stack[--top][w]);
+      ++visits;
+      if (nd.left != kInvalid32) {
+        const float g0 = fmaxf(fmaxf(fmaxf(nd.lo[0] - qx, qx - nd.hi[0]), 0.f) * (1.f - 0x1p-22f) - dq, 0.f);
+        const float g1 = fmaxf(fmaxf(fmaxf(nd.lo[1] - qy, qy - nd.hi[1]), 0.f) * (1.f - 0x1p-22f) - dq, 0.f);
+        const float g2 = fmaxf(fmaxf(fmaxf(nd.lo[2] - qz, qz - nd.hi[2]), 0.f) * (1.f - 0x1p-22f) - dq, 0.f);
+        if ((g0 * g0 + g1 * g1 + g2 * g2) * (1.f - 0x1p-20f) > R2f) continue;
+        if (top + 2 > kStepStack) {
+          open = true;
+          break;
+        }
+        stack[top++][w] = nd.left;
+        stack[top++][w] = nd.right;
+        continue;
       }
-      stepped = 1;
-      return kArmOk;
-    };
-    const int why = step();
-    if (why != kArmOk) {  // failed arms, and the least of them with its status
-      atomicAdd(stats + 2, 1ull);
-      atomicMin(stats + 3, (unsigned long long)a << 8 | (unsigned long long)why);
-    } else {
-      const uint32_t h = probe_facet(d, G, k);
-      go_on = h == kInvalid32;
-      if (!go_on) term[a] = h;
+      const uint32_t q = nd.right;
+      const double dx = d.px[q] - cx, dy = d.py[q] - cy, dz = d.pz[q] - cz;
+      const double dd = dx * dx + dy * dy + dz * dz;
+      if (dd > out2 || q == T[0] || q == T[1] || q == T[2] || q == T[3]) continue;
+      if (!(dd < in2) || n_in == (uint32_t)kStepIn) {
+        open = true;
+        break;
+      }
+      inside[n_in++][w] = q;
+    }
+    const QFacet& e = in_fac[i];
+    uint32_t k = 0;
+#pragma unroll
+    for (int j = 0; j < kMaxFacet; ++j) k += e.F[j] != kInvalid32 ? 1u : 0u;
+    open = open || n_in > k || n_in + (uint32_t)ts < k;
+    if (!open) {
+      // G ascending: the inside points, then the least support points
+#pragma unroll
+      for (int j = 0; j < kMaxFacet; ++j) G[j] = kInvalid32;
+      auto put = [&](uint32_t x) {
+#pragma unroll
+        for (int j = 0; j < kMaxFacet; ++j) {
+          const uint32_t lo = min(G[j], x);
+          x = max(G[j], x);
+          G[j] = lo;
+        }
+      };
+      for (uint32_t q = 0; q < n_in; ++q) put(inside[q][w]);
+      const bool at_level = n_in < k;  // the cutoff is beta(F): beta(G) must be shown to be less
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (n_in + j < k) put(T[j]);
+      bool same = true;
+#pragma unroll
+      for (int j = 0; j < kMaxFacet; ++j) same &= G[j] == e.F[j];
+      const uint32_t h = same ? kInvalid32 : probe_facet(d, G, (int)k);
+      open = same;
+      if (h != kInvalid32) {
+        const uint32_t ev = d.birth_event[h - d.n];
+        if (at_level && !(d.lmid[ev] + d.lerr[ev] < llo)) open = true;
+        else term[in_arm[i]] = h;
+      } else {
+        go_on = !open;
+        if (!at_level) T[0] = kInvalid32;  // a cutoff below the level: nothing to check
+      }
+      if (!open) {
+        stepped = 1;
+        equal = at_level ? 1u : 0u;
+      }
     }
   }
   __syncwarp();
-  const uint32_t b = __ballot_sync(0xffffffffu, go_on);
-  uint32_t base = 0;
-  if (lane == 0 && b) base = atomicAdd(out_count, (uint32_t)__popc(b));
-  base = __shfl_sync(0xffffffffu, base, 0);
+  const uint32_t slot = warp_slot(go_on, out_count), hslot = warp_slot(open, hard_count);
   if (go_on) {
-    const uint32_t slot = base + __popc(b & ((1u << lane) - 1u));
-    out_arm[slot] = a;
-    for (int j = 0; j < kMaxFacet; ++j) out_fac[(uint64_t)slot * kMaxFacet + j] = j < k ? G[j] : kInvalid32;
+    out_arm[slot] = in_arm[i];
+    QFacet q;
+#pragma unroll
+    for (int j = 0; j < kMaxFacet; ++j) q.F[j] = G[j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q.prev[j] = T[j];
+    q.prev_lo = llo;
+    out_fac[slot] = q;
   }
+  if (open) hard[hslot] = i;
   visits = __reduce_add_sync(0xffffffffu, visits);
   stepped = __reduce_add_sync(0xffffffffu, stepped);
   equal = __reduce_add_sync(0xffffffffu, equal);
-  strict = __reduce_add_sync(0xffffffffu, strict);
   if (lane != 0) return;
   atomicAdd(s_count + 0, visits);
   atomicAdd(s_count + 1, stepped);
   atomicAdd(s_count + 2, equal);
-  atomicAdd(s_count + 3, strict);
   __threadfence_block();
-  if (atomicAdd(&s_warps, 1u) + 1 < blockDim.x / 32) return;
+  if (atomicAdd(&s_warps, 1u) + 1 < kFT / 32) return;
   __threadfence_block();
   atomicAdd(&g_descent_visits[blockIdx.x % kVisitStripes], (unsigned long long)atomicAdd(s_count + 0, 0u));
-  atomicAdd(stats, (unsigned long long)atomicAdd(s_count + 1, 0u));
-  atomicAdd(&g_descent_slow[6], (unsigned long long)atomicAdd(s_count + 2, 0u));
-  atomicAdd(stats + 1, (unsigned long long)atomicAdd(s_count + 3, 0u));
+  const unsigned int n_step = atomicAdd(s_count + 1, 0u), n_equal = atomicAdd(s_count + 2, 0u);
+  atomicAdd(stats, (unsigned long long)n_step);
+  atomicAdd(stats + 1, (unsigned long long)n_equal);
+  atomicAdd(&g_descent_slow[6], (unsigned long long)n_equal);
+}
+
+// The whole step of the queue entries in `hard`, with the exact fallbacks.
+__global__ void __launch_bounds__(128)
+k_facet_exact(DescentParams d, uint32_t m, const uint32_t* __restrict__ hard, const uint32_t* __restrict__ in_arm,
+              const QFacet* __restrict__ in_fac, uint32_t* __restrict__ out_arm, QFacet* __restrict__ out_fac,
+              uint32_t* __restrict__ out_count, uint32_t* __restrict__ term, unsigned long long* __restrict__ stats) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t F[kMaxFacet], G[kMaxFacet], a = 0, visits = 0;
+  int k = 0;
+  bool go_on = false;
+  Mini mb;
+  int cut_below = 0;
+  double flo = 0.0, fhi = 0.0;
+  if (t < m) {
+    const uint32_t i = hard[t];
+    const QFacet e = in_fac[i];
+    a = in_arm[i];
+    for (int j = 0; j < kMaxFacet; ++j) {
+      F[j] = e.F[j];
+      k += F[j] != kInvalid32;
+    }
+    const Cloud c{d.px, d.py, d.pz, d.S};
+    // level(lo, hi, S) strictly below the interval or the support it is compared with
+    auto below = [&](const Mini& x, const uint32_t* T, int ts, double tlo) {
+      double lo, hi;
+      if (!flevel(x.fs, lo, hi)) exact_level_fp(c, x.T, x.ts, lo, hi);
+      return hi < tlo || level_cmp_exact(c, x.T, x.ts, T, ts) < 0;
+    };
+    auto step = [&]() -> int {
+      if (!facet_miniball(c, F, k, mb)) return kArmInternal;
+      if (e.prev[0] != kInvalid32) {
+        int ts = 1;
+        while (ts < 4 && e.prev[ts] != kInvalid32) ++ts;
+        if (!below(mb, e.prev, ts, e.prev_lo)) return kArmPlateau;
+      }
+      const int s = topk_choice(d, c, mb, k, G, &cut_below, &visits);
+      if (s != kArmOk) return s;
+      bool same = true;
+      for (int j = 0; j < k; ++j) same &= G[j] == F[j];
+      return same ? kArmUnresolved : kArmOk;
+    };
+    int why = step();
+    if (why == kArmOk) {
+      if (!flevel(mb.fs, flo, fhi)) exact_level_fp(c, mb.T, mb.ts, flo, fhi);
+      if (!cut_below) slow(6);
+      const uint32_t h = probe_facet(d, G, k);
+      go_on = h == kInvalid32;
+      if (!go_on) {
+        Mini mg;  // beta(G) <= cutoff = beta(F): the decrease must be strict
+        if (!cut_below && !facet_miniball(c, G, k, mg)) why = kArmInternal;
+        else if (!cut_below && !below(mg, mb.T, mb.ts, flo)) why = kArmPlateau;
+        else term[a] = h;
+      }
+    }
+    if (why != kArmOk) {  // failed arms, and the least of them with its status
+      atomicAdd(stats + 2, 1ull);
+      atomicMin(stats + 3, (unsigned long long)a << 8 | (unsigned long long)why);
+    } else {
+      atomicAdd(stats, 1ull);
+      if (!cut_below) atomicAdd(stats + 1, 1ull);
+    }
+    atomicAdd(&g_descent_visits[blockIdx.x % kVisitStripes], (unsigned long long)visits);
+  }
+  __syncwarp();
+  const uint32_t slot = warp_slot(go_on, out_count);
+  if (!go_on) return;
+  out_arm[slot] = a;
+  QFacet q;
+  for (int j = 0; j < kMaxFacet; ++j) q.F[j] = j < k ? G[j] : kInvalid32;
+  for (int j = 0; j < 4; ++j) q.prev[j] = !cut_below && j < mb.ts ? mb.T[j] : kInvalid32;
+  q.prev_lo = flo;
+  out_fac[slot] = q;
 }
 
 }  // namespace
@@ -1461,11 +1873,11 @@ int hier_run(Ctx& ctx, uint32_t K) {
     cudaMemcpyAsync(h.tie_pos, idx.data(), (uint64_t)cnt * 4, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(h.run_off, run_off.data(), (uint64_t)(nruns + 1) * 4, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(h.run_lo, run_lo.data(), (uint64_t)nruns * 4, cudaMemcpyHostToDevice, st);
-    k_run_gather<<<nblk(cnt, kT), kT, 0, st>>>(cnt, h.tie_pos, h.ev, h.ev_raw);
+    k_run_gather<<<nblk(cnt, kT), kT, 0, st>>>(cnt, h.tie_pos, h.ev, h.lmid, h.lerr, h.ev_raw, h.lmid_raw, h.lerr_raw);
     const Cloud dc{b.px, b.py, b.pz, h.S};
     k_tie_keys<<<nblk(cnt, 128), 128, 0, st>>>(cnt, h.tie_pos, h.ev, dc, h.tie_num, h.tie_a2);
-    k_tie_sort<<<nblk(nruns, 64), 64, 0, st>>>(nruns, h.run_off, h.run_lo, h.tie_num, h.tie_a2, h.ev_raw, h.tie_idx,
-                                               h.tie_tmp, h.ev, h.eqprev);
+    k_tie_sort<<<nblk(nruns, 64), 64, 0, st>>>(nruns, h.run_off, h.run_lo, h.tie_num, h.tie_a2, h.ev_raw, h.lmid_raw,
+                                               h.lerr_raw, h.tie_idx, h.tie_tmp, h.ev, h.lmid, h.lerr, h.eqprev);
     launches += 3;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "facade tie runs");
     ms_ties = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tt0).count();
@@ -1555,13 +1967,17 @@ int hier_run(Ctx& ctx, uint32_t K) {
   const uint64_t journal = journal_bytes(in);
   // queue entries: about a third of the arms miss their first probe; a longer queue grows
   uint64_t q_cap = std::min<uint64_t>(narms, std::max<uint64_t>(narms * 3 / 8, 1u << 16)) + 32;
-  uint32_t *q_arm[2], *q_fac[2];
+  uint32_t *q_arm[2], *q_hard;
+  QFacet* q_fac[2];
+  uint4* q_sup;
   auto queues = [&]() -> cudaError_t {
-    cudaError_t r = h.mem.reset(std::max(journal, q_cap * 2 * (4 + 4 * kMaxFacet) + 4096));
+    cudaError_t r = h.mem.reset(std::max(journal, q_cap * (2 * (4 + sizeof(QFacet)) + 4 + 16) + 4096));
     for (int i = 0; i < 2; ++i) {
       if (r == cudaSuccess) r = h.mem.take(&q_arm[i], q_cap);
-      if (r == cudaSuccess) r = h.mem.take(&q_fac[i], q_cap * kMaxFacet);
+      if (r == cudaSuccess) r = h.mem.take(&q_fac[i], q_cap);
     }
+    if (r == cudaSuccess) r = h.mem.take(&q_hard, q_cap);
+    if (r == cudaSuccess) r = h.mem.take(&q_sup, q_cap);
     return r;
   };
   auto no_queue = [&] {
@@ -1572,7 +1988,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
   if (!h.qcount && (e = halloc(h, &h.qcount, 4)) != cudaSuccess)
     return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "descent queue");
   const DescentParams dp{n, 2 * n - 2, g.tnodes, b.px, b.py, b.pz, h.S, h.slots, (uint32_t)(h.cap_slots - 1), h.bfac,
-                         (uint32_t)nb_higher};
+                         (uint32_t)nb_higher, in.ev, h.lmid, h.lerr};
   uint32_t misses = 0, max_rounds = 0;
   h.descent_steps = 0;
   h.ms_steps = 0;
@@ -1605,8 +2021,8 @@ int hier_run(Ctx& ctx, uint32_t K) {
         h.decision = EHGP_ERR_DEGENERATE;
         return abi_fail(&ctx, EHGP_ERR_DEGENERATE, "a strict arm descent exceeded its step budget");
       }
-      uint32_t* oc = h.qcount + 1 + (1 - cur);
-      cudaMemsetAsync(oc, 0, sizeof(uint32_t), st);
+      uint32_t* oc = h.qcount + 1;  // [1] queued for the next round, [2] left open
+      cudaMemsetAsync(oc, 0, 2 * sizeof(uint32_t), st);
       if (h.ev_step[0]) cudaEventRecord(h.ev_step[0], st);
       int spasses = -1;  // large queues run in Morton order of their facets
       if (pending >= kSortQueueMin && pending <= h.cap_events) {
@@ -1614,14 +2030,25 @@ int hier_run(Ctx& ctx, uint32_t K) {
         ++launches;
         spasses = radix_sort_kv(st, pending, h.order0, h.order1, h.key, h.key2, 24, rs, &launches);
       }
-      k_arm_step<<<nblk(pending, 128), 128, 0, st>>>(dp, pending, q_arm[cur], q_fac[cur], ctx.radix.state, spasses,
-                                                     h.order0, h.order1, q_arm[1 - cur], q_fac[1 - cur], oc, h.term,
-                                                     h.dstats);
-      if (h.ev_step[1]) cudaEventRecord(h.ev_step[1], st);
-      ++launches;
+      k_facet_ball<<<nblk(pending, kFT), kFT, 0, st>>>(dp, pending, q_fac[cur], ctx.radix.state, spasses, h.order0, h.order1,
+                                                       q_sup, q_hard, oc + 1);
+      k_facet_step<<<nblk(pending, kFT), kFT, 0, st>>>(dp, pending, q_arm[cur], q_fac[cur], q_sup, ctx.radix.state, spasses,
+                                                       h.order0, h.order1, q_arm[1 - cur], q_fac[1 - cur], oc, h.term,
+                                                       h.dstats, q_hard, oc + 1);
+      launches += 2;
       ++h.step_launches;
-      cudaMemcpyAsync(&pending, oc, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+      uint32_t hq[2] = {0, 0};
+      cudaMemcpyAsync(hq, oc, sizeof(hq), cudaMemcpyDeviceToHost, st);
       if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "strict-arm descent");
+      if (hq[1]) {
+        k_facet_exact<<<nblk(hq[1], 128), 128, 0, st>>>(dp, hq[1], q_hard, q_arm[cur], q_fac[cur], q_arm[1 - cur],
+                                                        q_fac[1 - cur], oc, h.term, h.dstats);
+        ++launches;
+        cudaMemcpyAsync(hq, oc, sizeof(hq), cudaMemcpyDeviceToHost, st);
+      }
+      if (h.ev_step[1]) cudaEventRecord(h.ev_step[1], st);
+      if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "strict-arm descent");
+      pending = hq[0];
       if (h.ev_step[0] && h.ev_step[1]) {
         float sm = 0.f;
         if (cudaEventElapsedTime(&sm, h.ev_step[0], h.ev_step[1]) == cudaSuccess) h.ms_steps += sm;
