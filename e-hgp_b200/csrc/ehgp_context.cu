@@ -148,6 +148,7 @@ int ehgp_ctx_create(int device, const ehgp_limits* limits, ehgp_ctx** out_ctx) {
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->evs1);
   if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_status, 64 * sizeof(uint32_t));
   if (e == cudaSuccess) e = ehgp::ctx_alloc(*ctx, (void**)&ctx->d_err, sizeof(uint32_t));
+  ctx->radix.err = ctx->d_err;
   if (e == cudaSuccess) {
     // admission: the context's resident buffers must fit the HBM fraction
     size_t free_b = 0, total_b = 0;

@@ -1716,7 +1716,7 @@ cudaError_t ensure_events(HierState& h, uint64_t m) {
   HA(h.lclass, cap);
   HA(h.rank_order, cap);
   HA(h.counters, 32);
-  HA(h.radix_counts, 256ull * ((cap + kRadixTile - 1) / kRadixTile) + 256);
+  HA(h.radix_counts, radix_counts_words(cap));
   HA(h.bfac, cap * kMaxFacet);
   HA(h.d_cls_rp, cap);
   HA(h.d_size_rp, cap);
@@ -1804,7 +1804,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
   const uint32_t m = (uint32_t)(total - hc[0]);
   h.events = m;
   // facade order by the FP64 level midpoints (diagnostics sort last)
-  RadixScratch rs{h.radix_counts, ctx.radix.state, (uint32_t)((h.cap_events + kRadixTile - 1) / kRadixTile)};
+  RadixScratch rs{h.radix_counts, ctx.radix.state, ctx.d_err};
   if (total) {
     k_iota<<<nblk(total, kT), kT, 0, st>>>((uint32_t)total, h.order0);
     ++launches;
@@ -2062,7 +2062,9 @@ int hier_run(Ctx& ctx, uint32_t K) {
   cudaMemcpyAsync(dst, h.dstats, sizeof(dst), cudaMemcpyDeviceToHost, st);
   cudaMemcpyFromSymbolAsync(h.slow, g_descent_slow, sizeof(h.slow), 0, cudaMemcpyDeviceToHost, st);
   cudaMemcpyFromSymbolAsync(h.visits, g_descent_visits, sizeof(h.visits), 0, cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(&herr, ctx.d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "strict-arm descent");
+  if (herr) return abi_device_status(&ctx, herr);
   h.first_misses = misses;
   h.descent_rounds = max_rounds;
   h.descent_steps = dst[0];

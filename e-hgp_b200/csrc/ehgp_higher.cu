@@ -2082,7 +2082,7 @@ static void higher_record_bytes(uint64_t c, uint64_t* b) {
   b[3] = c * sizeof(uint64_t);
   b[4] = c * sizeof(uint32_t);
   b[5] = c * sizeof(uint32_t);
-  b[6] = 256ull * ((c + kRadixTile - 1) / kRadixTile) * sizeof(uint32_t);
+  b[6] = radix_counts_words(c) * sizeof(uint32_t);
 }
 
 cudaError_t higher_records_alloc(Ctx& ctx, uint64_t capacity) {
@@ -2545,7 +2545,7 @@ int higher_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
   const uint32_t m = hc[0];
   if (m) {
     k_higher_keys<<<nblocks(m, 256), 256, 0, st>>>(m, (const HigherRec*)h.raw, h.khi, h.klo, h.order0);
-    RadixScratch rs{h.radix_counts, ctx.radix.state, (uint32_t)((h.capacity + kRadixTile - 1) / kRadixTile)};
+    RadixScratch rs{h.radix_counts, ctx.radix.state, ctx.d_err};
     const IndirectKey stages[2] = {{h.klo, 0}, {h.khi, 0}};
     const int bits[2] = {64, 64};
     const int passes = radix_sort_indirect(st, m, h.order0, h.order1, stages, bits, 2, rs, &launches);

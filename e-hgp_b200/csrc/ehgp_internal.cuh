@@ -46,16 +46,17 @@ __host__ __device__ __forceinline__ uint64_t order_key(uint64_t bits) {
 
 // ---- radix sort of u32 indices by an indirect 64-bit key -----------------
 struct RadixScratch {
-  uint32_t* counts = nullptr;   // [256 * max_tiles]
-  uint32_t* state = nullptr;    // per pass: [cur_in, trivial] pairs, kMaxPasses + 1 entries
-  uint32_t max_tiles = 0;
+  uint32_t* counts = nullptr;   // [radix_counts_words(n)] tile counts of two passes
+  uint32_t* state = nullptr;    // [kRadixStateWords]
+  uint32_t* err = nullptr;      // device error word (a bounded wait that ran out)
 };
-constexpr int kRadixThreads = 256;
-constexpr int kRadixItems = 4;
-constexpr int kRadixTile = kRadixThreads * kRadixItems;
-constexpr int kRadixMaxPasses = 32;
-// State words: per pass (input buffer, trivial flag), then 256 digit totals.
-constexpr int kRadixStateWords = 2 * (kRadixMaxPasses + 1) + 256;
+constexpr int kRadixTile = 2048;        // items of one block and pass
+constexpr int kRadixMaxPasses = 24;     // three 64-bit stages
+// State words: per pass (input buffer, trivial flag), digit bases of every pass, tile tickets.
+constexpr int kRadixStateWords = 2 * (kRadixMaxPasses + 1) + 257 * kRadixMaxPasses;
+__host__ __device__ constexpr uint64_t radix_counts_words(uint64_t n) {
+  return 2ull * 256 * ((n + kRadixTile - 1) / kRadixTile);
+}
 
 // Key source for one sorting stage: key(v) = order_key(words[v]) when
 // `order` is set, else words[v].

@@ -1156,7 +1156,7 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
   const uint64_t M = sh.m;
   // sorts m keys; returns the buffers that hold the result
   auto sort = [&](uint64_t m, uint64_t** key, uint32_t** val, int bits, uint64_t** rk, uint32_t** rv, int* passes) -> int {
-    RadixScratch rs{rcounts, ctx.radix.state, nblk(m, kRadixTile)};
+    RadixScratch rs{rcounts, ctx.radix.state, ctx.d_err};
     *passes = radix_sort_kv(st, (uint32_t)m, val[0], val[1], key[0], key[1], bits, rs, launches);
     uint32_t which = 0;
     if ((e = cudaMemcpyAsync(&which, ctx.radix.state + 2 * *passes, 4, cudaMemcpyDeviceToHost, st)) == cudaSuccess)
@@ -1186,7 +1186,7 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
       TAKE(cval[i], 4 * M);
       TAKE(pkey[i], 4 * M);
     }
-    TAKE(rcounts, 256ull * nblk(4 * M, kRadixTile));
+    TAKE(rcounts, radix_counts_words(4 * M));
     prefix_sums<1>(st, F, SharedFlagIn{j}, tot, SharedFlagOut{sh.fam, sh.slot_q}, launches);
     prefix_sums<1>(st, (uint32_t)M, RunIn{j, sh.fam}, tot, RunOut{j, t, sh.fam, pkey[0], cval[0]}, launches);
     uint64_t* key;
@@ -1263,11 +1263,11 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
     TAKE(ncls, Nn);
     TAKE(nidx, Nn);
     uint32_t* ncounts;
-    TAKE(ncounts, 256ull * nblk(Nn, kRadixTile));
+    TAKE(ncounts, radix_counts_words(Nn));
     k_fj_node_keys<<<nblk(F), kT, 0, st>>>(j, sh, gs, car, gc, gp, node_slot, key[0], val[0]);
     int bits = 8;
     while (bits < 32 && (H >> bits)) bits += 8;
-    RadixScratch rs{ncounts, ctx.radix.state, nblk(Nn, kRadixTile)};
+    RadixScratch rs{ncounts, ctx.radix.state, ctx.d_err};
     const int passes = radix_sort_kv(st, Nn, val[0], val[1], key[0], key[1], bits, rs, launches);
     k_fj_node_ranges<<<nblk(Nn), kT, 0, st>>>(Nn, val[0], val[1], key[0], key[1], ctx.radix.state, passes, j.cls, node_slot,
                                               t.range, ncls, nidx);

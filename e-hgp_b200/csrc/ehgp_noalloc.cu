@@ -73,7 +73,7 @@ constexpr uint64_t scratch_bytes() {
   L.take(4);                    // frame_done
   L.take(8 * 4);                // stats
   L.take(2 * n * sizeof(ehgp_lbvh_node) + n * sizeof(ehgp_lbvh_leaf) + n * 8);  // export
-  L.take(256ull * ((n + ehgp::kRadixTile - 1) / ehgp::kRadixTile) * 4);         // radix counts
+  L.take(ehgp::radix_counts_words(n) * 4);  // radix counts
   L.take(ehgp::kRadixStateWords * 4);  // radix state
   L.take(4);                    // error word
   return L.off;
@@ -135,10 +135,10 @@ void carve(ehgp::Ctx& c, unsigned char* base) {
   b.stats = (uint32_t*)at(8 * 4);
   b.export_bytes = 2 * n * sizeof(ehgp_lbvh_node) + n * sizeof(ehgp_lbvh_leaf) + n * 8;
   b.export_buf = at(b.export_bytes);
-  c.radix.max_tiles = (uint32_t)((n + ehgp::kRadixTile - 1) / ehgp::kRadixTile);
-  c.radix.counts = (uint32_t*)at(256ull * c.radix.max_tiles * 4);
+  c.radix.counts = (uint32_t*)at(ehgp::radix_counts_words(n) * 4);
   c.radix.state = (uint32_t*)at(ehgp::kRadixStateWords * 4);
   c.d_err = (uint32_t*)at(4);
+  c.radix.err = c.d_err;
   c.max_points = n;
   // the carve takes exactly the blocks that scratch_bytes() sized
   if (L.off != kScratchBytes) c.max_points = 0;

@@ -657,7 +657,7 @@ static void pair_record_bytes(uint64_t c, uint64_t* b) {
   b[3] = c * sizeof(uint32_t);
   b[4] = c * sizeof(uint32_t);
   b[5] = c * 4 * sizeof(uint64_t);
-  b[6] = 256ull * ((c + kRadixTile - 1) / kRadixTile) * sizeof(uint32_t);
+  b[6] = radix_counts_words(c) * sizeof(uint32_t);
 }
 
 cudaError_t pairs_records_alloc(Ctx& ctx, uint64_t capacity) {
@@ -780,7 +780,7 @@ int pairs_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
   const uint32_t m = hc[0];
   if (m) {
     k_pair_keys<<<(m + 255) / 256, 256, 0, st>>>(m, (const PairRec*)p.raw, p.key, p.order0);
-    RadixScratch rs{p.radix_counts, ctx.radix.state, (uint32_t)((p.capacity + kRadixTile - 1) / kRadixTile)};
+    RadixScratch rs{p.radix_counts, ctx.radix.state, ctx.d_err};
     const IndirectKey stage[1] = {{p.key, 0}};
     const int bits[1] = {64};
     const int passes = radix_sort_indirect(st, m, p.order0, p.order1, stage, bits, 1, rs, &launches);

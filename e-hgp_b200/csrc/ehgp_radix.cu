@@ -1,225 +1,348 @@
-// Stable LSD radix sort of 32-bit indices by indirect 64-bit keys (sm_100a).
+// Stable LSD radix sort of 32-bit indices by 64-bit keys (sm_100a), 8 bits per pass.
 //
-// Used twice on the LBVH path:
-//  * the canonical PointId order: lexicographic (x, y, z) binary64 total-order
-//    keys, i.e. the std::sort of src/cpu/spatial/point_cloud.cpp:58-62;
-//  * the Morton leaf order: (code, PointId), i.e. std::sort with
-//    morton_leaf_less (src/cpu/spatial/lbvh.cpp:93-100,512) -- stability of
-//    the LSD passes over an input in PointId order gives the PointId tie-break.
+// Serves every ordered output of the library: the canonical PointId order and the Morton leaf
+// order (std::sort of src/cpu/spatial/point_cloud.cpp:58-62 and lbvh.cpp:93-100,512; stability over
+// an input in PointId order gives the PointId tie-break), the EMST edge order, the support
+// catalogues, the facade and its rank partition, the descent queues.
 //
-// Each 8-bit pass is four kernels: a per-tile histogram (upsweep), a row scan
-// of the histogram (one block per digit), a digit-base scan that also detects a
-// pass in which every key has the same digit, and a stable scatter (downsweep).  Trivial passes are skipped on the
-// device (the scatter returns at once and the ping-pong buffer is not
-// flipped), so the host never synchronises inside a sort and the whole
-// sequence can be captured in a CUDA graph.
+// The digit counts of a pass do not depend on the order of its input, so one kernel counts the digits
+// of every pass, a second one turns them into digit bases and marks the passes whose keys share
+// one digit (their scatter returns at once and the ping-pong buffer is not flipped), and a pass is one
+// kernel: a block ranks a tile in shared memory, publishes its digit counts, sums those of the
+// tiles before it while they appear (decoupled look-back: a tile's number is a ticket, so every
+// tile it waits for has already started; the wait has a limit all the same), and writes the tile in
+// digit order.  The host never synchronises inside a sort.  Up to kSmall items one block runs all
+// passes in shared memory in one launch.
+// Bound: HBM for large inputs, launches for small ones.  With four kernels per pass (tile histogram,
+// row scan, digit bases, scatter of 1,024-item tiles) an LBVH build was 144 launches: 0.82 ms for 1,021
+// points, 0.32 now.
 #include "ehgp_internal.cuh"
 
 namespace ehgp {
 namespace {
 
-__device__ __forceinline__ uint32_t digit_of(const IndirectKey& k, uint32_t v, int shift) {
-  uint64_t w = __ldg(k.words + v);
-  if (k.order) w = order_key(w);
-  return (uint32_t)(w >> shift) & 0xffu;
+constexpr int kT = 256, kWarps = kT / 32;
+constexpr uint32_t kSmall = 2048;    // items that one block sorts on its own
+constexpr int kSmallT = 512, kSmallWarps = kSmallT / 32, kSmallRows = kSmall / kSmallT;
+constexpr int kRows = kRadixTile / kT;  // rows of 32 items per warp and tile
+constexpr uint32_t kSpinLimit = 1u << 24;
+
+// State words: per pass (input buffer, trivial flag), then the digit bases of every pass, then the
+// tile tickets.
+constexpr int kBases = 2 * (kRadixMaxPasses + 1);
+constexpr int kTickets = kBases + 256 * kRadixMaxPasses;
+static_assert(kRadixStateWords >= kTickets + kRadixMaxPasses, "state layout");
+
+struct Passes {  // of one sort: key source and shift
+  IndirectKey stage[3];
+  int first[4];  // first pass of each stage, then their number
+  int stages;
+};
+
+// Key of item v in pass p (indirect sorts), its digit in place.
+__device__ __forceinline__ uint32_t indirect_digit(const Passes& ps, int p, uint32_t v) {
+  int s = 0;
+  while (s + 1 < ps.stages && p >= ps.first[s + 1]) ++s;
+  uint64_t w = __ldg(ps.stage[s].words + v);
+  if (ps.stage[s].order) w = order_key(w);
+  return (uint32_t)(w >> (8 * (p - ps.first[s]))) & 0xffu;
 }
 
-__global__ void __launch_bounds__(kRadixThreads)
-k_radix_upsweep(uint32_t n, const uint32_t* __restrict__ vals0, const uint32_t* __restrict__ vals1,
-                IndirectKey key, int shift, const uint32_t* __restrict__ state, int pass,
-                uint32_t* __restrict__ counts, uint32_t tiles) {
-  __shared__ uint32_t hist[256];
-  const uint32_t tile = blockIdx.x;
-  hist[threadIdx.x] = 0;
-  __syncthreads();
-  const uint32_t* in = state[2 * pass] ? vals1 : vals0;
-  const uint32_t base = tile * kRadixTile;
-#pragma unroll
-  for (int r = 0; r < kRadixItems; ++r) {
-    const uint32_t i = base + r * kRadixThreads + threadIdx.x;
-    if (i < n) atomicAdd(&hist[digit_of(key, in[i], shift)], 1u);
+// Digit counts of every pass.  A warp whose lanes share a digit adds once (the high digits of most keys).
+__device__ __forceinline__ void count_digit(uint32_t* hist, uint32_t d, bool on) {
+  const uint32_t act = __ballot_sync(0xffffffffu, on);
+  if (!act) return;
+  const uint32_t first = __shfl_sync(0xffffffffu, d, __ffs((int)act) - 1);
+  if (__all_sync(0xffffffffu, !on || d == first)) {
+    if ((threadIdx.x & 31u) == 0) atomicAdd(hist + first, (uint32_t)__popc(act));
+  } else if (on) {
+    atomicAdd(hist + d, 1u);
   }
-  __syncthreads();
-  counts[threadIdx.x * tiles + tile] = hist[threadIdx.x];
 }
 
-// Row scan: block d turns row d of the tile histogram (counts[d * tiles ..]) into
-// exclusive offsets within the digit and stores the digit total (coalesced, one
-// block per digit).
-__global__ void __launch_bounds__(256)
-k_radix_rowscan(uint32_t* __restrict__ counts, uint32_t tiles, uint32_t* __restrict__ state) {
-  __shared__ uint32_t warp_tot[8];
-  __shared__ uint32_t carry;
-  const uint32_t d = blockIdx.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  uint32_t* row = counts + (uint64_t)d * tiles;
-  if (tid == 0) carry = 0;
+template <bool kKv>
+__global__ void __launch_bounds__(kT) k_radix_counts(uint32_t n, const uint32_t* __restrict__ vals,
+                                                     const uint64_t* __restrict__ keys, Passes ps, int passes,
+                                                     uint32_t* __restrict__ state) {
+  extern __shared__ uint32_t hist[];  // [passes][256]
+  for (int i = threadIdx.x; i < passes * 256; i += kT) hist[i] = 0;
   __syncthreads();
-  for (uint32_t base = 0; base < tiles; base += 256) {
-    const uint32_t t = base + tid;
-    const uint32_t v = t < tiles ? row[t] : 0u;
-    uint32_t x = v;  // inclusive warp scan
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-      if ((int)lane >= off) x += y;
+  for (uint32_t b = blockIdx.x * kT; b < n; b += gridDim.x * kT) {
+    const uint32_t i = b + threadIdx.x;
+    const bool on = i < n;
+    if (kKv) {
+      const uint64_t key = on ? keys[i] : 0;
+      for (int p = 0; p < passes; ++p) count_digit(hist + 256 * p, (uint32_t)(key >> (8 * p)) & 0xffu, on);
+    } else {
+      const uint32_t v = on ? vals[i] : 0;
+      for (int s = 0; s < ps.stages; ++s) {
+        uint64_t w = on ? __ldg(ps.stage[s].words + v) : 0;
+        if (ps.stage[s].order) w = order_key(w);
+        for (int p = ps.first[s]; p < ps.first[s + 1]; ++p)
+          count_digit(hist + 256 * p, (uint32_t)(w >> (8 * (p - ps.first[s]))) & 0xffu, on);
+      }
     }
-    if (lane == 31) warp_tot[warp] = x;
-    __syncthreads();
-    uint32_t wbase = 0;
-    for (uint32_t w = 0; w < warp; ++w) wbase += warp_tot[w];
-    const uint32_t c0 = carry;
-    if (t < tiles) row[t] = c0 + wbase + x - v;
-    __syncthreads();
-    if (tid == 255) carry = c0 + wbase + x;
-    __syncthreads();
   }
-  if (tid == 0) state[2 * (kRadixMaxPasses + 1) + d] = carry;
+  __syncthreads();
+  for (int i = threadIdx.x; i < passes * 256; i += kT)
+    if (hist[i]) atomicAdd(state + kBases + i, hist[i]);
 }
 
-// Digit bases: exclusive scan of the 256 digit totals; a pass whose keys share one
-// digit is marked trivial (its scatter is skipped and the buffers do not flip).
-__global__ void __launch_bounds__(256)
-k_radix_digits(uint32_t n, uint32_t* __restrict__ state, int pass) {
-  __shared__ uint32_t totals[256];
-  __shared__ uint32_t trivial;
-  const uint32_t d = threadIdx.x;
-  if (d == 0) trivial = 0;
-  const uint32_t sum = state[2 * (kRadixMaxPasses + 1) + d];
-  totals[d] = sum;
-  __syncthreads();
-  if (sum == n) trivial = 1;
-  uint32_t v = sum;
-  for (int off = 1; off < 256; off <<= 1) {
-    __syncthreads();
-    const uint32_t add = (d >= (uint32_t)off) ? totals[d - off] : 0u;
-    __syncthreads();
-    v += add;
-    totals[d] = v;
-  }
-  __syncthreads();
-  state[2 * (kRadixMaxPasses + 1) + d] = v - sum;  // exclusive base of digit d
-  __syncthreads();
-  if (d == 0) {
-    const uint32_t cur = state[2 * pass];
-    state[2 * pass + 1] = trivial;
-    state[2 * (pass + 1)] = trivial ? cur : (cur ^ 1u);
-  }
-}
-
-__global__ void __launch_bounds__(kRadixThreads)
-k_radix_downsweep(uint32_t n, uint32_t* __restrict__ vals0, uint32_t* __restrict__ vals1,
-                  IndirectKey key, int shift, const uint32_t* __restrict__ state, int pass,
-                  const uint32_t* __restrict__ counts, uint32_t tiles) {
-  if (state[2 * pass + 1]) return;  // every key has the same digit: order unchanged
-  constexpr int kWarps = kRadixThreads / 32;
-  __shared__ uint32_t base[256];
-  __shared__ uint32_t warp_cnt[kWarps][256];
-  const uint32_t tile = blockIdx.x;
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t* in = state[2 * pass] ? vals1 : vals0;
-  uint32_t* out = state[2 * pass] ? vals0 : vals1;
-  base[tid] = counts[tid * tiles + tile] + state[2 * (kRadixMaxPasses + 1) + tid];
-  const uint32_t lanemask_lt = (1u << lane) - 1u;
-  for (int r = 0; r < kRadixItems; ++r) {
-    const uint32_t i = tile * kRadixTile + r * kRadixThreads + tid;
-    const bool valid = i < n;
-    const uint32_t v = valid ? in[i] : 0u;
-    const uint32_t dig = valid ? digit_of(key, v, shift) : 256u;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) warp_cnt[w][tid] = 0;
-    __syncthreads();
-    const uint32_t peers = __match_any_sync(0xffffffffu, dig);
-    const uint32_t rank = __popc(peers & lanemask_lt);
-    if (valid && rank == 0) warp_cnt[warp][dig] = __popc(peers);
-    __syncthreads();
-    // exclusive prefix over warps, per digit (thread tid owns digit tid)
-    uint32_t run = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const uint32_t c = warp_cnt[w][tid];
-      warp_cnt[w][tid] = run;
-      run += c;
+// Digit bases (a warp per pass) and the buffer every pass starts from.
+__global__ void __launch_bounds__(1024) k_radix_plan(uint32_t n, int passes, uint32_t* __restrict__ state) {
+  __shared__ uint32_t trivial[32];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  if ((int)warp < passes) {
+    uint32_t* h = state + kBases + 256 * warp;
+    uint32_t c[8], sum = 0;
+    bool all = false;
+    for (int q = 0; q < 8; ++q) {
+      c[q] = h[8 * lane + q];
+      all |= c[q] == n;
+      sum += c[q];
     }
-    __syncthreads();
-    if (valid) out[base[dig] + warp_cnt[warp][dig] + rank] = v;
-    __syncthreads();
-    base[tid] += run;
-    __syncthreads();
+    uint32_t incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((int)lane >= o) incl += y;
+    }
+    uint32_t run = incl - sum;
+    for (int q = 0; q < 8; ++q) {
+      h[8 * lane + q] = run;
+      run += c[q];
+    }
+    const bool any = __any_sync(0xffffffffu, all);
+    if (lane == 0) trivial[warp] = any;
   }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  uint32_t cur = 0;
+  for (int p = 0; p < passes; ++p) {
+    state[2 * p] = cur;
+    state[2 * p + 1] = trivial[p];
+    cur ^= trivial[p] ? 0u : 1u;
+  }
+  state[2 * passes] = cur;
 }
 
-// Key-value variant: the 64-bit keys move with the indices (keys0/keys1 ping-pong with
-// vals0/vals1 under the same pass state), so every pass reads and writes both coalesced
-// instead of gathering the key of each index.
-__global__ void __launch_bounds__(kRadixThreads)
-k_radix_upsweep_kv(uint32_t n, const uint64_t* __restrict__ keys0, const uint64_t* __restrict__ keys1, int shift,
-                   const uint32_t* __restrict__ state, int pass, uint32_t* __restrict__ counts, uint32_t tiles) {
-  __shared__ uint32_t hist[256];
-  const uint32_t tile = blockIdx.x;
-  hist[threadIdx.x] = 0;
-  __syncthreads();
-  const uint64_t* in = state[2 * pass] ? keys1 : keys0;
-  const uint32_t base = tile * kRadixTile;
+// Ranks of a warp's rows: rank[r] = items of the same digit before it in this warp; cnt[256] ends as the
+// warp's digit counts.  digit 256 marks an absent item.
+template <int R>
+__device__ __forceinline__ void rank_rows(const uint32_t (&dig)[R], uint32_t (&rank)[R], uint32_t* cnt) {
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
 #pragma unroll
-  for (int r = 0; r < kRadixItems; ++r) {
-    const uint32_t i = base + r * kRadixThreads + threadIdx.x;
-    if (i < n) atomicAdd(&hist[(uint32_t)(in[i] >> shift) & 0xffu], 1u);
+  for (int r = 0; r < R; ++r) {
+    const uint32_t peers = __match_any_sync(0xffffffffu, dig[r]);
+    const int leader = __ffs((int)peers) - 1;
+    uint32_t base = 0;
+    if ((int)lane == leader && dig[r] < 256u) {
+      base = cnt[dig[r]];
+      cnt[dig[r]] = base + __popc(peers);
+    }
+    __syncwarp();
+    rank[r] = __shfl_sync(0xffffffffu, base, leader) + __popc(peers & lt);
   }
-  __syncthreads();
-  counts[threadIdx.x * tiles + tile] = hist[threadIdx.x];
 }
 
-__global__ void __launch_bounds__(kRadixThreads)
-k_radix_downsweep_kv(uint32_t n, uint32_t* __restrict__ vals0, uint32_t* __restrict__ vals1,
-                     uint64_t* __restrict__ keys0, uint64_t* __restrict__ keys1, int shift,
-                     const uint32_t* __restrict__ state, int pass, const uint32_t* __restrict__ counts,
-                     uint32_t tiles) {
+// Exclusive scan of one value per thread over the first 256 threads (all threads call).
+__device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t* tmp) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  uint32_t x = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if ((int)lane >= o) x += y;
+  }
+  if (lane == 31 && warp < 8) tmp[warp] = x;
+  __syncthreads();
+  uint32_t before = 0;
+  for (uint32_t w = 0; w < 8 && w < warp; ++w) before += tmp[w];
+  __syncthreads();
+  return before + x - v;
+}
+
+constexpr uint32_t kAggregate = 1u << 30, kInclusive = 2u << 30, kCountMask = (1u << 30) - 1u;
+
+// One pass.  look: [2][tiles][256] tile counts; the pass uses the half of its input buffer and clears
+// the other half for the next one.
+template <bool kKv>
+__global__ void __launch_bounds__(kT) k_radix_pass(uint32_t n, uint32_t* __restrict__ vals0, uint32_t* __restrict__ vals1,
+                                                   uint64_t* __restrict__ keys0, uint64_t* __restrict__ keys1, Passes ps,
+                                                   int pass, uint32_t* __restrict__ state, uint32_t* look, uint32_t tiles,
+                                                   uint32_t* __restrict__ err) {
   if (state[2 * pass + 1]) return;  // every key has the same digit: order unchanged
-  constexpr int kWarps = kRadixThreads / 32;
-  __shared__ uint32_t base[256];
-  __shared__ uint32_t warp_cnt[kWarps][256];
-  const uint32_t tile = blockIdx.x;
+  __shared__ uint32_t cnt[kWarps][256];
+  __shared__ uint32_t start[256], gbase[256], tmp[8], s_tile, s_bad;
+  __shared__ uint32_t sval[kRadixTile];
+  __shared__ uint64_t skey[kKv ? kRadixTile : 1];
+  __shared__ uint8_t sdig[kKv ? 1 : kRadixTile];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const bool flip = state[2 * pass] != 0;
   const uint32_t* in = flip ? vals1 : vals0;
   uint32_t* out = flip ? vals0 : vals1;
   const uint64_t* kin = flip ? keys1 : keys0;
   uint64_t* kout = flip ? keys0 : keys1;
-  base[tid] = counts[tid * tiles + tile] + state[2 * (kRadixMaxPasses + 1) + tid];
-  const uint32_t lanemask_lt = (1u << lane) - 1u;
-  for (int r = 0; r < kRadixItems; ++r) {
-    const uint32_t i = tile * kRadixTile + r * kRadixThreads + tid;
-    const bool valid = i < n;
-    const uint32_t v = valid ? in[i] : 0u;
-    const uint64_t key = valid ? kin[i] : 0u;
-    const uint32_t dig = valid ? (uint32_t)(key >> shift) & 0xffu : 256u;
+  if (tid == 0) {
+    s_tile = atomicAdd(state + kTickets + pass, 1u);
+    s_bad = 0;
+  }
+  for (int w = 0; w < kWarps; ++w) cnt[w][tid] = 0;
+  __syncthreads();
+  const uint32_t tile = s_tile;
+  uint32_t* mine = look + ((uint64_t)(flip ? tiles : 0) + tile) * 256 + tid;
+  look[((uint64_t)(flip ? 0 : tiles) + tile) * 256 + tid] = 0;
+  uint32_t v[kRows], dig[kRows], rank[kRows];
+  uint64_t key[kKv ? kRows : 1];
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) warp_cnt[w][tid] = 0;
-    __syncthreads();
-    const uint32_t peers = __match_any_sync(0xffffffffu, dig);
-    const uint32_t rank = __popc(peers & lanemask_lt);
-    if (valid && rank == 0) warp_cnt[warp][dig] = __popc(peers);
-    __syncthreads();
-    uint32_t run = 0;
+  for (int r = 0; r < kRows; ++r) {
+    const uint32_t i = tile * kRadixTile + warp * (kRows * 32) + r * 32 + lane;
+    v[r] = i < n ? in[i] : 0u;
+    if (kKv) {
+      key[r] = i < n ? kin[i] : 0u;
+      dig[r] = i < n ? (uint32_t)(key[r] >> (8 * pass)) & 0xffu : 256u;
+    } else {
+      dig[r] = i < n ? indirect_digit(ps, pass, v[r]) : 256u;
+    }
+  }
+  rank_rows<kRows>(dig, rank, cnt[warp]);
+  __syncthreads();
+  uint32_t total = 0;  // of digit tid
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const uint32_t c = warp_cnt[w][tid];
-      warp_cnt[w][tid] = run;
-      run += c;
+  for (int w = 0; w < kWarps; ++w) {
+    const uint32_t c = cnt[w][tid];
+    cnt[w][tid] = total;
+    total += c;
+  }
+  atomicExch(mine, total | (tile == 0 ? kInclusive : kAggregate));
+  const uint32_t local = scan256(total, tmp);
+  start[tid] = local;
+  uint32_t before = 0;
+  for (uint32_t t = tile, spin = 0; t > 0;) {
+    const uint32_t x = *(volatile const uint32_t*)(look + ((uint64_t)(flip ? tiles : 0) + t - 1) * 256 + tid);
+    if (x == 0) {
+      if (++spin > kSpinLimit) {
+        s_bad = 1;
+        break;
+      }
+      continue;
     }
-    __syncthreads();
-    if (valid) {
-      const uint32_t at = base[dig] + warp_cnt[warp][dig] + rank;
-      out[at] = v;
-      kout[at] = key;
-    }
-    __syncthreads();
-    base[tid] += run;
-    __syncthreads();
+    before += x & kCountMask;
+    if (x & kInclusive) break;
+    --t;
+  }
+  if (tile) atomicExch(mine, (before + total) | kInclusive);
+  gbase[tid] = state[kBases + 256 * pass + tid] + before - local;
+  __syncthreads();
+  if (s_bad) {  // uniform
+    if (tid == 0) atomicOr(err, kErrTimeout);
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    if (dig[r] > 255u) continue;
+    const uint32_t at = start[dig[r]] + cnt[warp][dig[r]] + rank[r];
+    sval[at] = v[r];
+    if (kKv) skey[at] = key[r];
+    else sdig[at] = (uint8_t)dig[r];
+  }
+  __syncthreads();
+  const uint32_t items = min((uint32_t)kRadixTile, n - tile * kRadixTile);
+  for (uint32_t j = tid; j < items; j += kT) {
+    const uint32_t d = kKv ? (uint32_t)(skey[j] >> (8 * pass)) & 0xffu : sdig[j];
+    const uint32_t to = gbase[d] + j;
+    out[to] = sval[j];
+    if (kKv) kout[to] = skey[j];
   }
 }
 
-__global__ void k_radix_init(uint32_t* state) {
-  if (threadIdx.x == 0) state[0] = 0;
+// All passes of a sort of at most kSmall items; the result is in the first buffer.
+template <bool kKv>
+__global__ void __launch_bounds__(kSmallT) k_radix_small(uint32_t n, uint32_t* __restrict__ vals, uint64_t* __restrict__ keys,
+                                                         Passes ps, int passes, uint32_t* __restrict__ state) {
+  __shared__ uint32_t cnt[kSmallWarps][256];
+  __shared__ uint32_t start[256], tmp[8], s_one;
+  __shared__ uint32_t sval[kSmall];
+  __shared__ uint64_t skey[kKv ? kSmall : 1];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  uint32_t v[kSmallRows], dig[kSmallRows], rank[kSmallRows];
+  uint64_t key[kKv ? kSmallRows : 1];
+  const uint32_t i0 = warp * (kSmallRows * 32) + lane;
+#pragma unroll
+  for (int r = 0; r < kSmallRows; ++r) {
+    const uint32_t i = i0 + r * 32;
+    v[r] = i < n ? vals[i] : 0u;
+    if (kKv) key[r] = i < n ? keys[i] : 0u;
+  }
+  for (int p = 0; p < passes; ++p) {
+    for (uint32_t q = tid; q < kSmallWarps * 256u; q += kSmallT) (&cnt[0][0])[q] = 0;
+    if (tid == 0) s_one = 0;
+#pragma unroll
+    for (int r = 0; r < kSmallRows; ++r)
+      dig[r] = i0 + r * 32 >= n ? 256u : kKv ? (uint32_t)(key[r] >> (8 * p)) & 0xffu : indirect_digit(ps, p, v[r]);
+    __syncthreads();
+    rank_rows<kSmallRows>(dig, rank, cnt[warp]);
+    __syncthreads();
+    uint32_t total = 0;
+    if (tid < 256) {
+      for (int w = 0; w < kSmallWarps; ++w) {
+        const uint32_t c = cnt[w][tid];
+        cnt[w][tid] = total;
+        total += c;
+      }
+      if (total == n) s_one = 1;
+    }
+    const uint32_t local = scan256(total, tmp);
+    if (tid < 256) start[tid] = local;
+    __syncthreads();
+    if (s_one) {  // one digit: order unchanged
+      __syncthreads();
+      continue;
+    }
+#pragma unroll
+    for (int r = 0; r < kSmallRows; ++r) {
+      if (dig[r] > 255u) continue;
+      const uint32_t at = start[dig[r]] + cnt[warp][dig[r]] + rank[r];
+      sval[at] = v[r];
+      if (kKv) skey[at] = key[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSmallRows; ++r) {
+      const uint32_t i = i0 + r * 32;
+      if (i >= n) continue;
+      v[r] = sval[i];
+      if (kKv) key[r] = skey[i];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kSmallRows; ++r) {
+    const uint32_t i = i0 + r * 32;
+    if (i >= n) continue;
+    vals[i] = v[r];
+    if (kKv) keys[i] = key[r];
+  }
+  if (tid == 0) state[2 * passes] = 0;
+}
+
+template <bool kKv>
+int sort(cudaStream_t st, uint32_t n, uint32_t* vals0, uint32_t* vals1, uint64_t* keys0, uint64_t* keys1, const Passes& ps,
+         int passes, RadixScratch& scratch, uint64_t* launches) {
+  if (n <= kSmall) {
+    k_radix_small<kKv><<<1, kSmallT, 0, st>>>(n, vals0, keys0, ps, passes, scratch.state);
+    ++*launches;
+    return passes;
+  }
+  const uint32_t tiles = (n + kRadixTile - 1) / kRadixTile;
+  cudaMemsetAsync(scratch.state, 0, kRadixStateWords * sizeof(uint32_t), st);
+  cudaMemsetAsync(scratch.counts, 0, (uint64_t)tiles * 256 * sizeof(uint32_t), st);
+  const uint32_t blocks = (n + 8 * kT - 1) / (8 * kT);
+  k_radix_counts<kKv><<<blocks < 1184 ? blocks : 1184, kT, passes * 256 * sizeof(uint32_t), st>>>(n, vals0, keys0, ps, passes,
+                                                                                                  scratch.state);
+  k_radix_plan<<<1, 1024, 0, st>>>(n, passes, scratch.state);
+  for (int p = 0; p < passes; ++p)
+    k_radix_pass<kKv><<<tiles, kT, 0, st>>>(n, vals0, vals1, keys0, keys1, ps, p, scratch.state, scratch.counts, tiles,
+                                            scratch.err);
+  *launches += 2 + passes;
+  return passes;
 }
 
 }  // namespace
@@ -227,23 +350,16 @@ __global__ void k_radix_init(uint32_t* state) {
 int radix_sort_indirect(cudaStream_t stream, uint32_t n, uint32_t* vals0, uint32_t* vals1,
                         const IndirectKey* stages, const int* stage_bits, int stage_count,
                         RadixScratch& scratch, uint64_t* launches) {
-  const uint32_t tiles = (n + kRadixTile - 1) / kRadixTile;
-  k_radix_init<<<1, 32, 0, stream>>>(scratch.state);
-  *launches += 1;
+  Passes ps{};
+  ps.stages = stage_count;
   int pass = 0;
   for (int s = 0; s < stage_count; ++s) {
-    for (int shift = 0; shift < stage_bits[s]; shift += 8) {
-      k_radix_upsweep<<<tiles, kRadixThreads, 0, stream>>>(n, vals0, vals1, stages[s], shift, scratch.state,
-                                                           pass, scratch.counts, tiles);
-      k_radix_rowscan<<<256, 256, 0, stream>>>(scratch.counts, tiles, scratch.state);
-      k_radix_digits<<<1, 256, 0, stream>>>(n, scratch.state, pass);
-      k_radix_downsweep<<<tiles, kRadixThreads, 0, stream>>>(n, vals0, vals1, stages[s], shift, scratch.state,
-                                                             pass, scratch.counts, tiles);
-      *launches += 4;
-      ++pass;
-    }
+    ps.stage[s] = stages[s];
+    ps.first[s] = pass;
+    pass += (stage_bits[s] + 7) / 8;
   }
-  return pass;
+  ps.first[stage_count] = pass;
+  return sort<false>(stream, n, vals0, vals1, nullptr, nullptr, ps, pass, scratch, launches);
 }
 
 // Stable LSD sort of (keys0[i], vals0[i]) pairs by the low `bits` bits of the keys; the
@@ -251,21 +367,7 @@ int radix_sort_indirect(cudaStream_t stream, uint32_t n, uint32_t* vals0, uint32
 // end beside it, in keys0 or keys1 under the same selection).
 int radix_sort_kv(cudaStream_t stream, uint32_t n, uint32_t* vals0, uint32_t* vals1, uint64_t* keys0,
                   uint64_t* keys1, int bits, RadixScratch& scratch, uint64_t* launches) {
-  const uint32_t tiles = (n + kRadixTile - 1) / kRadixTile;
-  k_radix_init<<<1, 32, 0, stream>>>(scratch.state);
-  *launches += 1;
-  int pass = 0;
-  for (int shift = 0; shift < bits; shift += 8) {
-    k_radix_upsweep_kv<<<tiles, kRadixThreads, 0, stream>>>(n, keys0, keys1, shift, scratch.state, pass,
-                                                            scratch.counts, tiles);
-    k_radix_rowscan<<<256, 256, 0, stream>>>(scratch.counts, tiles, scratch.state);
-    k_radix_digits<<<1, 256, 0, stream>>>(n, scratch.state, pass);
-    k_radix_downsweep_kv<<<tiles, kRadixThreads, 0, stream>>>(n, vals0, vals1, keys0, keys1, shift, scratch.state,
-                                                              pass, scratch.counts, tiles);
-    *launches += 4;
-    ++pass;
-  }
-  return pass;
+  return sort<true>(stream, n, vals0, vals1, keys0, keys1, Passes{}, (bits + 7) / 8, scratch, launches);
 }
 
 }  // namespace ehgp
