@@ -1347,12 +1347,12 @@ k_facet_ball(DescentParams d, uint32_t m, const QFacet* __restrict__ in_fac, con
 }
 
 constexpr int kStepStack = 32;  // traversal entries per thread (an arm that needs more is left open)
-constexpr int kStepIn = 20;     // points inside the ball per thread (likewise)
+constexpr int kStepIn = 20;     // points inside the ball per thread (likewise; their distances fit in the stack)
 
 // The step of every facet with a certified support: points strictly inside its miniball come from the LBVH;
 // with fewer than k of them the choice is those and the least support points (which lie on the sphere),
-// with exactly k those.  Any point that binary64 does not place, more than k inside points, or an arm that
-// would fail goes to `hard`.
+// with k or more the k nearest.  Any point that binary64 does not place, an order of distances that the
+// rounded ones leave open, or an arm that would fail goes to `hard`.
 __global__ void __launch_bounds__(kFT, 6)
 k_facet_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, const QFacet* __restrict__ in_fac,
              const uint4* __restrict__ support, const uint32_t* __restrict__ rstate, int passes,
@@ -1442,7 +1442,30 @@ k_facet_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, c
     uint32_t k = 0;
 #pragma unroll
     for (int j = 0; j < kMaxFacet; ++j) k += e.F[j] != kInvalid32 ? 1u : 0u;
-    open = open || n_in > k || n_in + (uint32_t)ts < k;
+    if (!open && n_in > k) {  // drop the farthest; the distances stand in the stack that the walk has left
+      for (uint32_t q = 0; q < n_in; ++q) {
+        const uint32_t p = inside[q][w];
+        const double dx = d.px[p] - cx, dy = d.py[p] - cy, dz = d.pz[p] - cz;
+        stack[q][w] = __float_as_uint((float)(dx * dx + dy * dy + dz * dz));  // >= 0: ordered as its bits
+      }
+      auto farthest = [&]() {
+        uint32_t at = 0;
+        for (uint32_t q = 1; q < n_in; ++q)
+          if (stack[q][w] > stack[at][w]) at = q;
+        return at;
+      };
+      float dropped = 0.f;
+      while (n_in > k) {
+        const uint32_t at = farthest();
+        dropped = __uint_as_float(stack[at][w]);
+        --n_in;
+        inside[at][w] = inside[n_in][w];
+        stack[at][w] = stack[n_in][w];
+      }
+      // the nearest dropped point is farther than every kept one for certain (both within ed, and rounded)
+      open = !(dropped - __uint_as_float(stack[farthest()][w]) > __double2float_ru(2.0 * ed) + 4e-7f * dropped);
+    }
+    open = open || n_in + (uint32_t)ts < k;
     if (!open) {
       // G ascending: the inside points, then the least support points
 #pragma unroll
