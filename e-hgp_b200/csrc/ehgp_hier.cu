@@ -36,18 +36,13 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
-#include <atomic>
 #include <cstring>
 #include <functional>
 #include <map>
 #include <memory>
 #include <numeric>
-#include <thread>
 #include <vector>
 
-#if defined(__x86_64__)
-#include <immintrin.h>
-#endif
 
 namespace ehgp {
 
@@ -1608,12 +1603,6 @@ k_facet_exact(DescentParams d, uint32_t m, const uint32_t* __restrict__ hard, co
 }  // namespace
 
 // ---- host state ---------------------------------------------------------------------
-constexpr int kStageSlots = 16;
-constexpr uint64_t kStageBytes = uint64_t{1} << 20;
-// Pageable bytes of one copy from which the pinned ring pays for its allocation (16 MB of page-locked
-// memory and the threads: a few ms, once per context).
-constexpr uint64_t kStageFrom = uint64_t{32} << 20;
-
 struct HierState {
   std::vector<void*> allocs;
   uint64_t cap_events = 0, cap_arms = 0, cap_births = 0, cap_slots = 0;
@@ -1674,17 +1663,11 @@ struct HierState {
   double ms_steps = 0;                          // summed k_arm_step launch times
   uint64_t step_launches = 0;
   uint32_t part_arms = 0;  // arms per part of the descent (0: one part); results never depend on it
-  // pinned ring through which results reach pageable memory
-  char* stage = nullptr;
-  cudaEvent_t stage_ev[kStageSlots] = {};
 };
 
 void hier_free(Ctx& ctx) {
   if (!ctx.hier) return;
   for (void* p : ctx.hier->allocs) cudaFree(p);
-  if (ctx.hier->stage) cudaFreeHost(ctx.hier->stage);
-  for (cudaEvent_t ev : ctx.hier->stage_ev)
-    if (ev) cudaEventDestroy(ev);
   for (void* q : {(void*)ctx.hier->tie_num, (void*)ctx.hier->tie_a2, (void*)ctx.hier->tie_idx,
                   (void*)ctx.hier->tie_tmp, (void*)ctx.hier->tie_pos, (void*)ctx.hier->run_off,
                   (void*)ctx.hier->run_lo})
@@ -2130,117 +2113,6 @@ int hier_run(Ctx& ctx, uint32_t K) {
   return EHGP_OK;
 }
 
-// One device range and the host memory it goes to.
-struct CopyOut {
-  char* dst;
-  const char* src;
-  uint64_t bytes;
-};
-
-namespace {
-
-// Streaming copy into memory that is not read back here (the caches keep the staging ring).
-void stream_copy(char* dst, const char* src, uint64_t bytes) {
-#if defined(__x86_64__)
-  const uint64_t lead = std::min<uint64_t>(bytes, (16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15);
-  std::memcpy(dst, src, lead);
-  dst += lead;
-  src += lead;
-  bytes -= lead;
-  uint64_t i = 0;
-  for (; i + 64 <= bytes; i += 64)
-    for (int q = 0; q < 4; ++q)
-      _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i) + q, _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i) + q));
-  std::memcpy(dst + i, src + i, bytes - i);
-  _mm_sfence();
-#else
-  std::memcpy(dst, src, bytes);
-#endif
-}
-
-}  // namespace
-
-// Copies device ranges to host memory.  Pinned destinations and small ranges go straight there;
-// large pageable ones go through a ring of pinned slots that host threads empty while the next
-// chunks cross the bus (a pageable cudaMemcpy stages through one thread instead).
-cudaError_t copy_out(Ctx& ctx, HierState& h, const std::vector<CopyOut>& list) {
-  cudaStream_t st = ctx.stream;
-  cudaError_t e = cudaSuccess;
-  std::vector<CopyOut> chunks;
-  uint64_t all = 0;
-  for (const CopyOut& c : list) all += c.bytes;
-  for (const CopyOut& c : list) {
-    cudaPointerAttributes at{};
-    const bool pinned = cudaPointerGetAttributes(&at, c.dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
-    cudaGetLastError();
-    if (pinned || c.bytes <= kStageBytes || all < kStageFrom) {
-      if ((e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-      continue;
-    }
-    for (uint64_t o = 0; o < c.bytes; o += kStageBytes)
-      chunks.push_back({c.dst + o, c.src + o, std::min(kStageBytes, c.bytes - o)});
-  }
-  if (chunks.empty()) return cudaStreamSynchronize(st);
-  if (!h.stage) {
-    if ((e = cudaMallocHost(reinterpret_cast<void**>(&h.stage), kStageSlots * kStageBytes)) != cudaSuccess) {
-      h.stage = nullptr;
-      return e;
-    }
-    for (cudaEvent_t& ev : h.stage_ev)
-      if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
-  }
-  const size_t total = chunks.size();
-  std::atomic<size_t> issued{0}, next{0};
-  std::atomic<int> failed{0};
-  std::vector<std::atomic<uint8_t>> done(total);
-  for (auto& d : done) d.store(0, std::memory_order_relaxed);
-  auto drain = [&] {
-    for (size_t t; (t = next.fetch_add(1)) < total;) {
-      while (issued.load(std::memory_order_acquire) <= t && !failed.load(std::memory_order_acquire)) std::this_thread::yield();
-      if (failed.load(std::memory_order_acquire)) return;
-      const int slot = (int)(t % kStageSlots);
-      if (cudaEventSynchronize(h.stage_ev[slot]) != cudaSuccess) {
-        failed.store(1, std::memory_order_release);
-        return;
-      }
-      stream_copy(chunks[t].dst, h.stage + slot * kStageBytes, chunks[t].bytes);
-      done[t].store(1, std::memory_order_release);
-    }
-  };
-  const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
-  const size_t workers = std::min<size_t>({total, (size_t)8, (size_t)(hw - 1)});
-  std::vector<std::thread> pool;
-  try {
-    for (size_t i = 0; i < workers; ++i) pool.emplace_back([&] {
-      cudaSetDevice(ctx.device);
-      drain();
-    });
-  } catch (...) {  // no more threads: the ones that started do the work
-  }
-  if (pool.empty()) {
-    for (const CopyOut& c : chunks)
-      if ((e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-    return cudaStreamSynchronize(st);
-  }
-  for (size_t t = 0; t < total && !failed.load(std::memory_order_acquire); ++t) {
-    if (t >= (size_t)kStageSlots)
-      while (!done[t - kStageSlots].load(std::memory_order_acquire) && !failed.load(std::memory_order_acquire))
-        std::this_thread::yield();
-    const int slot = (int)(t % kStageSlots);
-    e = cudaMemcpyAsync(h.stage + slot * kStageBytes, chunks[t].src, chunks[t].bytes, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaEventRecord(h.stage_ev[slot], st);
-    if (e != cudaSuccess) {
-      failed.store(1, std::memory_order_release);
-      break;
-    }
-    issued.store(t + 1, std::memory_order_release);
-  }
-  for (auto& th : pool) th.join();
-  const cudaError_t es = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return e;
-  return es != cudaSuccess ? es : failed.load() ? cudaErrorUnknown : cudaSuccess;
-}
-
 }  // namespace ehgp
 
 extern "C" {
@@ -2325,7 +2197,7 @@ int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out) {
     add(out->vertical, j.vert, j.n_vert, sizeof *j.vert);
     if (out->roots && !j.roots.empty()) std::memcpy(out->roots, j.roots.data(), j.roots.size() * sizeof j.roots[0]);
   }
-  const cudaError_t e = ehgp::copy_out(*ctx, h, list);
+  const cudaError_t e = ehgp::copy_out(*ctx, list);
   if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "hierarchy copy");
   return EHGP_OK;
 }
@@ -2371,8 +2243,7 @@ int ehgp_event_supports(ehgp_ctx* ctx, const uint32_t* events, uint64_t count, u
     cudaMemcpyAsync(h.order0, events + b0, (uint64_t)m * 4, cudaMemcpyHostToDevice, st);
     ehgp::k_event_supports<<<ehgp::nblk(m, ehgp::kT), ehgp::kT, 0, st>>>(m, h.order0, h.ev, (uint32_t)h.events,
                                                                         (uint32_t*)h.ev_raw);
-    cudaMemcpyAsync(out + 5 * b0, h.ev_raw, (uint64_t)m * 20, cudaMemcpyDeviceToHost, st);
-    const cudaError_t e = cudaStreamSynchronize(st);
+    const cudaError_t e = ehgp::copy_out(*ctx, {{(char*)(out + 5 * b0), (const char*)h.ev_raw, (uint64_t)m * 20}});
     if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "facade event supports");
   }
   return EHGP_OK;

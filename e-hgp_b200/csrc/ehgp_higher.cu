@@ -2061,15 +2061,33 @@ void cube_cells(const std::vector<float>& dirs, double delta, std::vector<uint16
         for (double s : {s0, s1})
           for (double t : {t0, t1}) eps = std::max(eps, angle(ctr, vec(face, s, t)));
         std::vector<std::pair<double, uint16_t>> near;
+        const double reach = delta + eps + 1e-6, cos_reach = std::cos(reach) - 1e-12;
         for (size_t d = 0; d < nd; ++d) {
           const std::array<double, 3> dv{dirs[3 * d], dirs[3 * d + 1], dirs[3 * d + 2]};
+          if (ctr[0] * dv[0] + ctr[1] * dv[1] + ctr[2] * dv[2] < cos_reach) continue;
           const double g = angle(ctr, dv);
-          if (g <= delta + eps + 1e-6) near.push_back({g, (uint16_t)d});
+          if (g <= reach) near.push_back({g, (uint16_t)d});
         }
         std::sort(near.begin(), near.end());
         uint16_t* out = &cells[((size_t)(face * kCube + i) * kCube + j) * kCellDirs];
         for (size_t q = 0; q < near.size() && q < (size_t)kCellDirs; ++q) out[q] = near[q].second;
       }
+}
+
+// The directions and their cells are the same for every context: made by the first one.
+struct DirectionTables {
+  std::vector<float> dirs;
+  std::vector<uint16_t> cells;
+  double delta = 0;
+};
+const DirectionTables& direction_tables() {
+  static const DirectionTables tables = [] {
+    DirectionTables t;
+    icosphere(t.dirs, t.delta);
+    cube_cells(t.dirs, t.delta, t.cells);
+    return t;
+  }();
+  return tables;
 }
 
 }  // namespace
@@ -2129,12 +2147,11 @@ cudaError_t higher_alloc(Ctx& ctx) {
   EHGP_ALLOC(h.todo, n * sizeof(uint8_t));
   EHGP_ALLOC(h.counters, 8 * sizeof(uint32_t));
   EHGP_ALLOC(h.stats, 8 * sizeof(unsigned long long));
-  std::vector<float> dirs;
-  double delta = 0;
-  icosphere(dirs, delta);
+  const DirectionTables& tables = direction_tables();
+  const std::vector<float>& dirs = tables.dirs;
+  const std::vector<uint16_t>& cells = tables.cells;
+  const double delta = tables.delta;
   if (dirs.size() != 3 * (size_t)kDirs) return cudaErrorInvalidValue;
-  std::vector<uint16_t> cells;
-  cube_cells(dirs, delta, cells);
   EHGP_ALLOC(h.dirs, dirs.size() * sizeof(float));
   EHGP_ALLOC(h.cells, cells.size() * sizeof(uint16_t));
   EHGP_ALLOC(h.rho, n * kDirs * sizeof(float));
@@ -2619,7 +2636,7 @@ int ehgp_higher(ehgp_ctx* ctx, uint32_t K, const ehgp_higher_out* out) {
   if (out && out->count) *out->count = m;
   if (out && out->records && m) {
     if (out->capacity < m) return ehgp::abi_fail(ctx, EHGP_ERR_CAPACITY, "the output capacity is below the record count");
-    e = cudaMemcpy(out->records, ctx->hb.sorted, (uint64_t)m * 64, cudaMemcpyDeviceToHost);
+    e = ehgp::copy_out(*ctx, {{(char*)out->records, (const char*)ctx->hb.sorted, (uint64_t)m * 64}});
     if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "higher-support copy");
   }
   return EHGP_OK;

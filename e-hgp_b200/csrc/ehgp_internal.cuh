@@ -249,6 +249,8 @@ struct HigherBuffers {
   uint64_t large_entries = 0;
 };
 
+constexpr int kStageSlots = 16;  // of the pinned ring that results reach pageable memory through
+
 struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -285,12 +287,24 @@ struct Ctx {
   uint32_t emst_minima = 0;        // total per-round minima logged
   bool emst_ready = false;
   struct HierState* hier = nullptr;  // direct hierarchy (ehgp_hier.cu)
+  char* stage = nullptr;             // pinned ring of copy_out, made by the first large copy
+  void* stage_map = nullptr;         // the mapping that holds it
+  cudaEvent_t stage_ev[kStageSlots] = {};
 };
 
 // Allocation helper: records the bytes on ctx.
 cudaError_t ctx_alloc(Ctx& ctx, void** ptr, size_t bytes);
 // Frees one allocation of ctx_alloc (bytes as allocated).
 void ctx_free(Ctx& ctx, void* ptr, size_t bytes);
+
+// One device range and the host memory it goes to.
+struct CopyOut {
+  char* dst;
+  const char* src;
+  uint64_t bytes;
+};
+// Copies device ranges to host memory and waits for them (ehgp_context.cu).
+cudaError_t copy_out(Ctx& ctx, const std::vector<CopyOut>& list);
 
 // LBVH stage (ehgp_lbvh.cu)
 // Launch constants of the build that also size its scratch, shared by the context

@@ -832,19 +832,13 @@ cudaError_t lbvh_export(Ctx& ctx, uint32_t n, const ehgp_lbvh_out* out) {
                                                         d_src, wl, wn, ws);
     ctx.last_launches += 1;
   }
-  cudaError_t e;
-  if (wn && (e = cudaMemcpyAsync(out->nodes, d_nodes, (2ull * n - 1) * sizeof(ehgp_lbvh_node),
-                                 cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-    return e;
-  if (wl && (e = cudaMemcpyAsync(out->leaves, d_leaves, n * sizeof(ehgp_lbvh_leaf), cudaMemcpyDeviceToHost, st)) !=
-                cudaSuccess)
-    return e;
-  if (ws && (e = cudaMemcpyAsync(out->source_index, d_src, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, st)) !=
-                cudaSuccess)
-    return e;
   uint64_t frame[12];
-  if ((e = cudaMemcpyAsync(frame, b.frame, sizeof(frame), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+  std::vector<CopyOut> list{{(char*)frame, (const char*)b.frame, sizeof(frame)}};
+  if (wn) list.push_back({(char*)out->nodes, (const char*)d_nodes, (2ull * n - 1) * sizeof(ehgp_lbvh_node)});
+  if (wl) list.push_back({(char*)out->leaves, (const char*)d_leaves, n * sizeof(ehgp_lbvh_leaf)});
+  if (ws) list.push_back({(char*)out->source_index, (const char*)d_src, n * sizeof(uint64_t)});
+  const cudaError_t e = copy_out(ctx, list);
+  if (e != cudaSuccess) return e;
   if (out->root_aabb_bits) std::memcpy(out->root_aabb_bits, frame, 6 * sizeof(uint64_t));
   if (out->root_node_index) *out->root_node_index = 2ull * n - 2;
   if (out->counters) {

@@ -830,9 +830,9 @@ int ehgp_pairs(ehgp_ctx* ctx, uint32_t K, const ehgp_pairs_out* out) {
   if (out && out->count) *out->count = m;
   if (out && out->records && m) {
     if (out->capacity < m) return ehgp::abi_fail(ctx, EHGP_ERR_CAPACITY, "the output capacity is below the record count");
-    e = cudaMemcpy(out->records, ctx->pb.sorted, (uint64_t)m * 64, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && out->level_num)
-      e = cudaMemcpy(out->level_num, ctx->pb.levelD, (uint64_t)m * 32, cudaMemcpyDeviceToHost);
+    std::vector<ehgp::CopyOut> list{{(char*)out->records, (const char*)ctx->pb.sorted, (uint64_t)m * 64}};
+    if (out->level_num) list.push_back({(char*)out->level_num, (const char*)ctx->pb.levelD, (uint64_t)m * 32});
+    e = ehgp::copy_out(*ctx, list);
     if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "pair copy");
   }
   return EHGP_OK;

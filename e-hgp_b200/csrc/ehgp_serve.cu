@@ -24,17 +24,63 @@
 #include "ehgp_internal.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <condition_variable>
+#include <cstdlib>
 #include <cstring>
 #include <deque>
 #include <memory>
 #include <thread>
 #include <unordered_map>
 
+#include <sys/mman.h>
+
 namespace {
 
 using Clock = std::chrono::steady_clock;
+
+// Result array of plain records, not initialised: its pages are first touched by the threads that fill
+// it (a vector's zeroing touched them all in one thread before).  Large arrays are mapped with huge
+// pages advised, so that touching them is a fault per 2 MB.
+template <class T>
+class ResultArray {
+ public:
+  ResultArray() = default;
+  ResultArray(const ResultArray&) = delete;
+  ResultArray& operator=(const ResultArray&) = delete;
+  ~ResultArray() { drop(); }
+  bool resize(uint64_t n) {
+    drop();
+    const size_t bytes = n * sizeof(T);
+    if (bytes == 0) return true;
+    if (bytes >= kMapped) {
+      void* p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+      if (p == MAP_FAILED) return false;
+      madvise(p, bytes, MADV_HUGEPAGE);
+      p_ = static_cast<T*>(p);
+    } else {
+      p_ = static_cast<T*>(std::malloc(bytes));
+      if (!p_) return false;
+    }
+    n_ = n;
+    return true;
+  }
+  T* data() const { return p_; }
+  uint64_t bytes() const { return n_ * sizeof(T); }
+  T& operator[](uint64_t i) const { return p_[i]; }
+
+ private:
+  static constexpr size_t kMapped = size_t{4} << 20;
+  void drop() {
+    if (p_ && bytes() >= kMapped) munmap(p_, bytes());
+    else std::free(p_);
+    p_ = nullptr;
+    n_ = 0;
+  }
+  T* p_ = nullptr;
+  uint64_t n_ = 0;
+};
 
 struct Request {
   uint64_t id = 0;
@@ -52,13 +98,13 @@ struct Request {
   double device_ms = 0;
   // result
   ehgp_hier_counts counts{};
-  std::vector<ehgp_forest_node> nodes;
-  std::vector<uint32_t> children;
-  std::vector<ehgp_forest_batch> batches;
-  std::vector<ehgp_forest_root> roots;
-  std::vector<ehgp_vertical_assignment> vertical;
-  std::vector<uint32_t> node_support;  // 5 words per node
-  std::vector<uint32_t> emst_u, emst_v;
+  ResultArray<ehgp_forest_node> nodes;
+  ResultArray<uint32_t> children;
+  ResultArray<ehgp_forest_batch> batches;
+  ResultArray<ehgp_forest_root> roots;
+  ResultArray<ehgp_vertical_assignment> vertical;
+  ResultArray<uint32_t> node_support;  // 5 words per node
+  ResultArray<uint32_t> emst_u, emst_v;
 };
 
 struct Worker {
@@ -77,7 +123,7 @@ struct ehgp_server {
   uint64_t reserved = 0;            // reservations of the running requests
   std::vector<Worker> workers;
   std::deque<uint64_t> queue;
-  std::unordered_map<uint64_t, std::unique_ptr<Request>> reqs;
+  std::unordered_map<uint64_t, std::shared_ptr<Request>> reqs;  // shared with result copies under way
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
   bool stop = false;
@@ -96,8 +142,7 @@ int run_request(ehgp_ctx* ctx, Request& r) {
   int st = r.f32 ? ehgp_lbvh_build_f32(ctx, r.xyz32.data(), r.n, &none) : ehgp_lbvh_build(ctx, r.xyz64.data(), r.n, &none);
   if (st != EHGP_OK) return st;
   if (r.n >= 2) {
-    r.emst_u.resize(r.n - 1);
-    r.emst_v.resize(r.n - 1);
+    if (!r.emst_u.resize(r.n - 1) || !r.emst_v.resize(r.n - 1)) return EHGP_ERR_OUT_OF_MEMORY;
     ehgp_emst_out eo{};
     eo.u = r.emst_u.data();
     eo.v = r.emst_v.data();
@@ -109,11 +154,9 @@ int run_request(ehgp_ctx* ctx, Request& r) {
   r.device_ms = ms;
   if (st != EHGP_OK) return st;
   const ehgp_hier_counts& c = r.counts;
-  r.nodes.resize(c.nodes);
-  r.children.resize(c.children);
-  r.batches.resize(c.journal_batches);
-  r.roots.resize(c.final_roots);
-  r.vertical.resize(c.vertical_assignments);
+  if (!r.nodes.resize(c.nodes) || !r.children.resize(c.children) || !r.batches.resize(c.journal_batches) ||
+      !r.roots.resize(c.final_roots) || !r.vertical.resize(c.vertical_assignments) || !r.node_support.resize(5 * c.nodes))
+    return EHGP_ERR_OUT_OF_MEMORY;
   ehgp_hier_out out{};
   out.nodes = r.nodes.data();
   out.children = r.children.data();
@@ -123,7 +166,6 @@ int run_request(ehgp_ctx* ctx, Request& r) {
   if ((st = ehgp_hier_copy(ctx, &out)) != EHGP_OK) return st;
   std::vector<uint32_t> lev(c.nodes);
   for (uint64_t i = 0; i < c.nodes; ++i) lev[i] = r.nodes[i].level_event;
-  r.node_support.resize(5 * c.nodes);
   return ehgp_event_supports(ctx, lev.data(), c.nodes, r.node_support.data());
 }
 
@@ -239,7 +281,7 @@ int ehgp_cloud_submit(ehgp_server* s, const ehgp_cloud_desc* d, ehgp_request_id*
   if (!s || !d || !id || !d->xyz || d->n == 0 || d->K == 0 || d->K > 10 || d->dtype > 1)
     return EHGP_ERR_INVALID_ARGUMENT;
   if (d->n > s->limits.max_points) return EHGP_ERR_CAPACITY;
-  std::unique_ptr<Request> r(new Request());
+  std::shared_ptr<Request> r(new Request());
   r->n = d->n;
   r->K = d->K;
   r->f32 = d->dtype == EHGP_DTYPE_F32;
@@ -307,12 +349,28 @@ const char* ehgp_request_error(ehgp_server* s, ehgp_request_id id) {
 
 int ehgp_result_copy(ehgp_server* s, ehgp_request_id id, const ehgp_served_out* out) {
   if (!s || !out) return EHGP_ERR_INVALID_ARGUMENT;
-  std::lock_guard<std::mutex> lock(s->mu);
-  Request* r = find(s, id);
-  if (!r) return EHGP_ERR_INVALID_ARGUMENT;
-  if (r->state != EHGP_REQ_DONE) return EHGP_ERR_NOT_BUILT;
-  auto put = [](auto* dst, const auto& v) {
-    if (dst && !v.empty()) std::memcpy(dst, v.data(), v.size() * sizeof(v[0]));
+  std::shared_ptr<Request> r;  // a finished request's result does not change: copied outside the lock
+  {
+    std::lock_guard<std::mutex> lock(s->mu);
+    auto it = s->reqs.find(id);
+    if (it == s->reqs.end()) return EHGP_ERR_INVALID_ARGUMENT;
+    if (it->second->state != EHGP_REQ_DONE) return EHGP_ERR_NOT_BUILT;
+    r = it->second;
+  }
+  struct Piece {
+    char* dst;
+    const char* src;
+    uint64_t bytes;
+  };
+  constexpr uint64_t kPiece = uint64_t{4} << 20;
+  std::vector<Piece> pieces;
+  uint64_t total = 0;
+  auto put = [&](auto* dst, const auto& v) {
+    if (!dst) return;
+    total += v.bytes();
+    for (uint64_t o = 0; o < v.bytes(); o += kPiece)
+      pieces.push_back({reinterpret_cast<char*>(dst) + o, reinterpret_cast<const char*>(v.data()) + o,
+                        std::min(kPiece, v.bytes() - o)});
   };
   put(out->nodes, r->nodes);
   put(out->children, r->children);
@@ -322,6 +380,20 @@ int ehgp_result_copy(ehgp_server* s, ehgp_request_id id, const ehgp_served_out* 
   put(out->node_supports, r->node_support);
   put(out->emst_u, r->emst_u);
   put(out->emst_v, r->emst_v);
+  std::atomic<size_t> next{0};
+  auto work = [&] {
+    for (size_t i; (i = next.fetch_add(1)) < pieces.size();) std::memcpy(pieces[i].dst, pieces[i].src, pieces[i].bytes);
+  };
+  std::vector<std::thread> pool;
+  if (total >= 4 * kPiece) {
+    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+    try {
+      for (unsigned i = 1; i < std::min(8u, hw); ++i) pool.emplace_back(work);
+    } catch (...) {  // no more threads: this one copies too
+    }
+  }
+  work();
+  for (auto& t : pool) t.join();
   return EHGP_OK;
 }
 
