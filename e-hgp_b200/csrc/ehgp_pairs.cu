@@ -44,6 +44,7 @@ namespace ehgp {
 namespace {
 
 constexpr int kThreads = 128;
+constexpr int kPairsBlocks = 5;  // resident blocks of k_pairs that the registers are shared out for (see there)
 constexpr uint32_t kStack = 512; // warp traversal stack
 // While the stack holds more than this, one node is taken per step: depth first, a walk adds at
 // most the tree's depth (63 + log2 n + 1) to it.
@@ -427,7 +428,10 @@ __device__ __forceinline__ void flush_records(const WarpShared& sh, uint32_t& ke
 // tasks == nullptr: warp i starts the walk of Morton position i at the root; else it goes on with
 // tasks[i].  Walks longer than kPairSteps leave the rest of their stack in next[0 .. *next_count)
 // (those that do not fit are counted only).
-__global__ void __launch_bounds__(kThreads)
+// Bound by the latency of the walk's dependent loads, so the registers are held to five blocks per SM
+// (102, against 147 and three): 29,791 lattice points 4.81 -> 3.86 ms, 50,653 at K = 4 3.46 -> 2.55,
+// 15,000 mixture points 8.82 -> 7.86; at six blocks 4.02 / 2.67 / 9.00 (the spills cost more).
+__global__ void __launch_bounds__(kThreads, kPairsBlocks)
 k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, const uint32_t* __restrict__ leaf_pid,
         const uint32_t* __restrict__ n_begin, const uint32_t* __restrict__ n_end, const double* __restrict__ px,
         const double* __restrict__ py, const double* __restrict__ pz, const int* __restrict__ scale,
