@@ -87,18 +87,18 @@ __host__ __device__ inline uint32_t nblk(uint64_t n, int t) {
 }
 
 // Device layouts of the support records (ehgp_pairs.cu, ehgp_higher.cu).
-struct PairRecD {
+struct alignas(16) PairRecD {
   uint32_t u, v, interior, shell, witness;
   uint32_t ids[9];
   uint32_t pad[2];
 };
-struct HigherRecD {
+struct alignas(16) HigherRecD {
   uint32_t size;
   uint32_t ids[4];
   uint32_t interior, shell, witness;
   uint32_t iids[8];
 };
-struct EvRec {
+struct alignas(16) EvRec {
   uint32_t size, ids[4], nint, rank, iids[9];
 };
 static_assert(sizeof(EvRec) == 64 && sizeof(PairRecD) == 64 && sizeof(HigherRecD) == 64, "64-byte records");
@@ -533,9 +533,11 @@ __global__ void k_rank_gather(uint32_t m, const uint32_t* __restrict__ v0, const
   if (i < m) out[i] = radix_result(state, passes, v0, v1)[i];
 }
 
-__host__ __device__ inline uint32_t facet_hash(const uint32_t* ids, int k) {
+__device__ __forceinline__ uint32_t facet_hash(const uint32_t* ids, int k) {
   uint64_t h = 0x9E3779B97F4A7C15ull ^ (uint64_t)k;
-  for (int i = 0; i < k; ++i) {
+#pragma unroll
+  for (int i = 0; i < kMaxFacet; ++i) {
+    if (i >= k) break;
     h ^= ids[i];
     h *= 0xFF51AFD7ED558CCDull;
     h ^= h >> 33;
@@ -545,17 +547,23 @@ __host__ __device__ inline uint32_t facet_hash(const uint32_t* ids, int k) {
   return (uint32_t)h;
 }
 
-__device__ __forceinline__ int event_facet(const EvRec& e, uint32_t* F) {  // I u U, ascending
-  int k = 0;
-  for (uint32_t j = 0; j < e.nint; ++j) F[k++] = e.iids[j];
-  for (uint32_t j = 0; j < e.size; ++j) F[k++] = e.ids[j];
-  for (int a = 1; a < k; ++a) {
-    const uint32_t x = F[a];
-    int b = a;
-    while (b > 0 && F[b - 1] > x) { F[b] = F[b - 1]; --b; }
-    F[b] = x;
-  }
-  return k;
+// I u U, ascending, filled up with kInvalid32: a compare network, so that the words stay in registers.
+__device__ __forceinline__ int event_facet(const EvRec& e, uint32_t (&F)[kMaxFacet + 1]) {
+#pragma unroll
+  for (int j = 0; j <= kMaxFacet; ++j) F[j] = kInvalid32;
+  auto put = [&](uint32_t x) {
+#pragma unroll
+    for (int j = 0; j <= kMaxFacet; ++j) {
+      const uint32_t lo = min(F[j], x);
+      x = max(F[j], x);
+      F[j] = lo;
+    }
+  };
+#pragma unroll
+  for (uint32_t j = 0; j < 9; ++j) put(j < e.nint ? e.iids[j] : kInvalid32);
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j) put(j < e.size ? e.ids[j] : kInvalid32);
+  return (int)(e.nint + e.size);
 }
 
 // Births of orders >= 2: handle = n + position in the rank partition; facets stored
@@ -568,8 +576,9 @@ __global__ void k_birth_insert(uint32_t nb, uint32_t n, uint32_t birth_base, con
   const uint32_t fi = rank_order[birth_base + b];
   uint32_t F[kMaxFacet + 1];
   const int k = event_facet(ev[fi], F);
-  uint32_t* out = bfac + (uint64_t)b * kMaxFacet;
-  for (int j = 0; j < kMaxFacet; ++j) out[j] = j < k ? F[j] : kInvalid32;
+  uint2* out = reinterpret_cast<uint2*>(bfac + (uint64_t)b * kMaxFacet);  // 40-byte rows
+#pragma unroll
+  for (int j = 0; j < kMaxFacet; j += 2) out[j / 2] = make_uint2(F[j], F[j + 1]);
   const uint32_t h = n + b;
   uint32_t s = facet_hash(F, k) & mask;
   for (uint32_t probe = 0; probe <= mask; ++probe) {
@@ -625,9 +634,13 @@ __device__ uint32_t probe_facet(const DescentParams& d, const uint32_t* F, int k
   for (uint32_t probe = 0; probe <= d.mask; ++probe) {
     const uint32_t h = __ldg(d.slots + s);
     if (h == kInvalid32) return kInvalid32;
-    const uint32_t* f = d.bfac + (uint64_t)(h - d.n) * kMaxFacet;
+    const uint2* f = reinterpret_cast<const uint2*>(d.bfac + (uint64_t)(h - d.n) * kMaxFacet);
     bool eq = true;
-    for (int j = 0; j < kMaxFacet && eq; ++j) eq = __ldg(f + j) == (j < k ? F[j] : kInvalid32);
+#pragma unroll
+    for (int j = 0; j < kMaxFacet; j += 2) {
+      const uint2 x = __ldg(f + j / 2);
+      eq &= x.x == (j < k ? F[j] : kInvalid32) && x.y == (j + 1 < k ? F[j + 1] : kInvalid32);
+    }
     if (eq) return h;
     s = (s + 1) & d.mask;
   }
@@ -1037,15 +1050,6 @@ __device__ __noinline__ int topk_choice(const DescentParams& d, const Cloud& c, 
   return kArmOk;
 }
 
-// Facet of arm a: F_u = (I u U) \ {u}, ascending.
-__device__ __forceinline__ int arm_facet(const EvRec& e, uint32_t removed, uint32_t* F) {
-  int k = event_facet(e, F);
-  int w = 0;
-  for (int j = 0; j < k; ++j)
-    if (F[j] != removed) F[w++] = F[j];
-  return w;
-}
-
 // Arm seeds and their first probe, one thread per saddle family: one arm per support point
 // (F_u = (I u U) \ {u}); most arms are themselves a birth facet of their order.  Misses are queued
 // with their facet for the descent steps while they fit (q_count counts them all).
@@ -1058,13 +1062,16 @@ __global__ void k_arm_probe(DescentParams d, uint32_t f0, uint32_t nfam, const u
   const uint32_t f = f0 + (on ? i : 0u), a0 = armoff[f];
   const EvRec e = ev[fam_event[f]];
   const uint32_t lane = threadIdx.x & 31u;
+  uint32_t S[kMaxFacet + 1];
+  const int k = event_facet(e, S) - 1;
+#pragma unroll
   for (uint32_t t = 0; t < 4; ++t) {  // the whole warp: its misses take their slots with one atomic
     const bool arm = on && t < e.size;
-    uint32_t F[kMaxFacet + 1];
-    int k = 0;
+    uint32_t F[kMaxFacet];  // of arm t: (I u U) \ {u}, ascending
+#pragma unroll
+    for (int j = 0; j < kMaxFacet; ++j) F[j] = S[j] < e.ids[t] ? S[j] : S[j + 1];
     bool miss = false;
     if (arm) {
-      k = arm_facet(e, e.ids[t], F);
       const uint32_t h = probe_facet(d, F, k);
       removed[a0 + t] = e.ids[t];
       term[a0 + t] = h;
@@ -1078,7 +1085,8 @@ __global__ void k_arm_probe(DescentParams d, uint32_t f0, uint32_t nfam, const u
     if (!miss || slot >= q_cap) continue;
     q_arm[slot] = a0 + t;
     QFacet q;
-    for (int j = 0; j < kMaxFacet; ++j) q.F[j] = j < k ? F[j] : kInvalid32;
+#pragma unroll
+    for (int j = 0; j < kMaxFacet; ++j) q.F[j] = F[j];
     for (int j = 0; j < 4; ++j) q.prev[j] = kInvalid32;
     q.prev_lo = 0.0;
     q_fac[slot] = q;
