@@ -295,12 +295,15 @@ __global__ void k_ev_gather(uint32_t m, const uint32_t* __restrict__ v0, const u
 struct OpMax {
   __device__ double operator()(double a, double b) const { return fmax(a, b); }
 };
+struct OpSum {
+  __device__ uint32_t operator()(uint32_t a, uint32_t b) const { return a + b; }
+};
 struct OpMin {
   __device__ double operator()(double a, double b) const { return fmin(a, b); }
 };
 
 // Inclusive prefix max of hi[i] = mid + err (forward) and suffix min of lo = mid - err
-// (backward), chunked: one block per 1024 items, then a sequential pass over blocks.
+// (backward), chunked: one block per 1024 items, then a pass over the blocks' results.
 template <class Op>
 __global__ void k_scan_blocks(uint32_t m, const double* __restrict__ mid, const double* __restrict__ err, double sgn,
                               int reverse, double* __restrict__ out, double* __restrict__ bsum, Op op, double ident) {
@@ -334,14 +337,34 @@ __global__ void k_scan_blocks(uint32_t m, const double* __restrict__ mid, const 
   if (threadIdx.x == 0) bsum[blockIdx.x] = sh[1023];
 }
 
-template <class Op>
-__global__ void k_scan_carry(uint32_t nb, double* __restrict__ bsum, Op op, double ident) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double run = ident;
-  for (uint32_t b = 0; b < nb; ++b) {
-    const double v = bsum[b];
-    bsum[b] = run;  // exclusive carry
-    run = op(run, v);
+// Exclusive scan of the block results, in place, by one block: bound by the chain of 1,024-item tiles.
+// One thread alone took 0.34 ms for the 4,818 results of 4.9 million events (the four such launches of
+// 24.8 million events: 4 ms of the hierarchy call).
+template <class T, class Op>
+__global__ void __launch_bounds__(1024) k_carry(uint32_t nb, T* __restrict__ bsum, Op op, T ident) {
+  __shared__ T w[32];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  T carry = ident;
+  for (uint32_t b = 0; b < nb; b += 1024) {
+    const uint32_t i = b + threadIdx.x;
+    T x = i < nb ? bsum[i] : ident;
+    for (int o = 1; o < 32; o <<= 1) {
+      const T y = __shfl_up_sync(0xffffffffu, x, o);
+      if ((int)lane >= o) x = op(y, x);
+    }
+    if (lane == 31) w[warp] = x;
+    x = __shfl_up_sync(0xffffffffu, x, 1);  // exclusive within the warp
+    if (lane == 0) x = ident;
+    __syncthreads();
+    T y = w[lane];
+    for (int o = 1; o < 32; o <<= 1) {  // every warp scans the warps' results
+      const T z = __shfl_up_sync(0xffffffffu, y, o);
+      if ((int)lane >= o) y = op(z, y);
+    }
+    const T before = __shfl_sync(0xffffffffu, y, (int)((warp + 31u) & 31u)), all = __shfl_sync(0xffffffffu, y, 31);
+    if (i < nb) bsum[i] = op(carry, warp ? op(before, x) : x);
+    carry = op(carry, all);
+    __syncthreads();
   }
 }
 
@@ -492,16 +515,6 @@ __global__ void k_sum_blocks(uint32_t m, const uint32_t* __restrict__ in, uint32
   for (uint32_t t = threadIdx.x; t < 1024; t += blockDim.x)
     if (base + t < m) out[base + t] = sh[t];
   if (threadIdx.x == 0) bsum[blockIdx.x] = sh[1023];
-}
-
-__global__ void k_sum_carry(uint32_t nb, uint32_t* __restrict__ bsum) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  uint32_t run = 0;
-  for (uint32_t b = 0; b < nb; ++b) {
-    const uint32_t v = bsum[b];
-    bsum[b] = run;
-    run += v;
-  }
 }
 
 __global__ void k_sum_apply(uint32_t m, uint32_t* __restrict__ out, const uint32_t* __restrict__ bsum, int minus1) {
@@ -1755,11 +1768,11 @@ void scan_minmax(cudaStream_t st, uint32_t m, const double* mid, const double* e
   const uint32_t nb = nblk(m, 1024);
   if (forward_max) {
     k_scan_blocks<<<nb, 256, 0, st>>>(m, mid, err, 1.0, 0, out, bsum, OpMax{}, -INFINITY);
-    k_scan_carry<<<1, 1, 0, st>>>(nb, bsum, OpMax{}, -INFINITY);
+    k_carry<<<1, 1024, 0, st>>>(nb, bsum, OpMax{}, -(double)INFINITY);
     k_scan_apply<<<nblk(m, kT), kT, 0, st>>>(m, 0, out, bsum, OpMax{});
   } else {
     k_scan_blocks<<<nb, 256, 0, st>>>(m, mid, err, -1.0, 1, out, bsum, OpMin{}, INFINITY);
-    k_scan_carry<<<1, 1, 0, st>>>(nb, bsum, OpMin{}, INFINITY);
+    k_carry<<<1, 1024, 0, st>>>(nb, bsum, OpMin{}, (double)INFINITY);
     k_scan_apply<<<nblk(m, kT), kT, 0, st>>>(m, 1, out, bsum, OpMin{});
   }
   *launches += 3;
@@ -1902,7 +1915,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
     k_level_class<<<nblk(m, kT), kT, 0, st>>>(m, h.eqprev, flag);
     const uint32_t nb = nblk(m, 1024);
     k_sum_blocks<<<nb, 256, 0, st>>>(m, flag, h.lclass, h.ubsum);
-    k_sum_carry<<<1, 1, 0, st>>>(nb, h.ubsum);
+    k_carry<<<1, 1024, 0, st>>>(nb, h.ubsum, OpSum{}, 0u);
     k_sum_apply<<<nblk(m, kT), kT, 0, st>>>(m, h.lclass, h.ubsum, 1);
     launches += 4;
   }
@@ -1948,7 +1961,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
   if (nfam) {  // arm offsets: inclusive sum of the family sizes into d_armoff + 1
     const uint32_t nb = nblk(nfam, 1024);
     k_sum_blocks<<<nb, 256, 0, st>>>((uint32_t)nfam, h.d_size_rp + fam_lo, h.d_armoff + 1, h.ubsum);
-    k_sum_carry<<<1, 1, 0, st>>>(nb, h.ubsum);
+    k_carry<<<1, 1024, 0, st>>>(nb, h.ubsum, OpSum{}, 0u);
     k_sum_apply<<<nblk(nfam, kT), kT, 0, st>>>((uint32_t)nfam, h.d_armoff + 1, h.ubsum, 0);
     cudaMemsetAsync(h.d_armoff, 0, sizeof(uint32_t), st);
     launches += 3;
