@@ -423,8 +423,9 @@ __device__ __forceinline__ void hook_entry(const uint32_t* cls, uint4 c, uint32_
   const uint32_t v[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    best_next[v[i]] = kNone;
-    if (v[i] == least || word<kShared>(best + v[i]) != f) continue;
+    if (word<kShared>(best + v[i]) != f) continue;
+    best_next[v[i]] = kNone;  // by the one entry that won v[i]: a store per entry queues on a large component
+    if (v[i] == least) continue;
     t.dead[v[i]] = make_uint2(least, cls[f]);
     lab[v[i]] = least;
   }
