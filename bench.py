@@ -13,7 +13,7 @@ descent, frozen-root quotient, hyper-Kruskal forest journal for orders 1..10).
 
 value : p95 over the K timed steps of the step time on the device timeline
         (CUDA events on the library's stream around the whole step; inputs
-        already resident in HBM; the host-side forest sweep is inside).
+        already resident in HBM; the k = 1 forest's host pass is inside).
 e2e   : p95 over K steps of the same step through the public C ABI with host
         buffers (the reference's warm_e2e protocol): pinned host input copied
         in, and the hgp_reduced payload copied back to pinned host memory:
@@ -299,8 +299,8 @@ def served_section(local: int) -> dict:
                 srv.release(r)
         return len(clouds_) / wall, bad
 
-    # the worker count is picked by measurement (each extra worker overlaps one cloud's host
-    # forest pass with another's device stages, and costs host threads and device memory)
+    # the worker count is picked by measurement (each extra worker overlaps one cloud's copies and
+    # host work with another's device stages, and costs a host thread and device memory)
     per_w = {w: served_rate(clouds, w) for w in WORKER_CHOICES}
     best_w = max(per_w, key=lambda w: per_w[w][0])
     served_cps, bad = per_w[best_w]
@@ -397,7 +397,7 @@ def run_ours(args, world, rank, local):
         torch.cuda.synchronize(local)
 
     def resident_step():
-        """Device-resident step: supports stay in HBM; the hierarchy's host passes are inside."""
+        """Device-resident step: supports stay in HBM; the k = 1 forest's host pass is inside."""
         ctx.step_begin()
         ctx._check(lib.ehgp_lbvh_build_device(ctx._h, C.c_void_p(d_pts.data_ptr()), n, C.byref(none_lbvh)))
         ctx._check(lib.ehgp_emst(ctx._h, None))
@@ -512,7 +512,7 @@ def run_ours(args, world, rank, local):
     hs = ctx.hier_stats()
     stage_ms["hierarchy_device"] = float(hs["device_ms"])
     stage_ms["hierarchy_descent"] = float(hs["descent_ms"])
-    stage_ms["hierarchy_forest_host"] = float(hs["forest_ms"])
+    stage_ms["hierarchy_forest"] = float(hs["forest_ms"])
     launches = launches_per_step * args.steps
     # roofline of the dominant device kernel of the step (triple/quad enumeration, k_higher):
     # algorithmic bytes per launch from its counters: 28 B per candidate-set entry staged
@@ -547,21 +547,19 @@ def run_ours(args, world, rank, local):
         "gpu_launches": int(launches),
         "gpu_launches_per_step": int(launches_per_step),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                     # DRAM bytes of one k_higher launch: ncu capture of the 24^3 lattice (102.9 MB read +
-                     # 1,755.9 MB written per launch over 13,824 owners at the 64-register budget),
-                     # scaled per owner to this cloud
-                     "traffic": (102938368 + 1755928576) * n / 13824,
+                     # DRAM bytes of one k_higher launch: ncu capture of the 24^3 lattice (45.2 MB read +
+                     # 386.2 MB written per emitting launch over 13,824 owners), scaled per owner to this cloud
+                     "traffic": (45209344 + 386202880) * n / 13824,
                      "traffic_source": "ncu dram__bytes_read/write.sum on the 13,824-point case, scaled per owner",
                      "kernel": "k_higher (triple/quad support enumeration)",
                      "kernel_ms": kmean, "algorithmic_bytes": alg_bytes,
                      "work": {"status_tests": tested, "classified": classified, "records": emitted,
                               "candidate_set_entries": set_entries},
-                     "note": "FP64 predicate-bound, not byte-bound; traffic is mostly local-memory spills",
+                     "note": "bound by the issue of its binary32 and binary64 tests, not by bytes; traffic is mostly the records",
                      "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"},
         "clocks": clocks.summary(),
     }
-    # roofline of the strict-arm descent step (k_arm_step), the largest share of the device
-    # launch list: 40 B per facet (one descent step) + 32 B per LBVH node its ball query visits
+    # roofline of the strict-arm descent rounds (k_facet_ball, k_facet_step, k_facet_exact): 40 B per facet (one descent step) + 32 B per LBVH node its ball query visits
     steps, visits = int(hs_last["descent_steps"]), int(hs_last["step_node_visits"])
     step_ms = float(hs_last["step_kernels_ms"])
     if step_ms > 0:
@@ -569,10 +567,10 @@ def run_ours(args, world, rank, local):
         d_ach = d_bytes / (step_ms * 1e-3) / 1e9
         line["roofline_descent"] = {
             "bound": "hbm", "achieved": d_ach, "peak": hbm, "unit": "GB/s", "frac": d_ach / hbm, "traffic": None,
-            "kernel": "k_arm_step (strict-arm descent step: exact facet miniball, ball query, exact top-k)",
+            "kernel": "k_facet_ball + k_facet_step + k_facet_exact (strict-arm descent rounds: facet miniball, ball query, top-k)",
             "kernel_ms_total": step_ms, "launches": int(hs_last["step_launches"]),
             "algorithmic_bytes": d_bytes, "work": {"descent_steps": steps, "node_visits": visits},
-            "note": "FP64 miniball and exact top-k per thread; latency-bound, not byte-bound",
+            "note": "bound by the walks' latency and divergence, not by bytes",
             "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"}
     if world == 1 and not args.no_served:
         try:

@@ -20,13 +20,12 @@
 //    on the device (2304-bit level comparisons), so the facade order is exact;
 //  * a stable partition by closed rank gives every order's births and saddle families in
 //    facade order at once; births are hashed by facet on the device;
-//  * each strict arm descends on its own thread: exact facet miniball (FP64 Welzl, then
-//    exact verification, exhaustive exact enumeration as the fallback), LBVH ball query at
-//    the miniball centre, exact top-k with the cutoff shell settled by 832-bit distance
-//    comparisons, the strict level decrease certified, until the facet hits a birth;
-//    the terminal facet does not depend on the locator state (a descent chain only
-//    reaches a minimum, and minima of lower level are bound before the arm's batch), so
-//    every arm of every batch descends in one launch;
+//  * all strict arms descend in rounds of one step per queued facet: miniball support, LBVH ball
+//    query at its centre, the k nearest, the strict level decrease certified, until the facet
+//    hits a birth; what binary64 leaves open takes the exact step (miniball by exhaustive exact
+//    enumeration, cutoff shell by 832-bit distance comparisons).  The terminal facet does not
+//    depend on the locator state (a descent chain only reaches a minimum, and minima of lower
+//    level are bound before the arm's batch), so the arms of all batches descend together;
 //  * the forest journal over the resolved arms is built on the device (ehgp_journal.cu).
 #include "ehgp_internal.cuh"
 #include "ehgp_exact.cuh"
@@ -602,7 +601,7 @@ __global__ void k_birth_insert(uint32_t nb, uint32_t n, uint32_t birth_base, con
   atomicOr(err, kErrCapacity);
 }
 
-// Rank-partition views read by the host pass in sequence: level class and support size
+// Rank-partition views that the forest journal reads in sequence: level class and support size
 // of the event at each rank position.
 __global__ void k_rank_info(uint32_t m, const uint32_t* __restrict__ rank_order, const EvRec* __restrict__ ev,
                             const uint32_t* __restrict__ lclass, uint32_t* __restrict__ cls_rp,
@@ -1681,7 +1680,7 @@ struct HierState {
   double ms_device = 0, ms_forest = 0, ms_descent = 0, ms_ties = 0;
   uint64_t descent_steps = 0, arms = 0, exact_boundaries = 0;
   cudaEvent_t ev_step[2] = {nullptr, nullptr};  // around each descent-step launch
-  double ms_steps = 0;                          // summed k_arm_step launch times
+  double ms_steps = 0;                          // summed launch times of the descent rounds
   uint64_t step_launches = 0;
   uint32_t part_arms = 0;  // arms per part of the descent (0: one part); results never depend on it
 };

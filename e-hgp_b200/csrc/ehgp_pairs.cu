@@ -429,7 +429,7 @@ __device__ __forceinline__ void flush_records(const WarpShared& sh, uint32_t& ke
 // tasks[i].  Walks longer than kPairSteps leave the rest of their stack in next[0 .. *next_count)
 // (those that do not fit are counted only).
 // Bound by the latency of the walk's dependent loads, so the registers are held to five blocks per SM
-// (102, against 147 and three): 29,791 lattice points 4.81 -> 3.86 ms, 50,653 at K = 4 3.46 -> 2.55,
+// (96, against 147 and three): 29,791 lattice points 4.81 -> 3.86 ms, 50,653 at K = 4 3.46 -> 2.55,
 // 15,000 mixture points 8.82 -> 7.86; at six blocks 4.02 / 2.67 / 9.00 (the spills cost more).
 __global__ void __launch_bounds__(kThreads, kPairsBlocks)
 k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, const uint32_t* __restrict__ leaf_pid,

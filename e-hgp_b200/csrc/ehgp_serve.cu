@@ -10,7 +10,7 @@
 //  * submit copies the request's points and queues it; a worker takes the oldest queued
 //    request as soon as it is idle and the request fits the memory budget, so requests
 //    that arrive while others run are admitted as workers and memory free up, and their
-//    device work and host passes overlap with the others' (continuous batching);
+//    device work and copies overlap with the others' (continuous batching);
 //  * admission by memory: every running request reserves an estimate of the device bytes
 //    its cloud needs (bytes per point, seeded conservatively and raised to the largest
 //    per-point footprint a worker's context has reached); a request is admitted when the
