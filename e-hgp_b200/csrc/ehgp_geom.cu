@@ -32,6 +32,11 @@ namespace ehgp {
 namespace {
 
 constexpr int kThreads = 256;
+// Threads per block of the walks (k_knn, k_bv_nearest): latency-bound, a thread per point, so 50,000 points
+// in blocks of 256 leave some SMs twice the walks of others.  k_knn at 256 / 128 / 64 / 32: 50,653 lattice
+// points 0.52 / 0.45 / 0.46 / 0.46 ms, 8,009 clustered 0.34 / 0.29 / 0.29 / 0.28; the EMST of 50,653 points
+// 2.39 / 2.32 / 2.36 / 2.46, of 100,003 clustered ones 3.22 / 3.21 / 3.31 / 3.36.
+constexpr int kWalkThreads = 128;
 constexpr int kStack = 128;
 constexpr int kKnnMax = 11;
 constexpr int kKnnCap = 48;
@@ -618,7 +623,7 @@ int emst_run(Ctx* ctx) {
     cudaMemsetAsync(g.nflag, 0, 2ull * n * sizeof(uint32_t), st);
     k_bv_node_labels<<<nblocks(n), kThreads, 0, st>>>(n, g.leaf_node, b.leaf_pid, g.labels, b.n_parent, b.n_left,
                                                        b.n_right, g.nlabel, g.nflag, ctx->d_err);
-    k_bv_nearest<<<nblocks(n), kThreads, 0, st>>>(n, root, g.tnodes, b.leaf_pid, g.labels, g.nlabel, b.px, b.py,
+    k_bv_nearest<<<nblocks(n, kWalkThreads), kWalkThreads, 0, st>>>(n, root, g.tnodes, b.leaf_pid, g.labels, g.nlabel, b.px, b.py,
                                                    b.pz, g.scale, g.best_q, g.best_d, ctx->d_err);
     cudaMemsetAsync(g.comp_dbits, 0xff, n * sizeof(unsigned long long), st);
     cudaMemsetAsync(g.comp_best, 0xff, n * sizeof(uint32_t), st);
@@ -698,7 +703,7 @@ int ehgp_knn(ehgp_ctx* ctx, uint32_t k, const ehgp_knn_out* out) {
   ehgp::GeomBuffers& g = ctx->gb;
   ehgp::LbvhBuffers& b = ctx->lb;
   cudaEventRecord(ctx->ev0, ctx->stream);
-  ehgp::k_knn<<<ehgp::nblocks(n), ehgp::kThreads, 0, ctx->stream>>>(n, k, 2 * n - 2, g.tnodes, b.leaf_pid, b.px,
+  ehgp::k_knn<<<ehgp::nblocks(n, ehgp::kWalkThreads), ehgp::kWalkThreads, 0, ctx->stream>>>(n, k, 2 * n - 2, g.tnodes, b.leaf_pid, b.px,
                                                                      b.py, b.pz, g.scale, g.knn_ids, g.knn_meta,
                                                                      g.knn_cut, ctx->d_err);
   cudaEventRecord(ctx->ev1, ctx->stream);
