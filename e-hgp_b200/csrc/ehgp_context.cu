@@ -406,6 +406,10 @@ int ehgp_tune(ehgp_ctx* ctx, uint32_t knob, uint64_t value) {
       if (value < 1 || value > 1024) return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "list capacity must be in [1, 1024]");
       ctx->hb.list_cap = (uint32_t)value;
       return EHGP_OK;
+    case EHGP_TUNE_PAIR_TASKS:
+      if (value > ctx->pb.task_cap) return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "handed-over walks are at most 2 * max_points + 4096");
+      ctx->pb.task_limit = (uint32_t)value;
+      return EHGP_OK;
     default:
       return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "unknown tuning knob");
   }

@@ -178,6 +178,7 @@ struct PairBuffers {
   uint32_t* W = nullptr;            // [n * 64] witness lists (64 nearest, FP64 order)
   void* tasks = nullptr;            // [2 * task_cap] walks handed over between rounds
   uint32_t task_cap = 0;
+  uint32_t task_limit = 0;          // of them used per round (<= task_cap)
   double* R2 = nullptr;             // [n] squared witness radius
   void* raw = nullptr;              // [capacity] 64-byte records, unordered
   void* sorted = nullptr;           // [capacity] records in (u, v) order

@@ -426,8 +426,10 @@ __device__ __forceinline__ void flush_records(const WarpShared& sh, uint32_t& ke
 }
 
 // tasks == nullptr: warp i starts the walk of Morton position i at the root; else it goes on with
-// tasks[i].  Walks longer than kPairSteps leave the rest of their stack in next[0 .. *next_count)
-// (those that do not fit are counted only).
+// tasks[i].  Walks longer than kPairSteps leave the rest of their stack in next[0 .. next_cap).  A
+// reservation is never given back (*next_count may end above next_cap): the ranges that warps are
+// given are disjoint and leave no slot below min(*next_count, next_cap) unwritten.  What does not fit is
+// walked on in place, by a warp that asks no more.
 // Bound by the latency of the walk's dependent loads, so the registers are held to five blocks per SM
 // (96, against 147 and three): 29,791 lattice points 4.81 -> 3.86 ms, 50,653 at K = 4 3.46 -> 2.55,
 // 15,000 mixture points 8.82 -> 7.86; at six blocks 4.02 / 2.67 / 9.00 (the spills cost more).
@@ -440,11 +442,12 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
         uint32_t* __restrict__ err, const PairTask* __restrict__ tasks, uint32_t ntask, PairTask* __restrict__ next,
         uint32_t next_cap, uint32_t* __restrict__ next_count) {
   __shared__ WarpShared shared[kWarpsPerBlock];
-  __shared__ unsigned long long s_stats[5];
-  if (threadIdx.x < 5) s_stats[threadIdx.x] = 0;
+  __shared__ unsigned long long s_stats[6];
+  if (threadIdx.x < 6) s_stats[threadIdx.x] = 0;
   __syncthreads();
   // work counters (identical in every lane; lane 0 publishes them)
   unsigned long long visits = 0, local_pairs = 0, ball_queries = 0, ball_nodes = 0, emitted = 0;
+  uint32_t refused = 0;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t wi = blockIdx.x * kWarpsPerBlock + warp;
   if (wi < (tasks ? ntask : n)) {  // uniform per warp
@@ -467,8 +470,9 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
                         __popc(__ballot_sync(0xffffffffu, w1 != kInvalid32));  // the first nw slots
     const uint32_t need = cap + 1;
     uint32_t top = 1, nleaf = 0, kept = 0, steps = 0;
+    bool list_full = false;
     if (tasks) {
-      top = tasks[wi].count;
+      top = min(tasks[wi].count, kTaskNodes);
       if (lane < top) sh.stack[lane] = tasks[wi].node[lane];
     } else if (lane == 0) {
       sh.stack[0] = root;
@@ -543,25 +547,25 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
         __syncwarp();
         continue;
       }
-      if (steps >= kPairSteps && top > 1) {  // hand the rest over (the top first: its nodes are the smallest)
+      if (steps >= kPairSteps && top > 1 && !list_full) {  // hand the rest over, from the top
         const uint32_t made = (top + kTaskNodes - 1) / kTaskNodes;
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(next_count, made);
+        uint32_t at = next_cap;
+        if (lane == 0 && *(volatile const uint32_t*)next_count < next_cap) at = atomicAdd(next_count, made);
         at = __shfl_sync(0xffffffffu, at, 0);
-        if (at + made <= next_cap) {
-          for (uint32_t i = lane; i < made; i += 32) {
-            PairTask t;
-            t.pos = pos;
-            t.count = min(kTaskNodes, top - i * kTaskNodes);
-            for (uint32_t j = 0; j < kTaskNodes; ++j) t.node[j] = j < t.count ? sh.stack[i * kTaskNodes + j] : 0u;
-            next[at + i] = t;
-          }
-          top = 0;
-          __syncwarp();
-          continue;
+        const uint32_t fit = at < next_cap ? min(made, next_cap - at) : 0u;
+        for (uint32_t i = lane; i < fit; i += 32) {
+          const uint32_t end = top - i * kTaskNodes, begin = end > kTaskNodes ? end - kTaskNodes : 0u;
+          PairTask t;
+          t.pos = pos;
+          t.count = end - begin;
+          for (uint32_t j = 0; j < kTaskNodes; ++j) t.node[j] = j < t.count ? sh.stack[begin + j] : 0u;
+          next[at + i] = t;
         }
-        if (lane == 0) atomicSub(next_count, made);  // no room: the walk goes on here
-        steps = 0;
+        list_full = fit < made;
+        refused = list_full ? 1u : 0u;
+        top -= min(top, fit * kTaskNodes);
+        __syncwarp();
+        continue;
       }
       const uint32_t batch = top > kStackWide ? 1u : min(top, 32u);
       uint32_t node = kInvalid32;
@@ -618,9 +622,10 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
     atomicAdd(s_stats + 2, ball_queries);
     atomicAdd(s_stats + 3, ball_nodes);
     atomicAdd(s_stats + 4, emitted);
+    if (refused) atomicAdd(s_stats + 5, 1ull);
   }
   __syncthreads();
-  if (threadIdx.x < 5 && s_stats[threadIdx.x]) atomicAdd(stats + threadIdx.x, s_stats[threadIdx.x]);
+  if (threadIdx.x < 6 && s_stats[threadIdx.x]) atomicAdd(stats + threadIdx.x, s_stats[threadIdx.x]);
 }
 
 __global__ void __launch_bounds__(256)
@@ -700,7 +705,7 @@ cudaError_t pairs_alloc(Ctx& ctx) {
   EHGP_ALLOC(p.R2, n * sizeof(double));
   EHGP_ALLOC(p.counters, 8 * sizeof(uint32_t));
   EHGP_ALLOC(p.stats, 8 * sizeof(unsigned long long));
-  p.task_cap = (uint32_t)(2 * n + 4096);  // handed-over walks per round (what does not fit goes on in place)
+  p.task_cap = p.task_limit = (uint32_t)(2 * n + 4096);  // handed-over walks per round (what does not fit goes on in place)
   EHGP_ALLOC(p.tasks, 2ull * p.task_cap * sizeof(PairTask));
 #undef EHGP_ALLOC
   // records: about 38 per point in lattices and uniform clouds; grown on demand
@@ -745,13 +750,14 @@ int pairs_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
     cudaEventRecord(ctx.evk0, st);
     unsigned long long hs[8];
     PairTask* task[2] = {(PairTask*)p.tasks, (PairTask*)p.tasks + p.task_cap};
+    uint64_t handed = 0;
     uint32_t ntask = 0;  // 0: the walks from the root; then those that were handed over, while there are any
     for (int round = 0;; ++round) {
       const uint32_t warps = round ? ntask : n;
       k_pairs<<<nblocks(warps, kWarpsPerBlock), kThreads, 0, st>>>(
           n, cap, root, g.tnodes, b.leaf_pid, b.n_begin, b.n_end, b.px, b.py, b.pz, g.scale, p.W, p.R2, (PairRec*)p.raw,
           p.capacity, p.counters, p.stats, ctx.d_err, round ? task[round & 1] : nullptr, ntask, task[(round + 1) & 1],
-          p.task_cap, p.counters + 1);
+          p.task_limit, p.counters + 1);
       ++launches;
       uint32_t hn[2];
       cudaEventRecord(ctx.evk1, st);
@@ -761,7 +767,8 @@ int pairs_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
       e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) return abi_cuda_fail(&ctx, e, "pair enumeration");
       hc[0] = hn[0];
-      ntask = hn[1];
+      ntask = hn[1] < p.task_limit ? hn[1] : p.task_limit;
+      handed += ntask;
       if (ntask == 0 || hc[1]) break;
       cudaMemsetAsync(p.counters + 1, 0, sizeof(uint32_t), st);
     }
@@ -770,6 +777,7 @@ int pairs_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
       cudaEventElapsedTime(&kms, ctx.evk0, ctx.evk1);
       ctx.kernel_ms = kms;
       for (int i = 0; i < 8; ++i) ctx.kernel_stats[i] = hs[i];
+      ctx.kernel_stats[6] = handed;
     }
     if (hc[1]) return abi_device_status(&ctx, hc[1]);
     if (hc[0] <= p.capacity) break;

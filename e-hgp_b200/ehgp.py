@@ -345,6 +345,7 @@ class Context:
         self._check(self.lib.ehgp_ctx_reserve(self._h, stage, records))
 
     TUNE_HIGHER_LIST = 1
+    TUNE_PAIR_TASKS = 2
 
     def tune(self, knob: int, value: int) -> None:
         """ehgp_tune: a tuning knob of later calls (results never depend on it)."""

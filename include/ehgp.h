@@ -99,8 +99,10 @@ int ehgp_checkpoint_load(ehgp_ctx* ctx, const char* path, uint32_t* K);
  * counterpart in the reference).
  *   EHGP_TUNE_HIGHER_LIST: neighbour-list entries (1..1024, default 1024) that a
  *     triple/quad owner may hold before its certificate moves to the
- *     large-neighbourhood path (arena lists of any length). */
-enum { EHGP_TUNE_HIGHER_LIST = 1 };
+ *     large-neighbourhood path (arena lists of any length).
+ *   EHGP_TUNE_PAIR_TASKS: walks of the pair enumeration (0..2 * max_points + 4096, the
+ *     default the largest) that may be handed over to further warps per round. */
+enum { EHGP_TUNE_HIGHER_LIST = 1, EHGP_TUNE_PAIR_TASKS = 2 };
 int ehgp_tune(ehgp_ctx* ctx, uint32_t knob, uint64_t value);
 
 /* ---- LBVH snapshot records (reference layout) ---------------------------- */
@@ -342,7 +344,8 @@ int ehgp_step_end(ehgp_ctx* ctx, double* elapsed_ms);
 /* CUDA-event time of the dominant kernel of the last pair stage (the pair
  * enumeration) and its work counters: [0] LBVH node visits, [1] witness-list
  * classifications, [2] exact ball queries, [3] ball-query node visits,
- * [4] emitted records. */
+ * [4] emitted records, [5] walks that found the hand-over list full, [6] walks
+ * handed over. */
 int ehgp_kernel_stats(const ehgp_ctx* ctx, double* kernel_ms, uint64_t* stats, uint32_t count);
 
 /* ---- direct Morse hierarchy ------------------------------------------------
