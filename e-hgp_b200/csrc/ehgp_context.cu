@@ -300,7 +300,6 @@ int ehgp_ctx_create(int device, const ehgp_limits* limits, ehgp_ctx** out_ctx) {
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->evs1);
   if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_status, 64 * sizeof(uint32_t));
   if (e == cudaSuccess) e = ehgp::ctx_alloc(*ctx, (void**)&ctx->d_err, sizeof(uint32_t));
-  ctx->radix.err = ctx->d_err;
   if (e == cudaSuccess) {
     // admission: the context's resident buffers must fit the HBM fraction
     size_t free_b = 0, total_b = 0;
@@ -409,6 +408,10 @@ int ehgp_tune(ehgp_ctx* ctx, uint32_t knob, uint64_t value) {
     case EHGP_TUNE_PAIR_TASKS:
       if (value > ctx->pb.task_cap) return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "handed-over walks are at most 2 * max_points + 4096");
       ctx->pb.task_limit = (uint32_t)value;
+      return EHGP_OK;
+    case EHGP_TUNE_SORT_WAIT:
+      if (value > ehgp::kRadixWait) return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "a sort looks at most 2^20 times");
+      ctx->radix.wait = (uint32_t)value;
       return EHGP_OK;
     default:
       return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "unknown tuning knob");

@@ -1830,7 +1830,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
   const uint32_t m = (uint32_t)(total - hc[0]);
   h.events = m;
   // facade order by the FP64 level midpoints (diagnostics sort last)
-  RadixScratch rs{h.radix_counts, ctx.radix.state, ctx.d_err};
+  RadixScratch rs{h.radix_counts, ctx.radix.state, ctx.radix.wait};
   if (total) {
     k_iota<<<nblk(total, kT), kT, 0, st>>>((uint32_t)total, h.order0);
     ++launches;

@@ -2562,7 +2562,7 @@ int higher_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
   const uint32_t m = hc[0];
   if (m) {
     k_higher_keys<<<nblocks(m, 256), 256, 0, st>>>(m, (const HigherRec*)h.raw, h.khi, h.klo, h.order0);
-    RadixScratch rs{h.radix_counts, ctx.radix.state, ctx.d_err};
+    RadixScratch rs{h.radix_counts, ctx.radix.state, ctx.radix.wait};
     const IndirectKey stages[2] = {{h.klo, 0}, {h.khi, 0}};
     const int bits[2] = {64, 64};
     const int passes = radix_sort_indirect(st, m, h.order0, h.order1, stages, bits, 2, rs, &launches);

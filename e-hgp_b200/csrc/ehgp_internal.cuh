@@ -45,10 +45,11 @@ __host__ __device__ __forceinline__ uint64_t order_key(uint64_t bits) {
 }
 
 // ---- radix sort of u32 indices by an indirect 64-bit key -----------------
+constexpr uint32_t kRadixWait = 1u << 20;  // looks at an earlier tile's counts (about a second)
 struct RadixScratch {
   uint32_t* counts = nullptr;   // [radix_counts_words(n)] tile counts of two passes
   uint32_t* state = nullptr;    // [kRadixStateWords]
-  uint32_t* err = nullptr;      // device error word (a bounded wait that ran out)
+  uint32_t wait = kRadixWait;   // looks before a block counts the earlier tiles itself
 };
 constexpr int kRadixTile = 2048;        // items of one block and pass
 constexpr int kRadixMaxPasses = 24;     // three 64-bit stages

@@ -1157,7 +1157,7 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
   const uint64_t M = sh.m;
   // sorts m keys; returns the buffers that hold the result
   auto sort = [&](uint64_t m, uint64_t** key, uint32_t** val, int bits, uint64_t** rk, uint32_t** rv, int* passes) -> int {
-    RadixScratch rs{rcounts, ctx.radix.state, ctx.d_err};
+    RadixScratch rs{rcounts, ctx.radix.state, ctx.radix.wait};
     *passes = radix_sort_kv(st, (uint32_t)m, val[0], val[1], key[0], key[1], bits, rs, launches);
     uint32_t which = 0;
     if ((e = cudaMemcpyAsync(&which, ctx.radix.state + 2 * *passes, 4, cudaMemcpyDeviceToHost, st)) == cudaSuccess)
@@ -1268,7 +1268,7 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
     k_fj_node_keys<<<nblk(F), kT, 0, st>>>(j, sh, gs, car, gc, gp, node_slot, key[0], val[0]);
     int bits = 8;
     while (bits < 32 && (H >> bits)) bits += 8;
-    RadixScratch rs{ncounts, ctx.radix.state, ctx.d_err};
+    RadixScratch rs{ncounts, ctx.radix.state, ctx.radix.wait};
     const int passes = radix_sort_kv(st, Nn, val[0], val[1], key[0], key[1], bits, rs, launches);
     k_fj_node_ranges<<<nblk(Nn), kT, 0, st>>>(Nn, val[0], val[1], key[0], key[1], ctx.radix.state, passes, j.cls, node_slot,
                                               t.range, ncls, nidx);

@@ -138,7 +138,6 @@ void carve(ehgp::Ctx& c, unsigned char* base) {
   c.radix.counts = (uint32_t*)at(ehgp::radix_counts_words(n) * 4);
   c.radix.state = (uint32_t*)at(ehgp::kRadixStateWords * 4);
   c.d_err = (uint32_t*)at(4);
-  c.radix.err = c.d_err;
   c.max_points = n;
   // the carve takes exactly the blocks that scratch_bytes() sized
   if (L.off != kScratchBytes) c.max_points = 0;

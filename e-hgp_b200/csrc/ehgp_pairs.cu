@@ -792,7 +792,7 @@ int pairs_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
   const uint32_t m = hc[0];
   if (m) {
     k_pair_keys<<<(m + 255) / 256, 256, 0, st>>>(m, (const PairRec*)p.raw, p.key, p.order0);
-    RadixScratch rs{p.radix_counts, ctx.radix.state, ctx.d_err};
+    RadixScratch rs{p.radix_counts, ctx.radix.state, ctx.radix.wait};
     const IndirectKey stage[1] = {{p.key, 0}};
     const int bits[1] = {64};
     const int passes = radix_sort_indirect(st, m, p.order0, p.order1, stage, bits, 1, rs, &launches);

@@ -11,7 +11,8 @@
 // kernel: a block ranks a tile in shared memory, publishes its digit counts, sums those of the
 // tiles before it while they appear (decoupled look-back: a tile's number is a ticket, so every
 // tile it waits for has already started; the wait has a limit all the same), and writes the tile in
-// digit order.  The host never synchronises inside a sort.  Up to kSmall items one block runs all
+// digit order.  A wait that runs out ends with the block counting those tiles itself, so a sort always
+// completes.  The host never synchronises inside a sort.  Up to kSmall items one block runs all
 // passes in shared memory in one launch.
 // Bound: HBM for large inputs, launches for small ones.  With four kernels per pass (tile histogram,
 // row scan, digit bases, scatter of 1,024-item tiles) an LBVH build was 144 launches: 0.82 ms for 1,021
@@ -25,7 +26,6 @@ constexpr int kT = 256, kWarps = kT / 32;
 constexpr uint32_t kSmall = 2048;    // items that one block sorts on its own
 constexpr int kSmallT = 512, kSmallWarps = kSmallT / 32, kSmallRows = kSmall / kSmallT;
 constexpr int kRows = kRadixTile / kT;  // rows of 32 items per warp and tile
-constexpr uint32_t kSpinLimit = 1u << 24;
 
 // State words: per pass (input buffer, trivial flag), then the digit bases of every pass, then the
 // tile tickets.
@@ -168,10 +168,10 @@ template <bool kKv>
 __global__ void __launch_bounds__(kT) k_radix_pass(uint32_t n, uint32_t* __restrict__ vals0, uint32_t* __restrict__ vals1,
                                                    uint64_t* __restrict__ keys0, uint64_t* __restrict__ keys1, Passes ps,
                                                    int pass, uint32_t* __restrict__ state, uint32_t* look, uint32_t tiles,
-                                                   uint32_t* __restrict__ err) {
+                                                   uint32_t wait) {
   if (state[2 * pass + 1]) return;  // every key has the same digit: order unchanged
   __shared__ uint32_t cnt[kWarps][256];
-  __shared__ uint32_t start[256], gbase[256], tmp[8], s_tile, s_bad;
+  __shared__ uint32_t start[256], gbase[256], tmp[8], s_tile;
   __shared__ uint32_t sval[kRadixTile];
   __shared__ uint64_t skey[kKv ? kRadixTile : 1];
   __shared__ uint8_t sdig[kKv ? 1 : kRadixTile];
@@ -181,10 +181,7 @@ __global__ void __launch_bounds__(kT) k_radix_pass(uint32_t n, uint32_t* __restr
   uint32_t* out = flip ? vals0 : vals1;
   const uint64_t* kin = flip ? keys1 : keys0;
   uint64_t* kout = flip ? keys0 : keys1;
-  if (tid == 0) {
-    s_tile = atomicAdd(state + kTickets + pass, 1u);
-    s_bad = 0;
-  }
+  if (tid == 0) s_tile = atomicAdd(state + kTickets + pass, 1u);
   for (int w = 0; w < kWarps; ++w) cnt[w][tid] = 0;
   __syncthreads();
   const uint32_t tile = s_tile;
@@ -216,26 +213,29 @@ __global__ void __launch_bounds__(kT) k_radix_pass(uint32_t n, uint32_t* __restr
   const uint32_t local = scan256(total, tmp);
   start[tid] = local;
   uint32_t before = 0;
+  bool late = false;
   for (uint32_t t = tile, spin = 0; t > 0;) {
     const uint32_t x = *(volatile const uint32_t*)(look + ((uint64_t)(flip ? tiles : 0) + t - 1) * 256 + tid);
     if (x == 0) {
-      if (++spin > kSpinLimit) {
-        s_bad = 1;
-        break;
-      }
-      continue;
+      if (spin++ < wait) continue;
+      late = true;
+      break;
     }
     before += x & kCountMask;
     if (x & kInclusive) break;
     --t;
   }
+  if (__syncthreads_or(late)) {  // the pass does not change its input: count the tiles before this one
+    sval[tid] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < tile * kRadixTile; i += kT)
+      atomicAdd(sval + (kKv ? (uint32_t)(kin[i] >> (8 * pass)) & 0xffu : indirect_digit(ps, pass, in[i])), 1u);
+    __syncthreads();
+    before = sval[tid];
+  }
   if (tile) atomicExch(mine, (before + total) | kInclusive);
   gbase[tid] = state[kBases + 256 * pass + tid] + before - local;
   __syncthreads();
-  if (s_bad) {  // uniform
-    if (tid == 0) atomicOr(err, kErrTimeout);
-    return;
-  }
 #pragma unroll
   for (int r = 0; r < kRows; ++r) {
     if (dig[r] > 255u) continue;
@@ -340,7 +340,7 @@ int sort(cudaStream_t st, uint32_t n, uint32_t* vals0, uint32_t* vals1, uint64_t
   k_radix_plan<<<1, 1024, 0, st>>>(n, passes, scratch.state);
   for (int p = 0; p < passes; ++p)
     k_radix_pass<kKv><<<tiles, kT, 0, st>>>(n, vals0, vals1, keys0, keys1, ps, p, scratch.state, scratch.counts, tiles,
-                                            scratch.err);
+                                            scratch.wait);
   *launches += 2 + passes;
   return passes;
 }

@@ -346,6 +346,7 @@ class Context:
 
     TUNE_HIGHER_LIST = 1
     TUNE_PAIR_TASKS = 2
+    TUNE_SORT_WAIT = 3
 
     def tune(self, knob: int, value: int) -> None:
         """ehgp_tune: a tuning knob of later calls (results never depend on it)."""

@@ -101,8 +101,10 @@ int ehgp_checkpoint_load(ehgp_ctx* ctx, const char* path, uint32_t* K);
  *     triple/quad owner may hold before its certificate moves to the
  *     large-neighbourhood path (arena lists of any length).
  *   EHGP_TUNE_PAIR_TASKS: walks of the pair enumeration (0..2 * max_points + 4096, the
- *     default the largest) that may be handed over to further warps per round. */
-enum { EHGP_TUNE_HIGHER_LIST = 1, EHGP_TUNE_PAIR_TASKS = 2 };
+ *     default the largest) that may be handed over to further warps per round.
+ *   EHGP_TUNE_SORT_WAIT: how often (0..2^20, the default the largest) a block of a sort
+ *     looks for an earlier block's counts before it counts that block's items itself. */
+enum { EHGP_TUNE_HIGHER_LIST = 1, EHGP_TUNE_PAIR_TASKS = 2, EHGP_TUNE_SORT_WAIT = 3 };
 int ehgp_tune(ehgp_ctx* ctx, uint32_t knob, uint64_t value);
 
 /* ---- LBVH snapshot records (reference layout) ---------------------------- */
