@@ -288,12 +288,13 @@ struct PairTask {
 };
 
 struct WarpShared {
-  float4 wit[kW];                 // w - u (binary32), |w - u|^2
+  float4 wit[kW];                 // scaled w - u (binary32), |w - u|^2
   uint32_t stack[kStack];
   uint32_t queue[kQueue];
   uint32_t ids[kMaxInterior + 64];
   uint32_t leaf[kLeaves + 32];
   PairRec rec[kRecs];
+  double su[4];                   // -u and 1, scaled
 };
 
 // Appends the ids of flagged lanes (two flags per lane) to sh.ids[base...];
@@ -457,13 +458,20 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
     const Pt u = point(px, py, pz, iu);
     const int S = scale[0];
     const double r2u = R2[iu];
+    // The binary32 tests work on differences scaled by a power of two that brings the cloud's largest
+    // coordinate to 2^30, so that their products neither overflow nor lose their margins to underflow
+    // (conversions of denormals and products add up to 2^-117; a witness closer than 2^-48 decides nothing).
+    const double f = __hiloint2double((1023 + min(30 - scale[1], 1000)) << 20, 0);
+    if (lane < 4) sh.su[lane] = lane == 0 ? -u.x * f : lane == 1 ? -u.y * f : lane == 2 ? -u.z * f : f;
     // this lane's two witnesses of u
     const uint32_t w0 = W[(uint64_t)iu * kW + lane], w1 = W[(uint64_t)iu * kW + 32 + lane];
     float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-    if (w0 != kInvalid32) { a0.x = (float)(px[w0] - u.x); a0.y = (float)(py[w0] - u.y); a0.z = (float)(pz[w0] - u.z); }
-    if (w1 != kInvalid32) { a1.x = (float)(px[w1] - u.x); a1.y = (float)(py[w1] - u.y); a1.z = (float)(pz[w1] - u.z); }
+    if (w0 != kInvalid32) { a0.x = (float)((px[w0] - u.x) * f); a0.y = (float)((py[w0] - u.y) * f); a0.z = (float)((pz[w0] - u.z) * f); }
+    if (w1 != kInvalid32) { a1.x = (float)((px[w1] - u.x) * f); a1.y = (float)((py[w1] - u.y) * f); a1.z = (float)((pz[w1] - u.z) * f); }
     a0.w = a0.x * a0.x + a0.y * a0.y + a0.z * a0.z;
     a1.w = a1.x * a1.x + a1.y * a1.y + a1.z * a1.z;
+    if (!(a0.w >= 0x1p-96f)) a0 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!(a1.w >= 0x1p-96f)) a1 = make_float4(0.f, 0.f, 0.f, 0.f);
     sh.wit[lane] = a0;
     sh.wit[32 + lane] = a1;
     const uint32_t nw = __popc(__ballot_sync(0xffffffffu, w0 != kInvalid32)) +
@@ -497,7 +505,7 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
           // reject the pair without a global query.  (w - u).(w - v) = |e|^2 - e.(q - p) with
           // e = w - p for the end p the witness belongs to and q the other end; the margin
           // covers binary32 differences.
-          const double vx = v.x - u.x, vy = v.y - u.y, vz = v.z - u.z;
+          const double sf = sh.su[3], vx = (v.x - u.x) * sf, vy = (v.y - u.y) * sf, vz = (v.z - u.z) * sf;
           auto inside = [&](double ex, double ey, double ez, double sx, double sy, double sz) {
             const double ee = ex * ex + ey * ey + ez * ez, tx = ex * sx, ty = ey * sy, tz = ez * sz;
             return ee - (tx + ty + tz) < -1e-5 * (ee + fabs(tx) + fabs(ty) + fabs(tz));
@@ -506,7 +514,7 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
             return w != kInvalid32 && w != iv && inside(a.x, a.y, a.z, vx, vy, vz);
           };
           auto of_v = [&](uint32_t w) {
-            return w != kInvalid32 && w != iu && inside(px[w] - v.x, py[w] - v.y, pz[w] - v.z, -vx, -vy, -vz);
+            return w != kInvalid32 && w != iu && inside((px[w] - v.x) * sf, (py[w] - v.y) * sf, (pz[w] - v.z) * sf, -vx, -vy, -vz);
           };
           const uint32_t cu = __popc(__ballot_sync(0xffffffffu, of_u(w0, a0))) +
                               __popc(__ballot_sync(0xffffffffu, of_u(w1, a1)));
@@ -581,8 +589,10 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
       if (node != kInvalid32 && n_end[node] > pos + 1) {  // every partner follows u in Morton order
         t = load_node(tn, node);
         open = true;
-        lx = (float)((double)t.lo[0] - u.x), ly = (float)((double)t.lo[1] - u.y), lz = (float)((double)t.lo[2] - u.z);
-        hx = (float)((double)t.hi[0] - u.x), hy = (float)((double)t.hi[1] - u.y), hz = (float)((double)t.hi[2] - u.z);
+        const double sx = sh.su[0], sy = sh.su[1], sz = sh.su[2], sf = sh.su[3];
+        lx = (float)__fma_rn((double)t.lo[0], sf, sx), ly = (float)__fma_rn((double)t.lo[1], sf, sy);
+        lz = (float)__fma_rn((double)t.lo[2], sf, sz), hx = (float)__fma_rn((double)t.hi[0], sf, sx);
+        hy = (float)__fma_rn((double)t.hi[1], sf, sy), hz = (float)__fma_rn((double)t.hi[2], sf, sz);
       }
       if (nw >= need) {
         // max over v in box of (w-u).(w-v) = sum_i a_i (a_i - (a_i >= 0 ? lo_i : hi_i)), a = w - u: below 0
