@@ -392,8 +392,8 @@ uint64_t ehgp_ctx_regrowths(const ehgp_ctx* ctx) { return ctx ? ctx->regrowths :
 
 int ehgp_ctx_counters(const ehgp_ctx* ctx, uint64_t* out, uint32_t count) {
   if (!ctx || !out) return EHGP_ERR_INVALID_ARGUMENT;
-  const uint64_t v[4] = {ctx->device_bytes, ctx->regrowths, ctx->pair_runs, ctx->higher_runs};
-  for (uint32_t i = 0; i < count && i < 4; ++i) out[i] = v[i];
+  const uint64_t v[5] = {ctx->device_bytes, ctx->regrowths, ctx->pair_runs, ctx->higher_runs, ctx->forest_rest};
+  for (uint32_t i = 0; i < count && i < 5; ++i) out[i] = v[i];
   return EHGP_OK;
 }
 
@@ -412,6 +412,9 @@ int ehgp_tune(ehgp_ctx* ctx, uint32_t knob, uint64_t value) {
     case EHGP_TUNE_SORT_WAIT:
       if (value > ehgp::kRadixWait) return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "a sort looks at most 2^20 times");
       ctx->radix.wait = (uint32_t)value;
+      return EHGP_OK;
+    case EHGP_TUNE_FOREST_ROUNDS:
+      ctx->forest_rounds = (uint32_t)std::min<uint64_t>(value, 0xffffffffu);
       return EHGP_OK;
     default:
       return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "unknown tuning knob");

@@ -1982,6 +1982,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
     in.fam0[k] = (uint32_t)(rb[std::min<uint32_t>(k + 1, 16)] - fam_lo);
     in.han0[k] = k == 1 ? 0 : (uint32_t)(n + rb[k] - rb[2]);
   }
+  in.rounds = std::min(ctx.forest_rounds, kForestRounds);
   in.ev = h.rank_order + fam_lo;
   in.cls = h.d_cls_rp + fam_lo;
   in.armoff = h.d_armoff;
@@ -2107,6 +2108,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
   // ---- forest journal, in the queues' memory ----
   if ((e = h.mem.reset(journal)) != cudaSuccess) return no_queue();
   const int js = journal_run(ctx, in, h.mem, h.journal, &launches);
+  ctx.forest_rest = h.journal.rest;
   if (js != EHGP_OK) return js;
   cudaEventRecord(ctx.ev1, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "forest journal");

@@ -289,6 +289,8 @@ struct Ctx {
   uint32_t emst_minima = 0;        // total per-round minima logged
   bool emst_ready = false;
   struct HierState* hier = nullptr;  // direct hierarchy (ehgp_hier.cu)
+  uint32_t forest_rounds = ~0u;      // limit on the forest journal's rounds (above its own: none)
+  uint64_t forest_rest = 0;          // families that the last journal's rounds left to the host
   char* stage = nullptr;             // pinned ring of copy_out, made by the first large copy
   void* stage_map = nullptr;         // the mapping that holds it
   cudaEvent_t stage_ev[kStageSlots] = {};

@@ -22,7 +22,9 @@
 //    earlier families, so at that family the chain is already one component, and the root's
 //    oldest handle is the component's.  Of two components whose first family is the same, the
 //    younger hooks, so every round makes progress; the number of rounds is the longest chain of
-//    ever older partners (10-20 on the clouds measured, not the number of merges).
+//    ever older partners: 10-60 on random clouds, but as many as points where
+//    the spacing shrinks along a curve.  What a bounded number of rounds leaves is applied family by
+//    family on the host (the contracted components and families are the same problem again).
 //  * Counts of carriers, reduced roots, nodes, children and groups before a batch are prefix
 //    sums over the families; the reduced root of a component at a level is the last node created
 //    under its oldest handle, found by binary search in the nodes sorted by handle.
@@ -35,6 +37,9 @@
 #include "ehgp_journal.cuh"
 
 #include <algorithm>
+#include <cstdlib>
+#include <memory>
+#include <new>
 
 namespace ehgp {
 
@@ -87,12 +92,12 @@ namespace {
 constexpr int kT = 256;
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kSaddle = 0x80000000u;    // role source: family index with this bit, else a handle
-constexpr uint32_t kTailFamilies = 1u << 13;  // active families that one block finishes on its own
+constexpr uint32_t kTailFamilies = 1u << 13;  // active families that one block takes on alone
 
 inline uint32_t nblk(uint64_t m, int t = kT) { return m ? (uint32_t)((m + t - 1) / t) : 1u; }
 
 // Journal error bits (device word).
-constexpr uint32_t kErrUnborn = 1u, kErrStuck = 2u, kErrNoRoot = 4u;
+constexpr uint32_t kErrUnborn = 1u, kErrNoRoot = 4u;
 
 struct J {  // kernel view of the input
   uint32_t n, keff, handles, families, arms;
@@ -487,19 +492,15 @@ __global__ void __launch_bounds__(kT) k_fj_advance(Active in, const uint32_t* __
     advance_block<false>(b, m, in, to, count_next, best_next, lab);
 }
 
-// The last active families: one block runs the remaining rounds without returning to the host
-// (their number is bounded by the entries: the least first family is mutual, so a component hooks).
+// The last active families: one block runs up to `rounds` rounds without returning to the host.
+// left[0]: the families still active then, left[1]: 1 when they are in `next`.
 __global__ void __launch_bounds__(1024) k_fj_tail(const uint32_t* __restrict__ cls, Active cur, Active next,
                                                   const uint32_t* __restrict__ count, uint32_t* best,
-                                                  uint32_t* best_next, Tree t, uint32_t* lab,
-                                                  uint32_t* __restrict__ err) {
+                                                  uint32_t* best_next, Tree t, uint32_t* lab, uint32_t rounds,
+                                                  uint32_t* __restrict__ left_over) {
   __shared__ uint32_t left;
-  uint32_t m = *count;
-  for (uint32_t round = 0; m > 0; ++round) {
-    if (round > kTailFamilies) {
-      if (threadIdx.x == 0) atomicOr(err, kErrStuck);
-      return;
-    }
+  uint32_t m = *count, round = 0;
+  for (; m > 0 && round < rounds; ++round) {
     if (threadIdx.x == 0) left = 0;
     for (uint32_t i = threadIdx.x; i < m; i += 1024)
       hook_entry<true>(cls, cur.comp[i], cur.fam[i], best, best_next, t, lab);
@@ -516,6 +517,55 @@ __global__ void __launch_bounds__(1024) k_fj_tail(const uint32_t* __restrict__ c
     uint32_t* q = best;
     best = best_next;
     best_next = q;
+  }
+  if (threadIdx.x == 0) {
+    left_over[0] = m;
+    left_over[1] = round & 1u;
+  }
+}
+
+__global__ void __launch_bounds__(kT) k_fj_rest_keys(uint32_t m, const uint32_t* __restrict__ fam,
+                                                     uint64_t* __restrict__ key, uint32_t* __restrict__ val) {
+  const uint32_t i = blockIdx.x * kT + threadIdx.x;
+  if (i >= m) return;
+  key[i] = fam[i];
+  val[i] = i;
+}
+
+// Deaths found on the host: (handle, older handle, family).
+__global__ void __launch_bounds__(kT) k_fj_deaths(uint32_t m, const uint32_t* __restrict__ cls,
+                                                  const uint4* __restrict__ deaths, Tree t) {
+  const uint32_t i = blockIdx.x * kT + threadIdx.x;
+  if (i >= m) return;
+  const uint4 d = deaths[i];
+  t.dead[d.x] = make_uint2(d.y, cls[d.z]);
+}
+
+// Kruskal's algorithm over families in ascending order: the deaths of the components' oldest handles.
+// val: the families' places in `comp`; key: the families.
+void deaths_in_order(uint32_t handles, const std::vector<uint4>& comp, const std::vector<uint64_t>& key,
+                     const std::vector<uint32_t>& val, std::vector<uint4>& deaths) {
+  // parent + 1, 0 = a root: zero pages that are never touched are never made
+  const std::unique_ptr<uint32_t, void (*)(void*)> hold(static_cast<uint32_t*>(std::calloc(handles, sizeof(uint32_t))), std::free);
+  uint32_t* up = hold.get();
+  if (!up) throw std::bad_alloc();
+  auto find = [up](uint32_t x) {
+    while (up[x]) {
+      const uint32_t p = up[x] - 1;
+      if (up[p]) up[x] = up[p];
+      x = p;
+    }
+    return x;
+  };
+  for (size_t i = 0; i < key.size(); ++i) {
+    const uint4 c = comp[val[i]];
+    uint32_t r[4] = {find(c.x), find(c.y), find(c.z), find(c.w)};
+    const uint32_t least = std::min(std::min(r[0], r[1]), std::min(r[2], r[3]));
+    for (uint32_t x : r) {
+      if (x == least || up[x]) continue;
+      up[x] = least + 1;
+      deaths.push_back(make_uint4(x, least, (uint32_t)key[i], 0u));
+    }
   }
 }
 
@@ -1097,7 +1147,8 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
   TAKE(lab, H);
   TAKE(best[0], H);
   TAKE(best[1], H);
-  TAKE(cnt, 8);  // [0], [1] active families (ping-pong), [2] errors, [3] saddles sharing a batch, [4] roots
+  TAKE(cnt, 8);  // [0], [1] active families (ping-pong), [2] errors, [3] saddles sharing a batch, [4] roots,
+                 // [5], [6] what the tail left
   TAKE(tot, 5ull * (nblk(R, kScanTile) + 1));
   for (Active& a : act) {
     TAKE(a.comp, F);
@@ -1114,47 +1165,13 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
       return abi_fail(&ctx, EHGP_ERR_DEGENERATE, "a strict arm descended to a minimum that is not yet born");
     if (hc[2] & kErrNoRoot)
       return abi_fail(&ctx, EHGP_ERR_DEGENERATE, "a reduced node has no lower-order image through its carrier saddle");
-    if (hc[2]) return abi_fail(&ctx, EHGP_ERR_CUDA, "the forest journal's rounds did not end");
     return EHGP_OK;
   };
   cudaMemsetAsync(cnt, 0, 8 * sizeof(uint32_t), st);
   k_fj_init<<<nblk(H), kT, 0, st>>>(H, t, lab, best[0], best[1]);
   ++*launches;
-  Shared sh;
-  int s;
-  if (F) {
-    k_fj_first<<<nblk(F, kT * kRows), kT, 0, st>>>(j, act[0], cnt, best[0], cnt + 2);
-    ++*launches;
-    if ((s = read("forest journal")) != EHGP_OK) return s;
-    uint32_t live = hc[0], cur = 0;
-    // Three rounds between looks at the count (each shrinks it to a half or less); every round
-    // hooks at least one component, so the loop ends.
-    while (live > kTailFamilies) {
-      for (int r = 0; r < 3; ++r) {
-        const uint32_t grid = std::min(nblk(live, kT * kRows), 148u * 8);
-        k_fj_hook<<<grid, kT, 0, st>>>(j.cls, act[cur], cnt + cur, best[cur], best[1 - cur], t, lab);
-        cudaMemsetAsync(cnt + (1 - cur), 0, sizeof(uint32_t), st);
-        k_fj_advance<<<grid, kT, 0, st>>>(act[cur], cnt + cur, act[1 - cur], cnt + (1 - cur), best[1 - cur], lab);
-        *launches += 2;
-        cur = 1 - cur;
-      }
-      if ((s = read("forest journal rounds")) != EHGP_OK) return s;
-      live = hc[cur];
-    }
-    if (live) {
-      k_fj_tail<<<1, 1024, 0, st>>>(j.cls, act[cur], act[1 - cur], cnt + cur, best[cur], best[1 - cur], t, lab, cnt + 2);
-      ++*launches;
-    }
-    k_fj_normalise<<<nblk(H), kT, 0, st>>>(H, t);
-    k_fj_carriers<<<nblk(F), kT, 0, st>>>(j, t, car, cnt + 3);
-    *launches += 2;
-    if ((s = read("forest journal carriers")) != EHGP_OK) return s;
-    sh.m = hc[3];
-  }
-  // ---- batches with several saddles ----
   uint64_t *ckey[2] = {nullptr, nullptr}, *pkey[2] = {nullptr, nullptr};
   uint32_t *cval[2] = {nullptr, nullptr}, *rcounts = nullptr;
-  const uint64_t M = sh.m;
   // sorts m keys; returns the buffers that hold the result
   auto sort = [&](uint64_t m, uint64_t** key, uint32_t** val, int bits, uint64_t** rk, uint32_t** rv, int* passes) -> int {
     RadixScratch rs{rcounts, ctx.radix.state, ctx.radix.wait};
@@ -1167,6 +1184,81 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
     *rv = val[which ? 1 : 0];
     return EHGP_OK;
   };
+  Shared sh;
+  int s;
+  if (F) {
+    k_fj_first<<<nblk(F, kT * kRows), kT, 0, st>>>(j, act[0], cnt, best[0], cnt + 2);
+    ++*launches;
+    if ((s = read("forest journal")) != EHGP_OK) return s;
+    uint32_t live = hc[0], cur = 0;
+    // Three rounds between looks at the count (on most clouds each shrinks it to a half or less).
+    for (uint32_t round = 0; live > kTailFamilies && round < in.rounds; round += 3) {
+      for (int r = 0; r < 3; ++r) {
+        const uint32_t grid = std::min(nblk(live, kT * kRows), 148u * 8);
+        k_fj_hook<<<grid, kT, 0, st>>>(j.cls, act[cur], cnt + cur, best[cur], best[1 - cur], t, lab);
+        cudaMemsetAsync(cnt + (1 - cur), 0, sizeof(uint32_t), st);
+        k_fj_advance<<<grid, kT, 0, st>>>(act[cur], cnt + cur, act[1 - cur], cnt + (1 - cur), best[1 - cur], lab);
+        *launches += 2;
+        cur = 1 - cur;
+      }
+      if ((s = read("forest journal rounds")) != EHGP_OK) return s;
+      live = hc[cur];
+    }
+    const bool tail = live <= kTailFamilies;
+    if (tail && live) {
+      k_fj_tail<<<1, 1024, 0, st>>>(j.cls, act[cur], act[1 - cur], cnt + cur, best[cur], best[1 - cur], t, lab, in.rounds, cnt + 5);
+      ++*launches;
+    }
+    auto carriers = [&] {
+      k_fj_normalise<<<nblk(H), kT, 0, st>>>(H, t);
+      k_fj_carriers<<<nblk(F), kT, 0, st>>>(j, t, car, cnt + 3);
+      *launches += 2;
+      return read("forest journal carriers");
+    };
+    // (as if the rounds had ended: one look at the counts tells)
+    if (tail && (s = carriers()) != EHGP_OK) return s;
+    const uint32_t rest = tail && live ? hc[5] : live;
+    out.rest = rest;
+    if (rest) {
+      const Active& a = act[tail ? cur ^ hc[6] : cur];
+      for (int i = 0; i < 2; ++i) {
+        TAKE(ckey[i], rest);
+        TAKE(cval[i], rest);
+      }
+      TAKE(rcounts, radix_counts_words(rest));
+      k_fj_rest_keys<<<nblk(rest), kT, 0, st>>>(rest, a.fam, ckey[0], cval[0]);
+      uint64_t* key;
+      uint32_t* val;
+      int passes;
+      if ((s = sort(rest, ckey, cval, 32, &key, &val, &passes)) != EHGP_OK) return s;
+      std::vector<uint4> deaths;
+      uint4* d_deaths;
+      try {
+        std::vector<uint4> comp(rest);
+        std::vector<uint64_t> keys(rest);
+        std::vector<uint32_t> vals(rest);
+        cudaMemcpyAsync(comp.data(), a.comp, rest * sizeof(uint4), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(keys.data(), key, rest * sizeof(uint64_t), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(vals.data(), val, rest * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "forest journal rest");
+        deaths_in_order(H, comp, keys, vals, deaths);
+      } catch (const std::bad_alloc&) {
+        return no_memory();
+      }
+      const uint32_t m = (uint32_t)deaths.size();
+      TAKE(d_deaths, m);
+      cudaMemcpyAsync(d_deaths, deaths.data(), m * sizeof(uint4), cudaMemcpyHostToDevice, st);
+      k_fj_deaths<<<nblk(m), kT, 0, st>>>(m, j.cls, d_deaths, t);
+      *launches += 2;
+      // the carriers of the unfinished tree are made again
+      cudaMemsetAsync(t.touch, 0xff, H * sizeof(uint32_t), st);
+      cudaMemsetAsync(cnt + 3, 0, sizeof(uint32_t), st);
+      if ((s = carriers()) != EHGP_OK) return s;
+    }
+    sh.m = hc[3];
+  }
+  // ---- batches with several saddles ----
+  const uint64_t M = sh.m;
   uint64_t* ck = nullptr;
   if (M) {
     uint32_t* prefix;

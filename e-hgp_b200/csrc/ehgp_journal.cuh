@@ -32,6 +32,9 @@ class DeviceArena {
   std::vector<Block> blocks_;
 };
 
+// Rounds of the forest journal over all families, and as many by its last block (12 to 21 and 1 to 47 on uniform,
+// lattice, mixture and graded clouds of 256 to 50,653 points).
+constexpr uint32_t kForestRounds = 64;
 constexpr int kJournalOrders = 18;  // orders 1..10 and the ends of their ranges
 
 // The resolved arms of every order.  Families (saddles) and birth handles of orders >= 2 are
@@ -40,6 +43,7 @@ constexpr int kJournalOrders = 18;  // orders 1..10 and the ends of their ranges
 struct JournalIn {
   uint32_t n = 0, keff = 0;
   uint32_t handles = 0, families = 0, arms = 0;
+  uint32_t rounds = kForestRounds;      // at most that
   uint32_t fam0[kJournalOrders] = {};   // first family of order k (k = 1..keff + 1)
   uint32_t han0[kJournalOrders] = {};   // first handle of order k
   const uint32_t* ev = nullptr;         // [families] facade index (ascending within an order)
@@ -63,6 +67,7 @@ struct JournalOut {
   ehgp_vertical_assignment* vert = nullptr;
   std::vector<ehgp_forest_root> roots;  // on the host (one per surviving component)
   uint64_t n_batches = 0, n_roles = 0, n_nodes = 0, n_children = 0, n_groups = 0, n_vert = 0;
+  uint32_t rest = 0;  // families that the rounds left to the host
 };
 
 // Device bytes the journal takes from its arena for these counts (nodes and children, which

@@ -347,16 +347,17 @@ class Context:
     TUNE_HIGHER_LIST = 1
     TUNE_PAIR_TASKS = 2
     TUNE_SORT_WAIT = 3
+    TUNE_FOREST_ROUNDS = 4
 
     def tune(self, knob: int, value: int) -> None:
         """ehgp_tune: a tuning knob of later calls (results never depend on it)."""
         self._check(self.lib.ehgp_tune(self._h, knob, value))
 
     def counters(self) -> dict:
-        """ehgp_ctx_counters: device bytes, regrowths, pair and triple/quad enumerations run."""
-        v = np.zeros(4, np.uint64)
-        self._check(self.lib.ehgp_ctx_counters(self._h, _ptr(v), 4))
-        return dict(zip(("device_bytes", "regrowths", "pair_runs", "higher_runs"), (int(x) for x in v)))
+        """ehgp_ctx_counters: device bytes, regrowths, pair and triple/quad enumerations run, families left to the host."""
+        v = np.zeros(5, np.uint64)
+        self._check(self.lib.ehgp_ctx_counters(self._h, _ptr(v), 5))
+        return dict(zip(("device_bytes", "regrowths", "pair_runs", "higher_runs", "forest_rest"), (int(x) for x in v)))
 
     def checkpoint_save(self, path: str, K: int = 10) -> None:
         """ehgp_checkpoint_save: cloud, K and support records of the resident cloud to `path`."""

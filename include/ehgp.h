@@ -78,7 +78,8 @@ int ehgp_ctx_reserve(ehgp_ctx* ctx, uint32_t stage, uint64_t records);
 uint64_t ehgp_ctx_regrowths(const ehgp_ctx* ctx);
 
 /* [0] device bytes, [1] record-buffer regrowths, [2] pair enumerations and [3]
- * triple/quad enumerations run on this context so far.  No reference counterpart. */
+ * triple/quad enumerations run on this context so far, [4] saddle families that
+ * the last hierarchy's forest rounds left to the host.  No reference counterpart. */
 int ehgp_ctx_counters(const ehgp_ctx* ctx, uint64_t* out, uint32_t count);
 
 /* Checkpoint and resume of a request after its support stages, in place of the
@@ -103,8 +104,10 @@ int ehgp_checkpoint_load(ehgp_ctx* ctx, const char* path, uint32_t* K);
  *   EHGP_TUNE_PAIR_TASKS: walks of the pair enumeration (0..2 * max_points + 4096, the
  *     default the largest) that may be handed over to further warps per round.
  *   EHGP_TUNE_SORT_WAIT: how often (0..2^20, the default the largest) a block of a sort
- *     looks for an earlier block's counts before it counts that block's items itself. */
-enum { EHGP_TUNE_HIGHER_LIST = 1, EHGP_TUNE_PAIR_TASKS = 2, EHGP_TUNE_SORT_WAIT = 3 };
+ *     looks for an earlier block's counts before it counts that block's items itself.
+ *   EHGP_TUNE_FOREST_ROUNDS: device rounds of the forest journal (0..; 64 at most, the
+ *     default) before the host applies the families that are left, in order. */
+enum { EHGP_TUNE_HIGHER_LIST = 1, EHGP_TUNE_PAIR_TASKS = 2, EHGP_TUNE_SORT_WAIT = 3, EHGP_TUNE_FOREST_ROUNDS = 4 };
 int ehgp_tune(ehgp_ctx* ctx, uint32_t knob, uint64_t value);
 
 /* ---- LBVH snapshot records (reference layout) ---------------------------- */
