@@ -160,7 +160,11 @@ __device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t* tmp) {
   return before + x - v;
 }
 
-constexpr uint32_t kAggregate = 1u << 30, kInclusive = 2u << 30, kCountMask = (1u << 30) - 1u;
+// A tile's published count of a digit: 0 not yet, 1 + its own (at most kRadixTile), or kInclusive + that of
+// the tiles up to it.  With two flag bits above the count, sorts of 2^30 items and more overflowed; the
+// largest record index is below 2^32 - 2^16.
+constexpr uint32_t kInclusive = 2u * kRadixTile;
+static_assert(1u + kRadixTile < kInclusive && kInclusive + 0xffff0000u > 0xffff0000u, "published counts are told apart");
 
 // One pass.  look: [2][tiles][256] tile counts; the pass uses the half of its input buffer and clears
 // the other half for the next one.
@@ -209,7 +213,7 @@ __global__ void __launch_bounds__(kT) k_radix_pass(uint32_t n, uint32_t* __restr
     cnt[w][tid] = total;
     total += c;
   }
-  atomicExch(mine, total | (tile == 0 ? kInclusive : kAggregate));
+  atomicExch(mine, total + (tile == 0 ? kInclusive : 1u));
   const uint32_t local = scan256(total, tmp);
   start[tid] = local;
   uint32_t before = 0;
@@ -221,8 +225,11 @@ __global__ void __launch_bounds__(kT) k_radix_pass(uint32_t n, uint32_t* __restr
       late = true;
       break;
     }
-    before += x & kCountMask;
-    if (x & kInclusive) break;
+    if (x >= kInclusive) {
+      before += x - kInclusive;
+      break;
+    }
+    before += x - 1u;
     --t;
   }
   if (__syncthreads_or(late)) {  // the pass does not change its input: count the tiles before this one
@@ -233,7 +240,7 @@ __global__ void __launch_bounds__(kT) k_radix_pass(uint32_t n, uint32_t* __restr
     __syncthreads();
     before = sval[tid];
   }
-  if (tile) atomicExch(mine, (before + total) | kInclusive);
+  if (tile) atomicExch(mine, before + total + kInclusive);
   gbase[tid] = state[kBases + 256 * pass + tid] + before - local;
   __syncthreads();
 #pragma unroll
