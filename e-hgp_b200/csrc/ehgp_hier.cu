@@ -904,9 +904,10 @@ __device__ __noinline__ int topk_choice(const DescentParams& d, const Cloud& c, 
   // 2^-22) and by dqf, clamped at 0; the sum of squares is lowered by a relative 2^-20 and
   // compared with R2_eff rounded up.  The bound never exceeds the exact one, so the prune skips
   // only boxes that hold no point within R2_eff (the FP64 prune skips at least those; the
-  // leaves decide membership in FP64 as before).  Far from the origin the FP64 prune stays.
+  // leaves decide membership in FP64 as before).  Far from the origin the FP64 prune stays, and for radii
+  // whose squares binary32 does not hold (a gap's square loses the margin to underflow).
   const double qv[3] = {cx, cy, cz};
-  const bool f32 = fabs(cx) < 0x1p60 && fabs(cy) < 0x1p60 && fabs(cz) < 0x1p60 && R2 < 0x1p100;
+  const bool f32 = fabs(cx) < 0x1p60 && fabs(cy) < 0x1p60 && fabs(cz) < 0x1p60 && R2 < 0x1p100 && R2 > 0x1p-126;
   float qf[3], dqf[3];
   for (int a = 0; a < 3; ++a) {
     qf[a] = (float)qv[a];
@@ -1416,7 +1417,8 @@ k_facet_step(DescentParams d, uint32_t m, const uint32_t* __restrict__ in_arm, c
       const double R = sqrt(lhi) * (1.0 + 1e-12) + dc;
       R2 = R * R * (1.0 + 1e-12);
       ed = 2.0 * R * dc + dc * dc + 8.0 * kU * R2 + kTiny;
-      open = !(relA < 0.5) || !isfinite(dc) || !(fabs(cx) < 0x1p60 && fabs(cy) < 0x1p60 && fabs(cz) < 0x1p60 && R2 < 0x1p100);
+      open = !(relA < 0.5) || !isfinite(dc) ||
+             !(fabs(cx) < 0x1p60 && fabs(cy) < 0x1p60 && fabs(cz) < 0x1p60 && R2 < 0x1p100 && R2 > 0x1p-126);
     }
     // binary32 prune as in topk_choice: a lower bound of the distance to a node box, from the rounded centre
     const float qx = (float)cx, qy = (float)cy, qz = (float)cz;

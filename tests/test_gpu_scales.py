@@ -35,3 +35,16 @@ def test_pairs_do_not_depend_on_the_unit(name, K):
             if e <= 0:  # squared lengths in units of the cloud's own grid
                 out[e] += r["level_num"].tobytes()
             assert out[e] == out[0][:len(out[e])], e
+
+
+@pytest.mark.parametrize("name", ["uniform300", "clustered600"])
+def test_hierarchies_do_not_depend_on_the_unit(name):
+    pts = CLOUDS[name]
+    with ehgp.Context(max_points=len(pts)) as ctx:
+        want = None
+        for e in (0, -100, -90, -80, -74, -70, -66, -62, -58, -40, 20, 60):
+            ctx.lbvh_build(scaled(pts, e), outputs=False)
+            got = ctx.hierarchy(6)
+            want = want or got
+            for k, v in want.items():
+                assert not isinstance(v, np.ndarray) or np.array_equal(got[k], v), (e, k)
