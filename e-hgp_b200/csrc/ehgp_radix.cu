@@ -232,17 +232,20 @@ __global__ void __launch_bounds__(kT) k_radix_pass(uint32_t n, uint32_t* __restr
     before += x - 1u;
     --t;
   }
+  if (tile && !late) atomicExch(mine, before + total + kInclusive);
+  gbase[tid] = state[kBases + 256 * pass + tid] + before - local;
   if (__syncthreads_or(late)) {  // the pass does not change its input: count the tiles before this one
     sval[tid] = 0;
     __syncthreads();
     for (uint32_t i = tid; i < tile * kRadixTile; i += kT)
       atomicAdd(sval + (kKv ? (uint32_t)(kin[i] >> (8 * pass)) & 0xffu : indirect_digit(ps, pass, in[i])), 1u);
     __syncthreads();
-    before = sval[tid];
+    if (late) {
+      atomicExch(mine, sval[tid] + total + kInclusive);
+      gbase[tid] += sval[tid] - before;
+    }
+    __syncthreads();
   }
-  if (tile) atomicExch(mine, before + total + kInclusive);
-  gbase[tid] = state[kBases + 256 * pass + tid] + before - local;
-  __syncthreads();
 #pragma unroll
   for (int r = 0; r < kRows; ++r) {
     if (dig[r] > 255u) continue;
