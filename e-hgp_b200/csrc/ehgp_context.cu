@@ -359,7 +359,7 @@ const char* ehgp_status_string(int status) {
   }
 }
 
-uint64_t ehgp_ctx_device_bytes(const ehgp_ctx* ctx) { return ctx ? ctx->device_bytes : 0; }
+uint64_t ehgp_ctx_device_bytes(const ehgp_ctx* ctx) { return ctx ? ctx->device_bytes + ctx->hier_bytes : 0; }
 
 int ehgp_ctx_reserve(ehgp_ctx* ctx, uint32_t stage, uint64_t records) {
   if (!ctx || stage > 1 || records == 0 || records >= 0xffff0000ull) return EHGP_ERR_INVALID_ARGUMENT;
@@ -392,7 +392,7 @@ uint64_t ehgp_ctx_regrowths(const ehgp_ctx* ctx) { return ctx ? ctx->regrowths :
 
 int ehgp_ctx_counters(const ehgp_ctx* ctx, uint64_t* out, uint32_t count) {
   if (!ctx || !out) return EHGP_ERR_INVALID_ARGUMENT;
-  const uint64_t v[5] = {ctx->device_bytes, ctx->regrowths, ctx->pair_runs, ctx->higher_runs, ctx->forest_rest};
+  const uint64_t v[5] = {ehgp_ctx_device_bytes(ctx), ctx->regrowths, ctx->pair_runs, ctx->higher_runs, ctx->forest_rest};
   for (uint32_t i = 0; i < count && i < 5; ++i) out[i] = v[i];
   return EHGP_OK;
 }

@@ -1626,7 +1626,9 @@ k_facet_exact(DescentParams d, uint32_t m, const uint32_t* __restrict__ hard, co
 
 // ---- host state ---------------------------------------------------------------------
 struct HierState {
-  std::vector<void*> allocs;
+  explicit HierState(Ctx& ctx) : held(ctx.hier_bytes), mem(ctx.hier_bytes) {}
+  std::atomic<uint64_t>& held;  // device bytes of everything below
+  std::vector<std::pair<void*, uint64_t>> allocs;
   uint64_t cap_events = 0, cap_arms = 0, cap_births = 0, cap_slots = 0;
   // device
   EvRec* ev_raw = nullptr;
@@ -1654,7 +1656,7 @@ struct HierState {
   uint32_t* term = nullptr;
   unsigned long long* dstats = nullptr;  // [0] descent steps, [1] strictness checks passed, [2] failed arms, [3] least (arm, status)
   uint32_t* qcount = nullptr;   // [0] first-probe misses, [1], [2] step outputs (ping-pong)
-  DeviceArena mem;              // the descent's queues, then the forest journal and its records
+  DeviceArena mem;              // (counted in held) the descent's queues, then the forest journal and its records
   uint32_t first_misses = 0, descent_rounds = 0;
   unsigned long long slow[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   unsigned long long visits[kVisitStripes] = {};  // ball-query node visits of the descent steps
@@ -1687,36 +1689,42 @@ struct HierState {
   uint32_t part_arms = 0;  // arms per part of the descent (0: one part); results never depend on it
 };
 
-void hier_free(Ctx& ctx) {
-  if (!ctx.hier) return;
-  for (void* p : ctx.hier->allocs) cudaFree(p);
-  for (void* q : {(void*)ctx.hier->tie_num, (void*)ctx.hier->tie_a2, (void*)ctx.hier->tie_idx,
-                  (void*)ctx.hier->tie_tmp, (void*)ctx.hier->tie_pos, (void*)ctx.hier->run_off,
-                  (void*)ctx.hier->run_lo})
-    if (q) cudaFree(q);
-  for (cudaEvent_t ev : ctx.hier->ev_step)
-    if (ev) cudaEventDestroy(ev);
-  delete ctx.hier;
-  ctx.hier = nullptr;
-}
-
 namespace {
 
 template <class T>
 cudaError_t halloc(HierState& h, T** p, uint64_t count) {
   void* q = nullptr;
-  const cudaError_t e = cudaMalloc(&q, count * sizeof(T) + 16);
+  const uint64_t bytes = count * sizeof(T) + 16;
+  const cudaError_t e = cudaMalloc(&q, bytes);
   if (e != cudaSuccess) return e;
-  h.allocs.push_back(q);
+  h.allocs.push_back({q, bytes});
+  h.held += bytes;
   *p = (T*)q;
   return cudaSuccess;
 }
 
+// Frees the event arrays; the facade goes with them.
 void hfree_all(HierState& h) {
-  for (void* p : h.allocs) cudaFree(p);
+  for (const auto& a : h.allocs) {
+    cudaFree(a.first);
+    h.held -= a.second;
+  }
   h.allocs.clear();
   h.qcount = nullptr;
+  h.events = 0;
+  h.complete = false;
+  h.decision = EHGP_ERR_NOT_BUILT;
   h.cap_events = h.cap_arms = h.cap_births = h.cap_slots = 0;
+}
+
+void free_ties(HierState& h) {
+  for (void* q : {(void*)h.tie_num, (void*)h.tie_a2, (void*)h.tie_idx, (void*)h.tie_tmp, (void*)h.tie_pos,
+                  (void*)h.run_off, (void*)h.run_lo})
+    if (q) cudaFree(q);
+  h.tie_num = h.tie_a2 = nullptr;
+  h.tie_idx = h.tie_tmp = h.tie_pos = h.run_off = h.run_lo = nullptr;
+  h.held -= h.tie_cap * (2 * sizeof(WL) + 12) + h.run_cap * 8;
+  h.tie_cap = h.run_cap = 0;
 }
 
 cudaError_t ensure_events(HierState& h, uint64_t m) {
@@ -1781,8 +1789,25 @@ void scan_minmax(cudaStream_t st, uint32_t m, const double* mid, const double* e
 
 }  // namespace
 
+void hier_trim(Ctx& ctx) {
+  if (!ctx.hier) return;
+  cudaSetDevice(ctx.device);
+  hfree_all(*ctx.hier);
+  free_ties(*ctx.hier);
+  ctx.hier->mem.release();
+}
+
+void hier_free(Ctx& ctx) {
+  if (!ctx.hier) return;
+  hier_trim(ctx);
+  for (cudaEvent_t ev : ctx.hier->ev_step)
+    if (ev) cudaEventDestroy(ev);
+  delete ctx.hier;
+  ctx.hier = nullptr;
+}
+
 int hier_run(Ctx& ctx, uint32_t K) {
-  if (!ctx.hier) ctx.hier = new HierState();
+  if (!ctx.hier) ctx.hier = new HierState(ctx);
   HierState& h = *ctx.hier;
   const uint32_t n = (uint32_t)ctx.built_n;
   cudaStream_t st = ctx.stream;
@@ -1879,12 +1904,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
     const uint32_t cnt = (uint32_t)idx.size(), nruns = (uint32_t)run_lo.size();
     // settled on the device: exact level keys per member, then a merge sort per run
     if (h.tie_cap < cnt || h.run_cap < nruns + 1) {
-      for (void* q : {(void*)h.tie_num, (void*)h.tie_a2, (void*)h.tie_idx, (void*)h.tie_tmp, (void*)h.tie_pos,
-                      (void*)h.run_off, (void*)h.run_lo})
-        if (q) cudaFree(q);
-      h.tie_num = h.tie_a2 = nullptr;
-      h.tie_idx = h.tie_tmp = h.tie_pos = h.run_off = h.run_lo = nullptr;
-      h.tie_cap = h.run_cap = 0;
+      free_ties(h);
       const uint64_t tc = cnt + cnt / 4 + 64, rc = nruns + nruns / 4 + 64;
       if (cudaMalloc(&h.tie_num, tc * sizeof(WL)) != cudaSuccess || cudaMalloc(&h.tie_a2, tc * sizeof(WL)) != cudaSuccess ||
           cudaMalloc(&h.tie_idx, tc * 4) != cudaSuccess || cudaMalloc(&h.tie_tmp, tc * 4) != cudaSuccess ||
@@ -1895,6 +1915,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
       }
       h.tie_cap = tc;
       h.run_cap = rc;
+      h.held += tc * (2 * sizeof(WL) + 12) + rc * 8;
     }
     // members' records are copied (ev_raw is free between the facade gather and the level
     // classes) so that the sort writes the facade in place
@@ -2188,7 +2209,7 @@ int ehgp_hierarchy(ehgp_ctx* ctx, uint32_t K, ehgp_hier_counts* counts) {
 int ehgp_hier_schedule(ehgp_ctx* ctx, uint32_t chunk_batches, uint32_t part_arms, uint32_t host_threads) {
   if (!ctx) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
-  if (!ctx->hier) ctx->hier = new ehgp::HierState();
+  if (!ctx->hier) ctx->hier = new ehgp::HierState(*ctx);
   (void)chunk_batches;  // the forest journal runs on the device
   (void)host_threads;
   ctx->hier->part_arms = part_arms;

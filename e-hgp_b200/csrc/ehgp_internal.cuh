@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -258,7 +259,8 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   uint64_t max_points = 0;
-  uint64_t device_bytes = 0;
+  std::atomic<uint64_t> device_bytes{0};  // of ctx_alloc
+  std::atomic<uint64_t> hier_bytes{0};    // of the hierarchy: event arrays, descent queues, journal and its records
   bool poisoned = false;
   std::mutex mutex;
   std::string last_error;
@@ -351,6 +353,8 @@ int higher_run(Ctx& ctx, uint32_t K, uint32_t* out_count);
 // Direct Morse hierarchy (ehgp_hier.cu)
 int hier_run(Ctx& ctx, uint32_t K);
 void hier_free(Ctx& ctx);
+// Gives the hierarchy's device memory back, its result with it.
+void hier_trim(Ctx& ctx);
 
 }  // namespace ehgp
 

@@ -51,12 +51,8 @@ cudaError_t DeviceArena::reset(uint64_t want) {
     return cudaSuccess;
   }
   release();
-  const uint64_t size = std::max(have, want + want / 16) + 4096;
   void* p = nullptr;
-  const cudaError_t e = cudaMalloc(&p, size);
-  if (e != cudaSuccess) return e;
-  blocks_.push_back({static_cast<char*>(p), size, 0});
-  return cudaSuccess;
+  return add(std::max(have, want + want / 16) + 4096, 0, &p);
 }
 
 cudaError_t DeviceArena::take(void** p, uint64_t bytes) {
@@ -67,24 +63,23 @@ cudaError_t DeviceArena::take(void** p, uint64_t bytes) {
       b.used += bytes;
       return cudaSuccess;
     }
-  void* q = nullptr;
-  const uint64_t size = bytes + bytes / 8 + 4096;
-  const cudaError_t e = cudaMalloc(&q, size);
+  return add(bytes + bytes / 8 + 4096, bytes, p);
+}
+
+cudaError_t DeviceArena::add(uint64_t size, uint64_t used, void** p) {
+  const cudaError_t e = cudaMalloc(p, size);
   if (e != cudaSuccess) return e;
-  blocks_.push_back({static_cast<char*>(q), size, bytes});
-  *p = q;
+  blocks_.push_back({static_cast<char*>(*p), size, used});
+  held_ += size;
   return cudaSuccess;
 }
 
 void DeviceArena::release() {
-  for (const Block& b : blocks_) cudaFree(b.p);
+  for (const Block& b : blocks_) {
+    cudaFree(b.p);
+    held_ -= b.size;
+  }
   blocks_.clear();
-}
-
-uint64_t DeviceArena::bytes() const {
-  uint64_t t = 0;
-  for (const Block& b : blocks_) t += b.size;
-  return t;
 }
 
 namespace {

@@ -10,7 +10,7 @@ namespace ehgp {
 // blocks, which the next reset folds into one of the total size.
 class DeviceArena {
  public:
-  DeviceArena() = default;
+  explicit DeviceArena(std::atomic<uint64_t>& held) : held_(held) {}  // counts the bytes of its blocks there
   DeviceArena(const DeviceArena&) = delete;
   DeviceArena& operator=(const DeviceArena&) = delete;
   ~DeviceArena() { release(); }
@@ -22,14 +22,15 @@ class DeviceArena {
     return take(reinterpret_cast<void**>(p), count * sizeof(T));
   }
   void release();
-  uint64_t bytes() const;
 
  private:
+  cudaError_t add(uint64_t size, uint64_t used, void** p);
   struct Block {
     char* p;
     uint64_t size, used;
   };
   std::vector<Block> blocks_;
+  std::atomic<uint64_t>& held_;
 };
 
 // Rounds of the forest journal over all families, and as many by its last block (12 to 21 and 1 to 47 on uniform,

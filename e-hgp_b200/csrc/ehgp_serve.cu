@@ -12,9 +12,10 @@
 //    that arrive while others run are admitted as workers and memory free up, and their
 //    device work and copies overlap with the others' (continuous batching);
 //  * admission by memory: every running request reserves an estimate of the device bytes
-//    its cloud needs (bytes per point, seeded conservatively and raised to the largest
+//    its cloud needs (bytes per point for its K, seeded conservatively and raised to the largest
 //    per-point footprint a worker's context has reached); a request is admitted when the
-//    reservations stay within hbm_fraction of the device's memory;
+//    reservations stay within hbm_fraction of the device's memory, with what idle workers keep from
+//    their last request; where that is in the way, they give it back first;
 //  * a request's LBVH, supports and event state stay on the device while it runs; when it
 //    completes, its result (forest nodes with the supports of their levels, child arena,
 //    forest batches, final roots, vertical maps, EMST edges) is copied to host memory the
@@ -26,6 +27,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstdlib>
 #include <cstring>
@@ -111,6 +113,8 @@ struct Worker {
   ehgp_ctx* ctx = nullptr;
   std::thread thread;
   uint64_t max_n_seen = 0;
+  uint64_t kept = 0;   // hierarchy memory of the idle context
+  bool trim = false;   // asked to give it back
 };
 
 }  // namespace
@@ -119,7 +123,8 @@ struct ehgp_server {
   int device = 0;
   ehgp_server_limits limits{};
   uint64_t budget = 0;              // bytes the running requests may reserve
-  double bytes_per_point = 0;       // admission estimate (raised by measurement)
+  double bytes_per_point[11] = {};  // admission estimate for each K (raised by measurement)
+  double records_per_point = 0;     // of them, the index and support buffers: submit refuses by these
   uint64_t reserved = 0;            // reservations of the running requests
   std::vector<Worker> workers;
   std::deque<uint64_t> queue;
@@ -133,7 +138,33 @@ struct ehgp_server {
 
 namespace {
 
-uint64_t estimate(const ehgp_server& s, uint64_t n) { return (uint64_t)(s.bytes_per_point * (double)n) + (64ull << 20); }
+uint64_t estimate(double per_point, uint64_t n) { return (uint64_t)(per_point * (double)n) + (64ull << 20); }
+
+// True when the memory that the other idle workers keep fits beside the reservations and `need` more;
+// else asks as many of them as it takes to give theirs back (the largest first).
+bool idle_memory_fits(ehgp_server& s, uint32_t w, uint64_t need) {
+  uint64_t all = 0, kept = 0;  // kept: by those that are not asked yet
+  for (uint32_t i = 0; i < s.workers.size(); ++i) {
+    const Worker& x = s.workers[i];
+    if (i == w) continue;
+    all += x.kept;
+    kept += x.trim ? 0 : x.kept;
+  }
+  if (all == 0 || s.reserved + need + all <= s.budget) return true;
+  while (s.reserved + need + kept > s.budget) {
+    Worker* most = nullptr;
+    for (uint32_t i = 0; i < s.workers.size(); ++i) {
+      Worker& x = s.workers[i];
+      if (i != w && x.kept && !x.trim && (!most || x.kept > most->kept)) most = &x;
+    }
+    if (!most) break;
+    most->trim = true;
+    kept -= most->kept;
+  }
+  s.cv_work.notify_all();
+  return false;
+}
+
 
 // The whole chain for one request on the worker's context; fills the request's result.
 int run_request(ehgp_ctx* ctx, Request& r) {
@@ -179,8 +210,14 @@ void worker_loop(ehgp_server* s, uint32_t w) {
         if (s->stop) return;
         if (!s->queue.empty()) {
           Request* head = s->reqs.at(s->queue.front()).get();
-          const uint64_t need = estimate(*s, head->n);
-          if (s->reserved + need <= s->budget || s->reserved == 0) {  // FIFO; a lone request always runs
+          const uint64_t est = estimate(s->bytes_per_point[head->K], head->n), need = std::max(est, me.kept);
+          if (s->reserved + est > s->budget && s->reserved != 0) {  // FIFO; a lone request always runs
+            ++s->waits_for_memory;
+          } else if (me.kept > est && s->reserved + need > s->budget) {
+            me.trim = true;
+          } else if (idle_memory_fits(*s, w, need)) {
+            me.kept = 0;  // within the reservation from here on
+            me.trim = false;
             s->queue.pop_front();
             head->reserved = need;
             s->reserved += need;
@@ -191,18 +228,31 @@ void worker_loop(ehgp_server* s, uint32_t w) {
             r = head;
             break;
           }
-          ++s->waits_for_memory;
+        }
+        if (me.trim) {
+          lock.unlock();
+          ehgp::hier_trim(*me.ctx);
+          lock.lock();
+          me.trim = false;
+          me.kept = 0;
+          s->cv_work.notify_all();
+          continue;
         }
         s->cv_work.wait(lock);
       }
     }
+    const uint64_t held_before = ehgp_ctx_device_bytes(me.ctx);
     const int st = run_request(me.ctx, *r);
-    const uint64_t held = ehgp_ctx_device_bytes(me.ctx);
+    const uint64_t held = ehgp_ctx_device_bytes(me.ctx), kept = me.ctx->hier_bytes;
     {
       std::lock_guard<std::mutex> lock(s->mu);
       me.max_n_seen = std::max(me.max_n_seen, r->n);
-      if (st == EHGP_OK && r->n >= 1024)  // the context's footprint per point of the largest cloud it holds
-        s->bytes_per_point = std::max(s->bytes_per_point, (double)held / (double)me.max_n_seen);
+      me.kept = kept;
+      if (st == EHGP_OK && r->n >= 1024) {  // the context's footprint per point of the largest cloud it holds
+        double& all = s->bytes_per_point[r->K];
+        if (held > held_before) all = std::max(all, (double)held / (double)me.max_n_seen);
+        s->records_per_point = std::max(s->records_per_point, (double)(held - kept) / (double)me.max_n_seen);
+      }
       r->status = st;
       if (st != EHGP_OK) r->error = ehgp_last_error(me.ctx);
       r->state = st == EHGP_OK ? EHGP_REQ_DONE : EHGP_REQ_FAILED;
@@ -245,9 +295,11 @@ int ehgp_server_create(int device, const ehgp_server_limits* limits, ehgp_server
   s->device = device;
   s->limits = *limits;
   s->budget = (uint64_t)(limits->hbm_fraction * (double)total_b);
-  // before any measurement: about 120 KB per point covers the 50,653-point lattice's
-  // supports and hierarchy with room
-  s->bytes_per_point = 120.0 * 1024.0;
+  s->records_per_point = 120.0 * 1024.0;  // before any measurement
+  // 37 KB per point for index, lists and first record buffers, 0.95 KB per support event with the
+  // hierarchy's: 502 KB per point at 50,653 lattice points and K = 10 (488 events), 82 KB at K = 4
+  for (uint32_t k = 1; k <= 10; ++k)
+    s->bytes_per_point[k] = 1024.0 * (40.0 + 1.05 * (7.0 + 483.0 * std::pow(k / 10.0, 2.3)));
   for (uint32_t w = 0; w < limits->workers; ++w) {
     ehgp_limits cl{limits->max_points, limits->hbm_fraction};
     Worker wk;
@@ -290,7 +342,7 @@ int ehgp_cloud_submit(ehgp_server* s, const ehgp_cloud_desc* d, ehgp_request_id*
   r->t_submit = Clock::now();
   {
     std::lock_guard<std::mutex> lock(s->mu);
-    if (estimate(*s, d->n) > s->budget) return EHGP_ERR_OUT_OF_MEMORY;
+    if (estimate(s->records_per_point, d->n) > s->budget) return EHGP_ERR_OUT_OF_MEMORY;
     r->id = s->next_id++;
     *id = r->id;
     s->queue.push_back(r->id);
@@ -413,7 +465,7 @@ int ehgp_server_info(ehgp_server* s, uint64_t* info, uint32_t count) {
   uint64_t held = 0, running = 0;
   for (const auto& w : s->workers) held += ehgp_ctx_device_bytes(w.ctx);
   for (const auto& kv : s->reqs) running += kv.second->state == EHGP_REQ_RUNNING;
-  const uint64_t v[8] = {s->budget, s->reserved, held, (uint64_t)s->bytes_per_point, s->queue.size(), running,
+  const uint64_t v[8] = {s->budget, s->reserved, held, (uint64_t)s->bytes_per_point[10], s->queue.size(), running,
                          s->completed, s->waits_for_memory};
   for (uint32_t i = 0; i < count && i < 8; ++i) info[i] = v[i];
   return EHGP_OK;

@@ -61,7 +61,8 @@ int ehgp_ctx_destroy(ehgp_ctx* ctx);
 const char* ehgp_last_error(const ehgp_ctx* ctx);
 /* Static name of a status code. */
 const char* ehgp_status_string(int status);
-/* Device bytes owned by the context (resident buffers). */
+/* Device bytes owned by the context: resident buffers, and the hierarchy's event arrays,
+ * queues and records. */
 uint64_t ehgp_ctx_device_bytes(const ehgp_ctx* ctx);
 
 /* Support records are produced count -> allocate -> emit, as the reference's
@@ -577,7 +578,7 @@ int ehgp_result_copy(ehgp_server* server, ehgp_request_id id, const ehgp_served_
 /* Drops a finished request and its result. */
 int ehgp_result_release(ehgp_server* server, ehgp_request_id id);
 /* [0] memory budget, [1] bytes reserved by running requests, [2] device bytes held
- * by the workers' contexts, [3] admission estimate in bytes per point, [4] queued,
+ * by the workers' contexts, [3] admission estimate in bytes per point at K = 10, [4] queued,
  * [5] running, [6] completed requests, [7] admissions deferred for memory. */
 int ehgp_server_info(ehgp_server* server, uint64_t* info, uint32_t count);
 
