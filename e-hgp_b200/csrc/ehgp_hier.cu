@@ -2219,7 +2219,10 @@ int ehgp_hier_schedule(ehgp_ctx* ctx, uint32_t chunk_batches, uint32_t part_arms
 int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out) {
   if (!ctx || !out) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
+  if (ctx->poisoned) return ehgp::abi_fail(ctx, EHGP_ERR_POISONED, "the context is poisoned by an earlier CUDA failure");
   if (!ctx->hier) return ehgp::abi_fail(ctx, EHGP_ERR_NOT_BUILT, "no hierarchy result is resident");
+  cudaError_t e = cudaSetDevice(ctx->device);  // the records are on it, and the copies' events belong to it
+  if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "cudaSetDevice");
   ehgp::HierState& h = *ctx->hier;
   const ehgp::JournalOut& j = h.journal;
   std::vector<ehgp::CopyOut> list;
@@ -2242,8 +2245,7 @@ int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out) {
     add(out->vertical, j.vert, j.n_vert, sizeof *j.vert);
     if (out->roots && !j.roots.empty()) std::memcpy(out->roots, j.roots.data(), j.roots.size() * sizeof j.roots[0]);
   }
-  const cudaError_t e = ehgp::copy_out(*ctx, list);
-  if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "hierarchy copy");
+  if ((e = ehgp::copy_out(*ctx, list)) != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "hierarchy copy");
   return EHGP_OK;
 }
 
@@ -2277,8 +2279,11 @@ int ehgp_hier_stats(const ehgp_ctx* ctx, double* ms, uint64_t* stats) {
 int ehgp_event_supports(ehgp_ctx* ctx, const uint32_t* events, uint64_t count, uint32_t* out) {
   if (!ctx || (count && (!events || !out))) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
+  if (ctx->poisoned) return ehgp::abi_fail(ctx, EHGP_ERR_POISONED, "the context is poisoned by an earlier CUDA failure");
   if (!ctx->hier || ctx->hier->decision != EHGP_OK || !ctx->hier->order0 || !ctx->hier->ev_raw)
     return ehgp::abi_fail(ctx, EHGP_ERR_NOT_BUILT, "ehgp_event_supports needs a hierarchy result");
+  cudaError_t e = cudaSetDevice(ctx->device);
+  if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "cudaSetDevice");
   ehgp::HierState& h = *ctx->hier;
   cudaStream_t st = ctx->stream;
   // chunks through the facade's scratch (index: order0, output: ev_raw), free after the call
@@ -2288,7 +2293,7 @@ int ehgp_event_supports(ehgp_ctx* ctx, const uint32_t* events, uint64_t count, u
     cudaMemcpyAsync(h.order0, events + b0, (uint64_t)m * 4, cudaMemcpyHostToDevice, st);
     ehgp::k_event_supports<<<ehgp::nblk(m, ehgp::kT), ehgp::kT, 0, st>>>(m, h.order0, h.ev, (uint32_t)h.events,
                                                                         (uint32_t*)h.ev_raw);
-    const cudaError_t e = ehgp::copy_out(*ctx, {{(char*)(out + 5 * b0), (const char*)h.ev_raw, (uint64_t)m * 20}});
+    e = ehgp::copy_out(*ctx, {{(char*)(out + 5 * b0), (const char*)h.ev_raw, (uint64_t)m * 20}});
     if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "facade event supports");
   }
   return EHGP_OK;
