@@ -158,12 +158,13 @@ cudaError_t copy_out(Ctx& ctx, const std::vector<CopyOut>& list) try {
   const cudaError_t es = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return e;
   return es != cudaSuccess ? es : failed.load() ? cudaErrorUnknown : cudaSuccess;
-} catch (const std::bad_alloc&) {
-  return cudaErrorMemoryAllocation;
+} catch (const std::bad_alloc&) {  // (thrown before the first thread starts)
+  return copy_direct(ctx, list);
 }
 
 cudaError_t ctx_alloc(Ctx& ctx, void** ptr, size_t bytes) {
   if (bytes == 0) bytes = 16;
+  ctx.allocations.reserve(ctx.allocations.size() + 1);  // (what is thrown is thrown before there is memory to lose)
   cudaError_t e = cudaMalloc(ptr, bytes);
   if (e == cudaSuccess) {
     ctx.allocations.push_back(*ptr);
@@ -198,6 +199,13 @@ namespace ehgp {
 int abi_fail(Ctx* ctx, int status, const char* msg) { return fail(ctx, status, msg); }
 int abi_cuda_fail(Ctx* ctx, cudaError_t e, const char* where) { return cuda_fail(ctx, e, where); }
 int abi_device_status(Ctx* ctx, uint32_t err) { return device_status(ctx, err); }
+int abi_no_memory(Ctx* ctx) noexcept {
+  try {
+    return fail(ctx, EHGP_ERR_OUT_OF_MEMORY, "host memory is exhausted");
+  } catch (...) {
+    return EHGP_ERR_OUT_OF_MEMORY;
+  }
+}
 }  // namespace ehgp
 
 namespace {
@@ -230,7 +238,7 @@ int device_status(Ctx* ctx, uint32_t err) {
 
 // Shared body of the three LBVH build entry points.  `src` is a host or
 // device pointer according to `where` (0 host f64, 1 host f32, 2 device f64).
-int lbvh_build_common(Ctx* ctx, const void* src, uint64_t n, const ehgp_lbvh_out* out, int where) {
+int lbvh_build_common(Ctx* ctx, const void* src, uint64_t n, const ehgp_lbvh_out* out, int where) try {
   if (!ctx) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   ctx->last_error.clear();
@@ -274,6 +282,8 @@ int lbvh_build_common(Ctx* ctx, const void* src, uint64_t n, const ehgp_lbvh_out
   if ((e = ehgp::lbvh_export(*ctx, n32, out)) != cudaSuccess) return cuda_fail(ctx, e, "LBVH export");
   ctx->built_n = n;
   return EHGP_OK;
+} catch (const std::bad_alloc&) {
+  return ehgp::abi_no_memory(ctx);
 }
 
 }  // namespace

@@ -1695,6 +1695,7 @@ template <class T>
 cudaError_t halloc(HierState& h, T** p, uint64_t count) {
   void* q = nullptr;
   const uint64_t bytes = count * sizeof(T) + 16;
+  h.allocs.reserve(h.allocs.size() + 1);
   const cudaError_t e = cudaMalloc(&q, bytes);
   if (e != cudaSuccess) return e;
   h.allocs.push_back({q, bytes});
@@ -2162,7 +2163,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
 
 extern "C" {
 
-int ehgp_hierarchy(ehgp_ctx* ctx, uint32_t K, ehgp_hier_counts* counts) {
+int ehgp_hierarchy(ehgp_ctx* ctx, uint32_t K, ehgp_hier_counts* counts) try {
   if (!ctx) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   ctx->last_error.clear();
@@ -2204,9 +2205,11 @@ int ehgp_hierarchy(ehgp_ctx* ctx, uint32_t K, ehgp_hier_counts* counts) {
     counts->decision = (uint32_t)s;
   }
   return s;
+} catch (const std::bad_alloc&) {
+  return ehgp::abi_no_memory(ctx);
 }
 
-int ehgp_hier_schedule(ehgp_ctx* ctx, uint32_t chunk_batches, uint32_t part_arms, uint32_t host_threads) {
+int ehgp_hier_schedule(ehgp_ctx* ctx, uint32_t chunk_batches, uint32_t part_arms, uint32_t host_threads) try {
   if (!ctx) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   if (!ctx->hier) ctx->hier = new ehgp::HierState(*ctx);
@@ -2214,9 +2217,11 @@ int ehgp_hier_schedule(ehgp_ctx* ctx, uint32_t chunk_batches, uint32_t part_arms
   (void)host_threads;
   ctx->hier->part_arms = part_arms;
   return EHGP_OK;
+} catch (const std::bad_alloc&) {
+  return ehgp::abi_no_memory(ctx);
 }
 
-int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out) {
+int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out) try {
   if (!ctx || !out) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   if (ctx->poisoned) return ehgp::abi_fail(ctx, EHGP_ERR_POISONED, "the context is poisoned by an earlier CUDA failure");
@@ -2247,6 +2252,8 @@ int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out) {
   }
   if ((e = ehgp::copy_out(*ctx, list)) != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "hierarchy copy");
   return EHGP_OK;
+} catch (const std::bad_alloc&) {
+  return ehgp::abi_no_memory(ctx);
 }
 
 int ehgp_hier_stats(const ehgp_ctx* ctx, double* ms, uint64_t* stats) {
@@ -2276,7 +2283,7 @@ int ehgp_hier_stats(const ehgp_ctx* ctx, double* ms, uint64_t* stats) {
   return EHGP_OK;
 }
 
-int ehgp_event_supports(ehgp_ctx* ctx, const uint32_t* events, uint64_t count, uint32_t* out) {
+int ehgp_event_supports(ehgp_ctx* ctx, const uint32_t* events, uint64_t count, uint32_t* out) try {
   if (!ctx || (count && (!events || !out))) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   if (ctx->poisoned) return ehgp::abi_fail(ctx, EHGP_ERR_POISONED, "the context is poisoned by an earlier CUDA failure");
@@ -2297,6 +2304,8 @@ int ehgp_event_supports(ehgp_ctx* ctx, const uint32_t* events, uint64_t count, u
     if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "facade event supports");
   }
   return EHGP_OK;
+} catch (const std::bad_alloc&) {
+  return ehgp::abi_no_memory(ctx);
 }
 
 int ehgp_event_level(ehgp_ctx* ctx, uint64_t event, uint64_t* num, uint64_t* den, int32_t* scale) {

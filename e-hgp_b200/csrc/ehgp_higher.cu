@@ -2615,7 +2615,7 @@ int ehgp_predicate_eval(ehgp_ctx* ctx, uint32_t predicate, const uint32_t* ids, 
   return EHGP_OK;
 }
 
-int ehgp_higher(ehgp_ctx* ctx, uint32_t K, const ehgp_higher_out* out) {
+int ehgp_higher(ehgp_ctx* ctx, uint32_t K, const ehgp_higher_out* out) try {
   if (!ctx) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   ctx->last_error.clear();
@@ -2640,6 +2640,8 @@ int ehgp_higher(ehgp_ctx* ctx, uint32_t K, const ehgp_higher_out* out) {
     if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "higher-support copy");
   }
   return EHGP_OK;
+} catch (const std::bad_alloc&) {
+  return ehgp::abi_no_memory(ctx);
 }
 
 int ehgp_higher_stats(const ehgp_ctx* ctx, double* kernel_ms, uint64_t* stats, uint32_t count) {

@@ -7,6 +7,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -367,4 +368,5 @@ namespace ehgp {
 int abi_fail(Ctx* ctx, int status, const char* msg);
 int abi_cuda_fail(Ctx* ctx, cudaError_t e, const char* where);
 int abi_device_status(Ctx* ctx, uint32_t err);
+int abi_no_memory(Ctx* ctx) noexcept;  // a std::bad_alloc that reached the C interface
 }  // namespace ehgp

@@ -67,6 +67,7 @@ cudaError_t DeviceArena::take(void** p, uint64_t bytes) {
 }
 
 cudaError_t DeviceArena::add(uint64_t size, uint64_t used, void** p) {
+  blocks_.reserve(blocks_.size() + 1);
   const cudaError_t e = cudaMalloc(p, size);
   if (e != cudaSuccess) return e;
   blocks_.push_back({static_cast<char*>(*p), size, used});

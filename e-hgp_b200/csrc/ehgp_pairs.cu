@@ -831,7 +831,7 @@ int pairs_run(Ctx& ctx, uint32_t K, uint32_t* out_count) {
 
 extern "C" {
 
-int ehgp_pairs(ehgp_ctx* ctx, uint32_t K, const ehgp_pairs_out* out) {
+int ehgp_pairs(ehgp_ctx* ctx, uint32_t K, const ehgp_pairs_out* out) try {
   if (!ctx) return EHGP_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mutex);
   ctx->last_error.clear();
@@ -858,6 +858,8 @@ int ehgp_pairs(ehgp_ctx* ctx, uint32_t K, const ehgp_pairs_out* out) {
     if (e != cudaSuccess) return ehgp::abi_cuda_fail(ctx, e, "pair copy");
   }
   return EHGP_OK;
+} catch (const std::bad_alloc&) {
+  return ehgp::abi_no_memory(ctx);
 }
 
 }  // extern "C"

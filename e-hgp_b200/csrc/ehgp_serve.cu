@@ -167,7 +167,7 @@ bool idle_memory_fits(ehgp_server& s, uint32_t w, uint64_t need) {
 
 
 // The whole chain for one request on the worker's context; fills the request's result.
-int run_request(ehgp_ctx* ctx, Request& r) {
+int run_request(ehgp_ctx* ctx, Request& r) try {
   if (ehgp_step_begin(ctx) != EHGP_OK) return EHGP_ERR_CUDA;
   ehgp_lbvh_out none{};
   int st = r.f32 ? ehgp_lbvh_build_f32(ctx, r.xyz32.data(), r.n, &none) : ehgp_lbvh_build(ctx, r.xyz64.data(), r.n, &none);
@@ -198,6 +198,8 @@ int run_request(ehgp_ctx* ctx, Request& r) {
   std::vector<uint32_t> lev(c.nodes);
   for (uint64_t i = 0; i < c.nodes; ++i) lev[i] = r.nodes[i].level_event;
   return ehgp_event_supports(ctx, lev.data(), c.nodes, r.node_support.data());
+} catch (const std::bad_alloc&) {
+  return ehgp::abi_no_memory(ctx);
 }
 
 void worker_loop(ehgp_server* s, uint32_t w) {
@@ -399,7 +401,7 @@ const char* ehgp_request_error(ehgp_server* s, ehgp_request_id id) {
   return r ? r->error.c_str() : "";
 }
 
-int ehgp_result_copy(ehgp_server* s, ehgp_request_id id, const ehgp_served_out* out) {
+int ehgp_result_copy(ehgp_server* s, ehgp_request_id id, const ehgp_served_out* out) try {
   if (!s || !out) return EHGP_ERR_INVALID_ARGUMENT;
   std::shared_ptr<Request> r;  // a finished request's result does not change: copied outside the lock
   {
@@ -447,6 +449,8 @@ int ehgp_result_copy(ehgp_server* s, ehgp_request_id id, const ehgp_served_out* 
   work();
   for (auto& t : pool) t.join();
   return EHGP_OK;
+} catch (const std::bad_alloc&) {
+  return EHGP_ERR_OUT_OF_MEMORY;
 }
 
 int ehgp_result_release(ehgp_server* s, ehgp_request_id id) {
