@@ -82,7 +82,7 @@ void stage_free(Ctx& ctx) {
 
 cudaError_t copy_direct(Ctx& ctx, const std::vector<CopyOut>& list) {
   for (const CopyOut& c : list) {
-    const cudaError_t e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, ctx.stream);
+    const cudaError_t e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDefault, ctx.stream);
     if (e != cudaSuccess) return e;
   }
   return cudaStreamSynchronize(ctx.stream);
@@ -104,7 +104,7 @@ cudaError_t copy_out(Ctx& ctx, const std::vector<CopyOut>& list) try {
     const bool pageable = cudaPointerGetAttributes(&at, c.dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
     if (!pageable || c.bytes <= kStageBytes || all < (ctx.stage ? kStageFrom : kStageMake)) {
-      if ((e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+      if ((e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDefault, st)) != cudaSuccess) return e;
       continue;
     }
     for (uint64_t o = 0; o < c.bytes; o += kStageBytes)
@@ -146,7 +146,7 @@ cudaError_t copy_out(Ctx& ctx, const std::vector<CopyOut>& list) try {
       while (!done[t - kStageSlots].load(std::memory_order_acquire) && !failed.load(std::memory_order_acquire))
         std::this_thread::yield();
     const int slot = (int)(t % kStageSlots);
-    e = cudaMemcpyAsync(ctx.stage + slot * kStageBytes, chunks[t].src, chunks[t].bytes, cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(ctx.stage + slot * kStageBytes, chunks[t].src, chunks[t].bytes, cudaMemcpyDefault, st);
     if (e == cudaSuccess) e = cudaEventRecord(ctx.stage_ev[slot], st);
     if (e != cudaSuccess) {
       failed.store(1, std::memory_order_release);
@@ -166,6 +166,11 @@ cudaError_t ctx_alloc(Ctx& ctx, void** ptr, size_t bytes) {
   if (bytes == 0) bytes = 16;
   ctx.allocations.reserve(ctx.allocations.size() + 1);  // (what is thrown is thrown before there is memory to lose)
   cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx.hier_bytes) {  // the last hierarchy gives way to this call's buffers
+    cudaGetLastError();
+    hier_trim(ctx);
+    e = cudaMalloc(ptr, bytes);
+  }
   if (e == cudaSuccess) {
     ctx.allocations.push_back(*ptr);
     ctx.device_bytes += bytes;
@@ -422,6 +427,9 @@ int ehgp_tune(ehgp_ctx* ctx, uint32_t knob, uint64_t value) {
     case EHGP_TUNE_SORT_WAIT:
       if (value > ehgp::kRadixWait) return fail(ctx, EHGP_ERR_INVALID_ARGUMENT, "a sort looks at most 2^20 times");
       ctx->radix.wait = (uint32_t)value;
+      return EHGP_OK;
+    case EHGP_TUNE_HIERARCHY_BLOCK:
+      ctx->hier_largest = value ? value : ~uint64_t{0};
       return EHGP_OK;
     case EHGP_TUNE_FOREST_ROUNDS:
       ctx->forest_rounds = (uint32_t)std::min<uint64_t>(value, 0xffffffffu);

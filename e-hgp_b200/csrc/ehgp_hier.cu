@@ -1628,7 +1628,7 @@ k_facet_exact(DescentParams d, uint32_t m, const uint32_t* __restrict__ hard, co
 struct HierState {
   explicit HierState(Ctx& ctx) : held(ctx.hier_bytes), mem(ctx.hier_bytes) {}
   std::atomic<uint64_t>& held;  // device bytes of everything below
-  std::vector<std::pair<void*, uint64_t>> allocs;
+  std::vector<std::pair<void*, uint64_t>> allocs, scratch;  // kept with a result / not used after the descent
   uint64_t cap_events = 0, cap_arms = 0, cap_births = 0, cap_slots = 0;
   // device
   EvRec* ev_raw = nullptr;
@@ -1692,25 +1692,30 @@ struct HierState {
 namespace {
 
 template <class T>
-cudaError_t halloc(HierState& h, T** p, uint64_t count) {
+cudaError_t halloc(HierState& h, T** p, uint64_t count, std::vector<std::pair<void*, uint64_t>>& list) {
   void* q = nullptr;
   const uint64_t bytes = count * sizeof(T) + 16;
-  h.allocs.reserve(h.allocs.size() + 1);
+  list.reserve(list.size() + 1);
   const cudaError_t e = cudaMalloc(&q, bytes);
   if (e != cudaSuccess) return e;
-  h.allocs.push_back({q, bytes});
+  list.push_back({q, bytes});
   h.held += bytes;
   *p = (T*)q;
   return cudaSuccess;
 }
 
-// Frees the event arrays; the facade goes with them.
-void hfree_all(HierState& h) {
-  for (const auto& a : h.allocs) {
+void hfree(HierState& h, std::vector<std::pair<void*, uint64_t>>& list) {
+  for (const auto& a : list) {
     cudaFree(a.first);
     h.held -= a.second;
   }
-  h.allocs.clear();
+  list.clear();
+}
+
+// Frees the event arrays; the facade goes with them.
+void hfree_all(HierState& h) {
+  hfree(h, h.allocs);
+  hfree(h, h.scratch);
   h.qcount = nullptr;
   h.events = 0;
   h.complete = false;
@@ -1729,34 +1734,35 @@ void free_ties(HierState& h) {
 }
 
 cudaError_t ensure_events(HierState& h, uint64_t m) {
-  if (m <= h.cap_events && h.cap_events) return cudaSuccess;
+  if (m <= h.cap_events && !h.scratch.empty()) return cudaSuccess;
   hfree_all(h);
   const uint64_t cap = m + m / 8 + 1024;
   cudaError_t e;
-#define HA(p, c) if ((e = halloc(h, &(p), (c))) != cudaSuccess) return e
+#define HA(p, c) if ((e = halloc(h, &(p), (c), h.allocs)) != cudaSuccess) return e
+#define HS(p, c) if ((e = halloc(h, &(p), (c), h.scratch)) != cudaSuccess) return e
   HA(h.ev_raw, cap);
   HA(h.ev, cap);
-  HA(h.lmid_raw, cap);
-  HA(h.lerr_raw, cap);
-  HA(h.lmid, cap);
-  HA(h.lerr, cap);
-  HA(h.key, cap);
-  HA(h.key2, cap);
+  HS(h.lmid_raw, cap);
+  HS(h.lerr_raw, cap);
+  HS(h.lmid, cap);
+  HS(h.lerr, cap);
+  HS(h.key, cap);
+  HS(h.key2, cap);
   HA(h.order0, cap);
-  HA(h.order1, cap);
-  HA(h.pre_hi, cap);
-  HA(h.suf_lo, cap);
+  HS(h.order1, cap);
+  HS(h.pre_hi, cap);
+  HS(h.suf_lo, cap);
   HA(h.bsum, cap / 1024 + 2);
   HA(h.ubsum, cap / 1024 + 2);
-  HA(h.uncertain, 1u << 20);
-  HA(h.eqprev, cap);
-  HA(h.lclass, cap);
+  HS(h.uncertain, 1u << 20);
+  HS(h.eqprev, cap);
+  HS(h.lclass, cap);
   HA(h.rank_order, cap);
   HA(h.counters, 32);
   HA(h.radix_counts, radix_counts_words(cap));
-  HA(h.bfac, cap * kMaxFacet);
+  HS(h.bfac, cap * kMaxFacet);
   HA(h.d_cls_rp, cap);
-  HA(h.d_size_rp, cap);
+  HS(h.d_size_rp, cap);
   HA(h.d_armoff, cap + 1);
   HA(h.dstats, 4);
   const uint64_t arms = 4 * cap;
@@ -1764,8 +1770,9 @@ cudaError_t ensure_events(HierState& h, uint64_t m) {
   HA(h.d_removed, arms);
   uint64_t slots = 1;
   while (slots < 2 * cap + 1024) slots <<= 1;
-  HA(h.slots, slots);
+  HS(h.slots, slots);
 #undef HA
+#undef HS
   h.cap_events = cap;
   h.cap_arms = arms;
   h.cap_slots = slots;
@@ -1836,7 +1843,13 @@ int hier_run(Ctx& ctx, uint32_t K) {
   nh = ctx.hb.count;
   cudaEventRecord(ctx.ev0, st);
   const uint64_t total = (uint64_t)np + nh;
+  h.mem.largest = ctx.hier_largest;
   cudaError_t e = ensure_events(h, total + 1);
+  if (e == cudaErrorMemoryAllocation) {  // the last call's working memory is made again below
+    cudaGetLastError();
+    h.mem.release();
+    e = ensure_events(h, total + 1);
+  }
   if (e != cudaSuccess) return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "hierarchy buffers do not fit the device");
   cudaMemsetAsync(h.counters, 0, 32 * sizeof(uint32_t), st);
   cudaMemsetAsync(h.dstats, 0, 4 * sizeof(unsigned long long), st);
@@ -2014,15 +2027,19 @@ int hier_run(Ctx& ctx, uint32_t K) {
   // ---- strict-arm descent ----
   // One part unless a schedule says otherwise: the fewer parts, the fewer rounds, and a round
   // is a few launches and a look at its queue's length.
-  const uint32_t part_fams = h.part_arms ? std::max(1u, h.part_arms / 4u) : (uint32_t)nfam;
+  uint32_t part_fams = h.part_arms ? std::max(1u, h.part_arms / 4u) : (uint32_t)nfam;
   const uint64_t journal = journal_bytes(in);
-  // queue entries: about a third of the arms miss their first probe; a longer queue grows
-  uint64_t q_cap = std::min<uint64_t>(narms, std::max<uint64_t>(narms * 3 / 8, 1u << 16)) + 32;
+  uint64_t q_cap = 0;
   uint32_t *q_arm[2], *q_hard;
   QFacet* q_fac[2];
   uint4* q_sup;
   auto queues = [&]() -> cudaError_t {
-    cudaError_t r = h.mem.reset(std::max(journal, q_cap * (2 * (4 + sizeof(QFacet)) + 4 + 16) + 4096));
+    const uint64_t bytes = q_cap * (2 * (4 + sizeof(QFacet)) + 4 + 16) + 4096;
+    cudaError_t r = h.mem.reset(std::max(journal, bytes));
+    if (r == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      r = h.mem.reset(bytes);
+    }
     for (int i = 0; i < 2; ++i) {
       if (r == cudaSuccess) r = h.mem.take(&q_arm[i], q_cap);
       if (r == cudaSuccess) r = h.mem.take(&q_fac[i], q_cap);
@@ -2031,12 +2048,23 @@ int hier_run(Ctx& ctx, uint32_t K) {
     if (r == cudaSuccess) r = h.mem.take(&q_sup, q_cap);
     return r;
   };
+  // Queues for `need` entries (0: a third of a part's arms, what misses the first probe, and some room); parts
+  // become smaller while the device has none.
+  auto room = [&](uint64_t need) -> bool {
+    for (;; need = 0, part_fams = (part_fams + 3) / 4) {
+      const uint64_t arms = std::min<uint64_t>(narms, 4ull * part_fams);
+      q_cap = need ? need : std::min<uint64_t>(arms, std::max<uint64_t>(arms * 3 / 8, 1u << 16)) + 32;
+      if (queues() == cudaSuccess) return true;
+      cudaGetLastError();
+      if (part_fams <= 1024) return false;
+    }
+  };
   auto no_queue = [&] {
     cudaGetLastError();
     return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "descent queue buffers do not fit the device");
   };
-  if (queues() != cudaSuccess) return no_queue();
-  if (!h.qcount && (e = halloc(h, &h.qcount, 4)) != cudaSuccess)
+  if (!room(0)) return no_queue();
+  if (!h.qcount && (e = halloc(h, &h.qcount, 4, h.allocs)) != cudaSuccess)
     return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "descent queue");
   const DescentParams dp{n, 2 * n - 2, g.tnodes, b.px, b.py, b.pz, h.S, h.slots, (uint32_t)(h.cap_slots - 1), h.bfac,
                          (uint32_t)nb_higher, in.ev, h.lmid, h.lerr};
@@ -2048,10 +2076,10 @@ int hier_run(Ctx& ctx, uint32_t K) {
     if (!ev && cudaEventCreate(&ev) != cudaSuccess) ev = nullptr;
   cudaEventRecord(ctx.evk0, st);
   cudaMemsetAsync(h.dstats + 3, 0xff, sizeof(unsigned long long), st);
-  for (uint32_t f0 = 0; f0 < nfam; f0 += part_fams) {
-    const uint32_t nf = std::min<uint32_t>(part_fams, (uint32_t)nfam - f0);
+  for (uint32_t f0 = 0, nf = 0; f0 < nfam; f0 += nf) {
     uint32_t pending = 0;
-    for (;;) {  // count -> grow -> queue
+    for (;;) {  // count -> grow (or cut the part) -> queue
+      nf = std::min<uint32_t>(part_fams, (uint32_t)nfam - f0);
       cudaMemsetAsync(h.qcount, 0, 4 * sizeof(uint32_t), st);
       k_arm_probe<<<nblk(nf, kT), kT, 0, st>>>(dp, f0, nf, in.ev, h.d_armoff, h.ev, h.d_removed, h.term, q_arm[0],
                                                q_fac[0], (uint32_t)q_cap, h.qcount);
@@ -2061,8 +2089,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
       if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "strict-arm seeds");
       if (herr) return abi_fail(&ctx, EHGP_ERR_CAPACITY, "the birth facet table is full");
       if (pending <= q_cap) break;
-      q_cap = pending;
-      if (queues() != cudaSuccess) return no_queue();
+      if (!room(pending)) return no_queue();
     }
     misses += pending;
     int cur = 0;
@@ -2130,8 +2157,18 @@ int hier_run(Ctx& ctx, uint32_t K) {
     return abi_fail(&ctx, status, msg[why < 6 ? why : 5]);
   }
   // ---- forest journal, in the queues' memory ----
-  if ((e = h.mem.reset(journal)) != cudaSuccess) return no_queue();
-  const int js = journal_run(ctx, in, h.mem, h.journal, &launches);
+  int js = EHGP_ERR_OUT_OF_MEMORY;
+  if (h.mem.reset(journal) == cudaSuccess) {
+    h.mem.release_host();
+    js = journal_run(ctx, in, h.mem, h.journal, &launches);
+  }
+  if (js == EHGP_ERR_OUT_OF_MEMORY) {  // no room: what only the descent needed goes, the records leave the device
+    cudaGetLastError();
+    hfree(h, h.scratch);
+    h.mem.reset(0);
+    h.mem.spilled = true;
+    js = journal_run(ctx, in, h.mem, h.journal, &launches);
+  }
   ctx.forest_rest = h.journal.rest;
   if (js != EHGP_OK) return js;
   cudaEventRecord(ctx.ev1, st);

@@ -293,6 +293,7 @@ struct Ctx {
   bool emst_ready = false;
   struct HierState* hier = nullptr;  // direct hierarchy (ehgp_hier.cu)
   uint32_t forest_rounds = ~0u;      // limit on the forest journal's rounds (above its own: none)
+  uint64_t hier_largest = ~uint64_t{0};  // larger blocks of the hierarchy's working memory are refused
   uint64_t forest_rest = 0;          // families that the last journal's rounds left to the host
   char* stage = nullptr;             // pinned ring of copy_out, made by the first large copy
   void* stage_map = nullptr;         // the mapping that holds it
@@ -304,7 +305,7 @@ cudaError_t ctx_alloc(Ctx& ctx, void** ptr, size_t bytes);
 // Frees one allocation of ctx_alloc (bytes as allocated).
 void ctx_free(Ctx& ctx, void* ptr, size_t bytes);
 
-// One device range and the host memory it goes to.
+// One range of device (or pinned host) memory and the host memory it goes to.
 struct CopyOut {
   char* dst;
   const char* src;

@@ -44,15 +44,20 @@
 namespace ehgp {
 
 cudaError_t DeviceArena::reset(uint64_t want) {
+  spilled = false;
+  for (Block& b : host_) b.used = 0;
   uint64_t have = 0;
   for (const Block& b : blocks_) have += b.size;
-  if (blocks_.size() == 1 && blocks_[0].size >= want) {
+  if (want && blocks_.size() == 1 && blocks_[0].size >= want && blocks_[0].size <= largest) {
     blocks_[0].used = 0;
     return cudaSuccess;
   }
-  release();
+  release_device();
+  if (want == 0) return cudaSuccess;
   void* p = nullptr;
-  return add(std::max(have, want + want / 16) + 4096, 0, &p);
+  if (add(std::max(have, want + want / 16) + 4096, 0, &p) == cudaSuccess) return cudaSuccess;
+  cudaGetLastError();
+  return add(want, 0, &p);
 }
 
 cudaError_t DeviceArena::take(void** p, uint64_t bytes) {
@@ -67,6 +72,7 @@ cudaError_t DeviceArena::take(void** p, uint64_t bytes) {
 }
 
 cudaError_t DeviceArena::add(uint64_t size, uint64_t used, void** p) {
+  if (size > largest) return cudaErrorMemoryAllocation;
   blocks_.reserve(blocks_.size() + 1);
   const cudaError_t e = cudaMalloc(p, size);
   if (e != cudaSuccess) return e;
@@ -75,12 +81,37 @@ cudaError_t DeviceArena::add(uint64_t size, uint64_t used, void** p) {
   return cudaSuccess;
 }
 
-void DeviceArena::release() {
+cudaError_t DeviceArena::take_host(void** p, uint64_t bytes) {
+  bytes = (bytes + 255) / 256 * 256;
+  for (Block& b : host_)
+    if (b.used + bytes <= b.size) {
+      *p = b.p + b.used;
+      b.used += bytes;
+      return cudaSuccess;
+    }
+  host_.reserve(host_.size() + 1);
+  const uint64_t size = bytes + bytes / 8 + 4096;
+  const cudaError_t e = cudaHostAlloc(p, size, cudaHostAllocPortable | cudaHostAllocMapped);
+  if (e == cudaSuccess) host_.push_back({static_cast<char*>(*p), size, bytes});
+  return e;
+}
+
+void DeviceArena::release_device() {
   for (const Block& b : blocks_) {
     cudaFree(b.p);
     held_ -= b.size;
   }
   blocks_.clear();
+}
+
+void DeviceArena::release_host() {
+  for (const Block& b : host_) cudaFreeHost(b.p);
+  host_.clear();
+}
+
+void DeviceArena::release() {
+  release_device();
+  release_host();
 }
 
 namespace {
@@ -1112,6 +1143,8 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
   };
 #define TAKE(p, c) \
   if ((e = mem.take(&(p), (c))) != cudaSuccess) return no_memory()
+#define TAKE_RECORD(p, c) \
+  if ((e = mem.take_record(&(p), (c))) != cudaSuccess) return no_memory()
   if ((uint64_t)H + F >= kSaddle)
     return abi_fail(&ctx, EHGP_ERR_CAPACITY, "the forest journal exceeds 32-bit record indices");
   J j{};
@@ -1316,9 +1349,9 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
   TAKE(rcls, R);
   TAKE(first, R);
   TAKE(fam_batch, F);
-  TAKE(out.roles, R);
-  TAKE(out.births, H);
-  TAKE(out.fam, F);
+  TAKE_RECORD(out.roles, R);
+  TAKE_RECORD(out.births, H);
+  TAKE_RECORD(out.fam, F);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "forest journal groups");
   const uint32_t Nn = ht[1];
   out.n_groups = ht[0];
@@ -1326,9 +1359,9 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
   out.n_children = ht[2];
   out.n_roles = R;
   out.n_vert = Nn - node1;
-  TAKE(out.nodes, out.n_nodes);
-  TAKE(out.children, out.n_children);
-  TAKE(out.vert, out.n_vert);
+  TAKE_RECORD(out.nodes, out.n_nodes);
+  TAKE_RECORD(out.children, out.n_children);
+  TAKE_RECORD(out.vert, out.n_vert);
   k_fj_singletons<<<nblk(in.n), kT, 0, st>>>(in.n, src, rcls, out.nodes);
   if (F) k_fj_roles<<<nblk(F), kT, 0, st>>>(j, H - in.n, src, rcls);
   *launches += 1 + (F ? 1 : 0);
@@ -1366,11 +1399,11 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
   }
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return abi_cuda_fail(&ctx, e, "forest journal batches");
   out.n_batches = nbatch;
-  TAKE(out.jb, out.n_batches);
-  TAKE(out.fb, out.n_batches);
-  TAKE(out.bindings, A);
-  TAKE(out.saddles, F);
-  TAKE(out.groups, out.n_groups);
+  TAKE_RECORD(out.jb, out.n_batches);
+  TAKE_RECORD(out.fb, out.n_batches);
+  TAKE_RECORD(out.bindings, A);
+  TAKE_RECORD(out.saddles, F);
+  TAKE_RECORD(out.groups, out.n_groups);
   k_fj_batches<<<nblk(nbatch), kT, 0, st>>>(j, nbatch, R, gs, src, first, out.jb, out.fb);
   ++*launches;
   if (F) {
@@ -1408,6 +1441,7 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
     cap = hc[4];
   }
 #undef TAKE
+#undef TAKE_RECORD
   std::sort(out.roots.begin(), out.roots.end(),
             [](const ehgp_forest_root& x, const ehgp_forest_root& y) { return x.node < y.node; });
   return EHGP_OK;

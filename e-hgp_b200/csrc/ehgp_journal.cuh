@@ -7,29 +7,46 @@
 namespace ehgp {
 
 // Device memory handed out in order from one kept block; what does not fit goes to further
-// blocks, which the next reset folds into one of the total size.
+// blocks, which the next reset folds into one of the total size.  Records that the device has no
+// room for go to pinned host memory, which the kernels write over the bus.
 class DeviceArena {
  public:
   explicit DeviceArena(std::atomic<uint64_t>& held) : held_(held) {}  // counts the bytes of its blocks there
   DeviceArena(const DeviceArena&) = delete;
   DeviceArena& operator=(const DeviceArena&) = delete;
   ~DeviceArena() { release(); }
-  // Forgets every piece handed out; nothing on the device may still use them.
+  // Forgets every piece handed out (nothing on the device may still use them) and makes room for `want`
+  // bytes in one block; 0: no block.
   cudaError_t reset(uint64_t want);
   cudaError_t take(void** p, uint64_t bytes);
   template <class T>
   cudaError_t take(T** p, uint64_t count) {
     return take(reinterpret_cast<void**>(p), count * sizeof(T));
   }
+  // A record array: on the device, or in host memory (always with `spilled`).
+  template <class T>
+  cudaError_t take_record(T** p, uint64_t count) {
+    if (!spilled) {
+      const cudaError_t e = take(p, count);
+      if (e != cudaErrorMemoryAllocation) return e;
+      cudaGetLastError();
+    }
+    return take_host(reinterpret_cast<void**>(p), count * sizeof(T));
+  }
+  void release_host();
   void release();
+  bool spilled = false;
+  uint64_t largest = ~uint64_t{0};  // larger blocks are refused (tests)
 
  private:
   cudaError_t add(uint64_t size, uint64_t used, void** p);
+  cudaError_t take_host(void** p, uint64_t bytes);
+  void release_device();
   struct Block {
     char* p;
     uint64_t size, used;
   };
-  std::vector<Block> blocks_;
+  std::vector<Block> blocks_, host_;
   std::atomic<uint64_t>& held_;
 };
 

@@ -348,6 +348,7 @@ class Context:
     TUNE_PAIR_TASKS = 2
     TUNE_SORT_WAIT = 3
     TUNE_FOREST_ROUNDS = 4
+    TUNE_HIERARCHY_BLOCK = 5
 
     def tune(self, knob: int, value: int) -> None:
         """ehgp_tune: a tuning knob of later calls (results never depend on it)."""

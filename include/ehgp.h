@@ -107,8 +107,11 @@ int ehgp_checkpoint_load(ehgp_ctx* ctx, const char* path, uint32_t* K);
  *   EHGP_TUNE_SORT_WAIT: how often (0..2^20, the default the largest) a block of a sort
  *     looks for an earlier block's counts before it counts that block's items itself.
  *   EHGP_TUNE_FOREST_ROUNDS: device rounds of the forest journal (0..; 64 at most, the
- *     default) before the host applies the families that are left, in order. */
-enum { EHGP_TUNE_HIGHER_LIST = 1, EHGP_TUNE_PAIR_TASKS = 2, EHGP_TUNE_SORT_WAIT = 3, EHGP_TUNE_FOREST_ROUNDS = 4 };
+ *     default) before the host applies the families that are left, in order.
+ *   EHGP_TUNE_HIERARCHY_BLOCK: bytes above which a device block of the hierarchy's working
+ *     memory counts as refused (0, the default: none).  Without room for one block the
+ *     descent runs in smaller parts and the records go to pinned host memory. */
+enum { EHGP_TUNE_HIGHER_LIST = 1, EHGP_TUNE_PAIR_TASKS = 2, EHGP_TUNE_SORT_WAIT = 3, EHGP_TUNE_FOREST_ROUNDS = 4, EHGP_TUNE_HIERARCHY_BLOCK = 5 };
 int ehgp_tune(ehgp_ctx* ctx, uint32_t knob, uint64_t value);
 
 /* ---- LBVH snapshot records (reference layout) ---------------------------- */

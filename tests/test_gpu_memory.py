@@ -83,3 +83,35 @@ def test_server_requests_wait_for_the_whole_footprint():
             t.join()
         assert srv.stats()["memory_waits"] > 0
     assert most[0] < budget + workers * (records + (128 << 20))
+
+
+def _arrays(ctx, K):
+    r = {k: v for k, v in ctx.hierarchy(K).items() if isinstance(v, np.ndarray)}
+    r["supports"] = ctx.event_supports(r["nodes"]["level_event"])
+    return r
+
+
+@pytest.mark.parametrize("pts", [workloads.jittered_lattice(10, 2),
+                                 np.concatenate([np.round(workloads.uniform_cube(150, 5) * 2.0**30) / 2.0**30 + [i, 0, 0]
+                                                 for i in (0.0, 2.0, 4.0)])], ids=["lattice", "copies"])
+def test_hierarchies_without_room_on_the_device(pts):
+    """Blocks above 8 MB (more than any one array needs, less than the journal) are refused: the descent
+    runs in parts, the records go to host memory."""
+    with ehgp.Context(max_points=len(pts)) as ctx:
+        ctx.lbvh_build(pts, outputs=False)
+        want = _arrays(ctx, 10)
+        roomy = ctx.device_bytes
+        for block in (8 << 20, 8 << 20, 0, 8 << 20):
+            ctx.tune(ctx.TUNE_HIERARCHY_BLOCK, block)
+            got = _arrays(ctx, 10)
+            assert got.keys() == want.keys()
+            for k in want:
+                assert np.array_equal(got[k], want[k]), (block, k)
+            assert (ctx.device_bytes < 0.8 * roomy) == (block > 0)
+        ctx.tune(ctx.TUNE_HIERARCHY_BLOCK, 4096)  # no room for anything
+        with pytest.raises(ehgp.EhgpError) as e:
+            ctx.hierarchy(10)
+        assert e.value.status == 4
+        ctx.tune(ctx.TUNE_HIERARCHY_BLOCK, 0)
+        got = _arrays(ctx, 10)
+        assert all(np.array_equal(got[k], want[k]) for k in want)
