@@ -1847,7 +1847,7 @@ int hier_run(Ctx& ctx, uint32_t K) {
   cudaError_t e = ensure_events(h, total + 1);
   if (e == cudaErrorMemoryAllocation) {  // the last call's working memory is made again below
     cudaGetLastError();
-    h.mem.release();
+    h.mem.reset(0);
     e = ensure_events(h, total + 1);
   }
   if (e != cudaSuccess) return abi_fail(&ctx, EHGP_ERR_OUT_OF_MEMORY, "hierarchy buffers do not fit the device");
