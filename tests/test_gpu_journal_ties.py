@@ -1,5 +1,5 @@
 """The tied copies of test_gpu_journal.py do tie: batches with several saddles, groups that join several
-where there are three copies to join, neither without copies; and a cloud whose saddles in shared batches are more than one block
+with three copies and more, neither without copies; and a cloud whose saddles in shared batches are more than one block
 sorts (2,048), against the restatement."""
 import numpy as np
 import pytest
@@ -23,7 +23,7 @@ def test_copies_share_batches_and_groups(count, tile, K):
     if count == 1:
         assert (batch, group, shared) == (1, 1, 0)
     else:
-        assert batch > 1 and shared > 0 and (group > 1) == (count > 2)
+        assert batch > 1 and shared > 0 and (group > 1 or count == 2)
 
 
 @pytest.mark.gpu
