@@ -82,7 +82,7 @@ void stage_free(Ctx& ctx) {
 
 cudaError_t copy_direct(Ctx& ctx, const std::vector<CopyOut>& list) {
   for (const CopyOut& c : list) {
-    const cudaError_t e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDefault, ctx.stream);
+    const cudaError_t e = cudaMemcpyAsync(c.dst, c.src, c.bytes, c.kind, ctx.stream);
     if (e != cudaSuccess) return e;
   }
   return cudaStreamSynchronize(ctx.stream);
@@ -104,11 +104,11 @@ cudaError_t copy_out(Ctx& ctx, const std::vector<CopyOut>& list) try {
     const bool pageable = cudaPointerGetAttributes(&at, c.dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
     if (!pageable || c.bytes <= kStageBytes || all < (ctx.stage ? kStageFrom : kStageMake)) {
-      if ((e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDefault, st)) != cudaSuccess) return e;
+      if ((e = cudaMemcpyAsync(c.dst, c.src, c.bytes, c.kind, st)) != cudaSuccess) return e;
       continue;
     }
     for (uint64_t o = 0; o < c.bytes; o += kStageBytes)
-      chunks.push_back({c.dst + o, c.src + o, std::min(kStageBytes, c.bytes - o)});
+      chunks.push_back({c.dst + o, c.src + o, std::min(kStageBytes, c.bytes - o), c.kind});
   }
   if (chunks.empty()) return cudaStreamSynchronize(st);
   if (!stage_ready(ctx)) return copy_direct(ctx, chunks);
@@ -146,7 +146,7 @@ cudaError_t copy_out(Ctx& ctx, const std::vector<CopyOut>& list) try {
       while (!done[t - kStageSlots].load(std::memory_order_acquire) && !failed.load(std::memory_order_acquire))
         std::this_thread::yield();
     const int slot = (int)(t % kStageSlots);
-    e = cudaMemcpyAsync(ctx.stage + slot * kStageBytes, chunks[t].src, chunks[t].bytes, cudaMemcpyDefault, st);
+    e = cudaMemcpyAsync(ctx.stage + slot * kStageBytes, chunks[t].src, chunks[t].bytes, chunks[t].kind, st);
     if (e == cudaSuccess) e = cudaEventRecord(ctx.stage_ev[slot], st);
     if (e != cudaSuccess) {
       failed.store(1, std::memory_order_release);

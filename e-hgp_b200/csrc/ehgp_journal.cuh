@@ -33,6 +33,7 @@ class DeviceArena {
     }
     return take_host(reinterpret_cast<void**>(p), count * sizeof(T));
   }
+  bool on_host(const void* p) const;
   void release_host();
   void release();
   bool spilled = false;
