@@ -308,7 +308,7 @@ def served_section(local: int) -> dict:
                            "served_over_plain": served_cps * plain_s / len(clouds), "workers": best_w,
                            "served_clouds_per_s_by_workers": {str(w): v[0] for w, v in per_w.items()},
                            "failed": bad})
-    # the same comparison on uniform clouds, whose step is dominated by the host forest pass
+    # the same comparison on uniform clouds, whose step is mostly the copy of its result
     ucl = [workloads.uniform_cube(int(n), 500 + i) for i, n in
            enumerate(np.exp(np.random.Generator(np.random.PCG64(5)).uniform(np.log(1000), np.log(20000), 32)))]
     with ehgp.Context(max_points=20000, device=local) as ctx:

@@ -553,8 +553,8 @@ class Context:
         return out
 
     def hier_schedule(self, chunk_batches: int = 0, part_arms: int = 0, host_threads: int = 0) -> None:
-        """ehgp_hier_schedule: chunk, descent-part and thread counts of later hierarchy calls
-        (0 = default); the result never depends on them."""
+        """ehgp_hier_schedule: arms per part of the descent of later hierarchy calls (0 = all in one; the other two
+        have no effect since the forest journal is built on the device); the result never depends on them."""
         self._check(self.lib.ehgp_hier_schedule(self._h, chunk_batches, part_arms, host_threads))
 
     def hier_stats(self) -> dict:
