@@ -156,13 +156,19 @@ struct Tree {
   const uint32_t* node_cls;  // [nodes] level class of the sorted nodes
   const uint32_t* node_idx;  // [nodes] their index among the created nodes
   uint32_t n;
+  uint2* skip;      // [handles] (the handle kSkip climbs up, the last death on the way), where climbs are long
 };
+constexpr int kSkip = 64;
 
 __device__ __forceinline__ uint32_t carrier_before(const Tree& t, uint32_t x, uint32_t cls) {
+  if (t.skip)
+    for (uint2 k = t.skip[x]; k.y < cls; k = t.skip[x]) x = k.x;
   for (uint2 d = t.dead[x]; d.y < cls; d = t.dead[x]) x = d.x;
   return x;
 }
 __device__ __forceinline__ uint32_t carrier_after(const Tree& t, uint32_t x, uint32_t cls) {
+  if (t.skip)
+    for (uint2 k = t.skip[x]; k.y <= cls && k.y != kNone; k = t.skip[x]) x = k.x;
   for (uint2 d = t.dead[x]; d.y <= cls && d.y != kNone; d = t.dead[x]) x = d.x;
   return x;
 }
@@ -611,6 +617,22 @@ __global__ void __launch_bounds__(kT) k_fj_normalise(uint32_t handles, Tree t) {
   if (d.y == kNone) return;
   const uint32_t p = carrier_after(t, d.x, d.y);
   if (p != d.x) t.dead[h].x = p;
+}
+
+// Deaths increase along a climb, so kSkip steps of it can be taken at once when the last one can.
+__global__ void __launch_bounds__(kT) k_fj_skips(uint32_t handles, Tree t, uint2* __restrict__ skip) {
+  const uint32_t h = blockIdx.x * kT + threadIdx.x;
+  if (h >= handles) return;
+  uint2 k = make_uint2(h, 0u);
+  for (int i = 0; i < kSkip; ++i) {
+    const uint2 d = t.dead[k.x];
+    if (d.y == kNone) {
+      k.y = kNone;
+      break;
+    }
+    k = d;
+  }
+  skip[h] = k;
 }
 
 // ---- 2. carriers and groups ----------------------------------------------------------------
@@ -1244,8 +1266,15 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
       k_fj_tail<<<1, 1024, 0, st>>>(j.cls, act[cur], act[1 - cur], cnt + cur, best[cur], best[1 - cur], t, lab, in.rounds, cnt + 5);
       ++*launches;
     }
+    uint2* skip = nullptr;
     auto carriers = [&] {
+      t.skip = nullptr;
       k_fj_normalise<<<nblk(H), kT, 0, st>>>(H, t);
+      if (skip) {
+        k_fj_skips<<<nblk(H), kT, 0, st>>>(H, t, skip);
+        ++*launches;
+      }
+      t.skip = skip;
       k_fj_carriers<<<nblk(F), kT, 0, st>>>(j, t, car, cnt + 3);
       *launches += 2;
       return read("forest journal carriers");
@@ -1285,6 +1314,7 @@ int journal_run(Ctx& ctx, const JournalIn& in, DeviceArena& mem, JournalOut& out
       cudaMemcpyAsync(d_deaths, deaths.data(), m * sizeof(uint4), cudaMemcpyHostToDevice, st);
       k_fj_deaths<<<nblk(m), kT, 0, st>>>(m, j.cls, d_deaths, t);
       *launches += 2;
+      TAKE(skip, H);  // a chain of deaths is as long as its components
       // the carriers of the unfinished tree are made again
       cudaMemsetAsync(t.touch, 0xff, H * sizeof(uint32_t), st);
       cudaMemsetAsync(cnt + 3, 0, sizeof(uint32_t), st);
