@@ -433,7 +433,8 @@ __device__ __forceinline__ void flush_records(const WarpShared& sh, uint32_t& ke
 // walked on in place, by a warp that asks no more.
 // Bound by the latency of the walk's dependent loads, so the registers are held to five blocks per SM
 // (96, against 147 and three): 29,791 lattice points 4.81 -> 3.86 ms, 50,653 at K = 4 3.46 -> 2.55,
-// 15,000 mixture points 8.82 -> 7.86; at six blocks 4.02 / 2.67 / 9.00 (the spills cost more).
+// 15,000 mixture points 8.82 -> 7.86; at six blocks 4.02 / 2.67 / 9.00 (the spills cost more); all of these
+// with a box per lane in the pruning test.  Now 3.01 / 1.20 ms, and 5.03 on another 15,000-point mixture.
 __global__ void __launch_bounds__(kThreads, kPairsBlocks)
 k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, const uint32_t* __restrict__ leaf_pid,
         const uint32_t* __restrict__ n_begin, const uint32_t* __restrict__ n_end, const double* __restrict__ px,
@@ -596,17 +597,25 @@ k_pairs(uint32_t n, uint32_t cap, uint32_t root, const TNode* __restrict__ tn, c
       }
       if (nw >= need) {
         // max over v in box of (w-u).(w-v) = sum_i a_i (a_i - (a_i >= 0 ? lo_i : hi_i)), a = w - u: below 0
-        // with certainty for `need` witnesses, no pair of u with the box is relevant
-        uint32_t in = 0;
-        for (uint32_t w = 0; w < nw; ++w) {
-          const float4 a = sh.wit[w];
-          const float tx = a.x * (a.x - (a.x >= 0.f ? lx : hx));
-          const float ty = a.y * (a.y - (a.y >= 0.f ? ly : hy));
-          const float tz = a.z * (a.z - (a.z >= 0.f ? lz : hz));
-          in += tx + ty + tz < -1e-5f * (fabsf(tx) + fabsf(ty) + fabsf(tz) + a.w) ? 1u : 0u;
-          if ((w & 7u) == 7u && __all_sync(0xffffffffu, !open || in >= need)) break;
+        // with certainty for `need` witnesses, no pair of u with the box is relevant.  Two witnesses per lane
+        // and one box after another: with a box per lane and one witness after another, the few boxes of a
+        // sparse walk cost 64 steps (50,000 points on a line, K = 2: 2.06 ms against 0.38; 50,653 lattice points,
+        // K = 4 2.57 against 1.20, 29,791 at K = 10 3.77 against 3.01).
+        const float4 w_lo = sh.wit[lane], w_hi = sh.wit[lane + 32];
+        for (uint32_t todo = __ballot_sync(0xffffffffu, open); todo; todo &= todo - 1) {
+          const uint32_t q = (uint32_t)__ffs((int)todo) - 1;
+          const float bx = __shfl_sync(0xffffffffu, lx, q), by = __shfl_sync(0xffffffffu, ly, q),
+                      bz = __shfl_sync(0xffffffffu, lz, q), cx = __shfl_sync(0xffffffffu, hx, q),
+                      cy = __shfl_sync(0xffffffffu, hy, q), cz = __shfl_sync(0xffffffffu, hz, q);
+          auto certain = [&](const float4& a) {
+            const float tx = a.x * (a.x - (a.x >= 0.f ? bx : cx));
+            const float ty = a.y * (a.y - (a.y >= 0.f ? by : cy));
+            const float tz = a.z * (a.z - (a.z >= 0.f ? bz : cz));
+            return tx + ty + tz < -1e-5f * (fabsf(tx) + fabsf(ty) + fabsf(tz) + a.w);
+          };
+          const uint32_t in = __popc(__ballot_sync(0xffffffffu, certain(w_lo))) + __popc(__ballot_sync(0xffffffffu, certain(w_hi)));
+          if (lane == q) open = in < need;
         }
-        open = open && in < need;
       }
       const bool is_leaf = open && t.left == kInvalid32, expand = open && !is_leaf;
       const uint32_t lb = __ballot_sync(0xffffffffu, is_leaf), eb = __ballot_sync(0xffffffffu, expand);
